@@ -14,6 +14,7 @@
 //   * coverage multiplicity cnt[x] = #{i : d(x,c_i) <= R} by marking every
 //     codeword's ball (covsearch2e.c:353-380, 958-967), with 32-bit atomics
 //     on packed uint16 pairs.
+#include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -299,6 +300,223 @@ k_dt_high(DtGeom g, int j0, int gsz, int lw, int last_, uint8_t *__restrict__ D,
         atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
 }
 
+// ------------------------------------------- the transform of few codewords --
+// When the code is small beside a tile of T = q^nl words (the low nl digits),
+// a tile needs no other tile: every codeword enters it at its low digits with
+// the distance of its high digits to the tile's as the starting value, and
+// the nl low axes finish the transform.  One launch writes each distance
+// once; nothing is read but the code.
+//
+// A line of the lowest axis is one 32-bit word, (m << 16) | mask: D = m at
+// the positions in mask and m + 1 elsewhere.  That is exact because distances
+// along an axis already taken differ by at most one (D is 1-Lipschitz in it),
+// and it stays true through the other axes.  With E the minimum over the q
+// lines of a fibre -- the least m, and the union of the masks that have it --
+// a line becomes min(line, E + 1): itself if its m is E's, the union of both
+// masks if it is one more, E + 1 otherwise.  A line element therefore costs
+// about 11 instructions a pass for q words, where a byte of its own costs
+// about two a word (and q bytes of shared memory instead of four).
+// Bound by instruction issue (72 % of the slots at 8^9, 19 lane-instructions
+// a word; DRAM 14 % busy): 8^10 with 2549 codewords takes 0.68 ms = 1.6 TB/s
+// of distances written, against 4.5 ms for a tile pass and two strip sweeps
+// of bytes.
+#define DT_TILES_NT 512
+#define DT_TILES_KEEP 8          // codewords a thread keeps between the two marking passes
+#define DT_TILES_SMEM (100 * 1024)
+
+// shared-memory slot of line l: for q = 8 the three low digits of l are
+// folded into the bank bits, so that a warp's fibres of the first three axes
+// fall in 32 banks (unswizzled: 8-way and 4-way conflicts).  XOR-linear.
+template <int Q>
+__device__ __forceinline__ uint32_t dt_slot(uint32_t l)
+{
+    if constexpr (Q == 8) return l ^ ((l >> 3) & 7u) ^ (((l >> 6) & 3u) << 3);
+    return l;
+}
+
+// per codeword: {nibbles of the high digits, (line of the low digits' tile << 4) | position}
+template <int Q>
+__global__ void k_dt_records(const uint8_t *__restrict__ code, int M, DtGeom g, int nl, uint2 *__restrict__ rec)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+        uint32_t x = 0;
+        for (int j = 0; j < g.n; j++) x = x * (uint32_t)Q + code[(size_t)i * g.n + j];
+        if (x >= g.N) x = 0xffffffffu;           // a digit outside the alphabet: no word
+        uint32_t hi = x / g.pw[nl], h = 0;
+        const uint32_t lo = x - hi * g.pw[nl];
+        for (int j = 0; j < g.n - nl; j++) { h |= (hi % (uint32_t)Q) << (4 * j); hi /= (uint32_t)Q; }
+        rec[i] = x == 0xffffffffu ? make_uint2(0u, 0xffffffffu)
+                                  : make_uint2(h, (dt_slot<Q>(lo / (uint32_t)Q) << 4) | (lo % (uint32_t)Q));
+    }
+}
+
+__device__ __forceinline__ uint32_t dt_nibble_dist(uint32_t a, uint32_t b)
+{
+    uint32_t x = a ^ b;
+    x |= x >> 1;
+    x |= x >> 2;
+    return (uint32_t)__popc(x & 0x11111111u);
+}
+
+// four distances from four mask bits: m where a bit is set, m + 1 elsewhere;
+// m1 holds m + 1 in every byte
+__device__ __forceinline__ uint32_t dt_expand4(uint32_t bits, uint32_t m1)
+{
+    return m1 - ((bits * 0x00204081u) & 0x01010101u);
+}
+
+template <int Q>
+__global__ void __launch_bounds__(DT_TILES_NT, Q <= 10 ? 3 : 1)
+k_dt_tiles(DtGeom g, int nl, const uint2 *__restrict__ rec, int M, uint8_t *__restrict__ D, unsigned long long *hist)
+{
+    extern __shared__ __align__(16) uint32_t dt_w[];
+    __shared__ int sh[COV_MAXN + 2];
+    constexpr uint32_t FULL = (1u << Q) - 1u;
+    const uint32_t T = g.pw[nl], lines = g.pw[nl - 1], ntile = g.N / T;
+    const uint32_t nt = blockDim.x;
+    const int nh = g.n - nl;
+    if (threadIdx.x < COV_MAXN + 2) sh[threadIdx.x] = 0;
+    for (uint32_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        uint32_t hp = 0;
+        {
+            uint32_t t = tile;
+            for (int j = 0; j < nh; j++) { hp |= (t % (uint32_t)Q) << (4 * j); t /= (uint32_t)Q; }
+        }
+        __syncthreads();
+        for (uint32_t l = threadIdx.x; l < lines; l += nt) dt_w[l] = ((uint32_t)g.inf << 16) | FULL;
+        __syncthreads();
+        // least starting value of every line, then the positions that have it
+        // kept: (starting value << 28) | (line << 4) | position, all ones for none
+        uint32_t kept[DT_TILES_KEEP];
+        const bool keep = (uint32_t)M <= nt * DT_TILES_KEEP;
+        if (keep) {
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++) {
+                const uint32_t i = threadIdx.x + (uint32_t)u * nt;
+                kept[u] = 0xffffffffu;
+                if ((uint32_t)u * nt < (uint32_t)M && i < (uint32_t)M) {
+                    const uint2 r = __ldg(&rec[i]);
+                    if (r.y != 0xffffffffu) kept[u] = (dt_nibble_dist(r.x, hp) << 28) | r.y;
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++)
+                if ((uint32_t)u * nt < (uint32_t)M && kept[u] != 0xffffffffu) atomicMin(&dt_w[(kept[u] & 0x0fffffffu) >> 4], (kept[u] >> 28) << 16);
+        } else {
+            for (uint32_t i = threadIdx.x; i < (uint32_t)M; i += nt) {
+                const uint2 r = __ldg(&rec[i]);
+                if (r.y != 0xffffffffu) atomicMin(&dt_w[r.y >> 4], dt_nibble_dist(r.x, hp) << 16);
+            }
+        }
+        __syncthreads();
+        if (keep) {
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++) {
+                if ((uint32_t)u * nt >= (uint32_t)M || kept[u] == 0xffffffffu) continue;
+                const uint32_t at = (kept[u] & 0x0fffffffu) >> 4;
+                if ((dt_w[at] >> 16) == kept[u] >> 28) atomicOr(&dt_w[at], 1u << (kept[u] & 15u));
+            }
+        } else {
+            for (uint32_t i = threadIdx.x; i < (uint32_t)M; i += nt) {
+                const uint2 r = __ldg(&rec[i]);
+                if (r.y != 0xffffffffu && (dt_w[r.y >> 4] >> 16) == dt_nibble_dist(r.x, hp))
+                    atomicOr(&dt_w[r.y >> 4], 1u << (r.y & 15u));
+            }
+        }
+        __syncthreads();
+        // the other low axes, a fibre of Q lines at a time
+        uint32_t inner = 1;
+        for (int j = 1; j < nl; j++, inner *= (uint32_t)Q) {
+            const float rinv = 1.0f / (float)inner;   // f < 2^24: one correction makes f / inner exact
+            const uint32_t p1 = dt_slot<Q>(inner), p2 = dt_slot<Q>(2u * inner), p4 = dt_slot<Q>(4u * inner);
+            for (uint32_t f = threadIdx.x; f < lines / (uint32_t)Q; f += nt) {
+                int o = (int)((float)f * rinv);
+                int i = (int)f - o * (int)inner;
+                if (i < 0) { o--; i += (int)inner; } else if (i >= (int)inner) { o++; i -= (int)inner; }
+                const uint32_t b = dt_slot<Q>((uint32_t)o * (uint32_t)Q * inner + (uint32_t)i);
+                uint32_t v[Q], ad[Q];
+#pragma unroll
+                for (int a = 0; a < Q; a++) {
+                    if constexpr (Q == 8)
+                        ad[a] = b ^ ((a & 1) ? p1 : 0u) ^ ((a & 2) ? p2 : 0u) ^ ((a & 4) ? p4 : 0u);
+                    else
+                        ad[a] = b + (uint32_t)a * inner;
+                    v[a] = dt_w[ad[a]];
+                }
+                uint32_t e = v[0];
+#pragma unroll
+                for (int a = 1; a < Q; a++) e = min(e, v[a]);
+                const uint32_t t0 = (e & 0xffff0000u) + 0x10000u, t1 = t0 + 0x10000u;   // m of E + 1, and one more
+                uint32_t w = t0;
+#pragma unroll
+                for (int a = 0; a < Q; a++)
+                    if (v[a] < t0) w |= v[a] & FULL;
+#pragma unroll
+                for (int a = 0; a < Q; a++)
+                    if (v[a] >= t0) dt_w[ad[a]] = v[a] < t1 ? v[a] | w : w;
+            }
+            __syncthreads();
+        }
+        if (hist) {
+            int m = -1, at = 0, more = 0;             // words at m and at m + 1 of a run of lines
+            for (uint32_t l = threadIdx.x; l < lines; l += nt) {
+                const uint32_t v = dt_w[l];
+                if ((int)(v >> 16) != m) {
+                    if (at) atomicAdd(&sh[m], at);
+                    if (more) atomicAdd(&sh[m + 1], more);
+                    m = (int)(v >> 16);
+                    at = more = 0;
+                }
+                const int c = __popc(v & FULL);
+                at += c;
+                more += Q - c;
+            }
+            if (at) atomicAdd(&sh[m], at);
+            if (more) atomicAdd(&sh[m + 1], more);
+        }
+        if (!D) continue;
+        uint8_t *const out = D + (size_t)tile * T;
+        if (Q == 8 && (reinterpret_cast<uintptr_t>(D) & 7u) == 0) {
+            for (uint32_t l = threadIdx.x; l < lines; l += nt) {
+                const uint32_t v = dt_w[dt_slot<Q>(l)];
+                const uint32_t m1 = ((v >> 16) + 1u) * 0x01010101u;
+                reinterpret_cast<uint2 *>(out)[l] = make_uint2(dt_expand4(v & 15u, m1), dt_expand4((v >> 4) & 15u, m1));
+            }
+            continue;
+        }
+        // aligned 32-bit words of the tile's T bytes, each from the one, two
+        // or (q = 2) three lines that its bytes lie in; the ends as bytes
+        const uint32_t head = min((4u - (uint32_t)(reinterpret_cast<uintptr_t>(out) & 3u)) & 3u, T);
+        const uint32_t nw = (T - head) >> 2;
+        for (uint32_t k = threadIdx.x; k < head + ((T - head) & 3u); k += nt) {
+            const uint32_t b = k < head ? k : 4 * nw + k;
+            const uint32_t v = dt_w[dt_slot<Q>(b / (uint32_t)Q)];
+            out[b] = (uint8_t)((v >> 16) + 1u - ((v >> (b % (uint32_t)Q)) & 1u));
+        }
+        for (uint32_t k = threadIdx.x; k < nw; k += nt) {
+            const uint32_t b = head + 4 * k;
+            uint32_t l = b / (uint32_t)Q, a = b - l * (uint32_t)Q;
+            uint32_t x = 0, done = 0;
+#pragma unroll
+            for (int part = 0; part < (Q == 2 ? 3 : 2); part++) {
+                if (done < 4u) {
+                    const uint32_t v = dt_w[dt_slot<Q>(l)];
+                    const uint32_t y = dt_expand4(((v & FULL) >> a) & 15u, ((v >> 16) + 1u) * 0x01010101u);
+                    const uint32_t keepm = 0xffffffffu << (8u * done);
+                    x = (x & ~keepm) | ((y << (8u * done)) & keepm);
+                    done += (uint32_t)Q - a;
+                    a = 0;
+                    l++;
+                }
+            }
+            *reinterpret_cast<uint32_t *>(out + b) = x;
+        }
+    }
+    __syncthreads();
+    if (hist && threadIdx.x < g.n + 2 && sh[threadIdx.x])
+        atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
+}
+
 // the transform kernels of every q, for a runtime q
 template <template <int> class F, class... A>
 int dt_for_q(int q, A... a)
@@ -317,8 +535,22 @@ template <int Q> struct DtAttrs {
     static int run()
     {
         if (cudaFuncSetAttribute(k_dt_low<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_TILE_BIG) != cudaSuccess ||
-            cudaFuncSetAttribute(k_dt_high<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_STRIP_MAX) != cudaSuccess)
+            cudaFuncSetAttribute(k_dt_high<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_STRIP_MAX) != cudaSuccess ||
+            cudaFuncSetAttribute(k_dt_tiles<Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_TILES_SMEM) != cudaSuccess)
             return -(100 + (int)cudaGetLastError());
+        return 0;
+    }
+};
+template <int Q> struct DtTiles {
+    static int run(int grid, int nt, size_t smem, cudaStream_t st, const uint8_t *code, int M, DtGeom g, int nl,
+                   uint2 *rec, uint8_t *D, unsigned long long *hist)
+    {
+        if (M > 0) {
+            k_dt_records<Q><<<std::min(1024, (M + 255) / 256), 256, 0, st>>>(code, M, g, nl, rec);
+            CK(cudaGetLastError());
+        }
+        k_dt_tiles<Q><<<grid, nt, smem, st>>>(g, nl, rec, M, D, hist);
+        CK(cudaGetLastError());
         return 0;
     }
 };
@@ -588,9 +820,59 @@ int ct_attrs()
     return 0;
 }
 
-// the transform on device buffers; hist (device, n+2 entries) may be null
-int dt_run(const DtGeom &g, const uint8_t *d_code, int M, uint8_t *d_D, unsigned long long *d_hist,
-           uint32_t *d_bm, cudaStream_t st)
+// How a transform runs: by tiles from the code alone (k_dt_tiles) or by the
+// bitmap and sweeps of the word array (k_dt_low, k_dt_high).
+struct DtPlan {
+    bool tiles;
+    int nl, nt, grid;
+    size_t smem;
+    size_t scratch;              // bytes of device scratch: the code's records, or its bitmap
+};
+
+// The tile form costs M code marks a tile, so the rule compares estimates in
+// SM cycles.  A tile takes about 25 lane-instructions a codeword (12 more
+// where the threads cannot keep them), 11 a line and pass, 4 a word of
+// output, at 64 lanes a cycle, and a latency chain of some 500 cycles a
+// barrier; the number of low digits with the least estimate is taken (of the
+// seven cells timed at every number it is the best or within 6 % of it).  The
+// sweep form's side is measured: 4.2 ps a word (8^10: 4.5 ms) after three
+// launches.  Measured, sweeps against tiles: 8^10 M 2549 4505 -> 680 us, 7^10
+// M 163 1076 -> 260, 7^9 M 1500 179 -> 50, 7^9 M 30000 179 -> 80, 6^6 M 41
+// 24.8 -> 10.6; near the line, 8^7 M 30000: 41.1 against 41.7.
+#define DT_SWEEP_CYCLES_WORD 0.0087
+#define DT_SWEEP_CYCLES_MIN 16000.0
+DtPlan dt_plan(const DtGeom &g, int M)
+{
+    DtPlan best{};
+    best.scratch = (size_t)((g.N + 31) / 32) * 4;
+    double least = DT_SWEEP_CYCLES_MIN + DT_SWEEP_CYCLES_WORD * g.N;
+    const double sms = std::max(1, cov_sm_count());
+    for (int nl = std::max(1, g.n - 8); nl <= g.n; nl++) {
+        const uint32_t T = g.pw[nl], lines = g.pw[nl - 1];
+        if ((size_t)lines * 4 > DT_TILES_SMEM) break;
+        const int nt = lines > 8192 ? 512 : lines > 256 ? 256 : 128;
+        const double tiles = g.N / T;
+        const double per_sm = std::min(std::min(1536.0 / nt, 220.0 * 1024 / (lines * 4.0 + 1200)), 32.0);
+        const double work = M * (M <= nt * DT_TILES_KEEP ? 25.0 : 37.0) + lines * 11.0 * (nl - 1) + T * 4.0;
+        const double waves = std::ceil(tiles / (sms * std::floor(per_sm)));
+        const double cyc = tiles * work / (64.0 * sms) + waves * (1500.0 + 500.0 * nl + work / (nt / 4.0));
+        if (cyc < least) {
+            least = cyc;
+            best.tiles = true;
+            best.nl = nl;
+            best.nt = nt;
+            best.smem = (size_t)lines * 4;
+            best.grid = (int)std::min(tiles, sms * std::floor(per_sm));
+            best.scratch = (size_t)std::max(M, 1) * 8;
+        }
+    }
+    return best;
+}
+
+// the transform on device buffers; hist (device, n+2 entries) may be null,
+// and d_D too when the plan is by tiles; scratch: plan.scratch bytes
+int dt_run(const DtGeom &g, const DtPlan &plan, const uint8_t *d_code, int M, uint8_t *d_D,
+           unsigned long long *d_hist, void *scratch, cudaStream_t st)
 {
     int dev = 0;
     if (!g_dt_attr.done(dev)) {
@@ -600,6 +882,10 @@ int dt_run(const DtGeom &g, const uint8_t *d_code, int M, uint8_t *d_D, unsigned
         }
         g_dt_attr.set(dev);
     }
+    if (plan.tiles)
+        return dt_for_q<DtTiles>(g.q, plan.grid, plan.nt, plan.smem, st, d_code, M, g, plan.nl, (uint2 *)scratch,
+                                 d_D, d_hist);
+    uint32_t *d_bm = (uint32_t *)scratch;
     CK(cudaMemsetAsync(d_bm, 0, (size_t)((g.N + 31) / 32) * 4, st));
     if (M > 0) {
         k_dt_bitmap<<<std::min(1024, (M + 255) / 256), 256, 0, st>>>(d_code, M, g, d_bm);
@@ -669,10 +955,11 @@ int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M, uint
     if (rc) return rc;
     if (M < 0 || (M > 0 && !d_code) || !d_dist) return COV_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    uint32_t *bm = nullptr;
-    CK(cudaMallocAsync(&bm, (size_t)((g.N + 31) / 32) * 4, st));
-    rc = dt_run(g, d_code, M, d_dist, nullptr, bm, st);
-    cudaFreeAsync(bm, st);
+    const DtPlan plan = dt_plan(g, M);
+    void *scratch = nullptr;
+    CK(cudaMallocAsync(&scratch, plan.scratch, st));
+    rc = dt_run(g, plan, d_code, M, d_dist, nullptr, scratch, st);
+    cudaFreeAsync(scratch, st);
     return rc;
 }
 
@@ -720,7 +1007,9 @@ int cov_mindist_dev_static(int32_t q, int32_t n, const uint8_t *d_code, int32_t 
         CK(cudaGetSymbolAddress(&ptr, g_dt_static_bitmap));
         g_dt_static_addr[dev] = (uint32_t *)ptr;
     }
-    return dt_run(g, d_code, M, d_dist, nullptr, g_dt_static_addr[dev], (cudaStream_t)stream);
+    DtPlan plan = dt_plan(g, M);
+    if (plan.scratch > sizeof g_dt_static_bitmap) plan = DtPlan{};       // more codewords than the array has records
+    return dt_run(g, plan, d_code, M, d_dist, nullptr, g_dt_static_addr[dev], (cudaStream_t)stream);
 }
 
 int64_t cov_count_above_dev(int32_t q, int32_t n, const uint8_t *d_dist, int32_t R, void *stream)
@@ -749,21 +1038,22 @@ int cov_mindist(int32_t q, int32_t n, const uint8_t *code, int32_t M, uint8_t *d
     if (M < 0 || (M > 0 && !code)) return COV_EINVAL;
     for (long long i = 0; i < (long long)M * n; i++) if (code[i] >= q) return COV_EINVAL;
     cudaStream_t st = nullptr;
+    const DtPlan plan = dt_plan(g, M);
+    const bool want_D = dist || !plan.tiles;      // the sweeps work in D; the tiles need none for the histogram
     uint8_t *d_code = nullptr, *d_D = nullptr;
-    uint32_t *d_bm = nullptr;
+    void *d_s = nullptr;
     unsigned long long *d_h = nullptr;
     const size_t cb = (size_t)std::max(M, 1) * n;
-    if (cudaMalloc(&d_code, cb) != cudaSuccess || cudaMalloc(&d_D, g.N) != cudaSuccess ||
-        cudaMalloc(&d_bm, (size_t)((g.N + 31) / 32) * 4) != cudaSuccess ||
-        cudaMalloc(&d_h, 8 * (COV_MAXN + 2)) != cudaSuccess) {
+    if (cudaMalloc(&d_code, cb) != cudaSuccess || (want_D && cudaMalloc(&d_D, g.N) != cudaSuccess) ||
+        cudaMalloc(&d_s, plan.scratch) != cudaSuccess || cudaMalloc(&d_h, 8 * (COV_MAXN + 2)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(d_code); cudaFree(d_D); cudaFree(d_bm); cudaFree(d_h);
+        cudaFree(d_code); cudaFree(d_D); cudaFree(d_s); cudaFree(d_h);
         return COV_ENOMEM;
     }
-    auto done = [&](int r) { cudaFree(d_code); cudaFree(d_D); cudaFree(d_bm); cudaFree(d_h); return r; };
+    auto done = [&](int r) { cudaFree(d_code); cudaFree(d_D); cudaFree(d_s); cudaFree(d_h); return r; };
     if (M > 0 && cudaMemcpy(d_code, code, (size_t)M * n, cudaMemcpyHostToDevice) != cudaSuccess) return done(-100);
     if (cudaMemset(d_h, 0, 8 * (COV_MAXN + 2)) != cudaSuccess) return done(-100);
-    rc = dt_run(g, d_code, M, d_D, d_h, d_bm, st);
+    rc = dt_run(g, plan, d_code, M, d_D, d_h, d_s, st);
     if (rc) return done(rc);
     unsigned long long hh[COV_MAXN + 2];
     cudaError_t e = cudaMemcpy(hh, d_h, 8 * (COV_MAXN + 2), cudaMemcpyDeviceToHost);
