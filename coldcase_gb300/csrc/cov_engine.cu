@@ -2693,26 +2693,20 @@ __global__ void k_mark_balls(CovSlot d, int first, int count, int sgn)
 // produces for k.  ul_bit must be clear beforehand.
 
 template <int Q>
-__global__ void __launch_bounds__(BT_NT) k_build_state(CovSlot d, unsigned long long *zeros)
+__global__ void __launch_bounds__(BT_NT) k_build_state(CovSlot d, BtCode code, unsigned long long *zeros)
 {
-    extern __shared__ __align__(16) unsigned char bt_raw[];
-    uint64_t *lpc = (uint64_t *)bt_raw;            // [BT_LCH] packed codewords of this chunk
-    uint32_t *lid = (uint32_t *)(lpc + BT_LCH);    // [BT_LCH] their ids
-    uint32_t *lbase = lid + BT_LCH;                // [BT_LCH] their low-digit index
-    uint32_t *tile = lbase + BT_LCH;               // [bt_tw]
-    __shared__ int gcnt[COV_MAXN + 2], gpos[COV_MAXN + 2], gfill[COV_MAXN + 2];
-
-    const int q = d.q, n = d.n, R = d.R, nh = d.bt_nh, nl = d.bt_nl;
+    extern __shared__ __align__(16) uint32_t bt_sm[];
+    const int q = Q > 0 ? Q : d.q, n = d.n, R = d.R, nh = d.bt_nh;
     const uint32_t T = d.bt_tw;
+    const BtTile tl = bt_layout(q, n, T);
+    bt_mark_tile<Q>(bt_sm, tl, blockIdx.x, q, n, R, d.M, code, nh, d.bt_nl, d.bt_v,
+                    [](uint32_t id) { return cov_cw_unit((int)id); });
+    const uint32_t *tile = bt_sm + tl.a0;
     uint64_t hp = 0;
     {
         uint32_t t = blockIdx.x;
         for (int j = nh - 1; j >= 0; --j) { hp |= (uint64_t)(t % (uint32_t)q) << (4 * j); t /= (uint32_t)q; }
     }
-    for (uint32_t x = threadIdx.x; x < T; x += BT_NT) tile[x] = 0;
-    BtScratch sc{lpc, lid, lbase, gcnt, gpos, gfill};
-    bt_mark_tile<Q>(tile, d.q, d.n, R, d.M, d.code, d.pw, nh, nl, d.bt_items, d.bt_last, d.bt_v, hp, sc,
-                    [](uint32_t id) { return cov_cw_unit((int)id); });
 
     uint32_t *gout = d.cw + (size_t)blockIdx.x * T;
     unsigned long long z = 0;
@@ -2942,9 +2936,9 @@ static int ensure_attrs()
     CK(cudaFuncSetAttribute(cov_run_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     CK(cudaFuncSetAttribute(cov_run_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(Smem)));
     CK(cudaFuncSetAttribute(cov_run_kernel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    CK(cudaFuncSetAttribute(k_build_state<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_smem_bytes(BT_MAX)));
+    CK(cudaFuncSetAttribute(k_build_state<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
 #define BS_ATTR_Q(QQ) \
-    CK(cudaFuncSetAttribute(k_build_state<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_smem_bytes(BT_MAX)));
+    CK(cudaFuncSetAttribute(k_build_state<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
     BT_Q_LIST(BS_ATTR_Q)
 #undef BS_ATTR_Q
     g_attr_done.set(dev);
@@ -3196,6 +3190,13 @@ int cov_pool_destroy(cov_pool *pool)
     return COV_OK;
 }
 
+// bytes of a slot's tabu table; the state build keeps its records of the
+// code there before the table is cleared
+static size_t tabu_bytes(int q, int n, int M)
+{
+    return std::max((size_t)M * n * q * 4, (size_t)M * BT_REC_BYTES);
+}
+
 size_t cov_slot_bytes(const cov_params *prm)
 {
     if (!prm) return 0;
@@ -3206,7 +3207,7 @@ size_t cov_slot_bytes(const cov_params *prm)
     auto add = [&](size_t x) { b += (x + 255) / 256 * 256; };
     add((size_t)N * 4);                              // cw
     add((size_t)M * 8 * 2);                          // code, best
-    add((size_t)M * n * q * 4);                      // tabu
+    add(tabu_bytes(q, n, M));                        // tabu
     add((size_t)M * (n + 1) * 4);                    // P
     add((size_t)UL_CAP_DEFAULT * 4);                 // ul_idx
     add((size_t)UL_CAP_DEFAULT * 8);                 // ul_pk
@@ -3216,15 +3217,6 @@ size_t cov_slot_bytes(const cov_params *prm)
     add(ce * 4 * 2 + (size_t)M * n * 4 + (size_t)M * 4);   // g_perm, g_dval, g_neg, g_list
     if (prm->wide) add((size_t)M * n * q * 4);      // g_negw
     add(65536);                                      // subset tables
-    {
-        int nh, nl;
-        bt_geom(q, n, &nh, &nl);
-        uint32_t vc[COV_MAXN + 2];
-        std::vector<uint8_t> lst;
-        const size_t ni = bt_items_h(q, n, std::min(R, n), nh, vc, lst).size();
-        add(ni * 8);                                 // state-build ball groups
-        add(ni);
-    }
     add(sizeof(CovSlotState));
     if (prm->trace) add((size_t)prm->trace_cap * sizeof(cov_move_rec));
     return b;
@@ -3315,7 +3307,7 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     d.cw = (uint32_t *)take_((size_t)N * 4);
     d.code = (uint64_t *)take_((size_t)Mw * 8);
     d.best = (uint64_t *)take_((size_t)Mw * 8);
-    d.tabu = (int32_t *)take_((size_t)Mw * n * q * 4);
+    d.tabu = (int32_t *)take_(tabu_bytes(q, n, Mw));
     d.P = (int32_t *)take_((size_t)Mw * (n + 1) * 4);
     d.ul_idx = (uint32_t *)take_((size_t)d.ul_cap * 4);
     d.ul_pk = (uint64_t *)take_((size_t)d.ul_cap * 8);
@@ -3331,14 +3323,9 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     uint8_t *dball = (uint8_t *)take_(balls.size());
     uint8_t *dsub1 = (uint8_t *)take_(subs1.size());
     d.sub = dsub; d.ball_sub = dball; d.sub1 = dsub1;
-    bt_geom(q, n, &d.bt_nh, &d.bt_nl);
+    bt_geom(q, n, R, Mw, &d.bt_nh, &d.bt_nl);
     d.bt_tw = (uint32_t)ipow_h(q, d.bt_nl);
-    std::vector<uint8_t> btl;
-    std::vector<uint64_t> bti = bt_items_h(q, n, R, d.bt_nh, d.bt_v, btl);
-    uint64_t *dbt = (uint64_t *)take_(bti.size() * 8);
-    uint8_t *dbl = (uint8_t *)take_(btl.size());
-    d.bt_items = dbt;
-    d.bt_last = dbl;
+    bt_vcum_h(q, n, R, d.bt_nl, d.bt_v);
     d.st = pool->d_states + s;
     d.trace = prm->trace ? take_((size_t)prm->trace_cap * sizeof(cov_move_rec)) : nullptr;
     d.trace_cap = prm->trace ? prm->trace_cap : 0;
@@ -3350,8 +3337,6 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     cudaError_t e = cudaMemcpyAsync(dsub, subs.data(), subs.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dball, balls.data(), balls.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dsub1, subs1.data(), subs1.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dbt, bti.data(), bti.size() * 8, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dbl, btl.data(), btl.size(), cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) { cudaFree(arena); return -(100 + (int)e); }
     pool->slots[s] = h;
@@ -3379,7 +3364,6 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
     }
     const bool incremental = m > M || (m < M && !random_init);   // repair or greedy
     if (incremental) CK(cudaMemsetAsync(d.cw, 0, (size_t)N * 4, st));
-    CK(cudaMemsetAsync(d.tabu, 0, (size_t)M * n * q * 4, st));
     CK(cudaMemsetAsync(d.P, 0, (size_t)M * (n + 1) * 4, st));
     CK(cudaMemsetAsync(d.ul_bit, 0, (size_t)((N + 31) / 32) * 4, st));
     CovSlotState hs;
@@ -3488,14 +3472,18 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
     CK(cudaMemsetAsync(d.P, 0, (size_t)M * (n + 1) * 4, st));
     CK(cudaMemsetAsync(d.ul_bit, 0, (size_t)((N + 31) / 32) * 4, st));
     CK(cudaMemsetAsync(d.zb, 0, (size_t)((N + 31) / 32) * 4, st));
-    switch (q) {
-#define BS_LAUNCH_Q(QQ) \
-    case QQ: k_build_state<QQ><<<(unsigned)ipow_h(q, d.bt_nh), BT_NT, bt_smem_bytes(d.bt_tw), st>>>(d, d_z); break;
+    const BtCode rec = bt_records(d.code, M, q, n, d.bt_nh, d.bt_nl, d.tabu, st);
+    CK(cudaGetLastError());
+    const unsigned bs_grid = (unsigned)ipow_h(q, d.bt_nh);
+    const size_t bs_smem = bt_smem_bytes(q, n, d.bt_tw);
+    switch (n < 2 ? 0 : q) {
+#define BS_LAUNCH_Q(QQ) case QQ: k_build_state<QQ><<<bs_grid, BT_NT, bs_smem, st>>>(d, rec, d_z); break;
     BT_Q_LIST(BS_LAUNCH_Q)
 #undef BS_LAUNCH_Q
-    default: k_build_state<0><<<(unsigned)ipow_h(q, d.bt_nh), BT_NT, bt_smem_bytes(d.bt_tw), st>>>(d, d_z); break;
+    default: k_build_state<0><<<bs_grid, BT_NT, bs_smem, st>>>(d, rec, d_z); break;
     }
     CK(cudaGetLastError());
+    CK(cudaMemsetAsync(d.tabu, 0, (size_t)M * n * q * 4, st));
     CK(cudaMemcpyAsync(d.best, d.code, (size_t)M * 8, cudaMemcpyDeviceToDevice, st));
     unsigned long long zl[2] = {0, 0};
     CK(cudaMemcpyAsync(zl, d_z, 16, cudaMemcpyDeviceToHost, st));

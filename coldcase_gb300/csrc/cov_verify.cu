@@ -581,56 +581,43 @@ __global__ void k_count_above(const uint8_t *__restrict__ D, uint32_t N, int R, 
 }
 
 // ------------------------------------------------ coverage multiplicity ----
-__global__ void k_pack_code(const uint8_t *__restrict__ code, int M, int n, uint64_t *__restrict__ out)
+// the tiles' records of a code given as digits (one outside the alphabet is
+// taken as the largest digit, so that every mark stays within its tile)
+__global__ void k_count_records(const uint8_t *__restrict__ code, int M, int q, int n, int nh, int nl, uint2 *mid,
+                                uint32_t *hi)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-        uint64_t v = 0;
-        for (int j = 0; j < n; j++) v |= (uint64_t)code[(size_t)i * n + j] << (4 * j);
-        out[i] = v;
+        const uint8_t *c = code + (size_t)i * n;
+        bt_record(i, q, n, nh, nl, mid, hi, [&](int j) { return (uint32_t)min((int)c[j], q - 1); });
     }
 }
 
 struct CountGeom {
     int q, n, R, M, nh, nl;
     uint32_t tw;                       // q^nl words per tile
-    uint32_t nitems;                   // ball groups (their last positions follow them)
-    uint32_t pw[COV_MAXN];             // q^(n-1-j)
     uint32_t vcum[COV_MAXN + 2];
 };
 
 // cnt[x] = #{i : d(x, c_i) <= R} saturated at 65535 (the cnt[] of
 // covsearch2e.c:958-967, the OUT=2 map of cov/gemm2/dct.cu:360-411), one CTA
-// per tile (cov_tiles.cuh); the tile's uncovered words are counted too.
+// per tile (cov_tiles.cuh).
 template <int Q>
-__global__ void __launch_bounds__(BT_NT) k_count_tiles(CountGeom g, const uint64_t *__restrict__ code,
-                                                       const uint64_t *__restrict__ items, uint16_t *cnt,
-                                                       unsigned long long *zeros)
+__global__ void __launch_bounds__(BT_NT) k_count_tiles(CountGeom g, BtCode code, uint16_t *cnt)
 {
-    extern __shared__ __align__(16) unsigned char ct_raw[];
-    uint64_t *lpc = (uint64_t *)ct_raw;
-    uint32_t *lid = (uint32_t *)(lpc + BT_LCH);
-    uint32_t *lbase = lid + BT_LCH;
-    uint32_t *tile = lbase + BT_LCH;
-    __shared__ int gcnt[COV_MAXN + 2], gpos[COV_MAXN + 2], gfill[COV_MAXN + 2];
-    uint64_t hp = 0;
-    {
-        uint32_t t = blockIdx.x;
-        for (int j = g.nh - 1; j >= 0; --j) { hp |= (uint64_t)(t % (uint32_t)g.q) << (4 * j); t /= (uint32_t)g.q; }
-    }
-    for (uint32_t x = threadIdx.x; x < g.tw; x += BT_NT) tile[x] = 0;
-    BtScratch sc{lpc, lid, lbase, gcnt, gpos, gfill};
-    bt_mark_tile<Q>(tile, g.q, g.n, g.R, g.M, code, g.pw, g.nh, g.nl, items,
-                 reinterpret_cast<const uint8_t *>(items + g.nitems), g.vcum, hp, sc,
-                 [](uint32_t) { return 1u; });
-    unsigned long long z = 0;
+    extern __shared__ __align__(16) uint32_t ct_sm[];
+    const BtTile tl = bt_layout(g.q, g.n, g.tw);
+    bt_mark_tile<Q>(ct_sm, tl, blockIdx.x, g.q, g.n, g.R, g.M, code, g.nh, g.nl, g.vcum,
+                    [](uint32_t) { return 1u; });
     uint16_t *out = cnt + (size_t)blockIdx.x * g.tw;
-    for (uint32_t x = threadIdx.x; x < g.tw; x += BT_NT) {
-        const uint32_t v = tile[x];
-        out[x] = (uint16_t)min(v, 65535u);
-        z += v == 0;
-    }
-    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    if ((threadIdx.x & 31) == 0 && z && zeros) atomicAdd(zeros, z);
+    const uint32_t *tile = ct_sm + tl.a0;
+    // whole 32-bit words between the first and the last 4-byte boundary
+    const uint32_t head = (uint32_t)(reinterpret_cast<uintptr_t>(out) >> 1) & 1u;
+    const uint32_t np = (g.tw - head) >> 1;
+    for (uint32_t k = threadIdx.x; k < np; k += BT_NT)
+        *reinterpret_cast<uint32_t *>(out + head + 2 * k) =
+            min(tile[head + 2 * k], 65535u) | (min(tile[head + 2 * k + 1], 65535u) << 16);
+    if (threadIdx.x == 0 && head) out[0] = (uint16_t)min(tile[0], 65535u);
+    if (threadIdx.x == 1 && ((g.tw - head) & 1u)) out[g.tw - 1] = (uint16_t)min(tile[g.tw - 1], 65535u);
 }
 
 // ------------------------------------------------------------ finisher ----
@@ -795,15 +782,28 @@ CovDeviceFlags g_dt_attr;   // shared-memory opt-in of the transform kernels, pe
 CovDeviceFlags g_ct_attr;   // the same for the tile count
 
 // the tile count of the alphabet size q (a kernel of its own for q = 5..8)
-void ct_launch(int q, unsigned grid, size_t smem, cudaStream_t st, const CountGeom &g, const uint64_t *code,
-               const uint64_t *items, uint16_t *cnt)
+void ct_launch(const CountGeom &g, BtCode code, uint16_t *cnt, cudaStream_t st)
 {
-    switch (q) {
-#define CT_LAUNCH_Q(QQ) case QQ: k_count_tiles<QQ><<<grid, BT_NT, smem, st>>>(g, code, items, cnt, nullptr); break;
+    const unsigned grid = (unsigned)ipw(g.q, g.nh);
+    const size_t smem = bt_smem_bytes(g.q, g.n, g.tw);
+    switch (g.n < 2 ? 0 : g.q) {
+#define CT_LAUNCH_Q(QQ) case QQ: k_count_tiles<QQ><<<grid, BT_NT, smem, st>>>(g, code, cnt); break;
     BT_Q_LIST(CT_LAUNCH_Q)
 #undef CT_LAUNCH_Q
-    default: k_count_tiles<0><<<grid, BT_NT, smem, st>>>(g, code, items, cnt, nullptr); break;
+    default: k_count_tiles<0><<<grid, BT_NT, smem, st>>>(g, code, cnt); break;
     }
+}
+
+// the tile geometry of a count of M codewords
+CountGeom count_geom(int q, int n, int R, int M)
+{
+    CountGeom g;
+    memset(&g, 0, sizeof g);
+    g.q = q; g.n = n; g.R = R; g.M = M;
+    bt_geom(q, n, R, M, &g.nh, &g.nl);
+    g.tw = (uint32_t)ipw(q, g.nl);
+    bt_vcum_h(q, n, R, g.nl, g.vcum);
+    return g;
 }
 
 int ct_attrs()
@@ -811,9 +811,9 @@ int ct_attrs()
     int dev = 0;
     if (g_ct_attr.done(dev)) return 0;
     CK(cudaFuncSetAttribute(k_count_tiles<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            (int)bt_smem_bytes(BT_MAX)));
+                            BT_SMEM_MAX));
 #define CT_ATTR_Q(QQ) \
-    CK(cudaFuncSetAttribute(k_count_tiles<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bt_smem_bytes(BT_MAX)));
+    CK(cudaFuncSetAttribute(k_count_tiles<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
     BT_Q_LIST(CT_ATTR_Q)
 #undef CT_ATTR_Q
     g_ct_attr.set(dev);
@@ -1094,30 +1094,17 @@ int cov_count_dev(int32_t q, int32_t n, int32_t R, const uint8_t *d_code, int32_
     cudaStream_t st = (cudaStream_t)stream;
     rc = ct_attrs();
     if (rc) return rc;
-    CountGeom g;
-    memset(&g, 0, sizeof g);
-    g.q = q; g.n = n; g.R = R; g.M = M;
-    bt_geom(q, n, &g.nh, &g.nl);
-    g.tw = (uint32_t)ipw(q, g.nl);
-    for (int j = 0; j < n; j++) g.pw[j] = dg.pw[n - 1 - j];
-    std::vector<uint8_t> last;
-    std::vector<uint64_t> items = bt_items_h(q, n, R, g.nh, g.vcum, last);
-    g.nitems = (uint32_t)items.size();
-    // one scratch allocation: the ball groups, their last positions, then
-    // the packed code
+    const CountGeom g = count_geom(q, n, R, M);
     void *tmp = nullptr;
-    const size_t ib = items.size() * 8, lb = (last.size() + 7) / 8 * 8;
-    CK(cudaMallocAsync(&tmp, ib + lb + (size_t)std::max(M, 1) * 8, st));
-    uint64_t *d_items = (uint64_t *)tmp, *d_pk = d_items + (ib + lb) / 8;
-    CK(cudaMemcpyAsync(d_items, items.data(), ib, cudaMemcpyHostToDevice, st));
-    CK(cudaMemcpyAsync(d_items + items.size(), last.data(), last.size(), cudaMemcpyHostToDevice, st));
+    CK(cudaMallocAsync(&tmp, (size_t)std::max(M, 1) * BT_REC_BYTES, st));
+    uint2 *mid = (uint2 *)tmp;
+    uint32_t *hi = (uint32_t *)(mid + M);
     if (M > 0) {
-        k_pack_code<<<std::min(1024, (M + 255) / 256), 256, 0, st>>>(d_code, M, n, d_pk);
+        k_count_records<<<std::min(1024, (M + 127) / 128), 128, 0, st>>>(d_code, M, q, n, g.nh, g.nl, mid, hi);
         CK(cudaGetLastError());
     }
-    ct_launch(q, (unsigned)ipw(q, g.nh), bt_smem_bytes(g.tw), st, g, d_pk, d_items, d_cnt);
+    ct_launch(g, BtCode{hi, mid}, d_cnt, st);
     CK(cudaGetLastError());
-    // items is pageable host memory: wait before it goes out of scope
     CK(cudaStreamSynchronize(st));
     CK(cudaFreeAsync(tmp, st));
     return COV_OK;
@@ -1170,15 +1157,8 @@ int cov_finish(int32_t q, int32_t n, int32_t R, int32_t M, const uint8_t *code, 
     rc = ct_attrs();
     if (rc) return rc;
     // tile count of the deduplicated words
-    CountGeom g;
-    memset(&g, 0, sizeof g);
-    g.q = q; g.n = n; g.R = R; g.M = m0;
-    bt_geom(q, n, &g.nh, &g.nl);
-    g.tw = (uint32_t)ipw(q, g.nl);
-    for (int j = 0; j < n; j++) g.pw[j] = dg.pw[n - 1 - j];
-    std::vector<uint8_t> tlast, blast;
-    std::vector<uint64_t> titems = bt_items_h(q, n, R, g.nh, g.vcum, tlast);
-    g.nitems = (uint32_t)titems.size();
+    const CountGeom g = count_geom(q, n, R, m0);
+    std::vector<uint8_t> blast;
     // whole-ball groups for the top-up (no high digits)
     uint32_t bcum[COV_MAXN + 2];
     std::vector<uint64_t> bitems = bt_items_h(q, n, R, 0, bcum, blast);
@@ -1187,30 +1167,28 @@ int cov_finish(int32_t q, int32_t n, int32_t R, int32_t M, const uint8_t *code, 
     fg.q = q; fg.n = n; fg.R = R; fg.M = M; fg.N = dg.N;
     for (int j = 0; j < n; j++) fg.pw[j] = dg.pw[n - 1 - j];
     fg.ngroups = bcum[std::min(R, n)];
-    const size_t tib = titems.size() * 8, tlb = (tlast.size() + 7) / 8 * 8;
+    const size_t trb = ((size_t)m0 * BT_REC_BYTES + 7) / 8 * 8;
     const size_t bib = bitems.size() * 8, blb = (blast.size() + 7) / 8 * 8;
     const size_t cb = ((size_t)dg.N * 2 + 15) / 16 * 16;
     char *buf = nullptr;
-    if (cudaMalloc(&buf, tib + tlb + bib + blb + (size_t)M * 8 + cb + 16) != cudaSuccess) {
+    if (cudaMalloc(&buf, trb + bib + blb + (size_t)M * 8 + cb + 16) != cudaSuccess) {
         cudaGetLastError();
         return COV_ENOMEM;
     }
-    uint64_t *d_ti = (uint64_t *)buf;
-    uint64_t *d_bi = (uint64_t *)(buf + tib + tlb);
-    uint8_t *d_bl = (uint8_t *)(buf + tib + tlb + bib);
-    uint64_t *d_code = (uint64_t *)(buf + tib + tlb + bib + blb);
-    uint16_t *d_cnt = (uint16_t *)(buf + tib + tlb + bib + blb + (size_t)M * 8);
-    unsigned long long *d_z = (unsigned long long *)(buf + tib + tlb + bib + blb + (size_t)M * 8 + cb);
+    uint64_t *d_bi = (uint64_t *)(buf + trb);
+    uint8_t *d_bl = (uint8_t *)(buf + trb + bib);
+    uint64_t *d_code = (uint64_t *)(buf + trb + bib + blb);
+    uint16_t *d_cnt = (uint16_t *)(buf + trb + bib + blb + (size_t)M * 8);
+    unsigned long long *d_z = (unsigned long long *)(buf + trb + bib + blb + (size_t)M * 8 + cb);
     auto done = [&](int r) { cudaFree(buf); return r; };
     cudaError_t e = cudaSuccess;
-    e = cudaMemcpy(d_ti, titems.data(), tib, cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_ti + titems.size(), tlast.data(), tlast.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess) e = cudaMemcpy(d_bi, bitems.data(), bib, cudaMemcpyHostToDevice);
+    e = cudaMemcpy(d_bi, bitems.data(), bib, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(d_bl, blast.data(), blast.size(), cudaMemcpyHostToDevice);
     if (e == cudaSuccess && m0 > 0) e = cudaMemcpy(d_code, pk.data(), (size_t)m0 * 8, cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemset(d_z, 0, 8);
     if (e != cudaSuccess) return done(-(100 + (int)e));
-    ct_launch(q, (unsigned)ipw(q, g.nh), bt_smem_bytes(g.tw), 0, g, d_code, d_ti, d_cnt);
+    const BtCode rec = bt_records(d_code, m0, q, n, g.nh, g.nl, buf, 0);
+    ct_launch(g, rec, d_cnt, 0);
     e = cudaGetLastError();
     if (e == cudaSuccess && m0 < M) {
         k_topup<<<1, 512>>>(fg, d_cnt, d_code, m0, d_bi, d_bl);
