@@ -14,14 +14,16 @@
 //    q^g rows x W words, all R+1 int32 layers of a tile at once, so a whole
 //    transform reads and writes the layers in a few sweeps instead of n.
 //    The same layers with the code itself marked give cnt.
-//  * Sequences.  A persistent kernel on one thread-block cluster runs the
-//    steps that are inherently one after another, with no host round trip:
-//    the lazy greedy placement (bounds from a gain map, the best bound
-//    re-counted exactly until it is current, then placed), the exact peel
-//    (codewords removed in a given order while each covers no word alone)
-//    and +-1 balls of a list of words.  Every CTA of the cluster walks a
-//    share of each ball; they meet at hardware cluster barriers and reduce
-//    through distributed shared memory.
+//  * Sequences.  The lazy greedy placement (bounds from a gain map, the best
+//    bounds re-counted exactly until the best is current, then placed) is one
+//    cooperative kernel over the whole GPU with no host round trip between
+//    its steps; it counts on masks of the uncovered words, a 64-bit word for
+//    the q^b words that share their high digits.  The exact peel (codewords
+//    removed in a given order while each covers no word alone) is a
+//    persistent kernel on one thread-block cluster: every CTA walks a share
+//    of each ball, and they meet at hardware cluster barriers and reduce
+//    through distributed shared memory.  The +-1 balls of a list of words
+//    commute and run at once.
 //
 // Words are indexed MSB-first (x = sum_j w_j q^(n-1-j)), as everywhere in
 // this library.  Extraction returns positions in increasing index order, and
@@ -48,6 +50,10 @@ namespace cg = cooperative_groups;
 #define SEQ_NT 512
 #define SEQ_CL 8                    // CTAs of the sequence cluster
 #define CAND_CAP (1 << 17)          // candidate bounds kept on the device per refresh
+#define GREEDY_NT 512
+#define GREEDY_MAXG 512             // most CTAs of the greedy kernel (one per SM)
+#define THR_BINS 1024               // histogram bins behind an extraction threshold
+#define EXT_CHUNK 8192              // words of one block of an ordered extraction
 
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { \
     fprintf(stderr, "covgpu: CUDA error %s at %s:%d\n", cudaGetErrorString(e_), __FILE__, __LINE__); \
@@ -59,10 +65,16 @@ struct SeqState {
     long long evals;             // exact ball counts made
     int placed, removed;         // words placed / removed by the launch
     int status;                  // SEQ_*
-    int pad;
+    int best;                    // greedy: no word's gain is higher at the end of the launch
+};
+
+// what a refresh of the greedy's candidates leaves on the device
+struct RefreshInfo {
+    int top;                     // maximum of the map
+    int thr;                     // candidates are the words with map >= thr
+    uint32_t found;              // how many there are (saturated)
 };
 enum { SEQ_DONE = 0, SEQ_REFRESH = 1, SEQ_COVERED = 2, SEQ_TARGET = 3, SEQ_GUARD = 5 };
-enum { MODE_GREEDY = 0, MODE_PEEL = 1, MODE_APPLY = 2 };
 
 struct cov_lns {
     int q, n, R;
@@ -76,9 +88,19 @@ struct cov_lns {
     uint32_t ngroups = 0;
     uint32_t *cand = nullptr;       // greedy candidates (positions, increasing)
     int32_t *bound = nullptr;       // their gain bounds
-    int32_t *fresh = nullptr;       // epoch at which a bound was last made exact
+    int nb = 0;                     // digits of a mask block: the most with q^nb <= 64
+    uint32_t blk = 1;               // its q^nb words
+    uint64_t *um = nullptr;         // uncovered words of every block (built by each greedy call)
+    uint64_t *pball = nullptr;      // ball groups on the n - nb high digits
+    uint8_t *pball_last = nullptr;
+    uint32_t npgroups = 0;
+    uint64_t *lowball = nullptr;    // [blk][nb + 1]: words of a block within 0..nb of each of its words
+    unsigned long long *nom = nullptr;   // [2 * GREEDY_MAXG] best keys of the greedy's CTAs
+    uint32_t *acc = nullptr;        // [3 * (GREEDY_MAXG + 1)] sums of the greedy's steps, then its barrier
+    RefreshInfo *info = nullptr;
     uint32_t *list = nullptr;       // words of a sequence (placed, peeled or applied)
     uint8_t *flag = nullptr;        // per listed word: removed by the peel
+    int list_cap = 0;
     SeqState *seq = nullptr;
     void *scratch = nullptr;        // small device buffers of the calls
     size_t scratch_bytes = 0;
@@ -274,43 +296,86 @@ __global__ void k_lns_max(const int32_t *A, uint32_t N, int *out)
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
 
-// histogram of values v >= 1 in nbins bins of [1, vmax]: bin = (v-1)*nbins/vmax
 // histogram of the positive values: value v in bin (min(v,vmax)-1)*nbins/vmax.
 // Counted per block in shared memory (the lanes of a warp that share a bin
 // add once), then one global add per bin and block: the values of a gain map
-// crowd into few bins, where per-element global atomics serialise.
-__global__ void k_lns_hist(const int32_t *A, uint32_t N, int nbins, int vmax, unsigned long long *hist)
+// crowd into few bins, where per-element global atomics serialise.  Eight
+// loads of a thread in flight (one at a time took 65 us at 6^9, bound by
+// latency).  vmax_dev (may be null) replaces vmax; top (may be null) receives
+// the maximum.
+__global__ void __launch_bounds__(LNS_NT) k_lns_hist(const int32_t *A, uint32_t N, int nbins, int vmax,
+                                                     const int *vmax_dev, unsigned long long *hist, int *top)
 {
     extern __shared__ uint32_t lh[];
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) lh[b] = 0;
+    if (vmax_dev) vmax = max(1, __ldcg(vmax_dev));
     __syncthreads();
     // (v-1)*nbins in 32 bits when it cannot overflow
     const bool narrow = (unsigned long long)vmax * (unsigned long long)nbins < (1ull << 32);
-    for (uint32_t x0 = blockIdx.x * blockDim.x; x0 < N; x0 += gridDim.x * blockDim.x) {
-        const uint32_t x = x0 + threadIdx.x;
-        int b = -1;
-        if (x < N) {
-            const int v = A[x];
-            if (v >= 1) {
-                const uint32_t t = (uint32_t)(min(v, vmax) - 1);
+    int m = INT_MIN;
+    for (unsigned long long x0 = (unsigned long long)blockIdx.x * (8 * LNS_NT); x0 < N;
+         x0 += (unsigned long long)gridDim.x * (8 * LNS_NT)) {
+        int v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const unsigned long long x = x0 + (unsigned)u * LNS_NT + threadIdx.x;
+            v[u] = x < N ? __ldcg(&A[x]) : INT_MIN;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            m = max(m, v[u]);
+            int b = -1;
+            if (v[u] >= 1) {
+                const uint32_t t = (uint32_t)(min(v[u], vmax) - 1);
                 b = narrow ? (int)(t * (uint32_t)nbins / (uint32_t)vmax)
                            : (int)((unsigned long long)t * (unsigned long long)nbins / (unsigned long long)vmax);
             }
+            const unsigned grp = __match_any_sync(0xffffffffu, b);
+            if (b >= 0 && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&lh[b], (uint32_t)__popc(grp));
         }
-        const unsigned grp = __match_any_sync(0xffffffffu, b);
-        if (b >= 0 && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&lh[b], (uint32_t)__popc(grp));
     }
     __syncthreads();
     for (int b = threadIdx.x; b < nbins; b += blockDim.x)
         if (lh[b]) atomicAdd(&hist[b], (unsigned long long)lh[b]);
+    if (top) {
+        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+        if ((threadIdx.x & 31) == 0) atomicMax(top, m);
+    }
 }
 
-// ordered compaction of {x : A[x] >= thr}: per-block counts, then positions
-__global__ void k_lns_count_ge(const int32_t *A, uint32_t N, int thr, uint32_t chunk, uint32_t *bcount)
+// extraction threshold that keeps {map >= thr} within cap, from the histogram
+// of [1, vmax] in THR_BINS bins: the least value of the lowest bin whose tail
+// fits (one thread: the walk ends after the few bins that hold cap words)
+__global__ void k_lns_threshold(const unsigned long long *hist, int vmax, const int *vmax_dev, long long cap,
+                                RefreshInfo *info)
 {
-    const uint32_t x0 = blockIdx.x * chunk, x1 = min(N, x0 + chunk);
+    const int nb = THR_BINS, top = info->top;
+    if (vmax_dev) vmax = max(1, *vmax_dev);
+    int thr = 1;
+    if (top > 1) {
+        long long above = 0;
+        int b = nb;
+        while (b > 0 && above + (long long)hist[b - 1] <= cap) { above += (long long)hist[b - 1]; b--; }
+        // bin b holds the values v with (v-1)*nb/vmax == b: the first such v
+        thr = b >= nb ? top : (int)(((long long)b * vmax + nb - 1) / nb) + 1;
+        thr = max(1, min(thr, top));
+    }
+    info->thr = thr;
+}
+
+// ordered compaction of {x : A[x] >= thr}: counts of chunks of EXT_CHUNK
+// words, their prefix sums, then positions; thr_dev (may be null) replaces thr
+__global__ void __launch_bounds__(LNS_NT) k_lns_count_ge(const int32_t *A, uint32_t N, int thr, const int *thr_dev,
+                                                         uint32_t *bcount)
+{
+    if (thr_dev) thr = __ldcg(thr_dev);
+    const uint32_t x0 = blockIdx.x * EXT_CHUNK;
     uint32_t c = 0;
-    for (uint32_t x = x0 + threadIdx.x; x < x1; x += blockDim.x) c += A[x] >= thr;
+#pragma unroll 8
+    for (uint32_t k = threadIdx.x; k < EXT_CHUNK; k += LNS_NT) {
+        const uint32_t x = x0 + k;
+        if (x < N) c += __ldcg(&A[x]) >= thr;
+    }
     __shared__ uint32_t red[LNS_NT / 32];
     for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = c;
@@ -322,13 +387,47 @@ __global__ void k_lns_count_ge(const int32_t *A, uint32_t N, int thr, uint32_t c
     }
 }
 
-__global__ void k_lns_emit_ge(const int32_t *A, uint32_t N, int thr, uint32_t chunk, const uint32_t *boff,
-                              uint32_t cap, uint32_t *oidx, int32_t *oval)
+// bcount[] -> its exclusive prefix sums (one block; saturated), the total to
+// *found
+__global__ void __launch_bounds__(1024) k_lns_scan(uint32_t *bcount, uint32_t nb, unsigned long long *found, uint32_t *found32)
 {
-    const uint32_t x0 = blockIdx.x * chunk, x1 = min(N, x0 + chunk);
+    __shared__ unsigned long long ws[32], run;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) run = 0;
+    __syncthreads();
+    for (uint32_t b0 = 0; b0 < nb; b0 += 1024) {
+        const uint32_t b = b0 + threadIdx.x;
+        const unsigned long long c = b < nb ? bcount[b] : 0;
+        unsigned long long x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) ws[warp] = x;
+        __syncthreads();
+        unsigned long long before = run;
+        for (int w = 0; w < warp; w++) before += ws[w];
+        if (b < nb) bcount[b] = (uint32_t)min(before + x - c, 0xffffffffull);
+        __syncthreads();
+        if (threadIdx.x == 1023) run = before + x;
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) {
+        if (found) *found = run;
+        if (found32) *found32 = (uint32_t)min(run, 0xffffffffull);
+    }
+}
+
+__global__ void __launch_bounds__(LNS_NT) k_lns_emit_ge(const int32_t *A, uint32_t N, int thr, const int *thr_dev,
+                                                        const uint32_t *boff, uint32_t cap, uint32_t *oidx, int32_t *oval)
+{
+    if (thr_dev) thr = __ldcg(thr_dev);
+    const uint32_t x0 = blockIdx.x * EXT_CHUNK, x1 = min(N, x0 + EXT_CHUNK);
+    const uint32_t first = boff[blockIdx.x];
+    if (first >= cap || (blockIdx.x + 1 < gridDim.x && boff[blockIdx.x + 1] == first)) return;
     __shared__ uint32_t wbase[LNS_NT / 32];
     __shared__ uint32_t run;
-    if (threadIdx.x == 0) run = boff[blockIdx.x];
+    if (threadIdx.x == 0) run = first;
     __syncthreads();
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     for (uint32_t xb = x0; xb < x1; xb += blockDim.x) {
@@ -336,7 +435,7 @@ __global__ void k_lns_emit_ge(const int32_t *A, uint32_t N, int thr, uint32_t ch
         const bool take = x < x1 && A[x] >= thr;
         const unsigned m = __ballot_sync(0xffffffffu, take);
         if (lane == 0) wbase[warp] = __popc(m);
-        __syncthreads();
+        if (!__syncthreads_or(take)) continue;
         if (threadIdx.x == 0) {
             uint32_t s = run;
             for (int w = 0; w < LNS_NT / 32; w++) { const uint32_t c = wbase[w]; wbase[w] = s; s += c; }
@@ -360,7 +459,7 @@ __device__ __forceinline__ uint64_t lns_pack(uint32_t x, int q, int n)
 }
 
 struct BallGeom {
-    int q, n;
+    int q, n, R;
     uint32_t pw[COV_MAXN];
     const uint64_t *items;
     const uint8_t *last;
@@ -429,55 +528,357 @@ __global__ void k_lns_zero(const uint16_t *cnt, uint32_t N, int target, unsigned
     if ((threadIdx.x & 31) == 0 && c) atomicAdd(out, c);
 }
 
-// ------------------------------------------------------- the sequences ----
-struct SeqArgs {
-    int mode;
+// ------------------------------------------------- uncovered-word masks ----
+// um[p]: bit y set iff the word p * blk + y is uncovered.  A block of words
+// (the blk = q^nb that share their high digits) is staged through shared
+// memory, so that the counts are read once in order.
+__global__ void __launch_bounds__(LNS_NT) k_lns_masks(const uint16_t *__restrict__ cnt, uint32_t nblk, int blk,
+                                                      uint64_t *__restrict__ um)
+{
+    __shared__ uint8_t z[LNS_NT * 64];
+    const uint32_t p0 = blockIdx.x * LNS_NT;
+    const uint32_t np = min((uint32_t)LNS_NT, nblk - p0);
+    const uint16_t *c = cnt + (size_t)p0 * blk;
+#pragma unroll 8
+    for (uint32_t k = threadIdx.x; k < np * (uint32_t)blk; k += LNS_NT) z[k] = __ldcg(&c[k]) == 0;
+    __syncthreads();
+    if (threadIdx.x < np) {
+        uint64_t m = 0;
+        for (int y = 0; y < blk; y++) m |= (uint64_t)z[threadIdx.x * blk + y] << y;
+        um[p0 + threadIdx.x] = m;
+    }
+}
+
+// -------------------------------------------------------- lists of balls ----
+// sgn over the balls of k listed words at once; the saturating updates of one
+// sign commute, so the counts are those of one word after another.  *delta
+// receives the change of the number of uncovered words.
+__global__ void __launch_bounds__(LNS_NT) k_lns_apply(uint16_t *cnt, BallGeom b, const uint32_t *list, int k, int sgn,
+                                                      uint32_t per, unsigned long long *delta)
+{
+    long long c = 0;
+    const unsigned long long total = (unsigned long long)k * per;
+    for (unsigned long long job = blockIdx.x; job < total; job += gridDim.x) {
+        const uint32_t base = list[job / per];
+        const uint32_t it = (uint32_t)(job % per) * LNS_NT + threadIdx.x;
+        if (it >= b.ngroups) continue;
+        const uint64_t pc = lns_pack(base, b.q, b.n);
+        ball_group(b, it, base, pc, [&](uint32_t w) {
+            unsigned short *p = reinterpret_cast<unsigned short *>(cnt) + w;
+            unsigned short v = __ldcg(p);
+            for (;;) {                                   // ends: a failed swap means another ball's succeeded
+                if (v == (sgn > 0 ? 65535 : 0)) break;
+                const unsigned short old = atomicCAS(p, v, (unsigned short)(v + sgn));
+                if (old == v) {
+                    if (sgn > 0) c -= v == 0;            // newly covered
+                    else c += v == 1;                    // newly uncovered
+                    break;
+                }
+                v = old;
+            }
+        });
+    }
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if ((threadIdx.x & 31) == 0 && c) atomicAdd(delta, (unsigned long long)c);
+}
+
+// --------------------------------------------------------------- the greedy ----
+struct GreedyArgs {
     uint16_t *cnt;
-    BallGeom b;
-    // greedy: candidates (increasing positions) and their bounds; placed
-    // words are appended to list[]
-    const uint32_t *cand;
-    int32_t *bound;
-    int32_t *fresh;
-    int ncand, thr, room;          // room: words still to place
+    uint64_t *um;
+    BallGeom b, whole;             // the ball on the n - nb high digits (b.n of them), and on all
+    const uint64_t *lowball;
+    int nb, blk;
+    uint64_t full;                 // the blk bits of a block
+    const uint32_t *cand;          // candidates (increasing positions) and their exact gains
+    const int32_t *bound;
+    const RefreshInfo *info;
+    uint32_t cand_cap;
+    int room;                      // words still to place
     int eval_cap;                  // exact counts since the last placement after which a
                                    // fresh map is cheaper (the host refreshes)
-    long long max_steps;           // bound on the steps of one launch
-    // peel / apply: the listed words in order
+    long long max_steps;           // bound on the steps of the launch
+    int team, nteam;               // CTAs that count one candidate together; candidates at once
+    int own;                       // most candidates of one CTA
+    unsigned long long *nom;       // [2 * G]
+    uint32_t *acc;                 // [3 * (GREEDY_MAXG + 1)]
+    unsigned *bar;                 // arrivals at the grid barrier (cleared by the host)
+    unsigned long long wait_ns;    // longest wait at a barrier
     uint32_t *list;
-    int nlist, sign;
+    SeqState *st;
+};
+
+// key of a candidate: larger bound first, then the lower position; 0: none
+__device__ __forceinline__ unsigned long long cand_key(int32_t bound, int pos)
+{
+    return ((unsigned long long)(uint32_t)(bound + 0x40000000) << 32) | (uint32_t)(0x7fffffff - pos);
+}
+__device__ __forceinline__ int key_pos(unsigned long long k) { return 0x7fffffff - (int)(uint32_t)k; }
+__device__ __forceinline__ int key_bound(unsigned long long k) { return (int)(uint32_t)(k >> 32) - 0x40000000; }
+
+__device__ __forceinline__ unsigned long long lns_ns()
+{
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    return t;
+}
+
+// All CTAs of the cooperative launch meet; every thread's writes before it
+// are visible after it.  False when the wait ran out.
+__device__ __forceinline__ bool grid_meet(unsigned *bar, unsigned target, unsigned long long wait_ns)
+{
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(bar, 1u);
+        const unsigned long long t0 = lns_ns();
+        int good = 1;
+        unsigned seen;
+        for (unsigned spin = 1;; spin++) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+            if (seen >= target) break;
+            if ((spin & 255u) == 0 && lns_ns() - t0 > wait_ns) { good = 0; break; }
+        }
+        __threadfence();
+        ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
+__device__ __forceinline__ unsigned long long warp_max64(unsigned long long k)
+{
+    for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
+    return k;
+}
+
+// Greedy placement over the whole GPU, one CTA per SM.  CTA c owns the
+// candidates p = c mod G, their bounds in its shared memory.  A step:
+//   nominate: every CTA publishes the best key among its current bounds and
+//     the best among its stale ones; the grid meets;
+//   act: every CTA reads all keys and takes the same decision.  The best of
+//     all is current: its ball is placed, and every bound becomes stale.  Else
+//     the nteam best stale nominees above the best current one are counted
+//     exactly, each by a team of CTAs; the grid meets.
+// A word is placed only when its exact gain is at least every bound, so it is
+// the word that counting one bound at a time would place.
+//
+// A count reads one mask per q^nb words instead of a counter per word (53,719
+// gathers for 182,791 at q7 n9 R4, from 6.6 MB instead of 81 MB), and a step
+// costs its two grid barriers and some six dependent trips to L2 whatever the
+// number of candidates counted: 11 us for 25 candidates at 6^9, against 15 us
+// for one on a cluster of 8 CTAs.  The fill of 6^9 (651 words) spends 42 ms
+// here where the cluster took 247.
+__global__ void __launch_bounds__(GREEDY_NT) k_lns_greedy(GreedyArgs a)
+{
+    extern __shared__ int gr_own[];                // [own] bounds, [own] epochs at which they were exact
+    __shared__ unsigned long long s_stale[GREEDY_MAXG], s_team[GREEDY_MAXG], s_w[2][GREEDY_NT / 32];
+    __shared__ unsigned long long s_kf, s_ks;
+    __shared__ uint64_t s_low[8];
+    __shared__ uint64_t s_pc, s_pw;                // the word's high digits, and all of them
+    __shared__ unsigned s_sum[GREEDY_NT / 32];
+    __shared__ int s_rank, s_count;
+    const int G = (int)gridDim.x, me = (int)blockIdx.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int *const sb = gr_own, *const sf = gr_own + a.own;
+    const int ncand = (int)min(a.info->found, a.cand_cap);
+    const int thr = a.info->thr;
+    const int mine = ncand > me ? (ncand - me + G - 1) / G : 0;
+    for (int i = threadIdx.x; i < mine; i += GREEDY_NT) { sb[i] = a.bound[me + i * G]; sf[i] = 1; }
+    long long uncov = a.st->uncov, evals = 0, steps = 0;
+    int epoch = 1, placed = 0, since = 0, status = SEQ_REFRESH, best = 0, buf = 0;
+    unsigned met = 0;
+    bool ok = ncand > 0;
+    __syncthreads();
+    while (ok) {
+        // ---- nominate
+        unsigned long long kf = 0, ks = 0;
+        for (int i = threadIdx.x; i < mine; i += GREEDY_NT) {
+            const unsigned long long k = cand_key(sb[i], me + i * G);
+            if (sf[i] == epoch) kf = max(kf, k);
+            else ks = max(ks, k);
+        }
+        kf = warp_max64(kf);
+        ks = warp_max64(ks);
+        if (lane == 0) { s_w[0][warp] = kf; s_w[1][warp] = ks; }
+        __syncthreads();
+        if (warp == 0) {
+            kf = warp_max64(lane < GREEDY_NT / 32 ? s_w[0][lane] : 0);
+            ks = warp_max64(lane < GREEDY_NT / 32 ? s_w[1][lane] : 0);
+            if (lane == 0) { __stcg(&a.nom[me], kf); __stcg(&a.nom[G + me], ks); }
+        }
+        if (!(ok = grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
+        // ---- the decision, the same in every CTA
+        kf = ks = 0;
+        for (int t = threadIdx.x; t < G; t += GREEDY_NT) {
+            kf = max(kf, __ldcg(&a.nom[t]));
+            const unsigned long long s = __ldcg(&a.nom[G + t]);
+            s_stale[t] = s;
+            ks = max(ks, s);
+        }
+        kf = warp_max64(kf);
+        ks = warp_max64(ks);
+        if (lane == 0) { s_w[0][warp] = kf; s_w[1][warp] = ks; }
+        __syncthreads();
+        if (warp == 0) {
+            kf = warp_max64(lane < GREEDY_NT / 32 ? s_w[0][lane] : 0);
+            ks = warp_max64(lane < GREEDY_NT / 32 ? s_w[1][lane] : 0);
+            if (lane == 0) { s_kf = kf; s_ks = ks; s_rank = -1; s_count = 0; }
+        }
+        __syncthreads();
+        kf = s_kf;
+        ks = s_ks;
+        const unsigned long long top = max(kf, ks);
+        const bool fresh = kf > ks;
+        best = top ? key_bound(top) : 0;
+        int stop = -1;
+        if (uncov <= 0) stop = SEQ_COVERED;
+        else if (placed >= a.room) stop = SEQ_TARGET;
+        else if (++steps > a.max_steps) stop = SEQ_GUARD;
+        // below the threshold a word outside the candidates could tie or beat
+        // the best: the host refreshes the bounds (and stops when the fresh
+        // map has no positive gain)
+        else if (!top || best < thr) stop = SEQ_REFRESH;
+        // so many bounds went stale that a fresh map is cheaper
+        else if (!fresh && since >= a.eval_cap) stop = SEQ_REFRESH;
+        if (stop >= 0) { status = stop; break; }
+        uint32_t *const acc = a.acc + buf * (GREEDY_MAXG + 1);
+        const int next = buf == 2 ? 0 : buf + 1;
+        if (me == 0)               // last read two steps ago, next written in the next step
+            for (int t = threadIdx.x; t <= a.nteam; t += GREEDY_NT) __stcg(&a.acc[next * (GREEDY_MAXG + 1) + t], 0u);
+        int pos = -1, share = me, shares = G;
+        if (fresh) {
+            pos = key_pos(top);
+        } else {
+            // the nominees to count: the nteam best stale keys above the best
+            // current one, each with its own team
+            for (int t = threadIdx.x; t < G; t += GREEDY_NT) {
+                const unsigned long long k = s_stale[t];
+                if (k <= kf) continue;
+                int rank = 0;
+                for (int u = 0; u < G; u++) rank += s_stale[u] > k;
+                if (rank < a.nteam) {
+                    s_team[rank] = k;
+                    if (t == me) s_rank = rank;
+                    atomicAdd(&s_count, 1);
+                }
+            }
+            __syncthreads();
+            const int team = me / a.team;
+            share = me - team * a.team;
+            shares = a.team;
+            if (team < s_count) pos = key_pos(s_team[team]);
+        }
+        unsigned c = 0;
+        if (pos >= 0) {
+            const uint32_t word = a.cand[pos];
+            const uint32_t pre = word / (uint32_t)a.blk, low = word - pre * (uint32_t)a.blk;
+            if (warp == 0) {
+                uint32_t d = 0;
+                if (lane < a.b.n) d = (pre / a.b.pw[lane]) % (uint32_t)a.b.q;
+                const uint32_t lo = __reduce_or_sync(0xffffffffu, lane < 8 ? d << (4 * lane) : 0u);
+                const uint32_t hi = __reduce_or_sync(0xffffffffu, lane >= 8 && lane < 16 ? d << (4 * (lane - 8)) : 0u);
+                if (lane == 0) {
+                    s_pc = ((uint64_t)hi << 32) | lo;
+                    s_pw = s_pc;
+                    for (uint32_t j = (uint32_t)a.whole.n, y = low; j-- > (uint32_t)a.b.n; y /= (uint32_t)a.b.q)
+                        s_pw |= (uint64_t)(y % (uint32_t)a.b.q) << (4 * j);
+                }
+            } else if (warp == 1 && lane <= a.nb) {
+                s_low[lane] = a.lowball[low * (uint32_t)(a.nb + 1) + (uint32_t)lane];
+            }
+            __syncthreads();
+            const uint64_t pc = s_pc;
+            const int R = (int)a.b.R;
+            for (uint32_t it = (uint32_t)share * GREEDY_NT + threadIdx.x; it < a.b.ngroups;
+                 it += (uint32_t)shares * GREEDY_NT) {
+                const int r = __popcll(cov_spread(a.b.items[it])) + (a.b.last[it] != 0xff);
+                const uint64_t m = R - r >= a.nb ? a.full : s_low[R - r];
+                // each block of the ball is this thread's alone
+                ball_group(a.b, it, pre, pc, [&](uint32_t p) {
+                    const uint64_t u = __ldcg(&a.um[p]);
+                    c += (unsigned)__popcll(u & m);
+                    if (fresh && (u & m)) __stcg(&a.um[p], u & ~m);
+                });
+            }
+            if (fresh) {
+                // the counters, a word at a time (a block at a time they are a
+                // chain of up to 64 dependent accesses: 130 us a placement)
+                for (uint32_t it = (uint32_t)me * GREEDY_NT + threadIdx.x; it < a.whole.ngroups;
+                     it += (uint32_t)G * GREEDY_NT)
+                    ball_group(a.whole, it, word, s_pw, [&](uint32_t w) {
+                        const uint16_t v = __ldcg(&a.cnt[w]);
+                        if (v != 65535u) __stcg(&a.cnt[w], (uint16_t)(v + 1));
+                    });
+            }
+            c = __reduce_add_sync(0xffffffffu, c);
+            if (lane == 0) s_sum[warp] = c;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                unsigned t = 0;
+                for (int w = 0; w < GREEDY_NT / 32; w++) t += s_sum[w];
+                if (t) atomicAdd(&acc[fresh ? 0 : me / a.team], t);
+            }
+        }
+        if (!(ok = grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
+        if (fresh) {
+            if (threadIdx.x == 0 && me == 0) a.list[placed] = a.cand[pos];
+            if (threadIdx.x == 0 && pos % G == me) sb[pos / G] = 0;      // a codeword now: its ball is covered
+            uncov -= (long long)__ldcg(&acc[0]);
+            placed++;
+            epoch++;
+            since = 0;
+        } else {
+            if (threadIdx.x == 0 && s_rank >= 0) {
+                const int i = key_pos(s_stale[me]) / G;
+                sb[i] = (int)__ldcg(&acc[s_rank]);
+                sf[i] = epoch;
+            }
+            since += s_count;
+            evals += s_count;
+        }
+        buf = next;
+        __syncthreads();
+    }
+    if (me == 0 && threadIdx.x == 0) {
+        a.st->uncov = uncov;
+        a.st->evals = evals;
+        a.st->placed = placed;
+        a.st->status = !ok && ncand > 0 ? SEQ_GUARD : status;
+        a.st->best = max(best, thr);
+    }
+}
+
+// ------------------------------------------------------------ the peel ----
+struct SeqArgs {
+    uint16_t *cnt;
+    BallGeom b;
+    long long max_steps;           // bound on the steps of one launch
+    uint32_t *list;                // the codewords in order
+    int nlist;
     uint8_t *flag;
     SeqState *st;
 };
 
 struct SeqShared {
-    unsigned long long cbest[SEQ_CL];  // greedy: each CTA's max key (plain stores, one per CTA)
     long long sum;                 // ball count / crossings over the cluster
-    int act, pos;                  // the leader's decision
+    int act;                       // the leader's decision
     uint32_t word;
-    int stop;
 };
 
-// a ball walked by the whole cluster: count (op 0: cnt == target) or add
-// sgn (op 1; returns the words that crossed between 0 and 1, signed as the
-// uncovered count changes).  All words of one ball are distinct.
-__device__ __forceinline__ long long cluster_ball(const SeqArgs &a, uint32_t base, int op, int target, int sgn,
-                                                  int rank)
+// a ball walked by the whole cluster: count (op 0: cnt == 1) or subtract (op
+// 1; returns the words that became uncovered).  All words of one ball are
+// distinct.
+__device__ __forceinline__ long long cluster_ball(const SeqArgs &a, uint32_t base, int op, int rank)
 {
     const uint64_t pc = lns_pack(base, a.b.q, a.b.n);
     long long c = 0;
     for (uint32_t it = (uint32_t)rank * SEQ_NT + threadIdx.x; it < a.b.ngroups; it += SEQ_CL * SEQ_NT) {
         ball_group(a.b, it, base, pc, [&](uint32_t w) {
             const uint32_t v = __ldcg(&a.cnt[w]);
-            if (op == 0) {
-                c += v == (uint32_t)target;
-            } else if (sgn > 0) {
-                if (v != 65535u) __stcg(&a.cnt[w], (uint16_t)(v + 1));
-                c -= v == 0;                          // newly covered
-            } else {
-                if (v != 0u) __stcg(&a.cnt[w], (uint16_t)(v - 1));
-                c += v == 1;                          // newly uncovered
-            }
+            c += v == 1u;
+            if (op && v != 0u) __stcg(&a.cnt[w], (uint16_t)(v - 1));
         });
     }
     return c;
@@ -490,139 +891,65 @@ __device__ __forceinline__ void cluster_add(long long v, SeqShared *lead)
     if ((threadIdx.x & 31) == 0 && v) atomicAdd((unsigned long long *)&lead->sum, (unsigned long long)v);
 }
 
-enum { ACT_STOP = 0, ACT_EVAL, ACT_PLACE, ACT_NEXT };
+enum { ACT_STOP = 0, ACT_EVAL, ACT_REMOVE, ACT_NEXT };
 
-// key of a candidate: larger bound first, then the lower position
-__device__ __forceinline__ unsigned long long cand_key(int32_t bound, int pos)
-{
-    return ((unsigned long long)(uint32_t)(bound + 0x40000000) << 32) | (uint32_t)(0x7fffffff - pos);
-}
-
-__global__ void __cluster_dims__(SEQ_CL, 1, 1) __launch_bounds__(SEQ_NT) k_lns_seq(SeqArgs a)
+__global__ void __cluster_dims__(SEQ_CL, 1, 1) __launch_bounds__(SEQ_NT) k_lns_peel(SeqArgs a)
 {
     __shared__ SeqShared sh;
-    __shared__ unsigned long long s_wmax[SEQ_NT / 32];
     __shared__ long long s_uncov, s_evals, s_steps;
-    __shared__ int s_epoch, s_placed, s_removed, s_i, s_since;
+    __shared__ int s_removed, s_i;
     cg::cluster_group cl = cg::this_cluster();
     const int rank = (int)cl.block_rank();
     SeqShared *lead = cl.map_shared_rank(&sh, 0);
     if (threadIdx.x == 0) {
-        for (int r = 0; r < SEQ_CL; r++) sh.cbest[r] = 0;
-        sh.sum = 0; sh.act = ACT_NEXT; sh.stop = 0; sh.pos = 0; sh.word = 0;
-        if (rank == 0) {
-            s_uncov = a.st->uncov; s_evals = 0; s_steps = 0;
-            s_epoch = 1; s_placed = 0; s_removed = 0; s_i = 0; s_since = 0;
-        }
+        sh.sum = 0; sh.act = ACT_NEXT; sh.word = 0;
+        if (rank == 0) { s_uncov = a.st->uncov; s_evals = 0; s_steps = 0; s_removed = 0; s_i = 0; }
     }
     __syncthreads();
     cl.sync();
     for (;;) {
-        // ---- the leader decides the next step
-        if (a.mode == MODE_GREEDY) {
-            unsigned long long k = 0;
-            for (int p = rank * SEQ_NT + threadIdx.x; p < a.ncand; p += SEQ_CL * SEQ_NT)
-                k = max(k, cand_key(__ldcg(&a.bound[p]), p));
-            for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
-            if ((threadIdx.x & 31) == 0) s_wmax[threadIdx.x >> 5] = k;
-            __syncthreads();
-            if (threadIdx.x == 0) {
-                unsigned long long kc = 0;
-                for (int w = 0; w < SEQ_NT / 32; w++) kc = max(kc, s_wmax[w]);
-                lead->cbest[rank] = kc;
+        // every CTA has read the previous step's decision before the leader
+        // writes the next one
+        cl.sync();
+        if (rank == 0 && threadIdx.x == 0) {
+            if (s_i >= a.nlist || ++s_steps > a.max_steps) {
+                sh.act = ACT_STOP;
+                a.st->status = s_i >= a.nlist ? SEQ_DONE : SEQ_GUARD;
+            } else {
+                sh.act = ACT_EVAL;
+                sh.word = a.list[s_i];
             }
-            cl.sync();
-            if (rank == 0 && threadIdx.x == 0) {
-                unsigned long long k0 = 0;
-                for (int r = 0; r < SEQ_CL; r++) k0 = max(k0, sh.cbest[r]);
-                const int pos = k0 ? 0x7fffffff - (int)(uint32_t)k0 : -1;
-                const int bnd = k0 ? (int)(uint32_t)(k0 >> 32) - 0x40000000 : 0;
-                int st = -1;
-                if (s_uncov <= 0) st = SEQ_COVERED;
-                else if (s_placed >= a.room) st = SEQ_TARGET;
-                else if (++s_steps > a.max_steps) st = SEQ_GUARD;
-                // below the threshold a word outside the candidates could tie
-                // or beat the best: the host refreshes the bounds (and stops
-                // when the fresh map has no positive gain)
-                else if (pos < 0 || bnd < a.thr) st = SEQ_REFRESH;
-                // so many bounds went stale that a fresh map is cheaper
-                else if (s_since >= a.eval_cap && __ldcg(&a.fresh[pos]) != s_epoch) st = SEQ_REFRESH;
-                if (st >= 0) {
-                    sh.act = ACT_STOP;
-                    a.st->status = st;
-                } else if (__ldcg(&a.fresh[pos]) == s_epoch) {
-                    // exact, and no other bound is higher: the best placement
-                    sh.act = ACT_PLACE; sh.pos = pos; sh.word = a.cand[pos];
-                } else {
-                    sh.act = ACT_EVAL; sh.pos = pos; sh.word = a.cand[pos];
-                }
-                sh.sum = 0;
-            }
-        } else {
-            // every CTA has read the previous step's decision before the
-            // leader writes the next one
-            cl.sync();
-            if (rank == 0 && threadIdx.x == 0) {
-                if (s_i >= a.nlist || ++s_steps > a.max_steps) {
-                    sh.act = ACT_STOP;
-                    a.st->status = s_i >= a.nlist ? SEQ_DONE : SEQ_GUARD;
-                } else {
-                    sh.act = a.mode == MODE_PEEL ? ACT_EVAL : ACT_PLACE;
-                    sh.pos = s_i; sh.word = a.list[s_i];
-                }
-                sh.sum = 0;
-            }
+            sh.sum = 0;
         }
         cl.sync();
-        const int act = lead->act;
-        const int pos = lead->pos;
         const uint32_t word = lead->word;
-        if (act == ACT_STOP) break;
-        // ---- the step on the whole cluster
-        if (act == ACT_EVAL) {
-            // greedy: the exact gain (count of uncovered ball words);
-            // peel: the exact loss (count of ball words covered only once)
-            cluster_add(cluster_ball(a, word, 0, a.mode == MODE_GREEDY ? 0 : 1, 0, rank), lead);
-            cl.sync();
-            if (rank == 0 && threadIdx.x == 0) {
-                s_evals++;
-                if (a.mode == MODE_GREEDY) {
-                    __stcg(&a.bound[pos], (int32_t)sh.sum);
-                    __stcg(&a.fresh[pos], s_epoch);
-                    s_since++;
-                    sh.act = ACT_NEXT;
-                } else {
-                    sh.act = sh.sum == 0 ? ACT_PLACE : ACT_NEXT;    // peel: remove if it covers nothing alone
-                    if (sh.act == ACT_NEXT) s_i++;
-                }
-                sh.sum = 0;
-            }
-            cl.sync();
-            if (a.mode == MODE_GREEDY || lead->act != ACT_PLACE) continue;
+        if (lead->act == ACT_STOP) break;
+        // the exact loss: ball words covered only once
+        cluster_add(cluster_ball(a, word, 0, rank), lead);
+        cl.sync();
+        if (rank == 0 && threadIdx.x == 0) {
+            s_evals++;
+            sh.act = sh.sum == 0 ? ACT_REMOVE : ACT_NEXT;    // remove it if it covers nothing alone
+            if (sh.act == ACT_NEXT) s_i++;
+            sh.sum = 0;
         }
-        // place (greedy, apply +1) or remove (peel, apply -1) the word's ball
-        const int sgn = a.mode == MODE_GREEDY ? 1 : a.mode == MODE_PEEL ? -1 : a.sign;
-        cluster_add(cluster_ball(a, word, 1, 0, sgn, rank), lead);
+        cl.sync();
+        if (lead->act != ACT_REMOVE) continue;
+        cluster_add(cluster_ball(a, word, 1, rank), lead);
         cl.sync();
         if (rank == 0 && threadIdx.x == 0) {
             s_uncov += sh.sum;
             sh.sum = 0;
-            if (a.mode == MODE_GREEDY) {
-                a.list[s_placed++] = word;
-                __stcg(&a.bound[pos], 0);         // a codeword now: its ball is covered
-                s_epoch++;
-                s_since = 0;
-            } else {
-                if (a.mode == MODE_PEEL) { a.flag[s_i] = 1; s_removed++; }
-                s_i++;
-            }
+            a.flag[s_i] = 1;
+            s_removed++;
+            s_i++;
         }
         cl.sync();
     }
     if (rank == 0 && threadIdx.x == 0) {
         a.st->uncov = s_uncov;
         a.st->evals = s_evals;
-        a.st->placed = s_placed;
+        a.st->placed = 0;
         a.st->removed = s_removed;
     }
     // no CTA may leave while another can still reach the leader's shared memory
@@ -803,34 +1130,21 @@ BallGeom ball_geom(const cov_lns *h)
 {
     BallGeom b;
     memset(&b, 0, sizeof b);
-    b.q = h->q; b.n = h->n;
+    b.q = h->q; b.n = h->n; b.R = h->R;
     for (int j = 0; j < h->n; j++) b.pw[j] = h->pw[j];
     b.items = h->ball; b.last = h->ball_last; b.ngroups = h->ngroups;
     return b;
 }
 
-// words in one ball of the cell
-long long ball_words(const cov_lns *h)
+// the ball on the high digits, whose words are the mask blocks
+BallGeom block_geom(const cov_lns *h)
 {
-    long long v = 0, c = 1;
-    for (int i = 0; i <= h->R; i++) {
-        v += c;
-        c = c * (h->n - i) / (i + 1) * (h->q - 1);
-    }
-    return std::max(1LL, v);
-}
-
-// one sequence launch; st in/out through h->seq
-int seq_run(cov_lns *h, SeqArgs &a, SeqState *io)
-{
-    a.cnt = h->cnt;
-    a.b = ball_geom(h);
-    a.st = h->seq;
-    CK(cudaMemcpy(h->seq, io, sizeof(SeqState), cudaMemcpyHostToDevice));
-    k_lns_seq<<<SEQ_CL, SEQ_NT>>>(a);
-    CK(cudaGetLastError());
-    CK(cudaMemcpy(io, h->seq, sizeof(SeqState), cudaMemcpyDeviceToHost));
-    return 0;
+    BallGeom b;
+    memset(&b, 0, sizeof b);
+    b.q = h->q; b.n = h->n - h->nb; b.R = h->R;
+    for (int j = 0; j < b.n; j++) b.pw[j] = h->pw[j] / h->blk;
+    b.items = h->pball; b.last = h->pball_last; b.ngroups = h->npgroups;
+    return b;
 }
 
 long long count_eq(cov_lns *h, int target)
@@ -845,34 +1159,49 @@ long long count_eq(cov_lns *h, int target)
 // room for a list of k words (and their flags) on the device
 int list_room(cov_lns *h, int k)
 {
-    if (h->list) { cudaFree(h->list); h->list = nullptr; }
-    if (h->flag) { cudaFree(h->flag); h->flag = nullptr; }
-    CK(cudaMalloc(&h->list, (size_t)std::max(k, 1) * 4));
-    CK(cudaMalloc(&h->flag, (size_t)std::max(k, 1)));
-    CK(cudaMemset(h->flag, 0, (size_t)std::max(k, 1)));
+    if (k > h->list_cap) {
+        cudaFree(h->list);
+        cudaFree(h->flag);
+        h->list = nullptr;
+        h->flag = nullptr;
+        h->list_cap = 0;
+        CK(cudaMalloc(&h->list, (size_t)k * 4));
+        CK(cudaMalloc(&h->flag, (size_t)k));
+        h->list_cap = k;
+    }
     return 0;
 }
 
-// ordered extraction into device buffers (oidx, oval) of at most cap entries
-int extract_dev(cov_lns *h, int32_t thr, int64_t cap, uint32_t *oidx, int32_t *oval, int64_t *found)
+// ordered extraction into device buffers (oidx, oval) of at most cap entries;
+// thr_dev (may be null) replaces thr.  bcount: extract_blocks(h) words.
+uint32_t extract_blocks(const cov_lns *h) { return (h->N + EXT_CHUNK - 1) / EXT_CHUNK; }
+
+int extract_launch(cov_lns *h, int32_t thr, const int *thr_dev, int64_t cap, uint32_t *bcount, uint32_t *oidx,
+                   int32_t *oval, unsigned long long *found, uint32_t *found32)
 {
-    const uint32_t chunk = 65536;
-    const uint32_t nb = (h->N + chunk - 1) / chunk;
-    int rc = lns_scratch(h, (size_t)nb * 8 + 16);
-    if (rc) return rc;
-    uint32_t *bcount = (uint32_t *)h->scratch, *boff = bcount + nb;
-    k_lns_count_ge<<<nb, LNS_NT>>>(h->map, h->N, thr, chunk, bcount);
-    CK(cudaGetLastError());
-    std::vector<uint32_t> c(nb), o(nb);
-    CK(cudaMemcpy(c.data(), bcount, (size_t)nb * 4, cudaMemcpyDeviceToHost));
-    unsigned long long tot = 0;
-    for (uint32_t b = 0; b < nb; b++) { o[b] = (uint32_t)std::min<unsigned long long>(tot, 0xffffffffull); tot += c[b]; }
-    *found = (int64_t)tot;
-    if (cap == 0 || tot == 0) return COV_OK;
-    CK(cudaMemcpy(boff, o.data(), (size_t)nb * 4, cudaMemcpyHostToDevice));
-    k_lns_emit_ge<<<nb, LNS_NT>>>(h->map, h->N, thr, chunk, boff, (uint32_t)cap, oidx, oval);
+    const uint32_t nb = extract_blocks(h);
+    k_lns_count_ge<<<nb, LNS_NT>>>(h->map, h->N, thr, thr_dev, bcount);
+    k_lns_scan<<<1, 1024>>>(bcount, nb, found, found32);
+    if (cap > 0)
+        k_lns_emit_ge<<<nb, LNS_NT>>>(h->map, h->N, thr, thr_dev, bcount,
+                                      (uint32_t)std::min<int64_t>(cap, 0xffffffffll), oidx, oval);
     CK(cudaGetLastError());
     return COV_OK;
+}
+
+// the greedy kernel's launch shape on the current device
+int greedy_shape(cov_lns *h, GreedyArgs &a, int *G, size_t *smem)
+{
+    *G = std::min(std::max(1, cov_sm_count()), GREEDY_MAXG);
+    a.own = (CAND_CAP + *G - 1) / *G;
+    *smem = (size_t)a.own * 8;
+    // a team's threads take about two groups each
+    a.team = (int)std::min<uint32_t>((uint32_t)*G, std::max(1u, (h->npgroups + 2 * GREEDY_NT - 1) / (2 * GREEDY_NT)));
+    a.nteam = *G / a.team;
+    if (*smem > 48 * 1024) CK(cudaFuncSetAttribute(k_lns_greedy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)*smem));
+    int per_sm = 0;
+    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_lns_greedy, GREEDY_NT, *smem));
+    return per_sm >= 1 ? COV_OK : COV_ENODEV;
 }
 
 }  // namespace
@@ -895,6 +1224,20 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
     uint32_t gcum[COV_MAXN + 2];
     std::vector<uint64_t> items = bt_items_h(q, n, R, 0, gcum, last);
     h->ngroups = gcum[std::min(R, n)];
+    // mask blocks: the ball groups on the high digits, and for each word of a
+    // block the words of it within 0..nb
+    while (h->nb < n && (long long)h->blk * q <= 64) { h->nb++; h->blk *= (uint32_t)q; }
+    std::vector<uint8_t> plast;
+    uint32_t pcum[COV_MAXN + 2];
+    std::vector<uint64_t> pitems = bt_items_h(q, n - h->nb, R, 0, pcum, plast);
+    h->npgroups = pcum[std::min(R, n - h->nb)];
+    std::vector<uint64_t> low((size_t)h->blk * (h->nb + 1), 0);
+    for (uint32_t x = 0; x < h->blk; x++)
+        for (uint32_t y = 0; y < h->blk; y++) {
+            int d = 0;
+            for (uint32_t u = x, v = y, k = 0; k < (uint32_t)h->nb; k++, u /= q, v /= q) d += u % q != v % q;
+            for (int sg = d; sg <= h->nb; sg++) low[(size_t)x * (h->nb + 1) + sg] |= 1ull << y;
+        }
     bool ok = cudaMalloc(&h->cnt, (size_t)N * 2) == cudaSuccess &&
               cudaMalloc(&h->map, (size_t)N * 4) == cudaSuccess &&
               cudaMalloc(&h->ball, items.size() * 8) == cudaSuccess &&
@@ -902,7 +1245,13 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
               cudaMalloc(&h->d_red, 64 * 8) == cudaSuccess &&
               cudaMalloc(&h->cand, (size_t)CAND_CAP * 4) == cudaSuccess &&
               cudaMalloc(&h->bound, (size_t)CAND_CAP * 4) == cudaSuccess &&
-              cudaMalloc(&h->fresh, (size_t)CAND_CAP * 4) == cudaSuccess &&
+              cudaMalloc(&h->um, (size_t)(N / h->blk) * 8) == cudaSuccess &&
+              cudaMalloc(&h->pball, pitems.size() * 8) == cudaSuccess &&
+              cudaMalloc(&h->pball_last, plast.size()) == cudaSuccess &&
+              cudaMalloc(&h->lowball, low.size() * 8) == cudaSuccess &&
+              cudaMalloc(&h->nom, sizeof(unsigned long long) * 2 * GREEDY_MAXG) == cudaSuccess &&
+              cudaMalloc(&h->acc, 4 * (3 * (GREEDY_MAXG + 1) + 1)) == cudaSuccess &&
+              cudaMalloc(&h->info, sizeof(RefreshInfo)) == cudaSuccess &&
               cudaMalloc(&h->seq, sizeof(SeqState)) == cudaSuccess;
     for (int d = 0; ok && d <= R; d++) ok = cudaMalloc(&h->layer[d], (size_t)N * 4) == cudaSuccess;
     if (!ok) {
@@ -912,6 +1261,9 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
     }
     if (cudaMemcpy(h->ball, items.data(), items.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(h->ball_last, last.data(), last.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(h->pball, pitems.data(), pitems.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(h->pball_last, plast.data(), plast.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMemcpy(h->lowball, low.data(), low.size() * 8, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemset(h->cnt, 0, (size_t)N * 2) != cudaSuccess) {
         cov_lns_destroy(h);
         return -100;
@@ -925,8 +1277,9 @@ int cov_lns_destroy(cov_lns *h)
     if (!h) return COV_OK;
     cudaDeviceSynchronize();
     cudaFree(h->cnt); cudaFree(h->map); cudaFree(h->ball); cudaFree(h->ball_last); cudaFree(h->d_red);
-    cudaFree(h->cand); cudaFree(h->bound); cudaFree(h->fresh); cudaFree(h->list); cudaFree(h->flag);
-    cudaFree(h->seq);
+    cudaFree(h->cand); cudaFree(h->bound); cudaFree(h->list); cudaFree(h->flag); cudaFree(h->seq);
+    cudaFree(h->um); cudaFree(h->pball); cudaFree(h->pball_last); cudaFree(h->lowball); cudaFree(h->nom);
+    cudaFree(h->acc); cudaFree(h->info);
     for (int d = 0; d <= LNS_MAXR; d++) cudaFree(h->layer[d]);
     cudaFree(h->scratch);
     delete h;
@@ -979,7 +1332,7 @@ int cov_lns_map_hist(cov_lns *h, int32_t nbins, int32_t vmax, int64_t *hist)
     if (rc) return rc;
     unsigned long long *d_h = (unsigned long long *)h->scratch;
     CK(cudaMemset(d_h, 0, (size_t)nbins * 8));
-    k_lns_hist<<<grid_of(h->N), LNS_NT, (size_t)nbins * 4>>>(h->map, h->N, nbins, vmax, d_h);
+    k_lns_hist<<<grid_of(h->N), LNS_NT, (size_t)nbins * 4>>>(h->map, h->N, nbins, vmax, nullptr, d_h, nullptr);
     CK(cudaGetLastError());
     CK(cudaMemcpy(hist, d_h, (size_t)nbins * 8, cudaMemcpyDeviceToHost));
     return COV_OK;
@@ -988,22 +1341,26 @@ int cov_lns_map_hist(cov_lns *h, int32_t nbins, int32_t vmax, int64_t *hist)
 int cov_lns_map_extract(cov_lns *h, int32_t thr, int64_t cap, uint32_t *idx, int32_t *val, int64_t *found)
 {
     if (!h || cap < 0 || (cap > 0 && (!idx || !val)) || !found) return COV_EINVAL;
-    uint32_t *d_i = nullptr;
-    int32_t *d_v = nullptr;
-    if (cap > 0) {
-        CK(cudaMalloc(&d_i, (size_t)cap * 4));
-        if (cudaMalloc(&d_v, (size_t)cap * 4) != cudaSuccess) { cudaGetLastError(); cudaFree(d_i); return COV_ENOMEM; }
+    const uint32_t nb = extract_blocks(h);
+    // at most N entries are written
+    const int64_t room = std::min<int64_t>(cap, (int64_t)h->N);
+    const size_t cb = ((size_t)nb * 4 + 7) / 8 * 8;
+    int rc = lns_scratch(h, cb + 8 + (size_t)room * 8);
+    if (rc) return rc;
+    uint32_t *bcount = (uint32_t *)h->scratch;
+    unsigned long long *d_f = (unsigned long long *)((char *)h->scratch + cb), tot = 0;
+    uint32_t *d_i = (uint32_t *)(d_f + 1);
+    int32_t *d_v = (int32_t *)(d_i + room);
+    rc = extract_launch(h, thr, nullptr, room, bcount, d_i, d_v, d_f, nullptr);
+    if (rc) return rc;
+    CK(cudaMemcpy(&tot, d_f, 8, cudaMemcpyDeviceToHost));
+    *found = (int64_t)tot;
+    const size_t k = (size_t)std::min<int64_t>(*found, room);
+    if (k) {
+        CK(cudaMemcpy(idx, d_i, k * 4, cudaMemcpyDeviceToHost));
+        CK(cudaMemcpy(val, d_v, k * 4, cudaMemcpyDeviceToHost));
     }
-    int rc = extract_dev(h, thr, cap, d_i, d_v, found);
-    if (!rc && cap > 0 && *found > 0) {
-        const size_t k = (size_t)std::min<int64_t>(*found, cap);
-        if (cudaMemcpy(idx, d_i, k * 4, cudaMemcpyDeviceToHost) != cudaSuccess ||
-            cudaMemcpy(val, d_v, k * 4, cudaMemcpyDeviceToHost) != cudaSuccess)
-            rc = -100;
-    }
-    cudaFree(d_i);
-    cudaFree(d_v);
-    return rc;
+    return COV_OK;
 }
 
 int cov_lns_map_read(cov_lns *h, const uint32_t *idx, int32_t k, int32_t *out)
@@ -1026,23 +1383,23 @@ int cov_lns_apply(cov_lns *h, const uint32_t *idx, int32_t k, int32_t sign, int6
 {
     if (!h || k < 0 || (k > 0 && !idx) || (sign != 1 && sign != -1) || !uncovered) return COV_EINVAL;
     for (int i = 0; i < k; i++) if (idx[i] >= h->N) return COV_EINVAL;
-    SeqState st;
-    memset(&st, 0, sizeof st);
-    st.uncov = count_eq(h, 0);
-    if (st.uncov < 0) return -100;
+    // the uncovered words before, and their change, in one counter
+    CK(cudaMemsetAsync(h->d_red, 0, 8));
+    k_lns_zero<<<grid_of(h->N), LNS_NT>>>(h->cnt, h->N, 0, h->d_red);
+    CK(cudaGetLastError());
     if (k > 0) {
         int rc = list_room(h, k);
         if (rc) return rc;
         CK(cudaMemcpy(h->list, idx, (size_t)k * 4, cudaMemcpyHostToDevice));
-        SeqArgs a;
-        memset(&a, 0, sizeof a);
-        a.mode = MODE_APPLY; a.list = h->list; a.nlist = k; a.sign = sign; a.flag = h->flag;
-        a.max_steps = (long long)k + 1;
-        rc = seq_run(h, a, &st);
-        if (rc) return rc;
-        if (st.status != SEQ_DONE) return COV_ETIMEOUT;
+        const uint32_t per = (h->ngroups + LNS_NT - 1) / LNS_NT;
+        const int grid = (int)std::min<unsigned long long>((unsigned long long)k * per,
+                                                           (unsigned long long)std::max(1, cov_sm_count()) * 8);
+        k_lns_apply<<<grid, LNS_NT>>>(h->cnt, ball_geom(h), h->list, k, sign, per, h->d_red);
+        CK(cudaGetLastError());
     }
-    *uncovered = st.uncov;
+    unsigned long long u = 0;
+    CK(cudaMemcpy(&u, h->d_red, 8, cudaMemcpyDeviceToHost));
+    *uncovered = (int64_t)u;
     return COV_OK;
 }
 
@@ -1080,35 +1437,22 @@ int cov_lns_peel(cov_lns *h, const uint32_t *idx, int32_t k, uint8_t *removed, i
         int rc = list_room(h, k);
         if (rc) return rc;
         CK(cudaMemcpy(h->list, idx, (size_t)k * 4, cudaMemcpyHostToDevice));
+        CK(cudaMemset(h->flag, 0, (size_t)k));
         SeqArgs a;
         memset(&a, 0, sizeof a);
-        a.mode = MODE_PEEL; a.list = h->list; a.nlist = k; a.flag = h->flag;
+        a.cnt = h->cnt; a.b = ball_geom(h); a.st = h->seq;
+        a.list = h->list; a.nlist = k; a.flag = h->flag;
         a.max_steps = 2LL * k + 2;
-        rc = seq_run(h, a, &st);
-        if (rc) return rc;
+        CK(cudaMemcpy(h->seq, &st, sizeof st, cudaMemcpyHostToDevice));
+        k_lns_peel<<<SEQ_CL, SEQ_NT>>>(a);
+        CK(cudaGetLastError());
+        CK(cudaMemcpy(&st, h->seq, sizeof st, cudaMemcpyDeviceToHost));
         if (st.status != SEQ_DONE) return COV_ETIMEOUT;
         CK(cudaMemcpy(removed, h->flag, (size_t)k, cudaMemcpyDeviceToHost));
         *nremoved = st.removed;
     }
     *uncovered = st.uncov;
     return COV_OK;
-}
-
-// extraction threshold that keeps {map >= thr} within cap (from a histogram)
-static int extract_threshold(cov_lns *h, int top, long long cap, int *thr_out)
-{
-    if (top <= 1) { *thr_out = 1; return 0; }
-    const int nb = 1024;
-    int64_t hist[1024];
-    int rc = cov_lns_map_hist(h, nb, top, hist);
-    if (rc) return rc;
-    long long above = 0;
-    int b = nb;                                      // smallest bin whose tail fits
-    while (b > 0 && above + hist[b - 1] <= cap) { above += hist[b - 1]; b--; }
-    // bin b holds the values v with (v-1)*nb/top == b: the first such v
-    const int thr = b >= nb ? top : (int)(((long long)b * top + nb - 1) / nb) + 1;
-    *thr_out = std::max(1, std::min(thr, top));
-    return 0;
 }
 
 int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed, int32_t *nplaced,
@@ -1118,56 +1462,79 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
     cand_cap = std::max<int64_t>(1, std::min<int64_t>(cand_cap > 0 ? cand_cap : CAND_CAP, CAND_CAP));
     int rc = list_room(h, room);
     if (rc) return rc;
+    GreedyArgs a;
+    memset(&a, 0, sizeof a);
+    int G = 1;
+    size_t smem = 0;
+    rc = greedy_shape(h, a, &G, &smem);
+    if (rc) return rc;
+    const uint32_t xb = extract_blocks(h), nblk = h->N / h->blk;
+    rc = lns_scratch(h, THR_BINS * 8 + (size_t)xb * 4);
+    if (rc) return rc;
+    unsigned long long *d_hist = (unsigned long long *)h->scratch;
+    uint32_t *bcount = (uint32_t *)(d_hist + THR_BINS);
     SeqState st;
     memset(&st, 0, sizeof st);
     st.uncov = count_eq(h, 0);
     if (st.uncov < 0) return -100;
-    int total = 0;
+    CK(cudaMemcpy(h->seq, &st, sizeof st, cudaMemcpyHostToDevice));
+    if (room > 0 && st.uncov > 0) {
+        k_lns_masks<<<(nblk + LNS_NT - 1) / LNS_NT, LNS_NT>>>(h->cnt, nblk, (int)h->blk, h->um);
+        CK(cudaGetLastError());
+    }
+    a.cnt = h->cnt; a.um = h->um; a.b = block_geom(h); a.whole = ball_geom(h); a.lowball = h->lowball;
+    a.nb = h->nb; a.blk = (int)h->blk;
+    a.full = h->blk == 64 ? ~0ull : (1ull << h->blk) - 1;
+    a.cand = h->cand; a.bound = h->bound; a.info = h->info; a.cand_cap = (uint32_t)cand_cap;
+    a.nom = h->nom; a.acc = h->acc; a.bar = h->acc + 3 * (GREEDY_MAXG + 1);
+    a.wait_ns = 2000000000ull;
+    a.st = h->seq;
+    // exact counts for one placement past which a map is the better buy.
+    // Fills with limits of 64, 256 and 1000: 6^9 116, 114, 151 ms; 7^9 518,
+    // 444, 475; 4^11 45, 48, 70.
+    a.eval_cap = (int)std::max<long long>(64, std::min<long long>(1024, (long long)h->N / 131072));
+    int total = 0, vmax = 0;
     long long refreshes = 0, evals = 0;
     // every refresh that finds a positive gain places at least one word (the
     // first placement of a launch needs no exact count: all bounds are fresh)
     for (int guard = 0; total < room && st.uncov > 0 && guard <= 2 * room + 2; guard++) {
         // bounds: the exact gain map, extracted above a threshold that keeps
-        // at most cand_cap candidates
-        rc = cov_lns_map(h, 0);
+        // at most cand_cap candidates.  A word outside the candidates had a
+        // gain below the threshold at the refresh (or, when even the map's
+        // maximum has more than cand_cap words, the same gain and a higher
+        // position): a candidate is placed only while its exact gain is at
+        // least the threshold, so it is always a best placement.
+        rc = lns_transform(h, h->cnt, 0, h->map, nullptr);
         if (rc) return rc;
         refreshes++;
-        int32_t top = 0;
-        rc = cov_lns_map_max(h, &top);
+        CK(cudaMemsetAsync(h->info, 0x80, sizeof(RefreshInfo)));         // top: a negative number
+        CK(cudaMemsetAsync(d_hist, 0, THR_BINS * 8));
+        const int *vmax_dev = nullptr;
+        if (vmax <= 0) {
+            // the first map of the call: its maximum first; later ones are
+            // bounded by the last launch's best bound (gains only fall)
+            k_lns_max<<<grid_of(h->N), LNS_NT>>>(h->map, h->N, &h->info->top);
+            vmax_dev = &h->info->thr;
+            CK(cudaMemcpyAsync(&h->info->thr, &h->info->top, 4, cudaMemcpyDeviceToDevice));
+        }
+        k_lns_hist<<<grid_of(h->N), LNS_NT, THR_BINS * 4>>>(h->map, h->N, THR_BINS, vmax, vmax_dev, d_hist,
+                                                            &h->info->top);
+        k_lns_threshold<<<1, 1>>>(d_hist, vmax, vmax_dev, (long long)cand_cap, h->info);
+        CK(cudaGetLastError());
+        rc = extract_launch(h, 1, &h->info->thr, cand_cap, bcount, h->cand, h->bound, nullptr, &h->info->found);
         if (rc) return rc;
-        if (top <= 0) break;
-        int thr = 1;
-        rc = extract_threshold(h, top, cand_cap, &thr);
-        if (rc) return rc;
-        int64_t found = 0;
-        rc = extract_dev(h, thr, cand_cap, h->cand, h->bound, &found);
-        if (rc) return rc;
-        const int ncand = (int)std::min<int64_t>(found, cand_cap);
-        if (ncand == 0) break;
-        // every bound is exact now (epoch 1 of the launch)
-        std::vector<int32_t> ones((size_t)ncand, 1);
-        CK(cudaMemcpy(h->fresh, ones.data(), (size_t)ncand * 4, cudaMemcpyHostToDevice));
-        SeqArgs a;
-        memset(&a, 0, sizeof a);
-        a.mode = MODE_GREEDY;
-        a.cand = h->cand; a.bound = h->bound; a.fresh = h->fresh; a.ncand = ncand;
-        // a word outside the candidates had a gain below thr at the refresh
-        // (or, when even the map's maximum has more than cand_cap words, the
-        // same gain and a higher position): a candidate is placed only while
-        // its exact gain is at least thr, so it is always a best placement
-        a.thr = thr;
+        CK(cudaMemsetAsync(h->acc, 0, 4 * (3 * (GREEDY_MAXG + 1) + 1)));
         a.room = room - total;
         a.list = h->list + total;
-        // a map costs about as much as N / (2 |ball|) exact counts: past
-        // that many counts for one placement, refresh instead
-        a.eval_cap = (int)std::max<long long>(8, std::min<long long>(4096, (long long)h->N / (2LL * ball_words(h))));
-        a.max_steps = 64LL * (room - total) + 4LL * ncand + 64;
-        rc = seq_run(h, a, &st);
-        if (rc) return rc;
+        a.max_steps = 64LL * (room - total) + 4LL * cand_cap + 64;
+        void *args[] = {&a};
+        CK(cudaLaunchCooperativeKernel((const void *)k_lns_greedy, dim3((unsigned)G), dim3(GREEDY_NT), args, smem, 0));
+        CK(cudaMemcpy(&st, h->seq, sizeof st, cudaMemcpyDeviceToHost));
         total += st.placed;
         evals += st.evals;
+        vmax = st.best;
         if (st.status == SEQ_GUARD) return COV_ETIMEOUT;
-        if (st.status != SEQ_REFRESH) break;
+        if (st.status != SEQ_REFRESH || st.placed == 0) break;
     }
     if (total > 0) CK(cudaMemcpy(placed, h->list, (size_t)total * 4, cudaMemcpyDeviceToHost));
     *nplaced = total;
@@ -1182,7 +1549,7 @@ int cov_lns_uncovered(cov_lns *h, int64_t cap, uint32_t *idx, int64_t *found)
     // the indicator of cnt == 0 into the map, then its ordered extraction
     k_lns_indicator<<<grid_of(h->N), LNS_NT>>>(h->cnt, 0, nullptr, h->N, h->map, nullptr);
     CK(cudaGetLastError());
-    std::vector<int32_t> val((size_t)std::max<int64_t>(cap, 1));
+    std::vector<int32_t> val((size_t)std::max<int64_t>(std::min<int64_t>(cap, h->N), 1));
     return cov_lns_map_extract(h, 1, cap, idx, val.data(), found);
 }
 
