@@ -5,15 +5,12 @@
 //  * Maps.  gain(x) = #{y : d(x,y) <= R, cnt[y] == 0} (the words a codeword
 //    at x would newly cover) and loss(x) = the same with cnt[y] == 1 (the
 //    words only a codeword at x covers) are computed for every x at once as
-//    layered counts: L_d[x] = #{marked y : d(x,y) = d}, d = 0..R, built one
-//    axis at a time -- along a line of q words with layer sums S_d, a word's
-//    L_d gains S_{d-1} - L_{d-1}[x] (the marked words that now differ from it
-//    in this coordinate too) -- and summed over d at the end.  The axes are
-//    not swept one by one through HBM: the low axes are done on contiguous
-//    tiles of q^k words in shared memory, the remaining ones on strips of
-//    q^g rows x W words, all R+1 int32 layers of a tile at once, so a whole
-//    transform reads and writes the layers in a few sweeps instead of n.
-//    The same layers with the code itself marked give cnt.
+//    layered counts over 64-bit masks of the marked words, one axis at a
+//    time.  The axes are not swept one by one through HBM: the low axes are
+//    done on contiguous tiles of q^k words in shared memory, the remaining
+//    ones on strips of q^g rows x W words, all int32 layers of a tile at once,
+//    and all sweeps but the last go part by part through L2.  The counts of a
+//    code come from the verifier's tiles.
 //  * Sequences.  The lazy greedy placement (bounds from a gain map, the best
 //    bounds re-counted exactly until the best is current, then placed) is one
 //    cooperative kernel over the whole GPU with no host round trip between
@@ -37,16 +34,18 @@
 #include <cooperative_groups.h>
 #include "cov_common.cuh"
 #include "cov_tiles.cuh"
+#include "cov_map.cuh"
 #include "../../include/covgpu.h"
 
 namespace cg = cooperative_groups;
 
-#define LNS_MAXR 8
 #define LNS_NT 256
 #define LNS_HIST_MAX 8192   // bins of cov_lns_map_hist (one shared-memory counter each)
-#define MAP_NT 512
 #define MAP_SMEM_MAX (200 * 1024)   // shared memory of one map tile (bytes)
-#define MAP_W_MIN 8                 // narrowest strip: 32 bytes of a layer per row
+#define MAP_SMEM_LOW (84 * 1024)    // of a low tile: two CTAs an SM at least
+#define MAP_SMEM_HIGH (112 * 1024)  // of a strip: two
+#define MAP_W_MIN 8                 // narrowest strip
+#define MAP_L2_BYTES (80 << 20)     // layers of the parts that are in flight between two sweeps
 #define SEQ_NT 512
 #define SEQ_CL 8                    // CTAs of the sequence cluster
 #define CAND_CAP (1 << 17)          // candidate bounds kept on the device per refresh
@@ -81,7 +80,11 @@ struct cov_lns {
     uint32_t N;
     uint32_t pw[COV_MAXN];          // q^(n-1-j)
     uint16_t *cnt = nullptr;        // coverage multiplicity (saturated)
-    int32_t *layer[LNS_MAXR + 1] = {};
+    int kl = 0, ng = 0, gs[COV_MAXN] = {}, slots[COV_MAXN] = {};   // low axes, strip groups: their axes and layers (map_plan)
+    uint32_t parts = 1, at_once = 1;
+    size_t scratch_ints = 0, whole_ints = 0;
+    int32_t *map_scratch = nullptr;      // the layers between the sweeps of a part (two of them from three groups on)
+    int32_t *map_whole = nullptr;        // the layers that reach the last sweep
     int32_t *map = nullptr;         // last map (gain or loss)
     uint64_t *ball = nullptr;       // whole-ball groups (cov_tiles.cuh, no high digits)
     uint8_t *ball_last = nullptr;
@@ -109,189 +112,39 @@ struct cov_lns {
 
 namespace {
 
-struct LayerPtrs { int32_t *a[LNS_MAXR + 1]; };
-
-struct MapGeom {
-    int q, n;
-    uint32_t N;
-    uint32_t pk[COV_MAXN + 1];      // q^k: the stride of axis k (the digit n-1-k)
-};
-
-// ----------------------------------------------------------- the maps -----
-// One axis over `nfib` lines of q elements at element stride st, held in
-// shared memory as R1 layers of E elements each.  Each thread owns whole
-// lines, so the update needs no synchronisation inside a pass.  With the
-// alphabet size Q known at compile time a line's Q x R1 counts are read
-// once into registers (R1 loads and R1 - 1 stores per element, no division
-// by st); Q = 0 is the form for any q.
-template <int R1, int Q>
-__device__ __forceinline__ void map_axis(int32_t *Ls, uint32_t E, int q, uint32_t nfib, uint32_t st)
-{
-    if constexpr (Q > 0) {
-        // f / st by a float reciprocal: f < 2^24, so the estimate is off by
-        // at most one and one correction makes it exact
-        const float rinv = 1.0f / (float)st;
-        for (uint32_t f = threadIdx.x; f < nfib; f += blockDim.x) {
-            int o = (int)((float)f * rinv);
-            int i = (int)f - o * (int)st;
-            if (i < 0) { o--; i += (int)st; } else if (i >= (int)st) { o++; i -= (int)st; }
-            const uint32_t e0 = (uint32_t)o * st * (uint32_t)Q + (uint32_t)i;
-            int32_t v[Q][R1];
-#pragma unroll
-            for (int a = 0; a < Q; a++)
-#pragma unroll
-                for (int d = 0; d < R1; d++) v[a][d] = Ls[d * E + e0 + (uint32_t)a * st];
-            int32_t S[R1 > 1 ? R1 - 1 : 1];
-#pragma unroll
-            for (int d = 0; d < R1 - 1; d++) {
-                S[d] = 0;
-#pragma unroll
-                for (int a = 0; a < Q; a++) S[d] += v[a][d];
-            }
-#pragma unroll
-            for (int a = 0; a < Q; a++)
-#pragma unroll
-                for (int d = 1; d < R1; d++) Ls[d * E + e0 + (uint32_t)a * st] = v[a][d] + S[d - 1] - v[a][d - 1];
-        }
-        return;
-    }
-    for (uint32_t f = threadIdx.x; f < nfib; f += blockDim.x) {
-        const uint32_t o = f / st, i = f - o * st;
-        const uint32_t e0 = o * st * (uint32_t)q + i;
-        int32_t S[R1 > 1 ? R1 - 1 : 1];
-#pragma unroll
-        for (int d = 0; d < R1 - 1; d++) S[d] = 0;
-        for (int a = 0; a < q; a++) {
-            const uint32_t e = e0 + (uint32_t)a * st;
-#pragma unroll
-            for (int d = 0; d < R1 - 1; d++) S[d] += Ls[d * E + e];
-        }
-        for (int a = 0; a < q; a++) {
-            const uint32_t e = e0 + (uint32_t)a * st;
-            int32_t below = Ls[e];                    // old L_{d-1}[x], starting at L_0
-#pragma unroll
-            for (int d = 1; d < R1; d++) {
-                const int32_t old = Ls[d * E + e];
-                Ls[d * E + e] = old + S[d - 1] - below;
-                below = old;
-            }
-        }
-    }
-}
-
-template <int R1>
-__device__ __forceinline__ void map_out(int32_t *Ls, uint32_t E, uint32_t e, uint32_t x, int fin, LayerPtrs L,
-                                        int32_t *out, uint16_t *cnt16)
-{
-    if (fin) {
-        int32_t s = 0;
-#pragma unroll
-        for (int d = 0; d < R1; d++) s += Ls[d * E + e];
-        if (out) out[x] = s;
-        else cnt16[x] = (uint16_t)min(s, 65535);
-    } else {
-#pragma unroll
-        for (int d = 0; d < R1; d++) L.a[d][x] = Ls[d * E + e];
-    }
-}
-
-// Axes 0..k-1 on contiguous tiles of T = q^k words.  Layer 0 starts as
-// [cnt == target] (cnt given) or as the layer-0 array (the code's word
-// counts); the higher layers start at 0.  With fin (k == n) the map is
-// written, else the layers.
-template <int R1, int Q>
-__global__ void __launch_bounds__(MAP_NT) k_map_low(MapGeom g, int k, const uint16_t *__restrict__ cnt, int target,
-                                                    LayerPtrs L, int fin, int32_t *out, uint16_t *cnt16)
-{
-    extern __shared__ __align__(16) int32_t Ls[];
-    uint32_t T = 1;
-    for (int j = 0; j < k; j++) T *= (uint32_t)g.q;
-    const uint32_t ntile = g.N / T;
-    for (uint32_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
-        const uint32_t x0 = tile * T;
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) {
-            const uint32_t x = x0 + e;
-            Ls[e] = cnt ? (int32_t)(__ldcg(&cnt[x]) == target) : L.a[0][x];
-#pragma unroll
-            for (int d = 1; d < R1; d++) Ls[d * T + e] = 0;
-        }
-        __syncthreads();
-        uint32_t st = 1;
-        for (int j = 0; j < k; j++, st *= (uint32_t)g.q) {
-            map_axis<R1, Q>(Ls, T, g.q, T / (uint32_t)g.q, st);
-            __syncthreads();
-        }
-        for (uint32_t e = threadIdx.x; e < T; e += blockDim.x) map_out<R1>(Ls, T, e, x0 + e, fin, L, out, cnt16);
-    }
-}
-
-// Axes j0..j0+gsz-1 on strips: q^gsz rows (row r at stride s = q^j0) of
-// W = 2^lw consecutive words, element (r, c) at base + r*s + c.
-template <int R1, int Q>
-__global__ void __launch_bounds__(MAP_NT) k_map_high(MapGeom g, int j0, int gsz, int lw, LayerPtrs L, int fin,
-                                                     int32_t *out, uint16_t *cnt16)
-{
-    extern __shared__ __align__(16) int32_t Ls[];
-    const uint32_t W = 1u << lw;
-    uint32_t s = 1, rows = 1;
-    for (int j = 0; j < j0; j++) s *= (uint32_t)g.q;
-    for (int j = 0; j < gsz; j++) rows *= (uint32_t)g.q;
-    const uint32_t E = rows << lw;
-    const uint32_t span = rows * s, outer = g.N / span;
-    const uint32_t nstrip = (s + W - 1) >> lw;
-    const unsigned long long ntiles = (unsigned long long)outer * nstrip;
-    for (unsigned long long tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t o = (uint32_t)(tile / nstrip);
-        const uint32_t c0 = (uint32_t)(tile - (unsigned long long)o * nstrip) << lw;
-        const uint32_t w = min(W, s - c0);
-        const uint32_t base = o * span + c0;
-        __syncthreads();
-        for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) {
-            const uint32_t r = e >> lw, c = e & (W - 1);
-            const uint32_t x = base + r * s + c;
-#pragma unroll
-            for (int d = 0; d < R1; d++) Ls[d * E + e] = c < w ? L.a[d][x] : 0;
-        }
-        __syncthreads();
-        uint32_t st = W;
-        for (int jj = 0; jj < gsz; jj++, st *= (uint32_t)g.q) {
-            map_axis<R1, Q>(Ls, E, g.q, E / (uint32_t)g.q, st);
-            __syncthreads();
-        }
-        for (uint32_t e = threadIdx.x; e < E; e += blockDim.x) {
-            const uint32_t r = e >> lw, c = e & (W - 1);
-            if (c < w) map_out<R1>(Ls, E, e, base + r * s + c, fin, L, out, cnt16);
-        }
-    }
-}
-
-__global__ void k_lns_zero_layer(int32_t *A0, uint32_t N)
-{
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x) A0[x] = 0;
-}
-
 __global__ void k_lns_scatter(int32_t *A0, const uint32_t *idx, int m)
 {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < m) atomicAdd(&A0[idx[i]], 1);
 }
 
-// R = 0: the map is the indicator itself
-__global__ void k_lns_indicator(const uint16_t *cnt, int target, const int32_t *A0, uint32_t N, int32_t *out,
-                                uint16_t *cnt16)
+// word counts to saturated counters (the counts at R = 0)
+__global__ void k_lns_narrow(const int32_t *A0, uint32_t N, uint16_t *cnt)
 {
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x) {
-        const int32_t v = cnt ? (int32_t)(cnt[x] == target) : A0[x];
-        if (out) out[x] = v;
-        else cnt16[x] = (uint16_t)min(v, 65535);
-    }
+    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x)
+        cnt[x] = (uint16_t)min(A0[x], 65535);
+}
+
+// the words whose count is target
+__global__ void k_lns_indicator(const uint16_t *cnt, int target, uint32_t N, int32_t *out)
+{
+    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x)
+        out[x] = (int32_t)(cnt[x] == target);
 }
 
 __global__ void k_lns_max(const int32_t *A, uint32_t N, int *out)
 {
     int m = INT_MIN;
-    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x) m = max(m, A[x]);
+    const uint32_t step = gridDim.x * blockDim.x;
+    unsigned long long x = blockIdx.x * blockDim.x + threadIdx.x;
+    for (; x + 7ull * step < N; x += 8ull * step) {
+        int v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = __ldcg(&A[x + (unsigned long long)u * step]);
+#pragma unroll
+        for (int u = 0; u < 8; u++) m = max(m, v[u]);
+    }
+    for (; x < N; x += step) m = max(m, A[x]);
     for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
     if ((threadIdx.x & 31) == 0) atomicMax(out, m);
 }
@@ -300,30 +153,25 @@ __global__ void k_lns_max(const int32_t *A, uint32_t N, int *out)
 // Counted per block in shared memory (the lanes of a warp that share a bin
 // add once), then one global add per bin and block: the values of a gain map
 // crowd into few bins, where per-element global atomics serialise.  Eight
-// loads of a thread in flight (one at a time took 65 us at 6^9, bound by
-// latency).  vmax_dev (may be null) replaces vmax; top (may be null) receives
-// the maximum.
+// loads of a thread are in flight.
 __global__ void __launch_bounds__(LNS_NT) k_lns_hist(const int32_t *A, uint32_t N, int nbins, int vmax,
-                                                     const int *vmax_dev, unsigned long long *hist, int *top)
+                                                     unsigned long long *hist)
 {
     extern __shared__ uint32_t lh[];
     for (int b = threadIdx.x; b < nbins; b += blockDim.x) lh[b] = 0;
-    if (vmax_dev) vmax = max(1, __ldcg(vmax_dev));
     __syncthreads();
     // (v-1)*nbins in 32 bits when it cannot overflow
     const bool narrow = (unsigned long long)vmax * (unsigned long long)nbins < (1ull << 32);
-    int m = INT_MIN;
     for (unsigned long long x0 = (unsigned long long)blockIdx.x * (8 * LNS_NT); x0 < N;
          x0 += (unsigned long long)gridDim.x * (8 * LNS_NT)) {
         int v[8];
 #pragma unroll
         for (int u = 0; u < 8; u++) {
             const unsigned long long x = x0 + (unsigned)u * LNS_NT + threadIdx.x;
-            v[u] = x < N ? __ldcg(&A[x]) : INT_MIN;
+            v[u] = x < N ? __ldcg(&A[x]) : 0;
         }
 #pragma unroll
         for (int u = 0; u < 8; u++) {
-            m = max(m, v[u]);
             int b = -1;
             if (v[u] >= 1) {
                 const uint32_t t = (uint32_t)(min(v[u], vmax) - 1);
@@ -337,30 +185,78 @@ __global__ void __launch_bounds__(LNS_NT) k_lns_hist(const int32_t *A, uint32_t 
     __syncthreads();
     for (int b = threadIdx.x; b < nbins; b += blockDim.x)
         if (lh[b]) atomicAdd(&hist[b], (unsigned long long)lh[b]);
-    if (top) {
-        for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
-        if ((threadIdx.x & 31) == 0) atomicMax(top, m);
-    }
 }
 
-// extraction threshold that keeps {map >= thr} within cap, from the histogram
-// of [1, vmax] in THR_BINS bins: the least value of the lowest bin whose tail
-// fits (one thread: the walk ends after the few bins that hold cap words)
-__global__ void k_lns_threshold(const unsigned long long *hist, int vmax, const int *vmax_dev, long long cap,
-                                RefreshInfo *info)
+// The values behind an extraction threshold: those in (vmax / 2, vmax] in
+// THR_BINS bins of `width` values, and the maximum of all.  vmax bounds the
+// map (*vmax_dev where it is given).  The values of a map below half its
+// maximum are nearly all of them and never reach the threshold, so a warp
+// without a higher one only compares.
+__device__ __forceinline__ int thr_width(int vmax) { return max(1, ((vmax + 1) / 2 + THR_BINS - 1) / THR_BINS); }
+
+__global__ void __launch_bounds__(LNS_NT) k_lns_tail(const int32_t *A, uint32_t N, int vmax, const int *vmax_dev,
+                                                     uint32_t *hist, int *top)
 {
-    const int nb = THR_BINS, top = info->top;
-    if (vmax_dev) vmax = max(1, *vmax_dev);
-    int thr = 1;
-    if (top > 1) {
-        long long above = 0;
-        int b = nb;
-        while (b > 0 && above + (long long)hist[b - 1] <= cap) { above += (long long)hist[b - 1]; b--; }
-        // bin b holds the values v with (v-1)*nb/vmax == b: the first such v
-        thr = b >= nb ? top : (int)(((long long)b * vmax + nb - 1) / nb) + 1;
-        thr = max(1, min(thr, top));
+    __shared__ uint32_t lh[THR_BINS];
+    for (int b = threadIdx.x; b < THR_BINS; b += LNS_NT) lh[b] = 0;
+    if (vmax_dev) vmax = max(1, __ldcg(vmax_dev));
+    __syncthreads();
+    const int floor = vmax / 2, width = thr_width(vmax);
+    int m = INT_MIN;
+    for (unsigned long long x0 = (unsigned long long)blockIdx.x * (8 * LNS_NT); x0 < N;
+         x0 += (unsigned long long)gridDim.x * (8 * LNS_NT)) {
+        int v[8], w = INT_MIN;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const unsigned long long x = x0 + (unsigned)u * LNS_NT + threadIdx.x;
+            v[u] = x < N ? __ldcg(&A[x]) : INT_MIN;
+            w = max(w, v[u]);
+        }
+        m = max(m, w);
+        if (!__any_sync(0xffffffffu, w > floor)) continue;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            // the lanes that share the first one's bin add once: early in a
+            // fill all gains are equal, later they spread over the bins
+            const int b = v[u] > floor ? min((v[u] - floor - 1) / width, THR_BINS - 1) : -1;
+            const unsigned in = __ballot_sync(0xffffffffu, b >= 0);
+            if (!in) continue;
+            const int lead = __ffs(in) - 1, b0 = __shfl_sync(0xffffffffu, b, lead);
+            const unsigned same = __ballot_sync(0xffffffffu, b == b0);
+            if ((int)(threadIdx.x & 31) == lead) atomicAdd(&lh[b0], (uint32_t)__popc(same));
+            else if (b >= 0 && b != b0) atomicAdd(&lh[b], 1u);
+        }
     }
-    info->thr = thr;
+    __syncthreads();
+    for (int b = threadIdx.x; b < THR_BINS; b += LNS_NT)
+        if (lh[b]) atomicAdd(&hist[b], lh[b]);
+    for (int o = 16; o > 0; o >>= 1) m = max(m, __shfl_xor_sync(0xffffffffu, m, o));
+    if ((threadIdx.x & 31) == 0) atomicMax(top, m);
+}
+
+// the threshold: the least value of the lowest bin whose tail holds at most
+// cap words, but at most the maximum (which more than cap words may have)
+__global__ void __launch_bounds__(THR_BINS) k_lns_threshold(const uint32_t *hist, int vmax, const int *vmax_dev,
+                                                            long long cap, RefreshInfo *info)
+{
+    __shared__ unsigned long long ws[THR_BINS / 32];
+    __shared__ int first;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (vmax_dev) vmax = max(1, *vmax_dev);
+    if (threadIdx.x == 0) first = THR_BINS;
+    // the bin's tail: a prefix sum from the highest bin down
+    const int b = THR_BINS - 1 - (int)threadIdx.x;
+    unsigned long long x = hist[b];
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    for (int w = 0; w < warp; w++) x += ws[w];
+    if (x <= (unsigned long long)cap) atomicMin(&first, b);
+    __syncthreads();
+    if (threadIdx.x == 0) info->thr = max(1, min(vmax / 2 + 1 + first * thr_width(vmax), info->top));
 }
 
 // ordered compaction of {x : A[x] >= thr}: counts of chunks of EXT_CHUNK
@@ -421,32 +317,30 @@ __global__ void __launch_bounds__(1024) k_lns_scan(uint32_t *bcount, uint32_t nb
 __global__ void __launch_bounds__(LNS_NT) k_lns_emit_ge(const int32_t *A, uint32_t N, int thr, const int *thr_dev,
                                                         const uint32_t *boff, uint32_t cap, uint32_t *oidx, int32_t *oval)
 {
+    constexpr uint32_t SPAN = EXT_CHUNK / (LNS_NT / 32);      // consecutive words of a warp
     if (thr_dev) thr = __ldcg(thr_dev);
-    const uint32_t x0 = blockIdx.x * EXT_CHUNK, x1 = min(N, x0 + EXT_CHUNK);
     const uint32_t first = boff[blockIdx.x];
     if (first >= cap || (blockIdx.x + 1 < gridDim.x && boff[blockIdx.x + 1] == first)) return;
-    __shared__ uint32_t wbase[LNS_NT / 32];
-    __shared__ uint32_t run;
-    if (threadIdx.x == 0) run = first;
-    __syncthreads();
+    __shared__ uint32_t wcount[LNS_NT / 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t xb = x0; xb < x1; xb += blockDim.x) {
-        const uint32_t x = xb + threadIdx.x;
-        const bool take = x < x1 && A[x] >= thr;
+    const uint32_t x0 = blockIdx.x * EXT_CHUNK + (uint32_t)warp * SPAN + (uint32_t)lane;
+    uint32_t c = 0;
+#pragma unroll 8
+    for (uint32_t k = 0; k < SPAN; k += 32) c += x0 + k < N && __ldcg(&A[x0 + k]) >= thr;
+    c = __reduce_add_sync(0xffffffffu, c);
+    if (lane == 0) wcount[warp] = c;
+    __syncthreads();
+    if (!c) return;
+    uint32_t at = first;
+    for (int w = 0; w < warp; w++) at += wcount[w];
+    for (uint32_t k = 0; k < SPAN; k += 32) {
+        const uint32_t x = x0 + k;
+        const int32_t v = x < N ? __ldcg(&A[x]) : INT_MIN;
+        const bool take = x < N && v >= thr;
         const unsigned m = __ballot_sync(0xffffffffu, take);
-        if (lane == 0) wbase[warp] = __popc(m);
-        if (!__syncthreads_or(take)) continue;
-        if (threadIdx.x == 0) {
-            uint32_t s = run;
-            for (int w = 0; w < LNS_NT / 32; w++) { const uint32_t c = wbase[w]; wbase[w] = s; s += c; }
-            run = s;
-        }
-        __syncthreads();
-        if (take) {
-            const uint32_t at = wbase[warp] + __popc(m & ((1u << lane) - 1));
-            if (at < cap) { oidx[at] = x; oval[at] = A[x]; }
-        }
-        __syncthreads();
+        const uint32_t to = at + __popc(m & ((1u << lane) - 1));
+        if (take && to < cap) { oidx[to] = x; oval[to] = v; }
+        at += __popc(m);
     }
 }
 
@@ -529,23 +423,32 @@ __global__ void k_lns_zero(const uint16_t *cnt, uint32_t N, int target, unsigned
 }
 
 // ------------------------------------------------- uncovered-word masks ----
-// um[p]: bit y set iff the word p * blk + y is uncovered.  A block of words
+// um[p]: bit y set iff the count of word p * blk + y is target.  A block of words
 // (the blk = q^nb that share their high digits) is staged through shared
 // memory, so that the counts are read once in order.
 __global__ void __launch_bounds__(LNS_NT) k_lns_masks(const uint16_t *__restrict__ cnt, uint32_t nblk, int blk,
-                                                      uint64_t *__restrict__ um)
+                                                      int target, uint64_t *__restrict__ um)
 {
     __shared__ uint8_t z[LNS_NT * 64];
     const uint32_t p0 = blockIdx.x * LNS_NT;
     const uint32_t np = min((uint32_t)LNS_NT, nblk - p0);
     const uint16_t *c = cnt + (size_t)p0 * blk;
 #pragma unroll 8
-    for (uint32_t k = threadIdx.x; k < np * (uint32_t)blk; k += LNS_NT) z[k] = __ldcg(&c[k]) == 0;
+    for (uint32_t k = threadIdx.x; k < np * (uint32_t)blk; k += LNS_NT) z[k] = (int)__ldcg(&c[k]) == target;
     __syncthreads();
     if (threadIdx.x < np) {
         uint64_t m = 0;
         for (int y = 0; y < blk; y++) m |= (uint64_t)z[threadIdx.x * blk + y] << y;
         um[p0 + threadIdx.x] = m;
+    }
+}
+
+// R = 0: the map is the marked words themselves
+__global__ void k_lns_mask_words(const uint64_t *um, uint32_t N, uint32_t blk, int32_t *out)
+{
+    for (uint32_t x = blockIdx.x * blockDim.x + threadIdx.x; x < N; x += gridDim.x * blockDim.x) {
+        const uint32_t z = x / blk;
+        out[x] = (int32_t)((um[z] >> (x - z * blk)) & 1u);
     }
 }
 
@@ -963,155 +866,151 @@ int grid_of(uint32_t N)
 
 CovDeviceFlags g_map_attr;      // shared-memory opt-in of the map kernels, per device
 
-// alphabet sizes with their own map kernels (others run the Q = 0 form)
-#define MAP_Q_LIST(X) X(5) X(6) X(7) X(8)
+// a sweep of `layers` layers: kernels for 3, 5, 7 and 9, so that the registers
+// and the shared memory of an element stay few where the layers are
+int map_slots(int layers) { return layers <= 3 ? 3 : layers <= 5 ? 5 : layers <= 7 ? 7 : 9; }
 
-template <int R1, int Q>
-int map_attrs_rq()
+void map_kernels(int q, int layers, MapLow *low, MapHigh *high)
 {
-    CK(cudaFuncSetAttribute(k_map_low<R1, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAP_SMEM_MAX));
-    CK(cudaFuncSetAttribute(k_map_high<R1, Q>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAP_SMEM_MAX));
-    return 0;
-}
-
-template <int R1>
-int map_attrs_one()
-{
-    int rc = map_attrs_rq<R1, 0>();
-#define MAP_ATTR_Q(QQ) if (!rc) rc = map_attrs_rq<R1, QQ>();
-    MAP_Q_LIST(MAP_ATTR_Q)
-#undef MAP_ATTR_Q
-    return rc;
+    switch (map_slots(layers)) {
+    case 3: map_kernels_3(q, low, high); break;
+    case 5: map_kernels_5(q, low, high); break;
+    case 7: map_kernels_7(q, low, high); break;
+    default: map_kernels_9(q, low, high); break;
+    }
 }
 
 int map_attrs()
 {
     int dev = 0;
     if (g_map_attr.done(dev)) return 0;
-    int rc = map_attrs_one<2>();
-    if (!rc) rc = map_attrs_one<3>();
-    if (!rc) rc = map_attrs_one<4>();
-    if (!rc) rc = map_attrs_one<5>();
-    if (!rc) rc = map_attrs_one<6>();
-    if (!rc) rc = map_attrs_one<7>();
-    if (!rc) rc = map_attrs_one<8>();
-    if (!rc) rc = map_attrs_one<9>();
-    if (rc) return rc;
+    for (int q = 2; q <= 11; q++)
+        for (int layers : {3, 5, 7, 9}) {
+            MapLow low;
+            MapHigh high;
+            map_kernels(q, layers, &low, &high);
+            CK(cudaFuncSetAttribute((const void *)low, cudaFuncAttributeMaxDynamicSharedMemorySize, MAP_SMEM_MAX));
+            CK(cudaFuncSetAttribute((const void *)high, cudaFuncAttributeMaxDynamicSharedMemorySize, MAP_SMEM_MAX));
+        }
     g_map_attr.set(dev);
     return 0;
 }
 
-template <int R1>
-int map_launch_low(int grid, size_t smem, const MapGeom &g, int k, const uint16_t *cnt, int target, LayerPtrs L,
-                   int fin, int32_t *out, uint16_t *cnt16)
+// layers that a strip sweep of axes j0 .. j0+gsz-1 holds of an element
+int map_strip_slots(int n, int R, int j0, int gsz) { return map_slots(map_hi(R, j0 + gsz) - map_lo(n, R, j0) + 1); }
+
+uint32_t map_cols(int q, int k) { return ((uint32_t)bt_ipow(q, k) + 3u) & ~3u; }
+
+// a low tile at `slots` layers an element: the layers, the table of the
+// blocks' balls, the masks
+size_t map_low_smem(int q, int slots, int k, int nb, uint32_t blk)
 {
-    switch (g.q) {
-#define MAP_LOW_Q(QQ) case QQ: k_map_low<R1, QQ><<<grid, MAP_NT, smem>>>(g, k, cnt, target, L, fin, out, cnt16); break;
-    MAP_Q_LIST(MAP_LOW_Q)
-#undef MAP_LOW_Q
-    default: k_map_low<R1, 0><<<grid, MAP_NT, smem>>>(g, k, cnt, target, L, fin, out, cnt16); break;
-    }
-    CK(cudaGetLastError());
-    return 0;
+    return (size_t)map_cols(q, k) * slots * 4 + (size_t)blk * (nb + 1) * 8 + (size_t)bt_ipow(q, k) / blk * 8;
 }
 
-template <int R1>
-int map_launch_high(int grid, size_t smem, const MapGeom &g, int j0, int gsz, int lw, LayerPtrs L, int fin,
-                    int32_t *out, uint16_t *cnt16)
+// How the axes are grouped: the low ones in tiles at two CTAs an SM or more,
+// the others in strips of at least eight columns at two, in as few groups as that
+// allows, the larger ones first.
+void map_plan(cov_lns *h)
 {
-    switch (g.q) {
-#define MAP_HIGH_Q(QQ) case QQ: k_map_high<R1, QQ><<<grid, MAP_NT, smem>>>(g, j0, gsz, lw, L, fin, out, cnt16); break;
-    MAP_Q_LIST(MAP_HIGH_Q)
-#undef MAP_HIGH_Q
-    default: k_map_high<R1, 0><<<grid, MAP_NT, smem>>>(g, j0, gsz, lw, L, fin, out, cnt16); break;
+    const int q = h->q, n = h->n, R = h->R;
+    h->kl = h->nb;
+    while (h->kl < n && map_low_smem(q, map_slots(map_hi(R, h->kl + 1) + 1), h->kl + 1, h->nb, h->blk) <= MAP_SMEM_LOW)
+        h->kl++;
+    const int m = n - h->kl;
+    int gmax = 1;
+    while (gmax < m && bt_ipow(q, gmax + 1) * MAP_W_MIN * map_slots(R + 1) * 4 <= MAP_SMEM_HIGH) gmax++;
+    h->ng = (m + gmax - 1) / gmax;
+    for (int i = 0, left = m; i < h->ng; i++) {
+        h->gs[i] = (left + h->ng - i - 1) / (h->ng - i);
+        left -= h->gs[i];
     }
-    CK(cudaGetLastError());
-    return 0;
+    for (int i = 0, j0 = h->kl; i < h->ng; j0 += h->gs[i++]) h->slots[i] = map_strip_slots(n, R, j0, h->gs[i]);
+    // All groups but the last work within the words that share the last
+    // group's digits.  A few such parts at a time go through them, so that
+    // what a sweep writes is still in L2 when the next one reads it.
+    h->parts = h->ng >= 2 ? (uint32_t)bt_ipow(q, h->gs[h->ng - 1]) : 1u;
+    int most = 0;
+    for (int i = 0; i < std::max(1, h->ng - 1); i++) most = std::max(most, h->slots[i]);
+    const long long cols = (long long)(h->N / h->parts) / bt_ipow(q, h->kl) * map_cols(q, h->kl);
+    h->at_once = (uint32_t)std::max(1LL, std::min<long long>(h->parts, MAP_L2_BYTES / (cols * most * 4)));
+    h->scratch_ints = h->ng ? (size_t)cols * h->at_once * most : 0;
+    h->whole_ints = h->ng >= 2 ? (size_t)cols * h->parts * h->slots[h->ng - 1] : 0;
 }
 
-int map_low_any(int R1, int grid, size_t smem, const MapGeom &g, int k, const uint16_t *cnt, int target,
-                LayerPtrs L, int fin, int32_t *out, uint16_t *cnt16)
+// The layered transform of the marked words (masks um) or of the word counts
+// A0, result to out (int32 map) or cnt16.
+int lns_transform(cov_lns *h, const int32_t *A0, int32_t *out, uint16_t *cnt16)
 {
-    switch (R1) {
-    case 2: return map_launch_low<2>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 3: return map_launch_low<3>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 4: return map_launch_low<4>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 5: return map_launch_low<5>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 6: return map_launch_low<6>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 7: return map_launch_low<7>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 8: return map_launch_low<8>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    case 9: return map_launch_low<9>(grid, smem, g, k, cnt, target, L, fin, out, cnt16);
-    default: return COV_EINVAL;
-    }
-}
-
-int map_high_any(int R1, int grid, size_t smem, const MapGeom &g, int j0, int gsz, int lw, LayerPtrs L, int fin,
-                 int32_t *out, uint16_t *cnt16)
-{
-    switch (R1) {
-    case 2: return map_launch_high<2>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 3: return map_launch_high<3>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 4: return map_launch_high<4>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 5: return map_launch_high<5>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 6: return map_launch_high<6>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 7: return map_launch_high<7>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 8: return map_launch_high<8>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    case 9: return map_launch_high<9>(grid, smem, g, j0, gsz, lw, L, fin, out, cnt16);
-    default: return COV_EINVAL;
-    }
-}
-
-// The layered transform: layer 0 from [cnt == target] (cnt given) or from
-// the layer-0 array (the code's counts), result to out (int32 map) or cnt16.
-int lns_transform(cov_lns *h, const uint16_t *cnt, int target, int32_t *out, uint16_t *cnt16)
-{
-    LayerPtrs L;
-    for (int d = 0; d <= LNS_MAXR; d++) L.a[d] = d <= h->R ? h->layer[d] : nullptr;
-    if (h->R == 0) {
-        k_lns_indicator<<<grid_of(h->N), LNS_NT>>>(cnt, target, h->layer[0], h->N, out, cnt16);
-        CK(cudaGetLastError());
-        return 0;
-    }
     int rc = map_attrs();
     if (rc) return rc;
-    const int R1 = h->R + 1, q = h->q, n = h->n;
+    const int q = h->q, n = h->n, R = h->R, sms = std::max(1, cov_sm_count());
+    MapLow low;
+    MapHigh high;
     MapGeom g;
     memset(&g, 0, sizeof g);
-    g.q = q; g.n = n; g.N = h->N;
-    g.pk[0] = 1;
-    for (int k = 1; k <= n; k++) g.pk[k] = g.pk[k - 1] * (uint32_t)q;
-    const size_t per = (size_t)R1 * 4;                    // bytes of one element's layers
-    const int sms = std::max(1, cov_sm_count());
-    // low axes: the widest contiguous tile the shared memory holds
-    int k = 1;
-    while (k < n && (size_t)g.pk[k + 1] * per <= MAP_SMEM_MAX) k++;
-    if ((size_t)g.pk[k] * per > MAP_SMEM_MAX) return COV_ERANGE;
-    {
-        const size_t smem = (size_t)g.pk[k] * per;
-        const int per_sm = std::max(1, (int)(220 * 1024 / smem));
-        const int grid = (int)std::min<uint32_t>(h->N / g.pk[k], (uint32_t)(sms * per_sm));
-        rc = map_low_any(R1, grid, smem, g, k, cnt, target, L, k == n, out, cnt16);
-        if (rc) return rc;
+    g.q = q; g.n = n; g.R = R;
+    g.T = (uint32_t)bt_ipow(q, h->kl);
+    g.Tp = map_cols(q, h->kl);
+    g.out = out; g.cnt16 = cnt16;
+    auto grid_for = [&](uint32_t tiles, size_t smem) {
+        const uint32_t per_sm = (uint32_t)std::max<size_t>(1, std::min<size_t>(8, 225 * 1024 / (smem + 1024)));
+        return std::min(tiles, (uint32_t)sms * per_sm);
+    };
+    // strip sweep i over `tiles` low tiles
+    auto strips = [&](int i, int j0, uint32_t tiles, const int32_t *from, int32_t *to, int slots) {
+        const int gsz = h->gs[i];
+        const uint32_t s = (uint32_t)bt_ipow(q, j0 - h->kl) * g.Tp, rows = (uint32_t)bt_ipow(q, gsz);
+        const size_t per = (size_t)rows * h->slots[i] * 4;
+        int lw = 3;
+        while (per * ((size_t)2 << lw) <= MAP_SMEM_HIGH && (1u << lw) < s && lw < 6) lw++;
+        const uint32_t nt = tiles / (uint32_t)bt_ipow(q, j0 + gsz - h->kl) * ((s + (1u << lw) - 1) >> lw);
+        map_kernels(q, h->slots[i], &low, &high);
+        high<<<grid_for(nt, per << lw), MAP_HIGH_NT, per << lw>>>(g, j0, gsz, lw, s, nt, from, to, slots);
+        CK(cudaGetLastError());
+        return 0;
+    };
+    // the low kernel works at the slots of its reader where they hold its layers
+    const int lslots = std::max(map_slots(map_hi(R, h->kl) + 1), h->ng ? h->slots[0] : 0);
+    const size_t lsm = map_low_smem(q, lslots, h->kl, h->nb, h->blk);
+    const uint32_t part_tiles = h->N / h->parts / g.T;
+    for (uint32_t p = 0; p < h->parts; p += h->at_once) {
+        const uint32_t t0 = p * part_tiles, tiles = std::min(h->at_once, h->parts - p) * part_tiles;
+        map_kernels(q, lslots, &low, &high);
+        low<<<grid_for(tiles, lsm), MAP_LOW_NT, lsm>>>(g, h->kl, h->nb, h->blk, A0 ? nullptr : h->um, h->lowball, A0, t0,
+                                                       tiles, h->map_scratch, h->ng ? h->slots[0] : 0);
+        CK(cudaGetLastError());
+        int j0 = h->kl;
+        int32_t *from = h->map_scratch, *other = h->map_scratch + h->scratch_ints;
+        for (int i = 0; i < h->ng && (i == 0 || i < h->ng - 1); i++) {
+            const bool last = h->ng >= 2 && i == h->ng - 2;
+            int32_t *to = last ? h->map_whole + (size_t)t0 * g.Tp * h->slots[h->ng - 1] : other;
+            rc = strips(i, j0, tiles, from, to, i + 1 < h->ng ? h->slots[i + 1] : 0);
+            if (rc) return rc;
+            other = from;
+            from = to;
+            j0 += h->gs[i];
+        }
     }
-    // the other axes in strips: as many axes as fit with rows of at least
-    // MAP_W_MIN words, then as wide as the shared memory allows
-    int j0 = k;
-    while (j0 < n) {
-        int gsz = 0;
-        while (j0 + gsz < n && (size_t)g.pk[gsz + 1] * MAP_W_MIN * per <= MAP_SMEM_MAX) gsz++;
-        if (gsz == 0) return COV_ERANGE;
-        const uint32_t s = g.pk[j0];
-        int lw = 0;
-        while ((size_t)g.pk[gsz] * ((size_t)2 << lw) * per <= MAP_SMEM_MAX && (1u << lw) < s) lw++;
-        const size_t smem = ((size_t)g.pk[gsz] << lw) * per;
-        const unsigned long long tiles =
-            (unsigned long long)(h->N / (g.pk[gsz] * s)) * ((s + (1u << lw) - 1) >> lw);
-        const int per_sm = std::max(1, (int)(220 * 1024 / smem));
-        const int grid = (int)std::min<unsigned long long>(tiles, (unsigned long long)sms * per_sm);
-        rc = map_high_any(R1, grid, smem, g, j0, gsz, lw, L, j0 + gsz == n, out, cnt16);
-        if (rc) return rc;
-        j0 += gsz;
-    }
+    if (h->ng >= 2) return strips(h->ng - 1, n - h->gs[h->ng - 1], h->N / g.T, h->map_whole, nullptr, 0);
+    return 0;
+}
+
+// masks of the words whose count is target
+int lns_masks(cov_lns *h, int target)
+{
+    const uint32_t nblk = h->N / h->blk;
+    k_lns_masks<<<(nblk + LNS_NT - 1) / LNS_NT, LNS_NT>>>(h->cnt, nblk, (int)h->blk, target, h->um);
+    CK(cudaGetLastError());
+    return 0;
+}
+
+// the map of the words whose masks are in um
+int lns_map_of_masks(cov_lns *h)
+{
+    if (h->R > 0) return lns_transform(h, nullptr, h->map, nullptr);
+    k_lns_mask_words<<<grid_of(h->N), LNS_NT>>>(h->um, h->N, h->blk, h->map);
+    CK(cudaGetLastError());
     return 0;
 }
 
@@ -1238,6 +1137,7 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
             for (uint32_t u = x, v = y, k = 0; k < (uint32_t)h->nb; k++, u /= q, v /= q) d += u % q != v % q;
             for (int sg = d; sg <= h->nb; sg++) low[(size_t)x * (h->nb + 1) + sg] |= 1ull << y;
         }
+    map_plan(h);
     bool ok = cudaMalloc(&h->cnt, (size_t)N * 2) == cudaSuccess &&
               cudaMalloc(&h->map, (size_t)N * 4) == cudaSuccess &&
               cudaMalloc(&h->ball, items.size() * 8) == cudaSuccess &&
@@ -1253,7 +1153,9 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
               cudaMalloc(&h->acc, 4 * (3 * (GREEDY_MAXG + 1) + 1)) == cudaSuccess &&
               cudaMalloc(&h->info, sizeof(RefreshInfo)) == cudaSuccess &&
               cudaMalloc(&h->seq, sizeof(SeqState)) == cudaSuccess;
-    for (int d = 0; ok && d <= R; d++) ok = cudaMalloc(&h->layer[d], (size_t)N * 4) == cudaSuccess;
+    if (ok && h->scratch_ints)
+        ok = cudaMalloc(&h->map_scratch, h->scratch_ints * 4 * (h->ng >= 3 ? 2 : 1)) == cudaSuccess;
+    if (ok && h->whole_ints) ok = cudaMalloc(&h->map_whole, h->whole_ints * 4) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         cov_lns_destroy(h);
@@ -1279,8 +1181,7 @@ int cov_lns_destroy(cov_lns *h)
     cudaFree(h->cnt); cudaFree(h->map); cudaFree(h->ball); cudaFree(h->ball_last); cudaFree(h->d_red);
     cudaFree(h->cand); cudaFree(h->bound); cudaFree(h->list); cudaFree(h->flag); cudaFree(h->seq);
     cudaFree(h->um); cudaFree(h->pball); cudaFree(h->pball_last); cudaFree(h->lowball); cudaFree(h->nom);
-    cudaFree(h->acc); cudaFree(h->info);
-    for (int d = 0; d <= LNS_MAXR; d++) cudaFree(h->layer[d]);
+    cudaFree(h->acc); cudaFree(h->info); cudaFree(h->map_scratch); cudaFree(h->map_whole);
     cudaFree(h->scratch);
     delete h;
     return COV_OK;
@@ -1290,25 +1191,45 @@ int cov_lns_recount(cov_lns *h, const uint32_t *idx, int32_t m)
 {
     if (!h || m < 0 || (m > 0 && !idx)) return COV_EINVAL;
     for (int i = 0; i < m; i++) if (idx[i] >= h->N) return COV_EINVAL;
-    k_lns_zero_layer<<<grid_of(h->N), LNS_NT>>>(h->layer[0], h->N);
-    CK(cudaGetLastError());
-    if (m > 0) {
-        int rc = lns_scratch(h, (size_t)m * 4);
+    // The verifier's tiles while the code is sparse, else the transform of its
+    // word counts; in ps a word: the tiles 1.6 + 0.9 a mark + 0.6 a codeword
+    // per word of a tile, the transform about 12.
+    int nh, nl;
+    bt_geom(h->q, h->n, h->R, m, &nh, &nl);
+    double v = 1, c = 1;
+    const int np = h->n - bt_block_digits(h->n);
+    for (int r = 0; r < std::min(h->R, np); r++) { c = c * (np - r) / (r + 1) * (h->q - 1); v += c; }
+    if (1.6 + 0.9 * m * v / h->N + 0.6 * m / (double)bt_ipow(h->q, nl) < 12.0) {
+        int rc = lns_scratch(h, (size_t)m * (4 + BT_REC_BYTES) + 8);
         if (rc) return rc;
-        CK(cudaMemcpy(h->scratch, idx, (size_t)m * 4, cudaMemcpyHostToDevice));
-        k_lns_scatter<<<(m + 255) / 256, 256>>>(h->layer[0], (const uint32_t *)h->scratch, m);
-        CK(cudaGetLastError());
+        uint2 *rec = (uint2 *)h->scratch;
+        uint32_t *d_i = (uint32_t *)((char *)h->scratch + (size_t)m * BT_REC_BYTES);
+        if (m > 0) CK(cudaMemcpy(d_i, idx, (size_t)m * 4, cudaMemcpyHostToDevice));
+        rc = cov_count_words(h->q, h->n, h->R, d_i, m, h->cnt, rec, nullptr);
+        if (rc) return rc;
+        CK(cudaDeviceSynchronize());
+        return COV_OK;
     }
-    int rc = lns_transform(h, nullptr, 0, nullptr, h->cnt);
+    int rc = lns_scratch(h, (size_t)m * 4);
     if (rc) return rc;
-    CK(cudaDeviceSynchronize());
-    return COV_OK;
+    int32_t *a0 = nullptr;
+    if (cudaMalloc(&a0, (size_t)h->N * 4) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+    auto done = [&](int r) { cudaFree(a0); return r; };
+    if (cudaMemset(a0, 0, (size_t)h->N * 4) != cudaSuccess ||
+        cudaMemcpy(h->scratch, idx, (size_t)m * 4, cudaMemcpyHostToDevice) != cudaSuccess)
+        return done(-100);
+    k_lns_scatter<<<(m + 255) / 256, 256>>>(a0, (const uint32_t *)h->scratch, m);
+    if (h->R == 0) k_lns_narrow<<<grid_of(h->N), LNS_NT>>>(a0, h->N, h->cnt);
+    else rc = lns_transform(h, a0, nullptr, h->cnt);
+    if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = -100;
+    return done(rc);
 }
 
 int cov_lns_map(cov_lns *h, int32_t target)
 {
     if (!h || target < 0) return COV_EINVAL;
-    int rc = lns_transform(h, h->cnt, target, h->map, nullptr);
+    int rc = lns_masks(h, target);
+    if (!rc) rc = lns_map_of_masks(h);
     if (rc) return rc;
     CK(cudaDeviceSynchronize());
     return COV_OK;
@@ -1332,7 +1253,7 @@ int cov_lns_map_hist(cov_lns *h, int32_t nbins, int32_t vmax, int64_t *hist)
     if (rc) return rc;
     unsigned long long *d_h = (unsigned long long *)h->scratch;
     CK(cudaMemset(d_h, 0, (size_t)nbins * 8));
-    k_lns_hist<<<grid_of(h->N), LNS_NT, (size_t)nbins * 4>>>(h->map, h->N, nbins, vmax, nullptr, d_h, nullptr);
+    k_lns_hist<<<grid_of(h->N), LNS_NT, (size_t)nbins * 4>>>(h->map, h->N, nbins, vmax, d_h);
     CK(cudaGetLastError());
     CK(cudaMemcpy(hist, d_h, (size_t)nbins * 8, cudaMemcpyDeviceToHost));
     return COV_OK;
@@ -1468,19 +1389,20 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
     size_t smem = 0;
     rc = greedy_shape(h, a, &G, &smem);
     if (rc) return rc;
-    const uint32_t xb = extract_blocks(h), nblk = h->N / h->blk;
-    rc = lns_scratch(h, THR_BINS * 8 + (size_t)xb * 4);
+    const uint32_t xb = extract_blocks(h);
+    rc = lns_scratch(h, THR_BINS * 4 + (size_t)xb * 4);
     if (rc) return rc;
-    unsigned long long *d_hist = (unsigned long long *)h->scratch;
+    uint32_t *d_hist = (uint32_t *)h->scratch;
     uint32_t *bcount = (uint32_t *)(d_hist + THR_BINS);
     SeqState st;
     memset(&st, 0, sizeof st);
     st.uncov = count_eq(h, 0);
     if (st.uncov < 0) return -100;
     CK(cudaMemcpy(h->seq, &st, sizeof st, cudaMemcpyHostToDevice));
+    // the uncovered words' masks, which the placements keep current
     if (room > 0 && st.uncov > 0) {
-        k_lns_masks<<<(nblk + LNS_NT - 1) / LNS_NT, LNS_NT>>>(h->cnt, nblk, (int)h->blk, h->um);
-        CK(cudaGetLastError());
+        rc = lns_masks(h, 0);
+        if (rc) return rc;
     }
     a.cnt = h->cnt; a.um = h->um; a.b = block_geom(h); a.whole = ball_geom(h); a.lowball = h->lowball;
     a.nb = h->nb; a.blk = (int)h->blk;
@@ -1504,11 +1426,11 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
         // maximum has more than cand_cap words, the same gain and a higher
         // position): a candidate is placed only while its exact gain is at
         // least the threshold, so it is always a best placement.
-        rc = lns_transform(h, h->cnt, 0, h->map, nullptr);
+        rc = lns_map_of_masks(h);
         if (rc) return rc;
         refreshes++;
         CK(cudaMemsetAsync(h->info, 0x80, sizeof(RefreshInfo)));         // top: a negative number
-        CK(cudaMemsetAsync(d_hist, 0, THR_BINS * 8));
+        CK(cudaMemsetAsync(d_hist, 0, THR_BINS * 4));
         const int *vmax_dev = nullptr;
         if (vmax <= 0) {
             // the first map of the call: its maximum first; later ones are
@@ -1517,9 +1439,8 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
             vmax_dev = &h->info->thr;
             CK(cudaMemcpyAsync(&h->info->thr, &h->info->top, 4, cudaMemcpyDeviceToDevice));
         }
-        k_lns_hist<<<grid_of(h->N), LNS_NT, THR_BINS * 4>>>(h->map, h->N, THR_BINS, vmax, vmax_dev, d_hist,
-                                                            &h->info->top);
-        k_lns_threshold<<<1, 1>>>(d_hist, vmax, vmax_dev, (long long)cand_cap, h->info);
+        k_lns_tail<<<grid_of(h->N), LNS_NT>>>(h->map, h->N, vmax, vmax_dev, d_hist, &h->info->top);
+        k_lns_threshold<<<1, THR_BINS>>>(d_hist, vmax, vmax_dev, (long long)cand_cap, h->info);
         CK(cudaGetLastError());
         rc = extract_launch(h, 1, &h->info->thr, cand_cap, bcount, h->cand, h->bound, nullptr, &h->info->found);
         if (rc) return rc;
@@ -1547,7 +1468,7 @@ int cov_lns_uncovered(cov_lns *h, int64_t cap, uint32_t *idx, int64_t *found)
 {
     if (!h || cap < 0 || (cap > 0 && !idx) || !found) return COV_EINVAL;
     // the indicator of cnt == 0 into the map, then its ordered extraction
-    k_lns_indicator<<<grid_of(h->N), LNS_NT>>>(h->cnt, 0, nullptr, h->N, h->map, nullptr);
+    k_lns_indicator<<<grid_of(h->N), LNS_NT>>>(h->cnt, 0, h->N, h->map);
     CK(cudaGetLastError());
     std::vector<int32_t> val((size_t)std::max<int64_t>(std::min<int64_t>(cap, h->N), 1));
     return cov_lns_map_extract(h, 1, cap, idx, val.data(), found);

@@ -460,3 +460,7 @@ static inline void bt_vcum_h(int q, int n, int R, int nl, uint32_t *vcum)
         if (in) c = c * (nm - r) / (r + 1) * (q - 1);
     }
 }
+
+// cov_verify.cu: the saturated coverage counts of the m listed words (device
+// word indices below q^n) into cnt; rec: m * BT_REC_BYTES bytes, 8-byte aligned
+int cov_count_words(int q, int n, int R, const uint32_t *d_idx, int m, uint16_t *cnt, uint2 *rec, cudaStream_t st);

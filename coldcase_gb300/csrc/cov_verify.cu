@@ -592,6 +592,18 @@ __global__ void k_count_records(const uint8_t *__restrict__ code, int M, int q, 
     }
 }
 
+// the same of word indices
+__global__ void k_count_records_idx(const uint32_t *__restrict__ idx, int M, int q, int n, int nh, int nl, uint2 *mid,
+                                    uint32_t *hi)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+        uint64_t pk = 0;
+        uint32_t x = idx[i];
+        for (int j = n - 1; j >= 0; j--) { pk |= (uint64_t)(x % (uint32_t)q) << (4 * j); x /= (uint32_t)q; }
+        bt_record(i, q, n, nh, nl, mid, hi, [&](int j) { return (uint32_t)cov_nib(pk, j); });
+    }
+}
+
 struct CountGeom {
     int q, n, R, M, nh, nl;
     uint32_t tw;                       // q^nl words per tile
@@ -945,6 +957,21 @@ int dt_run(const DtGeom &g, const DtPlan &plan, const uint8_t *d_code, int M, ui
 }
 
 }  // namespace
+
+int cov_count_words(int q, int n, int R, const uint32_t *d_idx, int m, uint16_t *cnt, uint2 *rec, cudaStream_t st)
+{
+    int rc = ct_attrs();
+    if (rc) return rc;
+    const CountGeom g = count_geom(q, n, std::min(R, n), m);
+    uint32_t *hi = (uint32_t *)(rec + m);
+    if (m > 0) {
+        k_count_records_idx<<<std::min(1024, (m + 127) / 128), 128, 0, st>>>(d_idx, m, q, n, g.nh, g.nl, rec, hi);
+        CK(cudaGetLastError());
+    }
+    ct_launch(g, BtCode{hi, rec}, cnt, st);
+    CK(cudaGetLastError());
+    return COV_OK;
+}
 
 extern "C" {
 
