@@ -1127,6 +1127,8 @@ sym_kernel(const SymSlot *slots, const int *list, int mode, unsigned long long b
         else if (op == SOP_COMMIT) sym_op_commit(d, S, LS, cl, rank, csize, oi, opos, oval);
         cl.sync();
     }
+    // no CTA may leave while another can still read the leader's shared memory
+    cl.sync();
     if (rank == 0 && threadIdx.x == 0) {
         SymState &st = *d.st;
         for (int k = 0; k < 4; k++) st.rng[k] = S.rng.s[k];
