@@ -211,6 +211,37 @@ __device__ __forceinline__ void cov_item_word(const CovSlot &d, const CovItem &i
     pk = cov_setnib(it.pk, it.last, val);
 }
 
+// ------------------------------------------------------- grid barrier -----
+// All CTAs of a cooperative launch meet: `arrivals` counts them (cleared
+// before the launch), `target` is the CTA count times the meetings so far.
+// Every thread's writes before it are visible after it to ld.global.cg.
+// False when the wait ran out; the caller then leaves.
+__device__ __forceinline__ bool cov_grid_meet(unsigned *arrivals, unsigned target, unsigned long long wait_ns)
+{
+    __shared__ int ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        atomicAdd(arrivals, 1u);
+        unsigned long long t0, t1;
+        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+        int good = 1;
+        unsigned seen;
+        for (unsigned spin = 1;; spin++) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(arrivals) : "memory");
+            if ((int)(seen - target) >= 0) break;
+            if ((spin & 255u) == 0) {
+                asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
+                if (t1 - t0 > wait_ns) { good = 0; break; }
+            }
+        }
+        __threadfence();
+        ok = good;
+    }
+    __syncthreads();
+    return ok != 0;
+}
+
 // ------------------------------------------------------ per device, host --
 // Host-side facts that belong to one device: its SM count, and whether a
 // kernel's attributes (the dynamic shared-memory opt-in, which

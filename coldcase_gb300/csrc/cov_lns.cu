@@ -519,37 +519,6 @@ __device__ __forceinline__ unsigned long long cand_key(int32_t bound, int pos)
 __device__ __forceinline__ int key_pos(unsigned long long k) { return 0x7fffffff - (int)(uint32_t)k; }
 __device__ __forceinline__ int key_bound(unsigned long long k) { return (int)(uint32_t)(k >> 32) - 0x40000000; }
 
-__device__ __forceinline__ unsigned long long lns_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-// All CTAs of the cooperative launch meet; every thread's writes before it
-// are visible after it.  False when the wait ran out.
-__device__ __forceinline__ bool grid_meet(unsigned *bar, unsigned target, unsigned long long wait_ns)
-{
-    __shared__ int ok;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const unsigned long long t0 = lns_ns();
-        int good = 1;
-        unsigned seen;
-        for (unsigned spin = 1;; spin++) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            if (seen >= target) break;
-            if ((spin & 255u) == 0 && lns_ns() - t0 > wait_ns) { good = 0; break; }
-        }
-        __threadfence();
-        ok = good;
-    }
-    __syncthreads();
-    return ok != 0;
-}
-
 __device__ __forceinline__ unsigned long long warp_max64(unsigned long long k)
 {
     for (int o = 16; o > 0; o >>= 1) k = max(k, __shfl_xor_sync(0xffffffffu, k, o));
@@ -611,7 +580,7 @@ __global__ void __launch_bounds__(GREEDY_NT) k_lns_greedy(GreedyArgs a)
             ks = warp_max64(lane < GREEDY_NT / 32 ? s_w[1][lane] : 0);
             if (lane == 0) { __stcg(&a.nom[me], kf); __stcg(&a.nom[G + me], ks); }
         }
-        if (!(ok = grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
+        if (!(ok = cov_grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
         // ---- the decision, the same in every CTA
         kf = ks = 0;
         for (int t = threadIdx.x; t < G; t += GREEDY_NT) {
@@ -724,7 +693,7 @@ __global__ void __launch_bounds__(GREEDY_NT) k_lns_greedy(GreedyArgs a)
                 if (t) atomicAdd(&acc[fresh ? 0 : me / a.team], t);
             }
         }
-        if (!(ok = grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
+        if (!(ok = cov_grid_meet(a.bar, ++met * (unsigned)G, a.wait_ns))) break;
         if (fresh) {
             if (threadIdx.x == 0 && me == 0) a.list[placed] = a.cand[pos];
             if (threadIdx.x == 0 && pos % G == me) sb[pos / G] = 0;      // a codeword now: its ball is covered

@@ -11,18 +11,21 @@
 // of every sampled move (each of its q sub-moves judged against the
 // unchanged counters), the reservoir tie-break and the kicks.
 //
-// Execution: one thread-block cluster per instance.  The leader CTA does the
-// serial, RNG-ordered steps (pick, candidates, sample, selection); the
-// cluster shares the three bulk operations -- the estimates of all sampled
+// Execution: one thread-block cluster per instance, or, for a single instance
+// that has the GPU to itself, one cooperative launch of a CTA per SM.  The
+// leader CTA does the serial, RNG-ordered steps (pick, candidates, sample,
+// selection); the CTAs share the three bulk operations -- the estimates of all sampled
 // moves (take x S' counter pairs, S' = C(n-1,R)(q-1)^R), the commit of the
 // chosen move (S' pairs) and the q balls of an orbit (init and kicks).  Ops
-// go out through the leader's shared memory and CTAs meet only at hardware
-// cluster barriers.  Counters are 16 bits (as the reference's), two to a
+// go out through the leader's shared memory and CTAs meet at hardware cluster
+// barriers; over the whole GPU they go through a global descriptor and the
+// CTAs meet at a counter with a bounded wait.  Counters are 16 bits (as the reference's), two to a
 // 32-bit word, updated by 32-bit atomics: a count never exceeds 65000 and
 // never drops below zero, so one half never carries into the other.  Beside
 // them a 2-bit shadow min(cnt, 2) (4 words a byte, the layout of
 // covsearch2e's opt_st = 2) serves the estimates and the pick: 8 MB for the
 // 16.7M quotient words of K_8(9,4), so that many instances stay in L2.
+#include <climits>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -39,12 +42,14 @@ namespace cg = cooperative_groups;
 #define SYM_MAXR 7              // symsearch.c:311
 #define SYM_PB 16               // pick probes drawn per batch
 #define SYM_CT 2048             // centre-table entries (sampled candidates x q)
+#define SYM_SLICE 1024LL        // moves of one launch over the whole GPU
+#define SYM_FY 512               // sample draws made at once
 #define SYM_INV 2048            // moduli with a reciprocal in shared memory
 #define SYM_CYCLES_PER_NS 2ull
 
 enum { SOP_STOP = 0, SOP_ORBIT = 1, SOP_EVAL = 2, SOP_COMMIT = 3 };
 enum { SPH_INIT = 0, SPH_MOVE = 1, SPH_SELECT = 2, SPH_AFTER_COMMIT = 3, SPH_KICK_DEL = 4,
-       SPH_KICK_ADD = 5, SPH_KICK_NEXT = 6, SPH_DONE = 7, SPH_EVAL = 8 };
+       SPH_KICK_ADD = 5, SPH_KICK_NEXT = 6, SPH_DONE = 7 };
 enum { SMODE_INIT = 0, SMODE_RUN = 1 };
 
 struct SymState {
@@ -56,11 +61,13 @@ struct SymState {
     // candidates, 2 sample, 3 estimate op, 4 selection, 5 commit op, 6 orbit
     // ops, 7 the rest; 8 moves counted
     unsigned long long prof[9];
-    // a move planned up to its estimates, which a grid-wide launch computes
-    // (the sample is in cands[0..take)); the next leader launch goes on
-    // from the selection
-    int eval_pending, take;
-    cov_move_rec rec;
+};
+
+// the op of a launch over the whole GPU, as the leader publishes it
+struct SymOp {
+    int op, oi, opos, oval, osign, take;
+    unsigned long long acc;      // uncovered change accumulated by the op
+    unsigned arrivals;           // at the grid barrier
 };
 
 struct SymSlot {
@@ -113,9 +120,8 @@ struct SymSmem {
     CovRng rng;
     long long it, unc, best_unc, since_improve, nkicks, trace_n, moves_left, it_limit;
     int init_i, status, finished, phase, kick_t, cand_sm;
-    int split, eval_pending;     // estimates by a grid-wide launch; one is due
-    unsigned long long deadline;
-    long long guard, est;
+    unsigned long long deadline, move_ns;   // move_ns: the budget is each move's (0: the launch's)
+    long long guard, est, slice_left;       // slice_left: moves this launch may still plan
     unsigned long long prof[9];
     long long t_mark;
     cov_move_rec rec;
@@ -132,6 +138,7 @@ struct SymSmem {
     uint64_t inv[SYM_INV + 1];   // floor((2^64-1)/m): leader's modular reductions
     int32_t cdv[SYM_TS];
     uint8_t skip[SYM_TS];
+    uint64_t fy[SYM_FY];         // draws of the sample
 };
 
 // ------------------------------------------------------------ helpers ----
@@ -299,9 +306,12 @@ __device__ __forceinline__ uint32_t sym_pick8(const uint4 &lo, const uint4 &hi, 
 // move itself on the counters; MODE 2: refresh the shadow of a and b.
 // cpk/base/dv: the centres' packed digits, word indices and move offsets,
 // indexed by delta.
+// MODE 1 and 2 do the inner values k0 .. k1-1 of the item's q-1 (an item of
+// radius 0 has the one).
 template <int MODE>
 __device__ __forceinline__ long long sym_walk_item(const SymSlot &d, const uint64_t *cpk, const uint32_t *cbase,
-                                                   const uint32_t *cdv, int p, uint32_t r)
+                                                   const uint32_t *cdv, int p, uint32_t r, int k0 = 0,
+                                                   int k1 = COV_MAXQ)
 {
     int delta = 0;
     uint32_t loc = r;
@@ -328,7 +338,7 @@ __device__ __forceinline__ long long sym_walk_item(const SymSlot &d, const uint6
     };
     if (rad == 0) {
         if (MODE == 0) du += (long long)(sym_st(d, base) == 1) - (long long)(sym_st(d, base + dv) == 0);
-        else visit(base);
+        else if (k0 == 0) visit(base);
         return du;
     }
     const uint32_t pp = d.ppow[rad - 1];
@@ -391,7 +401,7 @@ __device__ __forceinline__ long long sym_walk_item(const SymSlot &d, const uint6
             if (k < qm1) du += (long long)(ca[k] == 1) - (long long)(cb[k] == 0);
         return du;
     } else {
-        for (int k = 0; k < qm1; k++) visit(w + (uint32_t)((k + (k >= cl) - cl) * pl));
+        for (int k = k0; k < min(qm1, k1); k++) visit(w + (uint32_t)((k + (k >= cl) - cl) * pl));
         return du;
     }
 }
@@ -400,7 +410,8 @@ __device__ __forceinline__ long long sym_walk_item(const SymSlot &d, const uint6
 // it names (MODE 1, symsearch.c:135-174; returns the uncovered change) or
 // the refresh of their shadow (MODE 2)
 template <int MODE>
-__device__ __forceinline__ long long sym_ball_item(const SymSlot &d, const SymCentres &C, uint32_t r, int sign)
+__device__ __forceinline__ long long sym_ball_item(const SymSlot &d, const SymCentres &C, uint32_t r, int sign, int k0 = 0,
+                                                   int k1 = COV_MAXQ)
 {
     int delta = 0;
     uint32_t loc = r;
@@ -422,7 +433,7 @@ __device__ __forceinline__ long long sym_ball_item(const SymSlot &d, const SymCe
             du += old == 1;
         }
     };
-    if (loc == 0) { touch(base); return du; }
+    if (loc == 0) { if (k0 == 0) touch(base); return du; }
     loc -= 1;
     int rr = 1;
     while (rr <= SYM_MAXR && loc >= d.bcum[rr + 1]) rr++;
@@ -441,7 +452,7 @@ __device__ __forceinline__ long long sym_ball_item(const SymSlot &d, const SymCe
     }
     const int last = ps[rr - 1], cl = cov_nib(c, last);
     const int pl = (int)d.pw[last];
-    for (int k = 0; k < qm1; k++) touch(w + (uint32_t)((k + (k >= cl) - cl) * pl));
+    for (int k = k0; k < min(qm1, k1); k++) touch(w + (uint32_t)((k + (k >= cl) - cl) * pl));
     return du;
 }
 
@@ -449,19 +460,40 @@ __device__ __forceinline__ long long sym_ball_item(const SymSlot &d, const SymCe
 // The counters change first; after a cluster barrier the same words get
 // their shadow refreshed from the final counts (a word may be touched by
 // several threads, so the shadow is only written once its count is final).
-__device__ void sym_op_orbit(const SymSlot &d, SymSmem &S, SymSmem *LS, cg::cluster_group &cl, int rank,
-                             int csize, int i, int sign)
+// Over the whole GPU there are more threads than items, so a thread takes one
+// value of an item's last position (its q-1 values in one thread are a chain
+// of as many dependent atomics: the commit at K_8(9,4) 31 us instead of 20).
+// acc: the op's sum; meet: the CTAs' barrier (false: the wait ran out).
+template <bool GRID, class Work>
+__device__ __forceinline__ void sym_each(const SymSlot &d, uint32_t items, int rank, int csize, Work work)
+{
+    const uint32_t stride = (uint32_t)csize * SNT, first = (uint32_t)rank * SNT + threadIdx.x;
+    if constexpr (GRID) {
+        const uint32_t per = (uint32_t)max(1, d.q - 1);
+        for (unsigned long long t = first; t < (unsigned long long)items * per; t += stride) {
+            const uint32_t r = (uint32_t)(t / per);
+            const int k = (int)(t - (unsigned long long)r * per);
+            work(r, k, k + 1);
+        }
+    } else {
+        for (uint32_t r = first; r < items; r += stride) work(r, 0, COV_MAXQ);
+    }
+}
+
+template <bool GRID, class Meet>
+__device__ bool sym_op_orbit(const SymSlot &d, SymSmem &S, unsigned long long *acc, Meet meet, int rank, int csize, int i,
+                             int sign)
 {
     sym_centres(d, S.ct, cov_ldcg(&d.rep[i]), -1, 0);
     sym_bar();
     long long du = 0;
-    const uint32_t stride = (uint32_t)csize * SNT;
-    for (uint32_t r = (uint32_t)rank * SNT + threadIdx.x; r < d.opi; r += stride)
-        du += sym_ball_item<1>(d, S.ct, r, sign);
+    sym_each<GRID>(d, d.opi, rank, csize,
+                   [&](uint32_t r, int k0, int k1) { du += sym_ball_item<1>(d, S.ct, r, sign, k0, k1); });
     du = sym_block_sum(S, du);
-    if (threadIdx.x == 0 && du) atomicAdd(&LS->acc, (unsigned long long)du);
-    cl.sync();
-    for (uint32_t r = (uint32_t)rank * SNT + threadIdx.x; r < d.opi; r += stride) sym_ball_item<2>(d, S.ct, r, 0);
+    if (threadIdx.x == 0 && du) atomicAdd(acc, (unsigned long long)du);
+    if (!meet()) return false;
+    sym_each<GRID>(d, d.opi, rank, csize, [&](uint32_t r, int k0, int k1) { sym_ball_item<2>(d, S.ct, r, 0, k0, k1); });
+    return true;
 }
 
 // Estimates of the sampled moves.  Flat: every CTA holds the centres of all
@@ -569,29 +601,23 @@ __device__ void sym_eval_items(const SymSlot &d, SymSmem &S, int rank, int csize
     }
 }
 
-__device__ void sym_op_commit(const SymSlot &d, SymSmem &S, SymSmem *LS, cg::cluster_group &cl, int rank,
-                              int csize, int i, int p, int v)
+template <bool GRID, class Meet>
+__device__ bool sym_op_commit(const SymSlot &d, SymSmem &S, unsigned long long *acc, Meet meet, int rank, int csize,
+                              int i, int p, int v)
 {
     sym_centres(d, S.ct, cov_ldcg(&d.rep[i]), p, v);
     sym_bar();
     long long du = 0;
-    const uint32_t stride = (uint32_t)csize * SNT;
-    for (uint32_t r = (uint32_t)rank * SNT + threadIdx.x; r < d.ipc; r += stride)
-        du += sym_walk_item<1>(d, S.ct.cpk, S.ct.base, S.ct.dv, p, r);
+    sym_each<GRID>(d, d.ipc, rank, csize, [&](uint32_t r, int k0, int k1) {
+        du += sym_walk_item<1>(d, S.ct.cpk, S.ct.base, S.ct.dv, p, r, k0, k1);
+    });
     du = sym_block_sum(S, du);
-    if (threadIdx.x == 0 && du) atomicAdd(&LS->acc, (unsigned long long)du);
-    cl.sync();
-    for (uint32_t r = (uint32_t)rank * SNT + threadIdx.x; r < d.ipc; r += stride)
-        sym_walk_item<2>(d, S.ct.cpk, S.ct.base, S.ct.dv, p, r);
-}
-
-__device__ void sym_op_eval(const SymSlot &d, SymSmem &S, SymSmem *LS, int rank, int csize, int take)
-{
-    if (take <= SYM_TS && rank != 0) {
-        for (int s = threadIdx.x; s < take; s += SNT) S.cand[s] = LS->cand[s];
-        sym_bar();
-    }
-    sym_eval_items<false>(d, S, rank, csize, take);
+    if (threadIdx.x == 0 && du) atomicAdd(acc, (unsigned long long)du);
+    if (!meet()) return false;
+    sym_each<GRID>(d, d.ipc, rank, csize, [&](uint32_t r, int k0, int k1) {
+        sym_walk_item<2>(d, S.ct.cpk, S.ct.base, S.ct.dv, p, r, k0, k1);
+    });
+    return true;
 }
 
 // ------------------------------------------------------ leader routines ----
@@ -701,7 +727,9 @@ __device__ bool sym_plan_move(const SymSlot &d, SymSmem &S)
     const int q = d.q, NR = d.NR, R = d.R, norb = d.norb;
     if (tid == 0) {
         int stop = sym_should_stop(d, S) || S.unc <= 0 || S.moves_left <= 0 ||
-                   (S.it_limit >= 0 && S.it >= S.it_limit);
+                   (S.it_limit >= 0 && S.it >= S.it_limit) || S.slice_left <= 0;
+        S.slice_left--;
+        if (S.move_ns) S.deadline = (unsigned long long)sym_clock() + S.move_ns * SYM_CYCLES_PER_NS;
         S.ibc[1] = stop;
         if (!stop) {
             S.it++;
@@ -783,16 +811,44 @@ __device__ bool sym_plan_move(const SymSlot &d, SymSmem &S)
             nc = 1;
         }
         const int take = nc < d.cand ? nc : d.cand;
-        // Fisher-Yates sample (symsearch.c:425-430)
-        const bool sm = nc <= SYM_TS;
-        uint32_t *arr = sm ? S.cand : d.cands;
-        for (int s = 0; s < take; s++) {
-            const int j = s + (int)sym_mod(S, sym_draw(S), (uint64_t)(nc - s));
-            const uint32_t a = arr[s];
-            arr[s] = arr[j];
-            arr[j] = a;
-        }
         S.take = take;
+        S.ibc[3] = nc;
+    }
+    sym_bar();
+    // Fisher-Yates sample (symsearch.c:425-430): the draws one after another,
+    // their residues in parallel, then the swaps
+    nc = S.ibc[3];
+    const int take = S.take;
+    const bool sm = nc <= SYM_TS;
+    if (sm) {
+        for (int s0 = 0; s0 < take; s0 += SYM_FY) {
+            const int k = min(SYM_FY, take - s0);
+            if (tid == 0) {
+                CovRng r = S.rng;
+                for (int s = 0; s < k; s++) S.fy[s] = cov_rng_next(r);
+                S.rng = r;
+            }
+            sym_bar();
+            for (int s = tid; s < k; s += SNT) S.fy[s] = sym_mod(S, S.fy[s], (uint64_t)(nc - s0 - s));
+            sym_bar();
+            if (tid == 0)
+                for (int s = 0; s < k; s++) {
+                    const int at = s0 + s, j = at + (int)S.fy[s];
+                    const uint32_t a = S.cand[at], b = S.cand[j];
+                    S.cand[at] = b;
+                    S.cand[j] = a;
+                }
+            sym_bar();
+        }
+    }
+    if (tid == 0) {
+        if (!sm)
+            for (int s = 0; s < take; s++) {
+                const int j = s + (int)sym_mod(S, sym_draw(S), (uint64_t)(nc - s));
+                const uint32_t a = d.cands[s];
+                d.cands[s] = d.cands[j];
+                d.cands[j] = a;
+            }
         S.cand_sm = take <= SYM_TS && sm;
         S.rec.u = uw;
         S.rec.ncand = nc;
@@ -827,18 +883,40 @@ __device__ void sym_select(const SymSlot &d, SymSmem &S)
         }
     }
     sym_bar();
-    if (tid == 0) {
-        int bs = -1, nties = 0;
-        long long bestd = 1LL << 60;
-        for (int s = 0; s < take; s++) {
-            int cd, sk;
-            if (sm) { cd = S.cdv[s]; sk = S.skip[s]; }
-            else {
-                const uint32_t c = cov_ldcg(&d.cands[s]);
-                cd = cov_ldcg(&d.cd[s]);
-                sk = (int)(c & 15u) == cov_nib(cov_ldcg(&d.rep[c >> 8]), (int)((c >> 4) & 15u));
+    // The walk draws only where an estimate equals the least before it, so a
+    // warp finds the running minimum of 32 estimates at once and its leader
+    // visits just the places where it falls or is met again.
+    int bs = -1, nties = 0;
+    long long bestd = 1LL << 60;
+    if (sm && tid < 32) {
+        for (int s0 = 0; s0 < take; s0 += 32) {
+            const int s = s0 + tid;
+            const long long mine = s < take && !S.skip[s] ? (long long)S.cdv[s] : 1LL << 61;
+            long long before = mine;                         // least up to and with this lane
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long y = __shfl_up_sync(0xffffffffu, before, o);
+                if (tid >= o) before = min(before, y);
             }
-            if (sk) continue;
+            unsigned at = __ballot_sync(0xffffffffu, mine == before && mine <= bestd && mine < (1LL << 60));
+            while (at) {
+                const int l = __ffs((int)at) - 1;
+                at &= at - 1;
+                const long long cd = __shfl_sync(0xffffffffu, mine, l);
+                if (cd < bestd) { bestd = cd; bs = s0 + l; nties = 1; }
+                else if (cd == bestd) {
+                    nties++;
+                    int hit = 0;
+                    if (tid == 0) hit = sym_mod(S, sym_draw(S), (uint64_t)nties) == 0;
+                    if (__shfl_sync(0xffffffffu, hit, 0)) bs = s0 + l;
+                }
+            }
+        }
+    }
+    if (tid == 0) {
+        for (int s = 0; !sm && s < take; s++) {
+            const uint32_t c = cov_ldcg(&d.cands[s]);
+            const int cd = cov_ldcg(&d.cd[s]);
+            if ((int)(c & 15u) == cov_nib(cov_ldcg(&d.rep[c >> 8]), (int)((c >> 4) & 15u))) continue;
             if (cd < bestd) { bestd = cd; bs = s; nties = 1; }
             else if (cd == bestd) {
                 nties++;
@@ -934,28 +1012,7 @@ __device__ void sym_leader(const SymSlot &d, SymSmem &S, int mode)
                 sym_bar();
                 return;
             }
-            if (S.split) {
-                // the estimates run as a grid-wide launch: hand the sample
-                // over and end this launch
-                if (S.take <= SYM_TS)
-                    for (int x = tid; x < S.take; x += SNT) cov_stcg(&d.cands[x], S.cand[x]);
-                if (tid == 0) {
-                    S.phase = SPH_SELECT;
-                    S.eval_pending = 1;
-                    sym_emit(S, SOP_STOP, 0, 0, 0, 0);
-                }
-                sym_bar();
-                return;
-            }
             if (tid == 0) S.phase = SPH_SELECT;
-            sym_bar();
-            return;
-        }
-        if (ph == SPH_EVAL) {
-            // a move left planned for a grid-wide estimate, continued here
-            for (int x = tid; x < S.take; x += SNT) cov_stcg(&d.cd[x], 0);
-            sym_bar();
-            if (tid == 0) { sym_emit(S, SOP_EVAL, 0, 0, 0, 0); S.phase = SPH_SELECT; }
             sym_bar();
             return;
         }
@@ -1059,20 +1116,32 @@ __device__ void sym_leader(const SymSlot &d, SymSmem &S, int mode)
     }
 }
 
+// GRID: one instance on a cooperative launch over the whole GPU; else one
+// cluster per listed instance.  A move then costs the leader's serial steps,
+// five grid barriers (about 1.5 us each) and its bulk operations on every SM:
+// at K_8(9,4) 118 us, 80 of them the estimates (6.7 M random sectors of L2);
+// a cluster of 16 took 62 us for the commit alone (20 here), 188 for a move.
+template <bool GRID>
 __global__ void __launch_bounds__(SNT, 1)
-sym_kernel(const SymSlot *slots, const int *list, int mode, unsigned long long budget_ns, long long op_guard,
-           int split)
+sym_kernel(const SymSlot *slots, const int *list, int mode, unsigned long long budget_ns, long long op_guard, SymOp *gop,
+           long long slice)
 {
     extern __shared__ __align__(16) unsigned char sym_raw[];
     SymSmem &S = *reinterpret_cast<SymSmem *>(sym_raw);
     cg::cluster_group cl = cg::this_cluster();
-    const int csize = (int)cl.num_blocks();
-    const int rank = (int)cl.block_rank();
-    const int sidx = list[blockIdx.x / csize];
+    const int csize = GRID ? (int)gridDim.x : (int)cl.num_blocks();
+    const int rank = GRID ? (int)blockIdx.x : (int)cl.block_rank();
+    const int sidx = list[GRID ? 0 : blockIdx.x / csize];
+    unsigned met = 0;
+    auto meet = [&]() -> bool {
+        if constexpr (GRID) return cov_grid_meet(&gop->arrivals, ++met * (unsigned)csize, budget_ns + 10000000000ull);
+        cl.sync();
+        return true;
+    };
     if (threadIdx.x == 0) S.slot = slots[sidx];
     sym_bar();
     const SymSlot &d = S.slot;
-    SymSmem *LS = cl.map_shared_rank(&S, 0);
+    SymSmem *LS = GRID ? nullptr : cl.map_shared_rank(&S, 0);
     if (rank == 0)
         for (int m = threadIdx.x + 1; m <= SYM_INV; m += SNT) S.inv[m] = ~0ull / (uint64_t)m;
     if (rank == 0 && threadIdx.x == 0) {
@@ -1087,25 +1156,15 @@ sym_kernel(const SymSlot *slots, const int *list, int mode, unsigned long long b
         S.guard = 0;
         S.deadline = (unsigned long long)sym_clock() + budget_ns * SYM_CYCLES_PER_NS;
         if (S.status) S.phase = SPH_MOVE;
-        S.split = split;
-        S.eval_pending = st.eval_pending;
-        if (st.eval_pending) {
-            // the estimates of this move were left to a grid-wide launch
-            // (already run when this launch is split too)
-            S.take = st.take;
-            S.rec = st.rec;
-            S.phase = split ? SPH_SELECT : SPH_EVAL;
-            S.eval_pending = 0;
-        }
+        S.move_ns = GRID ? budget_ns : 0;
+        S.slice_left = slice;
     }
     sym_bar();
-    if (rank == 0 && S.phase == SPH_SELECT && S.take <= SYM_TS)
-        for (int x = threadIdx.x; x < S.take; x += SNT) S.cand[x] = cov_ldcg(&d.cands[x]);
-    if (rank == 0 && S.phase == SPH_EVAL && S.take <= SYM_TS)
-        for (int x = threadIdx.x; x < S.take; x += SNT) S.cand[x] = cov_ldcg(&d.cands[x]);
-    sym_bar();
+    bool ok = true;
     for (;;) {
         if (rank == 0) {
+            if (GRID && threadIdx.x == 0 && (S.op == SOP_ORBIT || S.op == SOP_COMMIT)) S.acc = cov_ldcg(&gop->acc);
+            sym_bar();
             if (S.status && S.phase != SPH_MOVE) {
                 if (threadIdx.x == 0) sym_emit(S, SOP_STOP, 0, 0, 0, 0);
                 sym_bar();
@@ -1117,50 +1176,56 @@ sym_kernel(const SymSlot *slots, const int *list, int mode, unsigned long long b
                 S.op = SOP_STOP;
             }
             sym_bar();
+            if (GRID) {
+                if (S.op == SOP_EVAL && S.take <= SYM_TS)
+                    for (int x = threadIdx.x; x < S.take; x += SNT) cov_stcg(&d.cands[x], S.cand[x]);
+                if (threadIdx.x == 0) {
+                    cov_stcg(&gop->op, S.op);
+                    cov_stcg(&gop->oi, S.oi);
+                    cov_stcg(&gop->opos, S.opos);
+                    cov_stcg(&gop->oval, S.oval);
+                    cov_stcg(&gop->osign, S.osign);
+                    cov_stcg(&gop->take, S.take);
+                    cov_stcg(&gop->acc, 0ull);
+                }
+            }
         }
-        cl.sync();
-        const int op = LS->op, oi = LS->oi, opos = LS->opos, oval = LS->oval, osign = LS->osign;
-        const int take = LS->take;
+        if (!(ok = meet())) break;
+        int op, oi, opos, oval, osign, take;
+        unsigned long long *acc;
+        if constexpr (GRID) {
+            op = cov_ldcg(&gop->op); oi = cov_ldcg(&gop->oi); opos = cov_ldcg(&gop->opos);
+            oval = cov_ldcg(&gop->oval); osign = cov_ldcg(&gop->osign); take = cov_ldcg(&gop->take);
+            acc = &gop->acc;
+        } else {
+            op = LS->op; oi = LS->oi; opos = LS->opos; oval = LS->oval; osign = LS->osign; take = LS->take;
+            acc = &LS->acc;
+        }
         if (op == SOP_STOP) break;
-        if (op == SOP_ORBIT) sym_op_orbit(d, S, LS, cl, rank, csize, oi, osign);
-        else if (op == SOP_EVAL) sym_op_eval(d, S, LS, rank, csize, take);
-        else if (op == SOP_COMMIT) sym_op_commit(d, S, LS, cl, rank, csize, oi, opos, oval);
-        cl.sync();
+        if (op == SOP_ORBIT) ok = sym_op_orbit<GRID>(d, S, acc, meet, rank, csize, oi, osign);
+        else if (op == SOP_COMMIT) ok = sym_op_commit<GRID>(d, S, acc, meet, rank, csize, oi, opos, oval);
+        else if (op == SOP_EVAL) {
+            if (take <= SYM_TS && rank != 0) {
+                for (int x = threadIdx.x; x < take; x += SNT) S.cand[x] = GRID ? cov_ldcg(&d.cands[x]) : LS->cand[x];
+                sym_bar();
+            }
+            sym_eval_items<GRID>(d, S, rank, csize, take);
+        }
+        if (!ok || !(ok = meet())) break;
     }
     // no CTA may leave while another can still read the leader's shared memory
     cl.sync();
     if (rank == 0 && threadIdx.x == 0) {
         SymState &st = *d.st;
+        if (!ok) S.status = COV_EDRIFT;          // a wait ran out: the counters may lack a share of an op
         for (int k = 0; k < 4; k++) st.rng[k] = S.rng.s[k];
         st.it = S.it; st.unc = S.unc; st.best_unc = S.best_unc; st.since_improve = S.since_improve;
         st.nkicks = S.nkicks; st.trace_n = S.trace_n; st.moves_left = S.moves_left;
         st.init_i = S.init_i;
         for (int k = 0; k < 9; k++) st.prof[k] = S.prof[k];
-        st.eval_pending = S.eval_pending;
-        st.take = S.take;
-        st.rec = S.rec;
         if (S.status) atomicCAS(&st.status, 0, S.status);
         st.finished = S.finished || S.unc <= 0;
     }
-}
-
-// The estimates of one instance's planned move over the whole grid
-// (symsearch.c:432-433 for every sampled candidate); the cluster kernel left
-// the sample in cands[0..take) and zeroed cd[0..take).
-__global__ void __launch_bounds__(SNT, 1) sym_eval_kernel(const SymSlot *slots, int slot)
-{
-    extern __shared__ __align__(16) unsigned char sym_raw[];
-    SymSmem &S = *reinterpret_cast<SymSmem *>(sym_raw);
-    if (threadIdx.x == 0) S.slot = slots[slot];
-    sym_bar();
-    const SymSlot &d = S.slot;
-    if (!cov_ldcg(&d.st->eval_pending) || cov_ldcg(&d.st->status)) return;
-    const int take = cov_ldcg(&d.st->take);
-    if (take <= SYM_TS) {
-        for (int x = threadIdx.x; x < take; x += SNT) S.cand[x] = cov_ldcg(&d.cands[x]);
-        sym_bar();
-    }
-    sym_eval_items<true>(d, S, (int)blockIdx.x, (int)gridDim.x, take);
 }
 
 __global__ void k_sym_budget(SymState *states, const int *list, int count, long long moves)
@@ -1226,9 +1291,9 @@ int sym_attrs()
 {
     int dev = 0;
     if (g_sym_attr.done(dev)) return 0;
-    SCK(cudaFuncSetAttribute(sym_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymSmem)));
-    SCK(cudaFuncSetAttribute(sym_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    SCK(cudaFuncSetAttribute(sym_eval_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymSmem)));
+    SCK(cudaFuncSetAttribute(sym_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymSmem)));
+    SCK(cudaFuncSetAttribute(sym_kernel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    SCK(cudaFuncSetAttribute(sym_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SymSmem)));
     g_sym_attr.set(dev);
     return 0;
 }
@@ -1244,6 +1309,7 @@ struct cov_sym {
     SymSlot *d_slots = nullptr;
     SymState *d_states = nullptr;
     int *d_list = nullptr;
+    SymOp *d_gop = nullptr;      // of a launch over the whole GPU
     cudaStream_t stream = nullptr;
 };
 
@@ -1288,23 +1354,25 @@ static int sym_launch(cov_sym *p, const std::vector<int> &slots, int mode, long 
         at[0].val.clusterDim.z = 1;
         cfg.attrs = at;
         cfg.numAttrs = 1;
-        if (mode == SMODE_RUN && p->grid_eval && slots.size() == 1) {
-            // one instance: each move is a cluster launch up to the
-            // estimates and a grid-wide launch for them; moves + 1 cluster
-            // launches close the last move (a finished instance's extra
-            // launches return at once)
-            for (long long m = 0; m <= moves; m++) {
-                SCK(cudaLaunchKernelEx(&cfg, sym_kernel, (const SymSlot *)p->d_slots, (const int *)p->d_list,
-                                       mode, budget_ns, guard, 1));
-                if (m < moves) {
-                    sym_eval_kernel<<<(unsigned)p->sms, SNT, sizeof(SymSmem), p->stream>>>(
-                        (const SymSlot *)p->d_slots, slots[0]);
-                }
-                SCK(cudaGetLastError());
+        if (p->grid_eval && slots.size() == 1) {
+            // one instance: the whole GPU shares its bulk operations, in
+            // launches of a bounded number of moves, the budget being each
+            // move's (a finished or stopped instance's launches return at once)
+            const SymSlot *ds = p->d_slots;
+            const int *dl = p->d_list;
+            long long left = mode == SMODE_RUN ? moves : 1;
+            while (left > 0) {
+                long long slice = std::min(left, SYM_SLICE);
+                left -= slice;
+                SCK(cudaMemsetAsync(p->d_gop, 0, sizeof(SymOp), p->stream));
+                void *args[] = {(void *)&ds, (void *)&dl, (void *)&mode, (void *)&budget_ns, (void *)&guard,
+                                (void *)&p->d_gop, (void *)&slice};
+                SCK(cudaLaunchCooperativeKernel((const void *)sym_kernel<true>, dim3((unsigned)p->sms), dim3(SNT), args,
+                                                sizeof(SymSmem), p->stream));
             }
         } else {
-            SCK(cudaLaunchKernelEx(&cfg, sym_kernel, (const SymSlot *)p->d_slots, (const int *)p->d_list, mode,
-                                   budget_ns, guard, 0));
+            SCK(cudaLaunchKernelEx(&cfg, sym_kernel<false>, (const SymSlot *)p->d_slots, (const int *)p->d_list, mode,
+                                   budget_ns, guard, (SymOp *)nullptr, LLONG_MAX));
             SCK(cudaGetLastError());
         }
         SCK(cudaStreamSynchronize(p->stream));
@@ -1332,9 +1400,10 @@ int cov_sym_create(int32_t max_slots, int32_t cluster, cov_sym **out)
     cudaError_t e = cudaMalloc(&p->d_slots, sizeof(SymSlot) * max_slots);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_states, sizeof(SymState) * max_slots);
     if (e == cudaSuccess) e = cudaMalloc(&p->d_list, sizeof(int) * max_slots);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_gop, sizeof(SymOp));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
-        cudaFree(p->d_slots); cudaFree(p->d_states); cudaFree(p->d_list);
+        cudaFree(p->d_slots); cudaFree(p->d_states); cudaFree(p->d_list); cudaFree(p->d_gop);
         delete p;
         return -(100 + (int)e);
     }
@@ -1347,7 +1416,7 @@ int cov_sym_destroy(cov_sym *p)
     if (!p) return COV_EINVAL;
     cudaStreamSynchronize(p->stream);
     for (auto &h : p->slots) if (h.used) cudaFree(h.arena);
-    cudaFree(p->d_slots); cudaFree(p->d_states); cudaFree(p->d_list);
+    cudaFree(p->d_slots); cudaFree(p->d_states); cudaFree(p->d_list); cudaFree(p->d_gop);
     cudaStreamDestroy(p->stream);
     delete p;
     return COV_OK;
@@ -1360,10 +1429,9 @@ int cov_sym_set_budget(cov_sym *p, double seconds)
     return COV_OK;
 }
 
-// Pool setting: "grid_eval" 1 runs a pool with one live instance with its
-// estimates spread over the whole GPU (a launch per move for them), 0 (the
-// default) keeps every move inside the instance's cluster.  Neither
-// changes a trajectory.
+// Pool setting: "grid_eval" 1 runs a call that advances one instance with its
+// bulk operations spread over the whole GPU, 0 (the default) keeps every move
+// inside the instance's cluster.  Neither changes a trajectory.
 int cov_sym_set_param(cov_sym *p, const char *name, int64_t value)
 {
     if (!p || !name) return COV_EINVAL;

@@ -47,8 +47,8 @@ class SymPool:
     """Quotient-search instances on one GPU (cov_sym_* in include/covgpu.h)."""
 
     def __init__(self, max_slots=1, cluster=1, budget_s=30.0, grid_eval=False):
-        """grid_eval: with one live instance, spread each move's estimates over
-        the whole GPU instead of the instance's cluster."""
+        """grid_eval: with one live instance, spread each move's estimates and
+        its commit over the whole GPU instead of the instance's cluster."""
         self.lib = L.load()
         h = ctypes.c_void_p()
         L.check(self.lib.cov_sym_create(int(max_slots), int(cluster), ctypes.byref(h)), "cov_sym_create")
