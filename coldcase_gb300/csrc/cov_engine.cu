@@ -50,6 +50,7 @@ namespace cg = cooperative_groups;
 #define RS_NCK    16           // checkpoints kept (RS_NCK * RS_CKI > RS + RS_CKI)
 static_assert(RS % RS_CKI == 0 && (RS & (RS - 1)) == 0 && (RS_CKI & (RS_CKI - 1)) == 0,
               "RNG ring: powers of two, whole checkpoint blocks");
+#define EV_CAP    96           // events a warp queues during a commit
 #define INV_N     1024         // moduli with a reciprocal in shared memory
 #define CODE_SM   2048         // codewords mirrored in every CTA's shared memory
 #define NEG_CLUSTER_PAIRS 4096  // list x candidate pairs above which the whole cluster helps
@@ -155,6 +156,7 @@ struct Smem {
     uint64_t st_H[ULS];        // staged list chunk: candidates at distance R+1 from the entry
     uint16_t st_E[ULS];        //                    positions where the entry equals the sampled word
     uint64_t inv[INV_N + 1];   // floor((2^64-1)/m), m = 1..INV_N
+    uint64_t inv_N;            // the same of q^n
     // RNG stream: draws generated ahead of use by an idle leader warp
     uint64_t rs_buf[RS];
     unsigned long long rs_gen, rs_use;
@@ -162,7 +164,8 @@ struct Smem {
     CovRng rs_ck[RS_NCK];      // generator at draw rs_ckpos[k]
     unsigned long long rs_ckpos[RS_NCK];
     uint64_t code_sm[CODE_SM]; // leader's mirror of the packed code (M <= CODE_SM)
-    uint8_t dist8[CODE_SM];    // distances to the sampled word
+    uint64_t ev_pk[NWARP][EV_CAP];   // a move's events, a queue per warp: the word,
+    uint32_t ev_tag[NWARP][EV_CAP];  // its coverer and what to do
 };
 
 static_assert(offsetof(Smem, fy_c) == offsetof(Smem, fy_a) + 2 * PERM_CAP * sizeof(int32_t),
@@ -261,19 +264,6 @@ __device__ __forceinline__ T warp_sum(T v)
     return v;
 }
 
-// block-wide sum of an int (all threads get the result)
-__device__ int block_sum_int(Smem &S, int v)
-{
-    v = warp_sum(v);
-    cov_bar();
-    if ((threadIdx.x & 31) == 0) S.red_i[threadIdx.x >> 5] = v;
-    cov_bar();
-    int t = 0;
-    for (int w = 0; w < NWARP; w++) t += S.red_i[w];
-    cov_bar();
-    return t;
-}
-
 __device__ unsigned block_min_u32(Smem &S, unsigned v)
 {
     for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -316,6 +306,14 @@ __device__ __forceinline__ uint64_t fastmod(const Smem &S, uint64_t x, uint64_t 
         return r;
     }
     return x % m;
+}
+
+// x mod q^n by the slot's reciprocal
+__device__ __forceinline__ uint32_t mod_words(const CovSlot &d, const Smem &S, uint64_t x)
+{
+    uint64_t r = x - __umul64hi(x, S.inv_N) * (uint64_t)d.N;
+    while (r >= (uint64_t)d.N) r -= (uint64_t)d.N;
+    return (uint32_t)r;
 }
 
 // ---- RNG stream.  The draws of the reference's single xoshiro256++ stream
@@ -703,9 +701,42 @@ __device__ __forceinline__ void group_add_h(int *partH, int key, int v, const ui
 //    Y = {w_p = c_p, d(w,c) = R-1} (in); X = Y + dv.  The counts of X and Y
 //    are not changed by the move, so they are read in the same pass.
 // The change of T_i / H_i goes to the leader's accT / accH.
+// What a counter's crossing leaves to do (an event): the word joins the
+// uncovered list (EV_OPEN), leaves the uncovered bitmap (EV_SHUT), or its only
+// coverer's private counts gain or lose it (EV_ALONE, EV_SHARED).
+enum { EV_OPEN = 0, EV_ALONE = 1, EV_SHUT = 2, EV_SHARED = 3 };
+
+// The newest `cnt` (<= 32) events of the warp's queue, a lane each.
+__device__ __forceinline__ void commit_events(const CovSlot &d, const OpParams &P, const uint64_t *qpk,
+                                              const uint32_t *qtag, int end, int cnt)
+{
+    const int lane = threadIdx.x & 31;
+    if (lane < cnt) {
+        const uint64_t pk = qpk[end - 1 - lane];
+        const uint32_t tag = qtag[end - 1 - lane];
+        const int kind = (int)(tag >> 16);
+        if (kind == EV_ALONE || kind == EV_SHARED) {
+            private_adjust(d, (int)(tag & 0xffffu), pk, kind == EV_ALONE ? +1 : -1);
+        } else {
+            const uint32_t x = widx_pk(d, pk);
+            if (kind == EV_OPEN) { ul_insert(d, P.ul_valid, x, pk); zb_set(d, x); }
+            else zb_clear(d, x);
+        }
+    }
+    __syncwarp();
+}
+
 // Leaving / entering pairs of a commit (covsearch2e.c:450-493): the S'
 // patterns of R positions avoiding p, q-1 values of the last one per item.
-// Per-lane form: each private-count event goes to P on its own.
+//
+// Lane form (few private-count events): a warp's 32 items touch 64 (q-1)
+// counters and a few of them have events, rarely the same lane's twice.
+// Acting on each where it is found makes the warp walk the event code once
+// per counter with one or two lanes active -- 1,230 warp-instructions for 32
+// items at q7 n9 R4, most of them there.  The events go to a queue of the warp
+// instead and are worked 32 at a time: the move phase of one instance at q7 n9
+// R4 takes 34 us for 54 on a cluster of 8, 103 for 155 on one of 2; 64
+// instances together are bound by random DRAM sectors (3 TB/s) either way.
 __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpParams &P, Smem &S, uint32_t wid,
                                                uint32_t wstride, int &T, long long &dunc)
 {
@@ -714,47 +745,95 @@ __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpPara
     const uint32_t nit = (uint32_t)d.nsub * d.ppow[R - 1];
     const uint32_t nstep = (nit + 31) / 32 * 32;
     const int qm1 = d.q - 1;
-
-        // few private-count events per move: each lane adds its own to P
+    const uint32_t unit = cov_cw_unit(P.mi);
+    uint64_t *const qpk = S.ev_pk[threadIdx.x >> 5];
+    uint32_t *const qtag = S.ev_tag[threadIdx.x >> 5];
+    const unsigned below = (1u << lane) - 1u;
+    int qn = 0;                                    // events in the queue
+    constexpr int CH = 8;
     for (uint32_t t0 = wid * 32; t0 < nstep; t0 += wstride) {
         const uint32_t t = t0 + lane;
+        const bool live = t < nit;
         int dt = 0;
         int key = -1;
         const uint8_t *ps = subp;
-        if (t < nit) {
-            // every word of the item is distinct: all 2(q-1) counters are
-            // loaded before any is written, so the loads are in flight together
-            CovItem it = cov_item(d, subp, R, t, P.base, P.pc);
+        // every word of the item is distinct: all 2(q-1) counters are
+        // loaded before any is written, so the loads are in flight together
+        CovItem it = cov_item(d, subp, R, live ? t : 0, P.base, P.pc);
+        if (live) {
             key = (int)(t / d.ppow[R - 1]);
             ps = it.ps;
-            uint32_t oa[COV_MAXQ - 1], ob[COV_MAXQ - 1];
+        }
+        // values of the last position in chunks of CH (one chunk for q <= 9)
+        for (int kb = 0; kb < qm1; kb += CH) {
+            uint32_t oa[CH], ob[CH];
+            if (live) {
 #pragma unroll
-            for (int kk = 0; kk < COV_MAXQ - 1; kk++) {
-                if (kk < qm1) {
-                    uint32_t a; uint64_t pka;
-                    cov_item_word(d, it, kk, a, pka);
-                    oa[kk] = cov_ldcg(&d.cw[a]);
-                    ob[kk] = cov_ldcg(&d.cw[a + P.dv]);
+                for (int kc = 0; kc < CH; kc++) {
+                    if (kb + kc < qm1) {
+                        uint32_t a; uint64_t pka;
+                        cov_item_word(d, it, kb + kc, a, pka);
+                        oa[kc] = cov_ldcg(&d.cw[a]);
+                        ob[kc] = cov_ldcg(&d.cw[a + P.dv]);
+                    }
                 }
             }
+            // leaving word a loses codeword i, entering word a + dv gains it
 #pragma unroll
-            for (int kk = 0; kk < COV_MAXQ - 1; kk++) {
-                if (kk < qm1) {
-                    uint32_t a; uint64_t pka;
-                    cov_item_word(d, it, kk, a, pka);
-                    dt -= (oa[kk] & 0xffffu) == 1;
-                    dt += (ob[kk] & 0xffffu) == 0;
-                    dunc += word_dec_v(d, P.ul_valid, P.mi, a, pka, oa[kk]);
-                    dunc += word_inc_v(d, P.mi, a + P.dv, cov_setnib(pka, P.mp, P.mv), ob[kk]);
+            for (int kc = 0; kc < CH; kc++) {
+                if (kb + kc < qm1) {
+                    int evd = -1, evi = -1;
+                    uint32_t kd = 0, ki = 0;
+                    uint64_t pka = 0;
+                    if (live) {
+                        uint32_t a;
+                        cov_item_word(d, it, kb + kc, a, pka);
+                        const uint32_t o1 = oa[kc], o2 = ob[kc];
+                        const uint32_t c1 = o1 & 0xffffu, c2 = o2 & 0xffffu;
+                        dt -= c1 == 1;
+                        dt += c2 == 0;
+                        if (c1 == 0 || c2 == 0xffffu) {
+                            set_error(d, COV_EDRIFT);
+                        } else {
+                            const uint32_t n1 = o1 - unit;
+                            cov_stcg(&d.cw[a], n1);
+                            cov_stcg(&d.cw[a + P.dv], o2 + unit);
+                            if (c1 == 1) { evd = EV_OPEN; dunc += 1; }
+                            else if (c1 == 2) { evd = EV_ALONE; kd = n1 >> 16; }
+                            if (c2 == 0) { evi = d.zbits ? EV_SHUT : -1; dunc -= 1; }
+                            else if (c2 == 1) { evi = EV_SHARED; ki = o2 >> 16; }
+                        }
+                    }
+                    const unsigned md = __ballot_sync(0xffffffffu, evd >= 0), mi = __ballot_sync(0xffffffffu, evi >= 0);
+                    if (md | mi) {
+                        if (evd >= 0) {
+                            const int at = qn + __popc(md & below);
+                            qpk[at] = pka;
+                            qtag[at] = ((uint32_t)evd << 16) | kd;
+                        }
+                        if (evi >= 0) {
+                            const int at = qn + __popc(md) + __popc(mi & below);
+                            qpk[at] = cov_setnib(pka, P.mp, P.mv);
+                            qtag[at] = ((uint32_t)evi << 16) | ki;
+                        }
+                        qn += __popc(md) + __popc(mi);
+                        __syncwarp();
+                        while (qn >= 32) {               // at most 31 + 64 are ever queued
+                            commit_events(d, P, qpk, qtag, qn, 32);
+                            qn -= 32;
+                        }
+                    }
                 }
             }
         }
         T += dt;
         if (t0 < nit) group_add_h(S.partH, key, dt, ps, R, -1);
     }
+    if (qn) commit_events(d, P, qpk, qtag, qn, qn);
 }
 
-// Warp-aggregated form: events collected into the shared table.
+// Warp-aggregated form (dense coverage, where most words have an event): acted
+// on at once, the private counts collected into the shared table.
 __device__ __forceinline__ void commit_pairs_warp(const CovSlot &d, const OpParams &P, Smem &S, const PAdjTab &tab,
                                                uint32_t wid, uint32_t wstride, int &T, long long &dunc)
 {
@@ -1383,40 +1462,46 @@ __device__ long long leader_pick(const CovSlot &d, Smem &S)
     if (tid == 0) rs_ensure(S, 65);
     __syncwarp();
     cov_bar();
-    if (tid < 64) {
-        uint32_t w = (uint32_t)(rs_peek(S, tid) % (uint64_t)d.N);
-        unsigned m = __ballot_sync(0xffffffffu, cnt_of(d, w) == 0);
-        if ((tid & 31) == 0) S.hitmask[tid >> 5] = m;
-    }
-    cov_bar();
-    int first = -1;
-    if (S.hitmask[0]) first = __ffs(S.hitmask[0]) - 1;
-    else if (S.hitmask[1]) first = 32 + __ffs(S.hitmask[1]) - 1;
-    const int consumed = first >= 0 ? first + 1 : 65;
-    long long result = -1;
-    uint32_t start = 0;
-    if (first >= 0) result = (long long)(rs_peek(S, first) % (uint64_t)d.N);
-    else start = (uint32_t)(rs_peek(S, 64) % (uint64_t)d.N);
-    cov_bar();
-    if (tid == 0) S.rs_use += consumed;
-    __syncwarp();
-    if (first >= 0 || S.unc <= 0) return result;     // no zero anywhere: -1
-    // Both searches below return the first zero after start.  The list is
+    // Two searches give the first zero after a random start: the list is
     // scanned whole; the linear scan stops at the first zero, about q^n/unc
-    // words on: it is the cheaper one while that distance is short.
-    if (S.ul_valid && (unsigned long long)S.unc * 16384ull < (unsigned long long)d.N) {
+    // words on, and is the cheaper one while that distance is short.  Where
+    // zeros are so few the probes nearly always fail, so the list is scanned
+    // while they are in flight.
+    const bool list = S.unc > 0 && S.ul_valid && (unsigned long long)S.unc * 16384ull < (unsigned long long)d.N;
+    const uint32_t start = mod_words(d, S, rs_peek(S, 64));
+    bool zero = false;
+    if (tid < 64) zero = cnt_of(d, mod_words(d, S, rs_peek(S, tid))) == 0;
+    unsigned best = 0xffffffffu;
+    if (list) {
         // every zero-count word is on the list: the first one after start is
         // the entry minimising (x - start) mod N
         // a thread reads the count only for an entry that would lower its
         // running minimum (a few per thread), not for every entry
         const int n0 = S.uln;
-        unsigned best = 0xffffffffu;
         for (int e = tid; e < n0; e += NT) {
             uint32_t x = cov_ldcg(&d.ul_idx[e]);
             unsigned key = x >= start ? x - start : x + (d.N - start);
             if (key < best && (cov_ldcg(&d.cw[x]) & 0xffffu) == 0) best = key;
         }
-        best = block_min_u32(S, best);
+        best = __reduce_min_sync(0xffffffffu, best);
+    }
+    if (tid < 64) {
+        const unsigned m = __ballot_sync(0xffffffffu, zero);
+        if ((tid & 31) == 0) S.hitmask[tid >> 5] = m;
+    }
+    if ((tid & 31) == 0) S.red_u[tid >> 5] = best;
+    cov_bar();
+    int first = -1;
+    if (S.hitmask[0]) first = __ffs(S.hitmask[0]) - 1;
+    else if (S.hitmask[1]) first = 32 + __ffs(S.hitmask[1]) - 1;
+    const int consumed = first >= 0 ? first + 1 : 65;
+    const long long result = first >= 0 ? (long long)mod_words(d, S, rs_peek(S, first)) : -1;
+    for (int w = 0; w < NWARP; w++) best = min(best, S.red_u[w]);
+    cov_bar();
+    if (tid == 0) S.rs_use += consumed;
+    __syncwarp();
+    if (first >= 0 || S.unc <= 0) return result;     // no zero anywhere: -1
+    if (list) {
         if (best != 0xffffffffu) {
             // (start + best) may pass 2^32 when q^n > 2^31
             unsigned long long x = (unsigned long long)start + best;
@@ -1648,44 +1733,70 @@ __device__ void leader_plan(const CovSlot &d, Smem &S, int csize)
     if (S.status) { if (tid == 0) { S.opp.op = OP_STOP; S.phase = PH_STOPPED; } return; }
     const uint64_t pu = S.pu;
 
-    // distances to all codewords and the target distance (covsearch2e.c:1342-1351)
+    // The target distance and the ordered list of codewords at it
+    // (covsearch2e.c:1342-1376): always in global memory, the first L_SM also
+    // in shared memory with their packed codes and one-hot masks.  The word is
+    // uncovered, so no codeword is nearer than R + 1 and nearly always one is
+    // that near: a warp walks its run of consecutive codewords once, eight
+    // loads in flight, and notes those at R + 1 in order; a second walk finds
+    // the others' distance if there was none.
     const bool csm = M <= CODE_SM;
-    unsigned dm = 0xffffffffu;
-    // (with --fix0 codeword 0 is not a candidate, covsearch2e.c:1343)
-    for (int i = tid; i < M; i += NT) {
-        if (i < d.fix0) { if (csm) S.dist8[i] = 0xff; continue; }
-        int dd = cov_dist(leader_code(d, S, i), pu);
-        if (csm) S.dist8[i] = (uint8_t)dd;
-        dm = min(dm, (unsigned)dd);
-    }
-    dm = block_min_u32(S, dm);
-    if (tid == 0) { long long t1 = cov_clock(); S.prof[10] += t1 - t0; }
-    __syncwarp();
-    const int dtar = ((int)dm <= R + 1) ? R + 1 : (int)dm;
-    // ordered list of codewords at distance dtar (covsearch2e.c:1359-1376):
-    // always in global memory, the first L_SM also in shared memory with
-    // their packed codes and one-hot masks
-    int nL = 0;
-    for (int c0 = 0; c0 < M; c0 += NT) {
-        int i = c0 + tid;
-        uint64_t pk = 0;
-        int f = 0;
-        if (i < M && i >= d.fix0) {
-            pk = leader_code(d, S, i);
-            f = (csm ? (int)S.dist8[i] : cov_dist(pk, pu)) == dtar;
-        }
-        int pos;
-        int tot = block_excl_scan(S, f, pos);
-        if (f) {
-            const int at = nL + pos;
-            d.g_list[at] = (uint32_t)i;
-            if (at < L_SM) {
-                S.L[at] = (uint32_t)i;
-                S.Lpk[at] = pk;
+    uint32_t *const note = csm ? reinterpret_cast<uint32_t *>(S.fy_a) : reinterpret_cast<uint32_t *>(d.g_neg);
+    const int lane = tid & 31, warp = tid >> 5;
+    const int run = ((M + NWARP - 1) / NWARP + 31) & ~31;        // codewords of a warp
+    const int lo = min(M, warp * run), hi = min(M, lo + run);
+    int dtar = R + 1, nL = 0;
+    for (int walk = 0; walk < 2; walk++) {
+        unsigned dm = 0xffffffffu;
+        int cnt = 0;                                             // the warp's notes
+        for (int c0 = lo; c0 < hi; c0 += 256) {
+            uint64_t pk[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int i = c0 + 32 * u + lane;
+                pk[u] = i < hi ? leader_code(d, S, i) : 0;
+            }
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                if (c0 + 32 * u >= hi) break;
+                const int i = c0 + 32 * u + lane;
+                // (with --fix0 codeword 0 is not a candidate, covsearch2e.c:1343)
+                const unsigned dd = i < hi && i >= d.fix0 ? (unsigned)cov_dist(pk[u], pu) : 0xffffffffu;
+                dm = min(dm, dd);
+                const unsigned m = __ballot_sync(0xffffffffu, dd == (unsigned)dtar);
+                if (dd == (unsigned)dtar) note[lo + cnt + __popc(m & ((1u << lane) - 1))] = (uint32_t)i;
+                cnt += __popc(m);
             }
         }
-        nL += tot;
+        if (lane == 0) S.red_i[warp] = cnt;
+        dm = __reduce_min_sync(0xffffffffu, dm);
+        if (lane == 0) S.red_u[warp] = dm;
+        cov_bar();
+        int before = 0;
+        nL = 0;
+        dm = 0xffffffffu;
+        for (int w = 0; w < NWARP; w++) {
+            if (w == warp) before = nL;
+            nL += S.red_i[w];
+            dm = min(dm, S.red_u[w]);
+        }
+        if (walk == 0 && tid == 0) { long long t1 = cov_clock(); S.prof[10] += t1 - t0; }
+        if (nL) {
+            for (int k = lane; k < cnt; k += 32) {
+                const uint32_t i = note[lo + k];
+                const int at = before + k;
+                d.g_list[at] = i;
+                if (at < L_SM) {
+                    S.L[at] = i;
+                    S.Lpk[at] = leader_code(d, S, (int)i);
+                }
+            }
+            break;
+        }
+        dtar = (int)dm <= R + 1 ? R + 1 : (int)dm;
+        cov_bar();
     }
+    cov_bar();
     int Lsm = nL <= L_SM;
     uint32_t *Lp = Lsm ? S.L : d.g_list;
     // --wide (covsearch2e.c:1353-1376): while the list is valid and
@@ -2075,74 +2186,68 @@ __device__ void leader_select(const CovSlot &d, Smem &S)
         }
     }
     cov_bar();
-    // Selection (covsearch2e.c:1503-1518) in parallel.  Scanning s in order
-    // with eligible keys d_s, a "reset" is an eligible s with d_s below the
-    // running minimum and an "event" one equal to it; each event draws once
-    // and, with nties = its rank in the current minimum's run (the reset
-    // counting 1), replaces the choice when draw % nties == 0.  Only events
-    // at the final minimum V can win: the last of them whose draw hits, else
-    // the first position holding V.  With nothing eligible one draw picks a
-    // random candidate.
-    int bs_par = -2, consumed = 0;
-    if (psm) {
+    // Selection (covsearch2e.c:1503-1518) by one warp, 32 candidates at a
+    // time.  Scanning s in order with eligible keys d_s, a "reset" is an
+    // eligible s with d_s below the running minimum and an "event" one equal
+    // to it; each event draws once and, with nties = its rank in the current
+    // minimum's run (the reset counting 1), replaces the choice when
+    // draw % nties == 0.  The running minimum is a prefix scan of the lanes,
+    // so the events of 32 candidates draw at once; with nothing eligible one
+    // draw picks a random candidate.
+    int bs_par = -2;
+    if (psm && tid < 32) {
         const long long unc = S.unc, best = S.best_unc;
-        const int CH = (take + NT - 1) / NT;
-        const int s_lo = min(take, tid * CH), s_hi = min(take, s_lo + CH);
         const int INF = 0x7fffffff;
-        auto keyof = [&](int s2) -> int {
-            const int dd = dval[s2];
-            return (S.tflag[s2] && unc + dd >= best) ? INF : dd;
-        };
-        int cmin = INF;
-        for (int s2 = s_lo; s2 < s_hi; s2++) cmin = min(cmin, keyof(s2));
-        int V;
-        const int pmin = block_scan_int(S, cmin, INF, [](int a2, int b2) { return min(a2, b2); }, V);
-        // events per chunk and the event count at the chunk's last reset
-        int m = pmin, nev = 0, ev_reset = -1;
-        for (int s2 = s_lo; s2 < s_hi; s2++) {
-            const int k2 = keyof(s2);
-            if (k2 == INF) continue;
-            if (k2 < m) { m = k2; ev_reset = nev; }
-            else if (k2 == m) nev++;
-        }
-        int E;
-        const int evbase = block_scan_int(S, nev, 0, [](int a2, int b2) { return a2 + b2; }, E);
-        int dummy;
-        const int in_reset = block_scan_int(S, ev_reset >= 0 ? evbase + ev_reset : -1, -1,
-                                            [](int a2, int b2) { return b2 != -1 ? b2 : a2; }, dummy);
-        if (V != INF && E <= RS / 2) {
-            if (tid == 0) rs_ensure(S, E);
-            __syncwarp();
-            cov_bar();
-            // first occurrence of V and the last winning event at V
-            int firstV = INF, win = -1;
-            m = pmin;
-            int cur_reset = in_reset, g = evbase;
-            for (int s2 = s_lo; s2 < s_hi; s2++) {
-                const int k2 = keyof(s2);
-                if (k2 == INF) continue;
-                if (k2 < m) {
-                    m = k2;
-                    cur_reset = g;
-                    if (k2 == V) firstV = min(firstV, s2);
-                } else if (k2 == m) {
-                    const int nties = 1 + (g + 1) - cur_reset;
-                    if (k2 == V && fastmod(S, rs_peek(S, g), (uint64_t)nties) == 0) win = s2;
-                    g++;
-                }
+        const unsigned below = (1u << tid) - 1u;
+        int run = INF, nties = 0, bs = -1;
+        for (int s0 = 0; s0 < take; s0 += 32) {
+            const int s2 = s0 + tid;
+            int key = INF;
+            if (s2 < take) {
+                const int dd = dval[s2];
+                key = S.tflag[s2] && unc + dd >= best ? INF : dd;
             }
-            int fv, wv;
-            block_scan_int(S, firstV, INF, [](int a2, int b2) { return min(a2, b2); }, fv);
-            block_scan_int(S, win, -1, [](int a2, int b2) { return max(a2, b2); }, wv);
-            bs_par = wv >= 0 ? wv : fv;
-            consumed = E;
-        } else if (V == INF) {
-            if (tid == 0) { rs_ensure(S, 1); }
-            __syncwarp();
-            cov_bar();
-            bs_par = (int)fastmod(S, rs_peek(S, 0), (uint64_t)take);
-            consumed = 1;
+            int least = key;                              // up to and with this lane
+            for (int o = 1; o < 32; o <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, least, o);
+                if (tid >= o) least = min(least, y);
+            }
+            int least_b = __shfl_up_sync(0xffffffffu, least, 1);
+            least_b = min(run, tid ? least_b : INF);      // before this lane
+            const unsigned rst = __ballot_sync(0xffffffffu, key < least_b);
+            const unsigned ev = __ballot_sync(0xffffffffu, key == least_b && key != INF);
+            unsigned hits = 0;
+            if (ev) {
+                if (tid == 0) rs_ensure(S, __popc(ev));
+                __syncwarp();
+                bool hit = false;
+                if ((ev >> tid) & 1u) {
+                    const unsigned rb = rst & below;
+                    const unsigned since = rb ? ~((2u << (31 - __clz((int)rb))) - 1u) : ~0u;   // lanes after the last reset
+                    const int rank = (rb ? 1 : nties) + __popc(ev & since & below) + 1;
+                    hit = fastmod(S, rs_peek(S, __popc(ev & below)), (uint64_t)rank) == 0;
+                }
+                hits = __ballot_sync(0xffffffffu, hit);
+                if (tid == 0) S.rs_use += (unsigned long long)__popc(ev);
+                __syncwarp();
+            }
+            unsigned at_run = ev;                         // events at the minimum the 32 end with
+            if (rst) {
+                const int lr = 31 - __clz((int)rst);
+                run = __shfl_sync(0xffffffffu, key, lr);
+                bs = s0 + lr;
+                nties = 1;
+                at_run &= ~((2u << lr) - 1u);
+            }
+            nties += __popc(at_run);
+            hits &= at_run;
+            if (hits) bs = s0 + 31 - __clz((int)hits);
         }
+        if (bs < 0) {
+            if (tid == 0) bs = (int)fastmod(S, rs_take(S), (uint64_t)take);
+            bs = __shfl_sync(0xffffffffu, bs, 0);
+        }
+        bs_par = bs;
     }
     if (tid == 0) {
         long long ts1 = cov_clock();
@@ -2150,25 +2255,19 @@ __device__ void leader_select(const CovSlot &d, Smem &S)
         int bs = -1;
         if (bs_par >= 0) {
             bs = bs_par;
-            S.rs_use += consumed;
         } else {
             long long bestd = 1LL << 60;
             int nties = 0;
             for (int s = 0; s < take; s++) {
-                long long dd;
-                int tb;
-                if (psm) { dd = dval[s]; tb = S.tflag[s]; }
-                else {
-                    uint32_t c = perm[s];
-                    int l = (int)(c / (uint32_t)cpw), rr = (int)(c - (uint32_t)l * cpw);
-                    int k = (int)Lp[l];
-                    uint64_t pk = cov_ldcg(&d.code[k]);
-                    int p, v;
-                    cand_pv(d, wide, rr, pk, pu, p, v);
-                    const int32_t *Pk = d.P + (size_t)k * (n + 1);
-                    dd = (cov_ldcg(&Pk[0]) - cov_ldcg(&Pk[1 + p])) - cand_neg(d, wide, negp, l, p, v);
-                    tb = (long long)cov_ldcg(&d.tabu[((size_t)k * n + p) * q + v]) > S.it;
-                }
+                uint32_t c = perm[s];
+                int l = (int)(c / (uint32_t)cpw), rr = (int)(c - (uint32_t)l * cpw);
+                int k = (int)Lp[l];
+                uint64_t pk = cov_ldcg(&d.code[k]);
+                int p, v;
+                cand_pv(d, wide, rr, pk, pu, p, v);
+                const int32_t *Pk = d.P + (size_t)k * (n + 1);
+                const long long dd = (cov_ldcg(&Pk[0]) - cov_ldcg(&Pk[1 + p])) - cand_neg(d, wide, negp, l, p, v);
+                const int tb = (long long)cov_ldcg(&d.tabu[((size_t)k * n + p) * q + v]) > S.it;
                 if (tb && S.unc + dd >= S.best_unc) continue;
                 if (dd < bestd) { bestd = dd; bs = s; nties = 1; }
                 else if (dd == bestd) {
@@ -2183,11 +2282,16 @@ __device__ void leader_select(const CovSlot &d, Smem &S)
         uint32_t c = perm[bs];
         int l = (int)(c / (uint32_t)cpw), rr = (int)(c - (uint32_t)l * cpw);
         int k = (int)Lp[l];
-        uint64_t pk = cov_ldcg(&d.code[k]);
+        uint64_t pk = Lsm ? S.Lpk[l] : cov_ldcg(&d.code[k]);
         int p, v;
         cand_pv(d, wide, rr, pk, pu, p, v);
-        const int32_t *Pk = d.P + (size_t)k * (n + 1);
-        long long dd = (cov_ldcg(&Pk[0]) - cov_ldcg(&Pk[1 + p])) - cand_neg(d, wide, negp, l, p, v);
+        long long dd;
+        if (psm) {
+            dd = dval[bs];
+        } else {
+            const int32_t *Pk = d.P + (size_t)k * (n + 1);
+            dd = (cov_ldcg(&Pk[0]) - cov_ldcg(&Pk[1 + p])) - cand_neg(d, wide, negp, l, p, v);
+        }
         issue_move(d, S, k, pk, p, v, dd);
         S.phase = PH_FINISH_MOVE;
         S.prof[3] += cov_clock() - t0;
@@ -2204,7 +2308,14 @@ __device__ void write_trace(const CovSlot &d, Smem &S)
 
 __device__ void copy_best(const CovSlot &d)
 {
-    for (int i = threadIdx.x; i < d.M; i += NT) cov_stcg(&d.best[i], cov_ldcg(&d.code[i]));
+    for (int i0 = threadIdx.x; i0 < d.M; i0 += 8 * NT) {      // eight loads in flight
+        uint64_t v[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) v[u] = i0 + u * NT < d.M ? cov_ldcg(&d.code[i0 + u * NT]) : 0;
+#pragma unroll
+        for (int u = 0; u < 8; u++)
+            if (i0 + u * NT < d.M) cov_stcg(&d.best[i0 + u * NT], v[u]);
+    }
 }
 
 // after OP_MOVE: covsearch2e.c:1525-1553
@@ -2213,6 +2324,10 @@ __device__ void leader_finish_move(const CovSlot &d, Smem &S)
     const int tid = threadIdx.x;
     const int n = d.n, q = d.q;
     const long long t0 = cov_clock();
+    if (tid >= 32 && tid <= 32 + n) {
+        int32_t *Pk = d.P + (size_t)S.opp.mi * (n + 1) + (tid - 32);
+        cov_stcg(Pk, cov_ldcg(Pk) + (tid == 32 ? S.acc.accT : S.acc.accH[tid - 33]));
+    }
     if (tid == 0) {
         long long dunc = (long long)S.acc.dunc;
         S.unc += dunc;
@@ -2220,9 +2335,6 @@ __device__ void leader_finish_move(const CovSlot &d, Smem &S)
         else if (dunc != S.chosen_delta) S.status = COV_EDRIFT;
         const OpParams &o = S.opp;
         leader_set_code(d, S, o.mi, o.pcn);
-        int32_t *Pk = d.P + (size_t)o.mi * (n + 1);
-        cov_stcg(&Pk[0], cov_ldcg(&Pk[0]) + S.acc.accT);
-        for (int j = 0; j < n; j++) cov_stcg(&Pk[1 + j], cov_ldcg(&Pk[1 + j]) + S.acc.accH[j]);
         const int oldv = S.ibc[3];
         uint64_t r4 = rs_take(S) % 4ull;
         cov_stcg(&d.tabu[((size_t)o.mi * n + o.mp) * q + oldv], (int32_t)(S.it + d.tenure + (long long)r4));
@@ -2518,6 +2630,7 @@ cov_run_kernel(const CovSlot *__restrict__ slots, const int *__restrict__ cluste
     if (leader)
         for (int m = threadIdx.x; m <= INV_N; m += NT)
             S.inv[m] = m ? 0xffffffffffffffffull / (uint64_t)m : 0;
+    if (leader && threadIdx.x == 0) S.inv_N = 0xffffffffffffffffull / (uint64_t)d.N;
     if (d.M <= CODE_SM)
         for (int i = threadIdx.x; i < d.M; i += NT) S.code_sm[i] = cov_ldcg(&d.code[i]);
     if (leader && threadIdx.x == 0) {
