@@ -2921,6 +2921,30 @@ __global__ void k_unique_cover(CovSlot d, int count, int *out)
     __syncwarp();
 }
 
+// A built slot is ready to run: its descriptor, its state (z: the build's
+// counts of uncovered and of listed words) and the best code so far.
+__global__ void k_slot_ready(CovSlot d, CovSlot *slot, CovRng rng, const unsigned long long *z)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < d.M; i += gridDim.x * blockDim.x) d.best[i] = d.code[i];
+    if (blockIdx.x || threadIdx.x) return;
+    *slot = d;
+    CovSlotState st;
+    memset(&st, 0, sizeof st);
+    for (int k = 0; k < 4; k++) st.rng[k] = rng.s[k];
+    st.unc = (long long)z[0];
+    st.best_unc = st.unc;
+    st.target = -1;
+    st.it_limit = -1;
+    st.sa_T = d.sa_t0;                   // --sa starts at --t0 (covsearch2e.c:1035)
+    // the list is in use from the first move when the uncovered words are at
+    // most half its capacity -- when the reference's first iteration would
+    // rebuild it (covsearch2e.c:1326-1329)
+    st.ul_valid = z[0] <= (unsigned long long)d.ul_cap / 2 && z[1] == z[0];
+    st.ul_n = st.ul_valid ? (int)z[0] : 0;
+    st.finished = st.unc == 0;
+    *d.st = st;
+}
+
 // per-launch budget of every listed slot, set on the device so that a run
 // needs no host round trip (and can be captured in a graph)
 __global__ void k_set_budget(CovSlotState *states, const int *map, int nslots, long long moves,
@@ -2998,6 +3022,7 @@ struct HostSlot {
     size_t arena_bytes = 0;
     int cluster = 1;
     int cap = 0;                 // codewords the storage holds
+    unsigned long long *d_z = nullptr;   // the state build's counts: uncovered words, listed words
     cov_params prm{};
 };
 
@@ -3310,6 +3335,10 @@ static size_t tabu_bytes(int q, int n, int M)
     return std::max((size_t)M * n * q * 4, (size_t)M * BT_REC_BYTES);
 }
 
+// entries of the uncovered list: its capacity is the reference's, but a word
+// is listed at most once (its membership bit), so there are at most q^n
+static long long ul_entries(long long N) { return std::min<long long>(UL_CAP_DEFAULT, N); }
+
 size_t cov_slot_bytes(const cov_params *prm)
 {
     if (!prm) return 0;
@@ -3322,10 +3351,11 @@ size_t cov_slot_bytes(const cov_params *prm)
     add((size_t)M * 8 * 2);                          // code, best
     add(tabu_bytes(q, n, M));                        // tabu
     add((size_t)M * (n + 1) * 4);                    // P
-    add((size_t)UL_CAP_DEFAULT * 4);                 // ul_idx
-    add((size_t)UL_CAP_DEFAULT * 8);                 // ul_pk
+    add((size_t)ul_entries(N) * 4);                  // ul_idx
+    add((size_t)ul_entries(N) * 8);                  // ul_pk
     add((size_t)((N + 31) / 32) * 4);                // ul_bit
     add((size_t)((N + 31) / 32) * 4);                // zb
+    add(16);                                         // build counters
     const size_t ce = (size_t)M * n * (prm->wide ? (size_t)(q - 1) : 1u);
     add(ce * 4 * 2 + (size_t)M * n * 4 + (size_t)M * 4);   // g_perm, g_dval, g_neg, g_list
     if (prm->wide) add((size_t)M * n * q * 4);      // g_negw
@@ -3421,20 +3451,25 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     d.code = (uint64_t *)take_((size_t)Mw * 8);
     d.best = (uint64_t *)take_((size_t)Mw * 8);
     d.tabu = (int32_t *)take_(tabu_bytes(q, n, Mw));
+    d.ul_idx = (uint32_t *)take_((size_t)ul_entries(N) * 4);
+    d.ul_pk = (uint64_t *)take_((size_t)ul_entries(N) * 8);
+    // what a state build starts from zero, in a row (slot_zero)
     d.P = (int32_t *)take_((size_t)Mw * (n + 1) * 4);
-    d.ul_idx = (uint32_t *)take_((size_t)d.ul_cap * 4);
-    d.ul_pk = (uint64_t *)take_((size_t)d.ul_cap * 8);
     d.ul_bit = (uint32_t *)take_((size_t)((N + 31) / 32) * 4);
     d.zb = (uint32_t *)take_((size_t)((N + 31) / 32) * 4);
+    h.d_z = (unsigned long long *)take_(16);
     const size_t ce = (size_t)Mw * n * (prm->wide ? (size_t)(q - 1) : 1u);
     d.g_perm = (uint32_t *)take_(ce * 4);
     d.g_dval = (int32_t *)take_(ce * 4);
     d.g_neg = (int32_t *)take_((size_t)Mw * n * 4);
     d.g_list = (uint32_t *)take_((size_t)Mw * 4);
     d.g_negw = prm->wide ? (int32_t *)take_((size_t)Mw * n * q * 4) : nullptr;
-    uint8_t *dsub = (uint8_t *)take_(subs.size());
-    uint8_t *dball = (uint8_t *)take_(balls.size());
-    uint8_t *dsub1 = (uint8_t *)take_(subs1.size());
+    // the subset tables: one copy
+    std::vector<uint8_t> tables(subs);
+    tables.insert(tables.end(), balls.begin(), balls.end());
+    tables.insert(tables.end(), subs1.begin(), subs1.end());
+    uint8_t *dsub = (uint8_t *)take_(tables.size());
+    uint8_t *dball = dsub + subs.size(), *dsub1 = dball + balls.size();
     d.sub = dsub; d.ball_sub = dball; d.sub1 = dsub1;
     bt_geom(q, n, R, Mw, &d.bt_nh, &d.bt_nl);
     d.bt_tw = (uint32_t)ipow_h(q, d.bt_nl);
@@ -3447,10 +3482,8 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     h.st = d.st;
     h.used = true;
     cudaStream_t st = pool->cur_stream();
-    cudaError_t e = cudaMemcpyAsync(dsub, subs.data(), subs.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dball, balls.data(), balls.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dsub1, subs1.data(), subs1.size(), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    // (pageable memory: staged when the call returns)
+    cudaError_t e = cudaMemcpyAsync(dsub, tables.data(), tables.size(), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) { cudaFree(arena); return -(100 + (int)e); }
     pool->slots[s] = h;
     pool->all_dirty = true;
@@ -3476,9 +3509,16 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
         if (rc) return rc;
     }
     const bool incremental = m > M || (m < M && !random_init);   // repair or greedy
-    if (incremental) CK(cudaMemsetAsync(d.cw, 0, (size_t)N * 4, st));
-    CK(cudaMemsetAsync(d.P, 0, (size_t)M * (n + 1) * 4, st));
-    CK(cudaMemsetAsync(d.ul_bit, 0, (size_t)((N + 31) / 32) * 4, st));
+    // P, ul_bit, zb and the build's counters, one after another in the arena
+    auto slot_zero = [&]() -> int {
+        CK(cudaMemsetAsync(d.P, 0, (size_t)((char *)(h.d_z + 2) - (char *)d.P), st));
+        return 0;
+    };
+    if (incremental) {
+        CK(cudaMemsetAsync(d.cw, 0, (size_t)N * 4, st));
+        int rc = slot_zero();
+        if (rc) return rc;
+    }
     CovSlotState hs;
     memset(&hs, 0, sizeof hs);
     CovRng rng;
@@ -3522,7 +3562,7 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
         for (int i = 0; i < M; i++) pk[i] = cur[i];
         have = M;
     }
-    unsigned long long *d_z = (unsigned long long *)d.g_dval;
+    unsigned long long *const d_z = h.d_z;
     if (have < M && !random_init) {
         // greedy placement runs on the device (it samples uncovered words)
         CK(cudaMemcpyAsync(d.code, pk.data(), (size_t)M * 8, cudaMemcpyHostToDevice, st));
@@ -3581,10 +3621,10 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
     }
     // coverage array, uncovered count, uncovered-word list and private
     // counts of the final M codewords, built tile by tile; then the best code
-    CK(cudaMemsetAsync(d_z, 0, 16, st));
-    CK(cudaMemsetAsync(d.P, 0, (size_t)M * (n + 1) * 4, st));
-    CK(cudaMemsetAsync(d.ul_bit, 0, (size_t)((N + 31) / 32) * 4, st));
-    CK(cudaMemsetAsync(d.zb, 0, (size_t)((N + 31) / 32) * 4, st));
+    {
+        int rc = slot_zero();
+        if (rc) return rc;
+    }
     const BtCode rec = bt_records(d.code, M, q, n, d.bt_nh, d.bt_nl, d.tabu, st);
     CK(cudaGetLastError());
     const unsigned bs_grid = (unsigned)ipow_h(q, d.bt_nh);
@@ -3597,27 +3637,10 @@ static int slot_init(cov_pool *pool, int s, uint64_t seed, const uint8_t *code, 
     }
     CK(cudaGetLastError());
     CK(cudaMemsetAsync(d.tabu, 0, (size_t)M * n * q * 4, st));
-    CK(cudaMemcpyAsync(d.best, d.code, (size_t)M * 8, cudaMemcpyDeviceToDevice, st));
-    unsigned long long zl[2] = {0, 0};
-    CK(cudaMemcpyAsync(zl, d_z, 16, cudaMemcpyDeviceToHost, st));
-    CK(cudaStreamSynchronize(st));
-    const unsigned long long z = zl[0];
-    memset(&hs, 0, sizeof hs);
-    for (int k = 0; k < 4; k++) hs.rng[k] = rng.s[k];
-    hs.unc = (long long)z;
-    hs.best_unc = hs.unc;
-    hs.target = -1;
-    hs.it_limit = -1;
-    hs.sa_T = d.sa_t0;                   // --sa starts at --t0 (covsearch2e.c:1035)
-    // the list is in use from the first move when the uncovered words are at
-    // most half its capacity -- when the reference's first iteration would
-    // rebuild it (covsearch2e.c:1326-1329)
-    hs.ul_valid = z <= (unsigned long long)d.ul_cap / 2 && zl[1] == z;
-    hs.ul_n = hs.ul_valid ? (int)z : 0;
-    hs.finished = hs.unc == 0;
-    CK(cudaMemcpyAsync(d.st, &hs, sizeof hs, cudaMemcpyHostToDevice, st));
-    int rc = push_slot(pool, s);
-    if (rc) return rc;
+    // the descriptor, the state and the best code, on the device: no counts
+    // come back, so the host waits once, for the whole initialisation
+    k_slot_ready<<<(unsigned)std::min(64, (M + 255) / 256), 256, 0, st>>>(d, pool->d_slots + s, rng, d_z);
+    CK(cudaGetLastError());
     CK(cudaStreamSynchronize(st));
     return COV_OK;
 }

@@ -15,6 +15,7 @@
 //     codeword's ball (covsearch2e.c:353-380, 958-967), with 32-bit atomics
 //     on packed uint16 pairs.
 #include <cmath>
+#include <mutex>
 #include <cstdio>
 #include <cstring>
 #include <vector>
@@ -790,6 +791,43 @@ int geom(int q, int n, DtGeom &g)
     return 0;
 }
 
+// Scratch of the verification calls: stream-ordered allocations from a memory
+// pool of the library's own, per device, that keeps at most SCRATCH_KEEP bytes
+// between calls (more goes back at the next synchronisation).  The default
+// pool gives everything back at each, and a call that maps memory anew takes
+// 100 to 200 us longer; so did a cudaMalloc and cudaFree for each buffer
+// (6^6: 213 us for a transform of 11).
+#define SCRATCH_KEEP (16ull << 20)
+
+int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
+{
+    static cudaMemPool_t pools[COV_MAX_DEVICES];
+    static std::mutex m;
+    int dev = 0;
+    CK(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= COV_MAX_DEVICES) return COV_ENODEV;
+    {
+        std::lock_guard<std::mutex> hold(m);
+        if (!pools[dev]) {
+            cudaMemPoolProps props;
+            memset(&props, 0, sizeof props);
+            props.allocType = cudaMemAllocationTypePinned;
+            props.location.type = cudaMemLocationTypeDevice;
+            props.location.id = dev;
+            cudaMemPool_t pool = nullptr;
+            CK(cudaMemPoolCreate(&pool, &props));
+            unsigned long long keep = SCRATCH_KEEP;
+            CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+            pools[dev] = pool;
+        }
+    }
+    if (cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pools[dev], st) != cudaSuccess) {
+        cudaGetLastError();
+        return COV_ENOMEM;
+    }
+    return 0;
+}
+
 CovDeviceFlags g_dt_attr;   // shared-memory opt-in of the transform kernels, per device
 CovDeviceFlags g_ct_attr;   // the same for the tile count
 
@@ -984,7 +1022,8 @@ int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M, uint
     cudaStream_t st = (cudaStream_t)stream;
     const DtPlan plan = dt_plan(g, M);
     void *scratch = nullptr;
-    CK(cudaMallocAsync(&scratch, plan.scratch, st));
+    rc = scratch_alloc(&scratch, plan.scratch, st);
+    if (rc) return rc;
     rc = dt_run(g, plan, d_code, M, d_dist, nullptr, scratch, st);
     cudaFreeAsync(scratch, st);
     return rc;
@@ -1046,7 +1085,8 @@ int64_t cov_count_above_dev(int32_t q, int32_t n, const uint8_t *d_dist, int32_t
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
     unsigned long long *d_c = nullptr, h = 0;
-    CK(cudaMallocAsync(&d_c, 8, st));
+    rc = scratch_alloc((void **)&d_c, 8, st);
+    if (rc) return rc;
     CK(cudaMemsetAsync(d_c, 0, 8, st));
     k_count_above<<<std::max(1, cov_sm_count()) * 8, 256, 0, st>>>(d_dist, g.N, R, d_c);
     CK(cudaGetLastError());
@@ -1067,28 +1107,24 @@ int cov_mindist(int32_t q, int32_t n, const uint8_t *code, int32_t M, uint8_t *d
     cudaStream_t st = nullptr;
     const DtPlan plan = dt_plan(g, M);
     const bool want_D = dist || !plan.tiles;      // the sweeps work in D; the tiles need none for the histogram
-    uint8_t *d_code = nullptr, *d_D = nullptr;
-    void *d_s = nullptr;
-    unsigned long long *d_h = nullptr;
-    const size_t cb = (size_t)std::max(M, 1) * n;
-    if (cudaMalloc(&d_code, cb) != cudaSuccess || (want_D && cudaMalloc(&d_D, g.N) != cudaSuccess) ||
-        cudaMalloc(&d_s, plan.scratch) != cudaSuccess || cudaMalloc(&d_h, 8 * (COV_MAXN + 2)) != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(d_code); cudaFree(d_D); cudaFree(d_s); cudaFree(d_h);
-        return COV_ENOMEM;
-    }
-    auto done = [&](int r) { cudaFree(d_code); cudaFree(d_D); cudaFree(d_s); cudaFree(d_h); return r; };
-    if (M > 0 && cudaMemcpy(d_code, code, (size_t)M * n, cudaMemcpyHostToDevice) != cudaSuccess) return done(-100);
-    if (cudaMemset(d_h, 0, 8 * (COV_MAXN + 2)) != cudaSuccess) return done(-100);
-    rc = dt_run(g, plan, d_code, M, d_D, d_h, d_s, st);
+    // one allocation: the histogram, the transform's scratch, the code, D
+    auto up = [](size_t x) { return (x + 255) / 256 * 256; };
+    const size_t hb = up(8 * (COV_MAXN + 2)), sb = up(plan.scratch), cb = up((size_t)std::max(M, 1) * n);
+    uint8_t *buf = nullptr;
+    rc = scratch_alloc((void **)&buf, hb + sb + cb + (want_D ? (size_t)g.N : 0), st);
+    if (rc) return rc;
+    unsigned long long *d_h = (unsigned long long *)buf;
+    uint8_t *d_code = buf + hb + sb, *d_D = want_D ? d_code + cb : nullptr;
+    auto done = [&](int r) { cudaFreeAsync(buf, st); return r; };
+    if (M > 0 && cudaMemcpyAsync(d_code, code, (size_t)M * n, cudaMemcpyHostToDevice, st) != cudaSuccess) return done(-100);
+    if (cudaMemsetAsync(d_h, 0, 8 * (COV_MAXN + 2), st) != cudaSuccess) return done(-100);
+    rc = dt_run(g, plan, d_code, M, d_D, d_h, buf + hb, st);
     if (rc) return done(rc);
     unsigned long long hh[COV_MAXN + 2];
-    cudaError_t e = cudaMemcpy(hh, d_h, 8 * (COV_MAXN + 2), cudaMemcpyDeviceToHost);
+    cudaError_t e = cudaMemcpyAsync(hh, d_h, 8 * (COV_MAXN + 2), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess && dist) e = cudaMemcpyAsync(dist, d_D, g.N, cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return done(-(100 + (int)e));
-    if (dist) {
-        e = cudaMemcpy(dist, d_D, g.N, cudaMemcpyDeviceToHost);
-        if (e != cudaSuccess) return done(-(100 + (int)e));
-    }
     int rad = 0;
     for (int v = 0; v <= n + 1; v++) {
         if (hist) hist[v] = (int64_t)hh[v];
@@ -1123,7 +1159,8 @@ int cov_count_dev(int32_t q, int32_t n, int32_t R, const uint8_t *d_code, int32_
     if (rc) return rc;
     const CountGeom g = count_geom(q, n, R, M);
     void *tmp = nullptr;
-    CK(cudaMallocAsync(&tmp, (size_t)std::max(M, 1) * BT_REC_BYTES, st));
+    rc = scratch_alloc(&tmp, (size_t)std::max(M, 1) * BT_REC_BYTES, st);
+    if (rc) return rc;
     uint2 *mid = (uint2 *)tmp;
     uint32_t *hi = (uint32_t *)(mid + M);
     if (M > 0) {
