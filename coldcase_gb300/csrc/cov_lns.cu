@@ -52,6 +52,9 @@ namespace cg = cooperative_groups;
 #define GREEDY_NT 512
 #define GREEDY_MAXG 512             // most CTAs of the greedy kernel (one per SM)
 #define THR_BINS 1024               // histogram bins behind an extraction threshold
+#define MAP_PS_WORD 20.0            // time of a map by transform, ps a word of the space
+#define MAP_PS_LAUNCH 20e6
+#define NOTE_CAP (1 << 16)          // most words whose balls a refresh counts by tiles
 #define EXT_CHUNK 8192              // words of one block of an ordered extraction
 
 #define CK(x) do { cudaError_t e_ = (x); if (e_ != cudaSuccess) { \
@@ -72,6 +75,7 @@ struct RefreshInfo {
     int top;                     // maximum of the map
     int thr;                     // candidates are the words with map >= thr
     uint32_t found;              // how many there are (saturated)
+    uint32_t noted;              // words that k_lns_note wrote
 };
 enum { SEQ_DONE = 0, SEQ_REFRESH = 1, SEQ_COVERED = 2, SEQ_TARGET = 3, SEQ_GUARD = 5 };
 
@@ -94,6 +98,8 @@ struct cov_lns {
     int nb = 0;                     // digits of a mask block: the most with q^nb <= 64
     uint32_t blk = 1;               // its q^nb words
     uint64_t *um = nullptr;         // uncovered words of every block (built by each greedy call)
+    uint64_t *um_map = nullptr;     // the masks of the greedy's last map
+    uint32_t *note = nullptr;       // [NOTE_CAP] words, then their tile records
     uint64_t *pball = nullptr;      // ball groups on the n - nb high digits
     uint8_t *pball_last = nullptr;
     uint32_t npgroups = 0;
@@ -441,6 +447,33 @@ __global__ void __launch_bounds__(LNS_NT) k_lns_masks(const uint16_t *__restrict
         for (int y = 0; y < blk; y++) m |= (uint64_t)z[threadIdx.x * blk + y] << y;
         um[p0 + threadIdx.x] = m;
     }
+}
+
+// The words of um (all), or those that um_map has and um has not, into note in
+// any order; um_map becomes um.  all < 0: none are noted.
+__global__ void __launch_bounds__(LNS_NT) k_lns_note(const uint64_t *__restrict__ um, uint64_t *um_map, uint32_t nblk,
+                                                     uint32_t blk, int all, uint32_t *note, uint32_t *noted)
+{
+    const uint32_t p = blockIdx.x * LNS_NT + threadIdx.x;
+    uint64_t m = 0;
+    if (p < nblk) {
+        const uint64_t u = um[p];
+        m = all > 0 ? u : all == 0 ? um_map[p] & ~u : 0;
+        um_map[p] = u;
+    }
+    const uint32_t c = (uint32_t)__popcll(m);
+    uint32_t at = c;
+    const int lane = threadIdx.x & 31;
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, at, o);
+        if (lane >= o) at += y;
+    }
+    const uint32_t sum = __shfl_sync(0xffffffffu, at, 31);
+    uint32_t base = 0;
+    if (sum && lane == 0) base = atomicAdd(noted, sum);
+    at += __shfl_sync(0xffffffffu, base, 0) - c;
+    for (; m; m &= m - 1, at++)
+        if (at < NOTE_CAP) note[at] = p * blk + (uint32_t)(__ffsll((long long)m) - 1);
 }
 
 // R = 0: the map is the marked words themselves
@@ -983,6 +1016,42 @@ int lns_map_of_masks(cov_lns *h)
     return 0;
 }
 
+// Estimate of counting the balls of m words by the verifier's tiles, in ps a
+// word of the space: 1.6 + 0.9 a mark + 0.6 a codeword per word of a tile.
+double tiles_ps(const cov_lns *h, long long m)
+{
+    int nh, nl;
+    bt_geom(h->q, h->n, h->R, (int)std::min<long long>(m, 1 << 30), &nh, &nl);
+    double v = 1, c = 1;
+    const int np = h->n - bt_block_digits(h->n);
+    for (int r = 0; r < std::min(h->R, np); r++) { c = c * (np - r) / (r + 1) * (h->q - 1); v += c; }
+    return 1.6 + 0.9 * (double)m * v / h->N + 0.6 * (double)m / (double)bt_ipow(h->q, nl);
+}
+
+// The greedy's map of the uncovered words (masks um, `left` of them).  Few
+// uncovered words are counted by tiles from their list; few words covered
+// since the last map (`gone` of them; < 0: there is no last map) are counted
+// off it; else the transform of the masks, some 22 ps a word and one launch
+// less (spaces below a million words gain nothing: 17 to 90 ms fills of 6^6 to
+// 7^7 with and without).  Map at 7^9: 0.92 ms by transform, 0.07 to 0.25 by
+// tiles of 10 to 3000 words.  Six rounds at 7^9 48 -> 29 ms, the fill of 6^9
+// 71 -> 65.
+int lns_greedy_map(cov_lns *h, long long left, long long gone)
+{
+    const double all_ps = left <= NOTE_CAP ? tiles_ps(h, left) + 0.6 : 1e300;
+    const double off_ps = gone >= 0 && gone <= NOTE_CAP ? tiles_ps(h, gone) + 1.2 : 1e300;
+    if (h->R == 0 || MAP_PS_WORD * h->N <= MAP_PS_LAUNCH) return lns_map_of_masks(h);
+    const bool tiles = (MAP_PS_WORD - std::min(all_ps, off_ps)) * h->N > MAP_PS_LAUNCH;
+    const int how = !tiles ? -1 : all_ps <= off_ps ? 1 : 0;
+    const uint32_t nblk = h->N / h->blk;
+    CK(cudaMemsetAsync(&h->info->noted, 0, 4));
+    k_lns_note<<<(nblk + LNS_NT - 1) / LNS_NT, LNS_NT>>>(h->um, h->um_map, nblk, h->blk, how, h->note, &h->info->noted);
+    CK(cudaGetLastError());
+    if (how < 0) return lns_map_of_masks(h);
+    return cov_count_words_map(h->q, h->n, h->R, h->note, (int)(how ? left : gone), h->map, !how,
+                               (uint2 *)(h->note + NOTE_CAP), nullptr);
+}
+
 int lns_scratch(cov_lns *h, size_t bytes)
 {
     if (bytes <= h->scratch_bytes) return 0;
@@ -1115,6 +1184,8 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
               cudaMalloc(&h->cand, (size_t)CAND_CAP * 4) == cudaSuccess &&
               cudaMalloc(&h->bound, (size_t)CAND_CAP * 4) == cudaSuccess &&
               cudaMalloc(&h->um, (size_t)(N / h->blk) * 8) == cudaSuccess &&
+              cudaMalloc(&h->um_map, (size_t)(N / h->blk) * 8) == cudaSuccess &&
+              cudaMalloc(&h->note, (size_t)NOTE_CAP * (4 + BT_REC_BYTES)) == cudaSuccess &&
               cudaMalloc(&h->pball, pitems.size() * 8) == cudaSuccess &&
               cudaMalloc(&h->pball_last, plast.size()) == cudaSuccess &&
               cudaMalloc(&h->lowball, low.size() * 8) == cudaSuccess &&
@@ -1149,7 +1220,7 @@ int cov_lns_destroy(cov_lns *h)
     cudaDeviceSynchronize();
     cudaFree(h->cnt); cudaFree(h->map); cudaFree(h->ball); cudaFree(h->ball_last); cudaFree(h->d_red);
     cudaFree(h->cand); cudaFree(h->bound); cudaFree(h->list); cudaFree(h->flag); cudaFree(h->seq);
-    cudaFree(h->um); cudaFree(h->pball); cudaFree(h->pball_last); cudaFree(h->lowball); cudaFree(h->nom);
+    cudaFree(h->um); cudaFree(h->um_map); cudaFree(h->note); cudaFree(h->pball); cudaFree(h->pball_last); cudaFree(h->lowball); cudaFree(h->nom);
     cudaFree(h->acc); cudaFree(h->info); cudaFree(h->map_scratch); cudaFree(h->map_whole);
     cudaFree(h->scratch);
     delete h;
@@ -1160,15 +1231,9 @@ int cov_lns_recount(cov_lns *h, const uint32_t *idx, int32_t m)
 {
     if (!h || m < 0 || (m > 0 && !idx)) return COV_EINVAL;
     for (int i = 0; i < m; i++) if (idx[i] >= h->N) return COV_EINVAL;
-    // The verifier's tiles while the code is sparse, else the transform of its
-    // word counts; in ps a word: the tiles 1.6 + 0.9 a mark + 0.6 a codeword
-    // per word of a tile, the transform about 12.
-    int nh, nl;
-    bt_geom(h->q, h->n, h->R, m, &nh, &nl);
-    double v = 1, c = 1;
-    const int np = h->n - bt_block_digits(h->n);
-    for (int r = 0; r < std::min(h->R, np); r++) { c = c * (np - r) / (r + 1) * (h->q - 1); v += c; }
-    if (1.6 + 0.9 * m * v / h->N + 0.6 * m / (double)bt_ipow(h->q, nl) < 12.0) {
+    // the verifier's tiles while the code is sparse, else the transform of its
+    // word counts (about 12 ps a word)
+    if (tiles_ps(h, m) < 12.0) {
         int rc = lns_scratch(h, (size_t)m * (4 + BT_REC_BYTES) + 8);
         if (rc) return rc;
         uint2 *rec = (uint2 *)h->scratch;
@@ -1385,7 +1450,7 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
     // 444, 475; 4^11 45, 48, 70.
     a.eval_cap = (int)std::max<long long>(64, std::min<long long>(1024, (long long)h->N / 131072));
     int total = 0, vmax = 0;
-    long long refreshes = 0, evals = 0;
+    long long refreshes = 0, evals = 0, mapped = -1;         // mapped: the words of the last map
     // every refresh that finds a positive gain places at least one word (the
     // first placement of a launch needs no exact count: all bounds are fresh)
     for (int guard = 0; total < room && st.uncov > 0 && guard <= 2 * room + 2; guard++) {
@@ -1395,10 +1460,11 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
         // maximum has more than cand_cap words, the same gain and a higher
         // position): a candidate is placed only while its exact gain is at
         // least the threshold, so it is always a best placement.
-        rc = lns_map_of_masks(h);
+        rc = lns_greedy_map(h, st.uncov, mapped < 0 ? -1 : mapped - st.uncov);
         if (rc) return rc;
+        mapped = st.uncov;
         refreshes++;
-        CK(cudaMemsetAsync(h->info, 0x80, sizeof(RefreshInfo)));         // top: a negative number
+        CK(cudaMemsetAsync(h->info, 0x80, offsetof(RefreshInfo, noted)));         // top: a negative number
         CK(cudaMemsetAsync(d_hist, 0, THR_BINS * 4));
         const int *vmax_dev = nullptr;
         if (vmax <= 0) {

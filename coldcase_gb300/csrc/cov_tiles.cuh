@@ -464,3 +464,6 @@ static inline void bt_vcum_h(int q, int n, int R, int nl, uint32_t *vcum)
 // cov_verify.cu: the saturated coverage counts of the m listed words (device
 // word indices below q^n) into cnt; rec: m * BT_REC_BYTES bytes, 8-byte aligned
 int cov_count_words(int q, int n, int R, const uint32_t *d_idx, int m, uint16_t *cnt, uint2 *rec, cudaStream_t st);
+// the same counts unsaturated into map, or (subtract) off it
+int cov_count_words_map(int q, int n, int R, const uint32_t *d_idx, int m, int32_t *map, int subtract, uint2 *rec,
+                        cudaStream_t st);

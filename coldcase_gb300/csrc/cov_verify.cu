@@ -633,6 +633,25 @@ __global__ void __launch_bounds__(BT_NT) k_count_tiles(CountGeom g, BtCode code,
     if (threadIdx.x == 1 && ((g.tw - head) & 1u)) out[g.tw - 1] = (uint16_t)min(tile[g.tw - 1], 65535u);
 }
 
+// The same sums as whole 32-bit words: map[x] = #{i : d(x, c_i) <= R}, or
+// that many less than before.
+template <int Q>
+__global__ void __launch_bounds__(BT_NT) k_count_tiles_map(CountGeom g, BtCode code, int32_t *map, int subtract)
+{
+    extern __shared__ __align__(16) uint32_t ct_sm[];
+    const BtTile tl = bt_layout(g.q, g.n, g.tw);
+    bt_mark_tile<Q>(ct_sm, tl, blockIdx.x, g.q, g.n, g.R, g.M, code, g.nh, g.nl, g.vcum,
+                    [](uint32_t) { return 1u; });
+    int32_t *out = map + (size_t)blockIdx.x * g.tw;
+    const uint32_t *tile = ct_sm + tl.a0;
+    if (subtract) {
+#pragma unroll 4
+        for (uint32_t k = threadIdx.x; k < g.tw; k += BT_NT) out[k] -= (int32_t)tile[k];
+    } else {
+        for (uint32_t k = threadIdx.x; k < g.tw; k += BT_NT) out[k] = (int32_t)tile[k];
+    }
+}
+
 // ------------------------------------------------------------ finisher ----
 struct FinishGeom {
     int q, n, R, M;
@@ -831,7 +850,7 @@ int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
 CovDeviceFlags g_dt_attr;   // shared-memory opt-in of the transform kernels, per device
 CovDeviceFlags g_ct_attr;   // the same for the tile count
 
-// the tile count of the alphabet size q (a kernel of its own for q = 5..8)
+// the tile count of the alphabet size q (BT_Q_LIST: a kernel of its own)
 void ct_launch(const CountGeom &g, BtCode code, uint16_t *cnt, cudaStream_t st)
 {
     const unsigned grid = (unsigned)ipw(g.q, g.nh);
@@ -841,6 +860,19 @@ void ct_launch(const CountGeom &g, BtCode code, uint16_t *cnt, cudaStream_t st)
     BT_Q_LIST(CT_LAUNCH_Q)
 #undef CT_LAUNCH_Q
     default: k_count_tiles<0><<<grid, BT_NT, smem, st>>>(g, code, cnt); break;
+    }
+}
+
+// the same into a map
+void ct_launch_map(const CountGeom &g, BtCode code, int32_t *map, int subtract, cudaStream_t st)
+{
+    const unsigned grid = (unsigned)ipw(g.q, g.nh);
+    const size_t smem = bt_smem_bytes(g.q, g.n, g.tw);
+    switch (g.n < 2 ? 0 : g.q) {
+#define CT_LAUNCH_Q(QQ) case QQ: k_count_tiles_map<QQ><<<grid, BT_NT, smem, st>>>(g, code, map, subtract); break;
+    BT_Q_LIST(CT_LAUNCH_Q)
+#undef CT_LAUNCH_Q
+    default: k_count_tiles_map<0><<<grid, BT_NT, smem, st>>>(g, code, map, subtract); break;
     }
 }
 
@@ -862,8 +894,10 @@ int ct_attrs()
     if (g_ct_attr.done(dev)) return 0;
     CK(cudaFuncSetAttribute(k_count_tiles<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                             BT_SMEM_MAX));
+    CK(cudaFuncSetAttribute(k_count_tiles_map<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
 #define CT_ATTR_Q(QQ) \
-    CK(cudaFuncSetAttribute(k_count_tiles<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
+    CK(cudaFuncSetAttribute(k_count_tiles<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX)); \
+    CK(cudaFuncSetAttribute(k_count_tiles_map<QQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, BT_SMEM_MAX));
     BT_Q_LIST(CT_ATTR_Q)
 #undef CT_ATTR_Q
     g_ct_attr.set(dev);
@@ -996,17 +1030,41 @@ int dt_run(const DtGeom &g, const DtPlan &plan, const uint8_t *d_code, int M, ui
 
 }  // namespace
 
-int cov_count_words(int q, int n, int R, const uint32_t *d_idx, int m, uint16_t *cnt, uint2 *rec, cudaStream_t st)
+// the records of the m listed words and the geometry of their count
+static int words_records(int q, int n, int R, const uint32_t *d_idx, int m, uint2 *rec, cudaStream_t st, CountGeom &g,
+                         BtCode &code)
 {
     int rc = ct_attrs();
     if (rc) return rc;
-    const CountGeom g = count_geom(q, n, std::min(R, n), m);
+    g = count_geom(q, n, std::min(R, n), m);
     uint32_t *hi = (uint32_t *)(rec + m);
+    code = BtCode{hi, rec};
     if (m > 0) {
         k_count_records_idx<<<std::min(1024, (m + 127) / 128), 128, 0, st>>>(d_idx, m, q, n, g.nh, g.nl, rec, hi);
         CK(cudaGetLastError());
     }
-    ct_launch(g, BtCode{hi, rec}, cnt, st);
+    return COV_OK;
+}
+
+int cov_count_words(int q, int n, int R, const uint32_t *d_idx, int m, uint16_t *cnt, uint2 *rec, cudaStream_t st)
+{
+    CountGeom g;
+    BtCode code;
+    int rc = words_records(q, n, R, d_idx, m, rec, st, g, code);
+    if (rc) return rc;
+    ct_launch(g, code, cnt, st);
+    CK(cudaGetLastError());
+    return COV_OK;
+}
+
+int cov_count_words_map(int q, int n, int R, const uint32_t *d_idx, int m, int32_t *map, int subtract, uint2 *rec,
+                        cudaStream_t st)
+{
+    CountGeom g;
+    BtCode code;
+    int rc = words_records(q, n, R, d_idx, m, rec, st, g, code);
+    if (rc) return rc;
+    ct_launch_map(g, code, map, subtract, st);
     CK(cudaGetLastError());
     return COV_OK;
 }
