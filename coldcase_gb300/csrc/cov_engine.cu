@@ -52,15 +52,17 @@ static_assert(RS % RS_CKI == 0 && (RS & (RS - 1)) == 0 && (RS_CKI & (RS_CKI - 1)
               "RNG ring: powers of two, whole checkpoint blocks");
 #define EV_CAP    96           // events a warp queues during a commit
 #define INV_N     1024         // moduli with a reciprocal in shared memory
+#define FAR_M     8192         // codewords from which the cluster finds the candidates together
+#define JCAP      64           // codewords changed since the best code was kept, at most, to copy them alone
 #define CODE_SM   2048         // codewords mirrored in every CTA's shared memory
 #define NEG_CLUSTER_PAIRS 4096  // list x candidate pairs above which the whole cluster helps
 #define LIST_COST 5             // one uncovered-list entry costs about five walked words
 #define UL_CAP_DEFAULT (1 << 20)
 
-enum { OP_STOP = 0, OP_MOVE, OP_NEGWALK, OP_BALL, OP_RECOMPUTE, OP_ZERO_TABU, OP_REBUILD_UL, OP_NEG };
+enum { OP_STOP = 0, OP_MOVE, OP_NEGWALK, OP_BALL, OP_RECOMPUTE, OP_ZERO_TABU, OP_REBUILD_UL, OP_NEG, OP_CAND };
 enum {
     PH_PLAN = 0, PH_SELECT, PH_FINISH_MOVE, PH_KICK_START, PH_KICK_PICK, PH_KICK_RECOMP,
-    PH_KICK_END, PH_KICK_DONE, PH_REBUILD_DONE, PH_GREEDY, PH_GREEDY_NEXT, PH_STOPPED, PH_SA_END
+    PH_KICK_END, PH_KICK_DONE, PH_REBUILD_DONE, PH_GREEDY, PH_GREEDY_NEXT, PH_STOPPED, PH_SA_END, PH_CAND
 };
 enum { MODE_SEARCH = 0, MODE_GREEDY = 1 };
 
@@ -164,6 +166,7 @@ struct Smem {
     CovRng rs_ck[RS_NCK];      // generator at draw rs_ckpos[k]
     unsigned long long rs_ckpos[RS_NCK];
     uint64_t code_sm[CODE_SM]; // leader's mirror of the packed code (M <= CODE_SM)
+    int jr[JCAP], jn;          // codewords changed since best was written; more than JCAP: any
     uint64_t ev_pk[NWARP][EV_CAP];   // a move's events, a queue per warp: the word,
     uint32_t ev_tag[NWARP][EV_CAP];  // its coverer and what to do
 };
@@ -401,6 +404,8 @@ __device__ __forceinline__ void leader_set_code(const CovSlot &d, Smem &S, int i
 {
     cov_stcg(&d.code[i], pk);
     if (d.M <= CODE_SM) S.code_sm[i] = pk;
+    if (S.jn < JCAP) S.jr[S.jn] = i;
+    if (S.jn <= JCAP) S.jn++;
 }
 
 // exclusive scan of an int over the block with an associative op (applied
@@ -982,7 +987,12 @@ __device__ __forceinline__ void op_move_t(const CovSlot &d, const OpParams &P, S
             const uint32_t pq = d.ppow[R - 2];
             const uint32_t nxy = (uint32_t)d.nsub1 * pq;
             const uint32_t nstep2 = (nxy + 31) / 32 * 32;
-            for (uint32_t t0 = wid * 32; t0 < nstep2; t0 += wstride) {
+            // the turns go on where the pairs above left off (the first warps
+            // had the odd round of both: 23.1 -> 21.2 us at q6 n9 R4 on a
+            // cluster of 8)
+            const uint32_t nw = wstride / 32;
+            const uint32_t turn = ((uint32_t)d.nsub * d.ppow[R - 1] + 31) / 32 % nw;
+            for (uint32_t t0 = (wid >= turn ? wid - turn : wid + nw - turn) * 32; t0 < nstep2; t0 += wstride) {
                 const uint32_t t = t0 + lane;
                 int dy = 0;
                 int key = -1;
@@ -1669,14 +1679,78 @@ __device__ void zero_acc(Smem &S)
 __device__ void issue_move(const CovSlot &d, Smem &S, int k, uint64_t pk, int p, int v, long long dd);
 __device__ bool method_pick(const CovSlot &d, Smem &S, uint32_t *Lp);
 __device__ void write_trace(const CovSlot &d, Smem &S);
-__device__ void copy_best(const CovSlot &d);
+__device__ void copy_best(const CovSlot &d, Smem &S);
+
+__device__ void leader_candidates(const CovSlot &d, Smem &S, int csize, int runs);
+
+// consecutive codewords of one of `runs` runs
+__device__ __forceinline__ int cand_run(int M, int runs) { return ((M + runs - 1) / runs + 31) & ~31; }
+
+// Codewords lo .. hi-1 at distance dtar from pu, noted in order from note[lo]
+// by a warp, eight loads in flight; returns how many, and the least distance
+// of the run in dm.
+__device__ __forceinline__ int cand_walk(const CovSlot &d, const Smem &S, uint64_t pu, int dtar, int lo, int hi,
+                                         uint32_t *note, unsigned &dm)
+{
+    const int lane = threadIdx.x & 31;
+    int cnt = 0;
+    for (int c0 = lo; c0 < hi; c0 += 256) {
+        uint64_t pk[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            const int i = c0 + 32 * u + lane;
+            pk[u] = i < hi ? leader_code(d, S, i) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+            if (c0 + 32 * u >= hi) break;
+            const int i = c0 + 32 * u + lane;
+            // (with --fix0 codeword 0 is not a candidate, covsearch2e.c:1343)
+            const unsigned dd = i < hi && i >= d.fix0 ? (unsigned)cov_dist(pk[u], pu) : 0xffffffffu;
+            dm = min(dm, dd);
+            const unsigned m = __ballot_sync(0xffffffffu, dd == (unsigned)dtar);
+            if (dd == (unsigned)dtar) note[lo + cnt + __popc(m & ((1u << lane) - 1))] = (uint32_t)i;
+            cnt += __popc(m);
+        }
+    }
+    dm = __reduce_min_sync(0xffffffffu, dm);
+    return cnt;
+}
+
+// codeword i is the at-th candidate
+__device__ __forceinline__ void cand_put(const CovSlot &d, Smem &S, int at, uint32_t i)
+{
+    d.g_list[at] = i;
+    if (at < L_SM) {
+        S.L[at] = i;
+        S.Lpk[at] = leader_code(d, S, (int)i);
+    }
+}
+
+// The walk shared by the cluster (M > FAR_M): 53,257 codewords are 426 KB that
+// one SM reads in 26 us of a move's 63 (q6 n8 R1, a cluster of 8: 36 us with
+// this and the best code kept by its changes).  The line: one SM walks 8192
+// codewords in 4 us, which is what the extra op costs.
+__device__ void op_cand(const CovSlot &d, const OpParams &P, Smem &S, Smem *LS, int rank, int csize)
+{
+    const int runs = csize * NWARP, r = rank * NWARP + (int)(threadIdx.x >> 5);
+    const int len = cand_run(d.M, runs);
+    const int lo = min(d.M, r * len), hi = min(d.M, lo + len);
+    unsigned dm = 0xffffffffu;
+    const int cnt = cand_walk(d, S, P.pc, d.R + 1, lo, hi, reinterpret_cast<uint32_t *>(d.g_neg), dm);
+    if ((threadIdx.x & 31) == 0) {
+        LS->fy_b[r] = cnt;
+        LS->fy_c[r] = (int32_t)dm;
+    }
+    __threadfence();
+}
 
 // Plan one iteration up to the point where the entering-side counts are
 // needed.  Returns with S.opp set.
 __device__ void leader_plan(const CovSlot &d, Smem &S, int csize)
 {
     const int tid = threadIdx.x;
-    const int n = d.n, R = d.R, M = d.M;
+    const int M = d.M;
     if (tid == 0) {
         const int u = cov_ldcg(&d.st->ul_n);
         if (S.ul_valid && u > d.ul_cap) S.ul_valid = 0;
@@ -1733,47 +1807,74 @@ __device__ void leader_plan(const CovSlot &d, Smem &S, int csize)
     if (S.status) { if (tid == 0) { S.opp.op = OP_STOP; S.phase = PH_STOPPED; } return; }
     const uint64_t pu = S.pu;
 
+    if (M > FAR_M && csize > 1) {
+        if (tid == 0) { S.opp.op = OP_CAND; S.opp.pc = pu; S.phase = PH_CAND; }
+        __syncwarp();
+        return;
+    }
+    leader_candidates(d, S, csize, 0);
+}
+
+// The rest of the plan, from the target word S.pu.  runs: 0, or the runs of
+// codewords that the cluster has walked (OP_CAND; their notes are in g_neg,
+// their counts in fy_b and their least distances in fy_c).
+__device__ void leader_candidates(const CovSlot &d, Smem &S, int csize, int runs)
+{
+    const int tid = threadIdx.x;
+    const int n = d.n, R = d.R, M = d.M;
+    const uint64_t pu = S.pu;
+    long long t0 = cov_clock();
+
     // The target distance and the ordered list of codewords at it
     // (covsearch2e.c:1342-1376): always in global memory, the first L_SM also
     // in shared memory with their packed codes and one-hot masks.  The word is
     // uncovered, so no codeword is nearer than R + 1 and nearly always one is
-    // that near: a warp walks its run of consecutive codewords once, eight
-    // loads in flight, and notes those at R + 1 in order; a second walk finds
-    // the others' distance if there was none.
+    // that near: a warp walks its run of consecutive codewords once and notes
+    // those at R + 1 in order; a second walk finds the others' distance if
+    // there was none.
     const bool csm = M <= CODE_SM;
     uint32_t *const note = csm ? reinterpret_cast<uint32_t *>(S.fy_a) : reinterpret_cast<uint32_t *>(d.g_neg);
     const int lane = tid & 31, warp = tid >> 5;
-    const int run = ((M + NWARP - 1) / NWARP + 31) & ~31;        // codewords of a warp
-    const int lo = min(M, warp * run), hi = min(M, lo + run);
+    const int run = cand_run(M, NWARP);
     int dtar = R + 1, nL = 0;
-    for (int walk = 0; walk < 2; walk++) {
-        unsigned dm = 0xffffffffu;
-        int cnt = 0;                                             // the warp's notes
-        for (int c0 = lo; c0 < hi; c0 += 256) {
-            uint64_t pk[8];
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                const int i = c0 + 32 * u + lane;
-                pk[u] = i < hi ? leader_code(d, S, i) : 0;
+    unsigned near = 0xffffffffu;                                     // least distance of all
+    if (runs) {
+        // the runs' places in the list (into dval), then a warp per run
+        const int len = cand_run(M, runs);
+        if (warp == 0) {
+            int acc = 0;
+            for (int k0 = 0; k0 < runs; k0 += 32) {
+                const int k = k0 + lane;
+                const int c = k < runs ? S.fy_b[k] : 0;
+                int x = c;
+                for (int o = 1; o < 32; o <<= 1) {
+                    const int y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (k < runs) { S.dval[k] = acc + x - c; near = min(near, (unsigned)S.fy_c[k]); }
+                acc += __shfl_sync(0xffffffffu, x, 31);
             }
-#pragma unroll
-            for (int u = 0; u < 8; u++) {
-                if (c0 + 32 * u >= hi) break;
-                const int i = c0 + 32 * u + lane;
-                // (with --fix0 codeword 0 is not a candidate, covsearch2e.c:1343)
-                const unsigned dd = i < hi && i >= d.fix0 ? (unsigned)cov_dist(pk[u], pu) : 0xffffffffu;
-                dm = min(dm, dd);
-                const unsigned m = __ballot_sync(0xffffffffu, dd == (unsigned)dtar);
-                if (dd == (unsigned)dtar) note[lo + cnt + __popc(m & ((1u << lane) - 1))] = (uint32_t)i;
-                cnt += __popc(m);
-            }
+            near = __reduce_min_sync(0xffffffffu, near);
+            if (lane == 0) { S.red_i[0] = acc; S.red_u[0] = near; }
         }
-        if (lane == 0) S.red_i[warp] = cnt;
-        dm = __reduce_min_sync(0xffffffffu, dm);
-        if (lane == 0) S.red_u[warp] = dm;
+        cov_bar();
+        nL = S.red_i[0];
+        near = S.red_u[0];
+        if (tid == 0) { long long t1 = cov_clock(); S.prof[10] += t1 - t0; }
+        for (int r = warp; r < runs; r += NWARP) {
+            const int lo = min(M, r * len), cnt = S.fy_b[r], before = S.dval[r];
+            for (int k = lane; k < cnt; k += 32) cand_put(d, S, before + k, cov_ldcg(&note[lo + k]));
+        }
+        if (!nL) dtar = (int)near <= R + 1 ? R + 1 : (int)near;
+    }
+    for (int walk = runs ? 1 : 0; walk < 2 && !nL; walk++) {
+        const int lo = min(M, warp * run), hi = min(M, lo + run);
+        unsigned dm = 0xffffffffu;
+        const int cnt = cand_walk(d, S, pu, dtar, lo, hi, note, dm);
+        if (runs) cov_bar();                      // red_i is still being read
+        if (lane == 0) { S.red_i[warp] = cnt; S.red_u[warp] = dm; }
         cov_bar();
         int before = 0;
-        nL = 0;
         dm = 0xffffffffu;
         for (int w = 0; w < NWARP; w++) {
             if (w == warp) before = nL;
@@ -1782,15 +1883,7 @@ __device__ void leader_plan(const CovSlot &d, Smem &S, int csize)
         }
         if (walk == 0 && tid == 0) { long long t1 = cov_clock(); S.prof[10] += t1 - t0; }
         if (nL) {
-            for (int k = lane; k < cnt; k += 32) {
-                const uint32_t i = note[lo + k];
-                const int at = before + k;
-                d.g_list[at] = i;
-                if (at < L_SM) {
-                    S.L[at] = i;
-                    S.Lpk[at] = leader_code(d, S, (int)i);
-                }
-            }
+            for (int k = lane; k < cnt; k += 32) cand_put(d, S, before + k, note[lo + k]);
             break;
         }
         dtar = (int)dm <= R + 1 ? R + 1 : (int)dm;
@@ -2135,7 +2228,7 @@ __device__ void leader_sa_end(const CovSlot &d, Smem &S)
     }
     __syncwarp();
     cov_bar();
-    if (S.improved) copy_best(d);
+    if (S.improved) copy_best(d, S);
     cov_bar();
     if (tid == 0) {
         S.rec.unc_end = S.unc;
@@ -2306,16 +2399,25 @@ __device__ void write_trace(const CovSlot &d, Smem &S)
     if (d.trace) S.trace_n++;
 }
 
-__device__ void copy_best(const CovSlot &d)
+// best = code: the codewords changed since the last time, or all of them (the
+// first time in a launch).  All of 53,257 take 9 us of a move's 63.
+__device__ void copy_best(const CovSlot &d, Smem &S)
 {
-    for (int i0 = threadIdx.x; i0 < d.M; i0 += 8 * NT) {      // eight loads in flight
-        uint64_t v[8];
+    const int jn = S.jn;
+    if (jn <= JCAP) {
+        for (int k = threadIdx.x; k < jn; k += NT) cov_stcg(&d.best[S.jr[k]], leader_code(d, S, S.jr[k]));
+    } else {
+        for (int i0 = threadIdx.x; i0 < d.M; i0 += 8 * NT) {      // eight loads in flight
+            uint64_t v[8];
 #pragma unroll
-        for (int u = 0; u < 8; u++) v[u] = i0 + u * NT < d.M ? cov_ldcg(&d.code[i0 + u * NT]) : 0;
+            for (int u = 0; u < 8; u++) v[u] = i0 + u * NT < d.M ? cov_ldcg(&d.code[i0 + u * NT]) : 0;
 #pragma unroll
-        for (int u = 0; u < 8; u++)
-            if (i0 + u * NT < d.M) cov_stcg(&d.best[i0 + u * NT], v[u]);
+            for (int u = 0; u < 8; u++)
+                if (i0 + u * NT < d.M) cov_stcg(&d.best[i0 + u * NT], v[u]);
+        }
     }
+    cov_bar();
+    if (threadIdx.x == 0) S.jn = 0;
 }
 
 // after OP_MOVE: covsearch2e.c:1525-1553
@@ -2346,7 +2448,7 @@ __device__ void leader_finish_move(const CovSlot &d, Smem &S)
     }
     __syncwarp();
     cov_bar();
-    if (S.improved) copy_best(d);
+    if (S.improved) copy_best(d, S);
     cov_bar();
     if (tid == 0) {
         if (S.dokick) { S.kick_t = 0; S.phase = PH_KICK_START; }
@@ -2371,9 +2473,10 @@ __device__ void leader_step(const CovSlot &d, Smem &S, int csize)
         const int ph = S.phase;
         cov_bar();
         if (ph == PH_STOPPED) { if (tid == 0) S.opp.op = OP_STOP; return; }
-        if (ph == PH_PLAN) {
-            if (S.mode == MODE_GREEDY) { if (tid == 0) S.phase = PH_GREEDY; continue; }
-            leader_plan(d, S, csize);
+        if (ph == PH_PLAN || ph == PH_CAND) {
+            if (ph == PH_PLAN && S.mode == MODE_GREEDY) { if (tid == 0) S.phase = PH_GREEDY; continue; }
+            if (ph == PH_PLAN) leader_plan(d, S, csize);
+            else leader_candidates(d, S, csize, csize * NWARP);
             cov_bar();
             if (S.phase == PH_SELECT && S.opp.op == -1) {
                 leader_select(d, S);
@@ -2645,6 +2748,7 @@ cov_run_kernel(const CovSlot *__restrict__ slots, const int *__restrict__ cluste
         S.phase = PH_PLAN;
         S.t_deadline = (unsigned long long)cov_clock() + budget_ns * COV_CYCLES_PER_NS;
         S.guard = 0;
+        S.jn = JCAP + 1;
         S.opp.op = -1;
         S.gh_seq = 0;
         S.code_gen = 0;
@@ -2702,6 +2806,8 @@ cov_run_kernel(const CovSlot *__restrict__ slots, const int *__restrict__ cluste
             op_recompute(d, P.basen, P.pcn, S, LS, rank, csize);
         } else if (op == OP_ZERO_TABU) {
             op_zero_tabu(d, rank, csize);
+        } else if (op == OP_CAND) {
+            op_cand(d, P, S, LS, rank, csize);
         } else if (op == OP_REBUILD_UL) {
             op_rebuild_ul(d, rank, csize, cl);
         }
@@ -2738,6 +2844,7 @@ cov_run_kernel(const CovSlot *__restrict__ slots, const int *__restrict__ cluste
         if (leader && threadIdx.x == 0) {
             const long long dt = cov_clock() - top;
             if (op == OP_MOVE) S.prof[4] += dt;
+            else if (op == OP_CAND) S.prof[1] += dt;
             else if (op == OP_NEGWALK || op == OP_NEG) { S.prof[2] += dt; S.prof[14] += dt; }
             else S.prof[7] += dt;
         }

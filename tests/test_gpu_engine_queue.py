@@ -64,3 +64,28 @@ def test_initialisation_of_small_and_large_slots(covlib):
         assert st["uncovered"] == o.uncovered() and st["best"] == o.best_uncovered()
         o.close()
     pool.close()
+
+
+@pytest.mark.parametrize("cluster", [1, 2, 16])
+def test_cluster_wide_candidates_match_oracle(covlib, cluster):
+    """Codes so long that the cluster walks them together, the best code kept
+    from the changed codewords alone, kicks and a first codeword held fixed
+    included; moves split over launches."""
+    from oracle.pyoracle import Oracle
+    for q, n, R, M, opt in ((6, 6, 1, 8400, dict(kick=70, stall=3)), (8, 6, 1, 8200, dict(fix0=True)),
+                            (7, 7, 2, 8193, {}), (6, 7, 1, 20011, dict(noise=200))):
+        rng = np.random.default_rng(M)
+        code = rng.integers(0, q, size=(M, n)).astype(np.uint8)
+        o = Oracle(q, n, R, M, seed=5, tabu=3, threads=4, **opt)
+        o.init(code)
+        want = o.run(90, trace=True)
+        pool = Pool(1, cluster=cluster)
+        s = pool.add(q, n, R, M, code=code, seed=5, tabu=3, trace=1, trace_cap=90, **opt)
+        for k in (1, 50, 39):
+            pool.run(k)
+        assert pool.status(s)["status"] == 0
+        assert pool.trace(s).tobytes() == want.tobytes()
+        assert (pool.best(s) == o.best()).all() and (pool.code(s) == o.code()).all()
+        assert (pool.cnt(s) == o.cnt()).all() and (pool.rng(s) == o.rng()).all()
+        pool.close()
+        o.close()
