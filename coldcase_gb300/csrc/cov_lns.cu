@@ -1036,10 +1036,12 @@ double tiles_ps(const cov_lns *h, long long m)
 // 7^7 with and without).  Map at 7^9: 0.92 ms by transform, 0.07 to 0.25 by
 // tiles of 10 to 3000 words.  Six rounds at 7^9 48 -> 29 ms, the fill of 6^9
 // 71 -> 65.
-int lns_greedy_map(cov_lns *h, long long left, long long gone)
+// *tiled: the map came from tiles.
+int lns_greedy_map(cov_lns *h, long long left, long long gone, bool *tiled)
 {
     const double all_ps = left <= NOTE_CAP ? tiles_ps(h, left) + 0.6 : 1e300;
     const double off_ps = gone >= 0 && gone <= NOTE_CAP ? tiles_ps(h, gone) + 1.2 : 1e300;
+    *tiled = false;
     if (h->R == 0 || MAP_PS_WORD * h->N <= MAP_PS_LAUNCH) return lns_map_of_masks(h);
     const bool tiles = (MAP_PS_WORD - std::min(all_ps, off_ps)) * h->N > MAP_PS_LAUNCH;
     const int how = !tiles ? -1 : all_ps <= off_ps ? 1 : 0;
@@ -1048,6 +1050,7 @@ int lns_greedy_map(cov_lns *h, long long left, long long gone)
     k_lns_note<<<(nblk + LNS_NT - 1) / LNS_NT, LNS_NT>>>(h->um, h->um_map, nblk, h->blk, how, h->note, &h->info->noted);
     CK(cudaGetLastError());
     if (how < 0) return lns_map_of_masks(h);
+    *tiled = true;
     return cov_count_words_map(h->q, h->n, h->R, h->note, (int)(how ? left : gone), h->map, !how,
                                (uint2 *)(h->note + NOTE_CAP), nullptr);
 }
@@ -1447,8 +1450,11 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
     a.st = h->seq;
     // exact counts for one placement past which a map is the better buy.
     // Fills with limits of 64, 256 and 1000: 6^9 116, 114, 151 ms; 7^9 518,
-    // 444, 475; 4^11 45, 48, 70.
-    a.eval_cap = (int)std::max<long long>(64, std::min<long long>(1024, (long long)h->N / 131072));
+    // 444, 475; 4^11 45, 48, 70.  A quarter of it where tiles make the map
+    // (six rounds at 7^9 with 40, 80, 160, 320: 24.8, 24.8, 25.6, 28.9 ms).
+    const int evals_map = (int)std::max<long long>(64, std::min<long long>(1024, (long long)h->N / 131072));
+    const int evals_tiles = std::max(64, evals_map / 4);
+    bool tiled = false;
     int total = 0, vmax = 0;
     long long refreshes = 0, evals = 0, mapped = -1;         // mapped: the words of the last map
     // every refresh that finds a positive gain places at least one word (the
@@ -1460,7 +1466,7 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
         // maximum has more than cand_cap words, the same gain and a higher
         // position): a candidate is placed only while its exact gain is at
         // least the threshold, so it is always a best placement.
-        rc = lns_greedy_map(h, st.uncov, mapped < 0 ? -1 : mapped - st.uncov);
+        rc = lns_greedy_map(h, st.uncov, mapped < 0 ? -1 : mapped - st.uncov, &tiled);
         if (rc) return rc;
         mapped = st.uncov;
         refreshes++;
@@ -1480,6 +1486,7 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
         rc = extract_launch(h, 1, &h->info->thr, cand_cap, bcount, h->cand, h->bound, nullptr, &h->info->found);
         if (rc) return rc;
         CK(cudaMemsetAsync(h->acc, 0, 4 * (3 * (GREEDY_MAXG + 1) + 1)));
+        a.eval_cap = tiled ? evals_tiles : evals_map;
         a.room = room - total;
         a.list = h->list + total;
         a.max_steps = 64LL * (room - total) + 4LL * cand_cap + 64;
