@@ -318,9 +318,9 @@ k_dt_high(DtGeom g, int j0, int gsz, int lw, int last_, uint8_t *__restrict__ D,
 // about 11 instructions a pass for q words, where a byte of its own costs
 // about two a word (and q bytes of shared memory instead of four).
 // Bound by instruction issue (72 % of the slots at 8^9, 19 lane-instructions
-// a word; DRAM 14 % busy): 8^10 with 2549 codewords takes 0.68 ms = 1.6 TB/s
-// of distances written, against 4.5 ms for a tile pass and two strip sweeps
-// of bytes.
+// a word; DRAM 14 % busy): 8^10 with 2549 codewords takes 0.68 ms, against
+// 4.5 ms for a tile pass and two strip sweeps of bytes.  q = 5..8 mostly take
+// the blocks below.
 #define DT_TILES_NT 512
 #define DT_TILES_KEEP 8          // codewords a thread keeps between the two marking passes
 #define DT_TILES_SMEM (100 * 1024)
@@ -516,6 +516,272 @@ k_dt_tiles(DtGeom g, int nl, const uint2 *__restrict__ rec, int M, uint8_t *__re
     __syncthreads();
     if (hist && threadIdx.x < g.n + 2 && sh[threadIdx.x])
         atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
+}
+
+// ------------------------------------------------ the same, block by block --
+// For q = 5..8 a block of the two lowest axes, q^2 <= 64 words, is one element:
+// its least distance e, the words at e (a0) and the words at e or e + 1 (a1)
+// as bit masks; all others are at e + 2, because two words of a block differ
+// by two steps at most.  A block starts from the codewords that enter it --
+// e is the least starting value, a0 the codewords with it, a1 their rows and
+// columns and the codewords one farther -- so that the two lowest axes cost
+// nothing; along another axis, with E the least e of a fibre's q blocks and
+// U0, U1 the words of the fibre at E and within E + 1, a block becomes
+// min(block, E + 1, ...) in a handful of mask operations for q^2 words.
+template <int Q> struct DtMask { typedef unsigned long long W; };
+template <> struct DtMask<5> { typedef uint32_t W; };
+#define DT_BLOCKS_SMEM (100 * 1024)
+
+// bit of word y of a block.  q = 8: the four words of a 32-bit store stand at
+// the same bit of the four bytes of a half, so that a shift and a mask make
+// four bytes of them.
+template <int Q>
+__host__ __device__ constexpr int dt_bit(int y)
+{
+    return Q == 8 ? (y & 3) * 8 + ((y >> 2) & 7) + 32 * (y >> 5) : y;
+}
+
+// per codeword: {nibbles of the high digits, (slot of the block << 6) | word}
+template <int Q>
+__global__ void k_dt_block_records(const uint8_t *__restrict__ code, int M, DtGeom g, int nl, uint2 *__restrict__ rec)
+{
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
+        uint32_t x = 0;
+        for (int j = 0; j < g.n; j++) x = x * (uint32_t)Q + code[(size_t)i * g.n + j];
+        if (x >= g.N) x = 0xffffffffu;           // a digit outside the alphabet: no word
+        uint32_t hi = x / g.pw[nl], h = 0;
+        const uint32_t lo = x - hi * g.pw[nl];
+        for (int j = 0; j < g.n - nl; j++) { h |= (hi % (uint32_t)Q) << (4 * j); hi /= (uint32_t)Q; }
+        rec[i] = x == 0xffffffffu ? make_uint2(0u, 0xffffffffu)
+                                  : make_uint2(h, (dt_slot<Q>(lo / (uint32_t)(Q * Q)) << 6) | (lo % (uint32_t)(Q * Q)));
+    }
+}
+
+// NT: the most threads of a CTA.  A fibre of q = 6..8 blocks wants the registers
+// of 256 threads (8^10 with 2549 codewords 409 -> 370 us, 7^10 with 163 155 ->
+// 137); many codewords want the threads (8^9 with 20000: 151 -> 119), and q = 5
+// has masks of half the size.
+//
+// Bound by the integer pipe (65 % at 8^9 with 1000 codewords, 7.2
+// lane-instructions a word) and, below some hundred tiles an SM, by the last
+// wave.  Against a line an element (k_dt_tiles): 8^10 M 2549 686 -> 370 us (2.9
+// TB/s of distances), 7^10 M 163 267 -> 137, 5^12 M 3000 295 -> 169, 6^11 M 300
+// 334 -> 230, 7^9 M 1500 57 -> 40.
+template <int Q, int NT>
+__global__ void __launch_bounds__(NT, NT > 256 ? 2 : 3)
+k_dt_blocks(DtGeom g, int nl, const uint2 *__restrict__ rec, int M, uint8_t *__restrict__ D, unsigned long long *hist)
+{
+    typedef typename DtMask<Q>::W W;
+    constexpr uint32_t QQ = Q * Q, HALVES = sizeof(W) / 4;
+    constexpr W ALL = (W)(~(W)0) >> (8 * sizeof(W) - QQ);
+    struct __align__(2 * sizeof(W)) Planes { W a0, a1; };
+    extern __shared__ __align__(16) uint32_t dt_w[];
+    __shared__ int sh[COV_MAXN + 4];
+    __shared__ W cross[QQ];                        // a word's row and column
+    const uint32_t T = g.pw[nl], nblk = T / QQ, ntile = g.N / T;
+    Planes *const pl = reinterpret_cast<Planes *>(dt_w);
+    uint32_t *const le = dt_w + (size_t)nblk * 2 * HALVES;
+    const uint32_t nt = blockDim.x;
+    const int nh = g.n - nl;
+    if (threadIdx.x < COV_MAXN + 4) sh[threadIdx.x] = 0;
+    if (threadIdx.x < QQ) {
+        W c = 0;
+        const int y = (int)threadIdx.x;
+        for (int k = 0; k < Q; k++) c |= ((W)1 << dt_bit<Q>(y / Q * Q + k)) | ((W)1 << dt_bit<Q>(k * Q + y % Q));
+        cross[y] = c;
+    }
+    for (uint32_t tile = blockIdx.x; tile < ntile; tile += gridDim.x) {
+        uint32_t hp = 0;
+        {
+            uint32_t t = tile;
+            for (int j = 0; j < nh; j++) { hp |= (t % (uint32_t)Q) << (4 * j); t /= (uint32_t)Q; }
+        }
+        __syncthreads();
+        for (uint32_t l = threadIdx.x; l < nblk; l += nt) le[l] = (uint32_t)g.inf;
+        __syncthreads();
+        // least starting value of every block, then the masks:
+        // (starting value << 28) | (slot << 6) | word, all ones for none
+        uint32_t kept[DT_TILES_KEEP];
+        const bool keep = (uint32_t)M <= nt * DT_TILES_KEEP;
+        auto entry = [&](uint32_t i) {
+            const uint2 r = __ldg(&rec[i]);
+            return r.y == 0xffffffffu ? r.y : (dt_nibble_dist(r.x, hp) << 28) | r.y;
+        };
+        auto lower = [&](uint32_t v) {
+            if (v != 0xffffffffu) atomicMin(&le[(v & 0x0fffffffu) >> 6], v >> 28);
+        };
+        auto mark = [&](uint32_t v) {
+            if (v == 0xffffffffu) return;
+            const uint32_t at = (v & 0x0fffffffu) >> 6, y = v & 63u, e = le[at], s = v >> 28;
+            if (s > e + 1u) return;
+            uint32_t *const p = dt_w + (size_t)at * 2 * HALVES;
+            const W bit = (W)1 << dt_bit<Q>((int)y), c = s == e ? cross[y] : bit;
+#pragma unroll
+            for (uint32_t h = 0; h < HALVES; h++) {
+                const uint32_t b = (uint32_t)(bit >> (16 * h) >> (16 * h)), x = (uint32_t)(c >> (16 * h) >> (16 * h));
+                if (s == e && b) atomicOr(&p[h], b);
+                if (x) atomicOr(&p[HALVES + h], x);
+            }
+        };
+        if (keep) {
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++) {
+                const uint32_t i = threadIdx.x + (uint32_t)u * nt;
+                kept[u] = (uint32_t)u * nt < (uint32_t)M && i < (uint32_t)M ? entry(i) : 0xffffffffu;
+            }
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++)
+                if ((uint32_t)u * nt < (uint32_t)M) lower(kept[u]);
+        } else {
+            for (uint32_t i = threadIdx.x; i < (uint32_t)M; i += nt) lower(entry(i));
+        }
+        __syncthreads();
+        for (uint32_t l = threadIdx.x; l < nblk; l += nt) {
+            const W x = le[l] == (uint32_t)g.inf ? ALL : 0;       // no codeword: every word is at inf
+            pl[l].a0 = x;
+            pl[l].a1 = x;
+        }
+        __syncthreads();
+        if (keep) {
+#pragma unroll
+            for (int u = 0; u < DT_TILES_KEEP; u++)
+                if ((uint32_t)u * nt < (uint32_t)M) mark(kept[u]);
+        } else {
+            for (uint32_t i = threadIdx.x; i < (uint32_t)M; i += nt) mark(entry(i));
+        }
+        __syncthreads();
+        // the other low axes, a fibre of Q blocks at a time
+        uint32_t inner = 1;
+        for (int j = 2; j < nl; j++, inner *= (uint32_t)Q) {
+            const float rinv = 1.0f / (float)inner;   // f < 2^24: one correction makes f / inner exact
+            const uint32_t p1 = dt_slot<Q>(inner), p2 = dt_slot<Q>(2u * inner), p4 = dt_slot<Q>(4u * inner);
+            for (uint32_t f = threadIdx.x; f < nblk / (uint32_t)Q; f += nt) {
+                int o = (int)((float)f * rinv);
+                int i = (int)f - o * (int)inner;
+                if (i < 0) { o--; i += (int)inner; } else if (i >= (int)inner) { o++; i -= (int)inner; }
+                const uint32_t b = dt_slot<Q>((uint32_t)o * (uint32_t)Q * inner + (uint32_t)i);
+                auto slot = [&](int a) {
+                    if constexpr (Q == 8) return b ^ ((a & 1) ? p1 : 0u) ^ ((a & 2) ? p2 : 0u) ^ ((a & 4) ? p4 : 0u);
+                    else return b + (uint32_t)a * inner;
+                };
+                uint32_t e[Q];
+                Planes v[Q];
+#pragma unroll
+                for (int a = 0; a < Q; a++) {
+                    e[a] = le[slot(a)];
+                    v[a] = pl[slot(a)];
+                }
+                uint32_t E = e[0];
+#pragma unroll
+                for (int a = 1; a < Q; a++) E = min(E, e[a]);
+                W u0 = 0, u1 = 0;
+#pragma unroll
+                for (int a = 0; a < Q; a++) {
+                    if (e[a] == E) { u0 |= v[a].a0; u1 |= v[a].a1; }
+                    if (e[a] == E + 1u) u1 |= v[a].a0;
+                }
+#pragma unroll
+                for (int a = 0; a < Q; a++) {
+                    if (e[a] == E) {
+                        pl[slot(a)].a1 = v[a].a1 | u0;
+                    } else {
+                        Planes w{u0, u1};
+                        if (e[a] == E + 1u) { w.a0 |= v[a].a0; w.a1 |= v[a].a1; }
+                        if (e[a] == E + 2u) w.a1 |= v[a].a0;
+                        pl[slot(a)] = w;
+                        le[slot(a)] = E + 1u;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+        auto bits = [](W x) {
+            if constexpr (sizeof(W) == 8) return __popcll(x);
+            else return __popc(x);
+        };
+        if (hist) {
+            int m = -1, at = 0, next = 0, more = 0;    // words at m, m + 1 and m + 2 of a run of blocks
+            auto put = [&] {
+                if (at) atomicAdd(&sh[m], at);
+                if (next) atomicAdd(&sh[m + 1], next);
+                if (more) atomicAdd(&sh[m + 2], more);
+            };
+            for (uint32_t l = threadIdx.x; l < nblk; l += nt) {
+                if ((int)le[l] != m) {
+                    put();
+                    m = (int)le[l];
+                    at = next = more = 0;
+                }
+                const int c0 = bits(pl[l].a0), c1 = bits(pl[l].a1);
+                at += c0;
+                next += c1 - c0;
+                more += (int)QQ - c1;
+            }
+            put();
+        }
+        if (!D) continue;
+        uint8_t *const out = D + (size_t)tile * T;
+        if constexpr (Q == 8) {
+            // sixteen words of a block, a quarter of it, a lane (D is 16-byte aligned)
+            for (uint32_t x = threadIdx.x; x < nblk * 4u; x += nt) {
+                const uint32_t l = dt_slot<Q>(x >> 2), h = (x >> 1) & 1u, sft = (x & 1u) * 4u;
+                const uint32_t a0 = dt_w[l * 4u + h] >> sft, a1 = dt_w[l * 4u + 2u + h] >> sft;
+                const uint32_t m2 = (le[l] + 2u) * 0x01010101u;
+                auto four = [&](int k) { return m2 - ((a0 >> k) & 0x01010101u) - ((a1 >> k) & 0x01010101u); };
+                reinterpret_cast<uint4 *>(out)[x] = make_uint4(four(0), four(1), four(2), four(3));
+            }
+        } else {
+            // aligned pieces of 16 bytes, each from the one or two blocks that
+            // its bytes lie in; the ends as bytes
+            const uint32_t head = min((16u - (uint32_t)(reinterpret_cast<uintptr_t>(out) & 15u)) & 15u, T);
+            const uint32_t np = (T - head) >> 4, ends = T - 16u * np;
+            for (uint32_t k = threadIdx.x; k < ends; k += nt) {
+                const uint32_t x = k < head ? k : 16u * np + k, l = x / QQ, y = x - l * QQ;
+                out[x] = (uint8_t)(le[l] + 2u - (uint32_t)((pl[l].a0 >> y) & 1u) - (uint32_t)((pl[l].a1 >> y) & 1u));
+            }
+            for (uint32_t k = threadIdx.x; k < np; k += nt) {
+                const uint32_t x = head + 16u * k, l = x / QQ, y = x - l * QQ;
+                const int left = (int)(QQ - y);          // words of block l in the piece
+                const Planes v = pl[l];
+                uint32_t a0 = (uint32_t)(v.a0 >> y), a1 = (uint32_t)(v.a1 >> y);
+                const uint32_t ma = (le[l] + 2u) * 0x01010101u;
+                uint32_t mb = ma;
+                if (left < 16) {
+                    const Planes w = pl[l + 1];
+                    a0 |= (uint32_t)w.a0 << left;
+                    a1 |= (uint32_t)w.a1 << left;
+                    mb = (le[l + 1] + 2u) * 0x01010101u;
+                }
+                uint32_t r[4];
+#pragma unroll
+                for (int k4 = 0; k4 < 4; k4++) {
+                    const int c = min(max(left - 4 * k4, 0), 4);
+                    const uint32_t first = (uint32_t)((1ull << (8 * c)) - 1ull);
+                    const uint32_t m2 = (ma & first) | (mb & ~first);
+                    r[k4] = m2 - ((((a0 >> (4 * k4)) & 15u) * 0x00204081u) & 0x01010101u) -
+                            ((((a1 >> (4 * k4)) & 15u) * 0x00204081u) & 0x01010101u);
+                }
+                *reinterpret_cast<uint4 *>(out + x) = make_uint4(r[0], r[1], r[2], r[3]);
+            }
+        }
+    }
+    __syncthreads();
+    if (hist && threadIdx.x < g.n + 2 && sh[threadIdx.x])
+        atomicAdd(&hist[threadIdx.x], (unsigned long long)sh[threadIdx.x]);
+}
+
+template <int Q>
+int dt_blocks_launch(int grid, int nt, size_t smem, cudaStream_t st, const uint8_t *code, int M, const DtGeom &g, int nl,
+                     uint2 *rec, uint8_t *D, unsigned long long *hist)
+{
+    if (M > 0) {
+        k_dt_block_records<Q><<<std::min(1024, (M + 255) / 256), 256, 0, st>>>(code, M, g, nl, rec);
+        CK(cudaGetLastError());
+    }
+    if (nt > 256) k_dt_blocks<Q, 512><<<grid, nt, smem, st>>>(g, nl, rec, M, D, hist);
+    else k_dt_blocks<Q, 256><<<grid, nt, smem, st>>>(g, nl, rec, M, D, hist);
+    CK(cudaGetLastError());
+    return 0;
 }
 
 // the transform kernels of every q, for a runtime q
@@ -907,7 +1173,7 @@ int ct_attrs()
 // How a transform runs: by tiles from the code alone (k_dt_tiles) or by the
 // bitmap and sweeps of the word array (k_dt_low, k_dt_high).
 struct DtPlan {
-    bool tiles;
+    bool tiles, blocks;          // blocks: tiles by k_dt_blocks
     int nl, nt, grid;
     size_t smem;
     size_t scratch;              // bytes of device scratch: the code's records, or its bitmap
@@ -920,12 +1186,14 @@ struct DtPlan {
 // barrier; the number of low digits with the least estimate is taken (of the
 // seven cells timed at every number it is the best or within 6 % of it).  The
 // sweep form's side is measured: 4.2 ps a word (8^10: 4.5 ms) after three
-// launches.  Measured, sweeps against tiles: 8^10 M 2549 4505 -> 680 us, 7^10
-// M 163 1076 -> 260, 7^9 M 1500 179 -> 50, 7^9 M 30000 179 -> 80, 6^6 M 41
-// 24.8 -> 10.6; near the line, 8^7 M 30000: 41.1 against 41.7.
+// launches.  Measured, sweeps against lines against blocks (q = 5..8: 30
+// lane-instructions a codeword and a block's pass, 2.5 to 5 a word of output):
+// 8^10 M 2549 4505, 686, 367 us; 7^10 M 163 1076, 267, 139; 7^9 M 1500 179,
+// 57, 40; 7^9 M 30000 179, 85; 6^6 M 41 24.8, 10.6; near the line, 8^7 M
+// 30000: sweeps 41.1, lines 41.7.
 #define DT_SWEEP_CYCLES_WORD 0.0087
 #define DT_SWEEP_CYCLES_MIN 16000.0
-DtPlan dt_plan(const DtGeom &g, int M)
+DtPlan dt_plan(const DtGeom &g, int M, const uint8_t *D)
 {
     DtPlan best{};
     best.scratch = (size_t)((g.N + 31) / 32) * 4;
@@ -950,6 +1218,29 @@ DtPlan dt_plan(const DtGeom &g, int M)
             best.scratch = (size_t)std::max(M, 1) * 8;
         }
     }
+    // blocks of two digits (q = 8 stores 16 bytes at a time)
+    if (g.q < 5 || g.q > 8 || (g.q == 8 && (reinterpret_cast<uintptr_t>(D) & 15u))) return best;
+    for (int nl = std::max(2, g.n - 8); nl <= g.n; nl++) {
+        const uint32_t T = g.pw[nl], nblk = T / (uint32_t)(g.q * g.q);
+        const size_t smem = (size_t)nblk * (g.q == 5 ? 12 : 20);
+        if (smem > DT_BLOCKS_SMEM) break;
+        const int nt = nblk <= 64 ? 128 : nblk > 1024 && (g.q == 5 || M > 4096) ? 512 : 256;
+        const double tiles = g.N / T;
+        const double per_sm = std::min(std::min((nt > 256 ? 1024.0 : 768.0) / nt, 220.0 * 1024 / (smem + 2048.0)), 32.0);
+        const double work = M * (M <= nt * DT_TILES_KEEP ? 30.0 : 45.0) + nblk * (30.0 * (nl - 2) + 15.0) +
+                            T * (g.q == 8 ? 2.5 : 5.0);
+        const double waves = std::ceil(tiles / (sms * std::floor(per_sm)));
+        const double cyc = tiles * work / (64.0 * sms) + waves * (2000.0 + 500.0 * (nl - 2) + work / (nt / 4.0));
+        if (cyc < least) {
+            least = cyc;
+            best.tiles = best.blocks = true;
+            best.nl = nl;
+            best.nt = nt;
+            best.smem = smem;
+            best.grid = (int)std::min(tiles, sms * std::floor(per_sm));
+            best.scratch = (size_t)std::max(M, 1) * 8;
+        }
+    }
     return best;
 }
 
@@ -964,7 +1255,20 @@ int dt_run(const DtGeom &g, const DtPlan &plan, const uint8_t *d_code, int M, ui
             const int rc = dt_for_q<DtAttrs>(q);
             if (rc) return rc;
         }
+        for (const void *k : {(const void *)k_dt_blocks<5, 256>, (const void *)k_dt_blocks<6, 256>,
+                              (const void *)k_dt_blocks<7, 256>, (const void *)k_dt_blocks<8, 256>,
+                              (const void *)k_dt_blocks<5, 512>, (const void *)k_dt_blocks<6, 512>,
+                              (const void *)k_dt_blocks<7, 512>, (const void *)k_dt_blocks<8, 512>})
+            CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, DT_BLOCKS_SMEM));
         g_dt_attr.set(dev);
+    }
+    if (plan.blocks) {
+        switch (g.q) {
+#define DT_BLOCKS_Q(QQ) case QQ: return dt_blocks_launch<QQ>(plan.grid, plan.nt, plan.smem, st, d_code, M, g, plan.nl, \
+                                                             (uint2 *)scratch, d_D, d_hist);
+        DT_BLOCKS_Q(5) DT_BLOCKS_Q(6) DT_BLOCKS_Q(7) DT_BLOCKS_Q(8)
+#undef DT_BLOCKS_Q
+        }
     }
     if (plan.tiles)
         return dt_for_q<DtTiles>(g.q, plan.grid, plan.nt, plan.smem, st, d_code, M, g, plan.nl, (uint2 *)scratch,
@@ -1078,7 +1382,7 @@ int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M, uint
     if (rc) return rc;
     if (M < 0 || (M > 0 && !d_code) || !d_dist) return COV_EINVAL;
     cudaStream_t st = (cudaStream_t)stream;
-    const DtPlan plan = dt_plan(g, M);
+    const DtPlan plan = dt_plan(g, M, d_dist);
     void *scratch = nullptr;
     rc = scratch_alloc(&scratch, plan.scratch, st);
     if (rc) return rc;
@@ -1131,7 +1435,7 @@ int cov_mindist_dev_static(int32_t q, int32_t n, const uint8_t *d_code, int32_t 
         CK(cudaGetSymbolAddress(&ptr, g_dt_static_bitmap));
         g_dt_static_addr[dev] = (uint32_t *)ptr;
     }
-    DtPlan plan = dt_plan(g, M);
+    DtPlan plan = dt_plan(g, M, d_dist);
     if (plan.scratch > sizeof g_dt_static_bitmap) plan = DtPlan{};       // more codewords than the array has records
     return dt_run(g, plan, d_code, M, d_dist, nullptr, g_dt_static_addr[dev], (cudaStream_t)stream);
 }
@@ -1163,7 +1467,7 @@ int cov_mindist(int32_t q, int32_t n, const uint8_t *code, int32_t M, uint8_t *d
     if (M < 0 || (M > 0 && !code)) return COV_EINVAL;
     for (long long i = 0; i < (long long)M * n; i++) if (code[i] >= q) return COV_EINVAL;
     cudaStream_t st = nullptr;
-    const DtPlan plan = dt_plan(g, M);
+    const DtPlan plan = dt_plan(g, M, nullptr);   // D will be 256-byte aligned
     const bool want_D = dist || !plan.tiles;      // the sweeps work in D; the tiles need none for the histogram
     // one allocation: the histogram, the transform's scratch, the code, D
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
