@@ -1669,6 +1669,54 @@ __device__ void fy_parallel(Smem &S, int take, int ncand)
     cov_bar();
 }
 
+// The same by one warp without a block barrier, 32 steps at a time, for short
+// lists: prevS and prevT come from the lanes below or from the table of the
+// last step that targeted a position, and W is complete up to the chunk.
+// fy_parallel's barriers and scans take 2.7 us whatever the list; with it and
+// without, the candidates of a move take 2.5 and 4.6 us for 23 of them (q4 n6
+// R1), 5.3 and 5.9 for 182 (q6 n9 R4).
+#define FY_WARP 256            // longest list (at most NT)
+__device__ void fy_warp(Smem &S, int take, int ncand)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned below = (1u << lane) - 1u;
+    int32_t *const last = S.fy_a, *const W = S.fy_b;
+    unsigned *const to = reinterpret_cast<unsigned *>(S.fy_c);     // steps of the chunk that target its positions
+    for (int x = lane; x < ncand; x += 32) last[x] = -1;
+    to[lane] = 0;
+    __syncwarp();
+    for (int s0 = 0; s0 < take; s0 += 32) {
+        const int s = s0 + lane;
+        const bool live = s < take;
+        const int j = live ? S.dval[s] : -1 - lane;
+        const unsigned same = __match_any_sync(0xffffffffu, j);
+        int ps = -1, pt = -1;
+        if (live) {
+            ps = same & below ? s0 + 31 - __clz((int)(same & below)) : last[j];
+            pt = last[s];
+            if (j < s0 + 32) atomicOr(&to[j - s0], 1u << lane);
+        }
+        __syncwarp();
+        if (to[lane] & below) pt = s0 + 31 - __clz((int)(to[lane] & below));
+        // W(s): a value, or the lane (as -1 - lane) that has it
+        int w = !live ? 0 : pt < 0 ? s : pt < s0 ? W[pt] : s0 - 1 - pt;
+        while (__any_sync(0xffffffffu, w < 0)) {
+            const int v = __shfl_sync(0xffffffffu, w, w < 0 ? -1 - w : lane);
+            if (w < 0) w = v;
+        }
+        if (live) W[s] = w;
+        __syncwarp();
+        if (live) {
+            S.perm[s] = (uint32_t)(ps >= 0 ? W[ps] : j);
+            if (same >> lane == 1u) last[j] = s;
+        }
+        to[lane] = 0;
+        __syncwarp();
+    }
+    if (lane == 0) S.rs_use += take;
+    __syncwarp();
+}
+
 __device__ void zero_acc(Smem &S)
 {
     if (threadIdx.x == 0) { S.acc.dunc = 0; S.acc.accT = 0; }
@@ -1909,43 +1957,62 @@ __device__ void leader_candidates(const CovSlot &d, Smem &S, int csize, int runs
     const int psm = ncand <= PERM_CAP;
     uint32_t *perm = psm ? S.perm : d.g_perm;
     int32_t *dval = psm ? S.dval : d.g_dval;
-    for (int c = tid; c < ncand; c += NT) perm[c] = (uint32_t)c;
-    // Fisher-Yates sample of `take` (covsearch2e.c:1383-1389): the draws are
-    // generated in order by one thread, reduced in parallel, applied in order.
-    for (int s0 = 0; s0 < take; s0 += RB) {
-        const int cnt = min(RB, take - s0);
-        cov_bar();
-        if (tid == 0) rs_ensure(S, cnt);
-        __syncwarp();
-        cov_bar();
-        for (int t = tid; t < cnt; t += NT) {
-            int s = s0 + t;
-            dval[s] = s + (int32_t)fastmod(S, rs_peek(S, t), (uint64_t)(ncand - s));
-        }
-        cov_bar();
-        if (tid == 0) S.rs_use += cnt;
-        __syncwarp();
-    }
-    cov_bar();
-    // the sample's permutation: in parallel in shared memory; the oversized
-    // case is swapped in order by one thread while the others work on the
-    // entering side (apply_swaps), which does not need it
     int pending = 1;
-    if (psm) {
-        // perm[c] = c was set above for c < ncand; fy_parallel rewrites
-        // perm[0..take) directly from the draws
-        fy_parallel(S, take, ncand);
+    auto count_words = [&] {                   // distinct codewords of a sample (thread 0)
+        int c = 0;
+        for (int s2 = 0; s2 < take; s2++) {
+            int l = (int)(perm[s2] / (uint32_t)cpw), dup = 0;
+            for (int t2 = 0; t2 < s2; t2++) if ((int)(perm[t2] / (uint32_t)cpw) == l) { dup = 1; break; }
+            c += !dup;
+        }
+        S.ibc[2] = c;
+    };
+    if (ncand <= FY_WARP) {
+        // a short list: one warp, while the others go on to the entering side
+        if (S.rs_gen < S.rs_use + (unsigned long long)take) {
+            cov_bar();
+            if (tid == 0) rs_ensure(S, take);
+            __syncwarp();
+            cov_bar();
+        }
+        if (tid < take) dval[tid] = tid + (int32_t)fastmod(S, rs_peek(S, tid), (uint64_t)(ncand - tid));
+        cov_bar();
+        if (tid < 32) {
+            fy_warp(S, take, ncand);
+            if (take < ncand && tid == 0) count_words();
+            __syncwarp();
+        }
         pending = 0;
-        if (take < ncand && tid == 0) {
-            int c = 0;
-            for (int s2 = 0; s2 < take; s2++) {
-                int l = (int)(perm[s2] / (uint32_t)cpw), dup = 0;
-                for (int t2 = 0; t2 < s2; t2++) if ((int)(perm[t2] / (uint32_t)cpw) == l) { dup = 1; break; }
-                c += !dup;
+    } else {
+        for (int c = tid; c < ncand; c += NT) perm[c] = (uint32_t)c;
+        // Fisher-Yates sample of `take` (covsearch2e.c:1383-1389): the draws are
+        // generated in order by one thread, reduced in parallel, applied in order.
+        for (int s0 = 0; s0 < take; s0 += RB) {
+            const int cnt = min(RB, take - s0);
+            cov_bar();
+            if (tid == 0) rs_ensure(S, cnt);
+            __syncwarp();
+            cov_bar();
+            for (int t = tid; t < cnt; t += NT) {
+                int s = s0 + t;
+                dval[s] = s + (int32_t)fastmod(S, rs_peek(S, t), (uint64_t)(ncand - s));
             }
-            S.ibc[2] = c;
+            cov_bar();
+            if (tid == 0) S.rs_use += cnt;
+            __syncwarp();
         }
         cov_bar();
+        // the sample's permutation: in parallel in shared memory; the oversized
+        // case is swapped in order by one thread while the others work on the
+        // entering side (apply_swaps), which does not need it
+        if (psm) {
+            // perm[c] = c was set above for c < ncand; fy_parallel rewrites
+            // perm[0..take) directly from the draws
+            fy_parallel(S, take, ncand);
+            pending = 0;
+            if (take < ncand && tid == 0) count_words();
+            cov_bar();
+        }
     }
     if (tid == 0) {
         S.swaps_pending = pending;
