@@ -731,6 +731,63 @@ __device__ __forceinline__ void commit_events(const CovSlot &d, const OpParams &
     __syncwarp();
 }
 
+// The 32 items of a warp, a lane each, and their 32 (q-1) words taken in the
+// order (item, value): step k's lane works word 32 k + lane, value `v` of item
+// `src`.  Neighbouring lanes then read neighbouring words -- the values of a low
+// position lie in one sector, and so do those of consecutive items, whose next
+// to last position differs -- where a lane that walks its own item's values
+// makes every access of a warp 32 lines, one tag lookup each: the commit of one
+// instance at q6 n9 R4 on a cluster of 8 was bound by those (5.5 us for the 320
+// loads and 320 stores of a warp's 32 items).  A move's op there 21.2 -> 16.8
+// us; 64 restarts of q7 n9 R4 on clusters of 2 177 -> 145; q7 n9 R3 M2691
+// (dense) 40.6 -> 39.6.
+struct ItemRow {
+    uint32_t w0, pl;           // word with digit 0 at the last position; its stride
+    uint32_t lc;               // last position, and the centre's digit there << 8
+    uint64_t pk;
+};
+__device__ __forceinline__ ItemRow item_row(const CovSlot &d, const CovItem &it)
+{
+    ItemRow r;
+    r.pl = d.pw[it.last];
+    r.w0 = it.w - (uint32_t)it.clast * r.pl;
+    r.lc = (uint32_t)it.last | ((uint32_t)it.clast << 8);
+    r.pk = it.pk;
+    return r;
+}
+struct ItemStep {
+    int src, v;
+};
+// inv: 65536 / (q-1) + 1 (exact below 32 * 15)
+__device__ __forceinline__ ItemStep item_step(int k, int qm1, uint32_t inv)
+{
+    const uint32_t f = (uint32_t)k * 32u + (threadIdx.x & 31u);
+    ItemStep s;
+    s.src = (int)((f * inv) >> 16);
+    s.v = (int)f - s.src * qm1;
+    return s;
+}
+__device__ __forceinline__ uint32_t step_word(const ItemRow &r, const ItemStep &s)
+{
+    const uint32_t w0 = __shfl_sync(0xffffffffu, r.w0, s.src), pl = __shfl_sync(0xffffffffu, r.pl, s.src);
+    const int cl = (int)(__shfl_sync(0xffffffffu, r.lc, s.src) >> 8);
+    return w0 + (uint32_t)(s.v + (s.v >= cl)) * pl;
+}
+__device__ __forceinline__ uint64_t step_pk(const ItemRow &r, const ItemStep &s)
+{
+    const uint32_t lc = __shfl_sync(0xffffffffu, r.lc, s.src);
+    const uint32_t lo = __shfl_sync(0xffffffffu, (uint32_t)r.pk, s.src);
+    const uint32_t hi = __shfl_sync(0xffffffffu, (uint32_t)(r.pk >> 32), s.src);
+    return cov_setnib(((uint64_t)hi << 32) | lo, (int)(lc & 255u), s.v + (s.v >= (int)(lc >> 8)));
+}
+// the lanes of step k that work the words of this lane's item
+__device__ __forceinline__ unsigned item_lanes(int k, int qm1)
+{
+    const int o = (int)(threadIdx.x & 31) * qm1 - k * 32;
+    const unsigned m = (1u << qm1) - 1u;
+    return o >= 32 || o <= -qm1 ? 0u : o >= 0 ? m << o : m >> -o;
+}
+
 // Leaving / entering pairs of a commit (covsearch2e.c:450-493): the S'
 // patterns of R positions avoiding p, q-1 values of the last one per item.
 //
@@ -740,8 +797,7 @@ __device__ __forceinline__ void commit_events(const CovSlot &d, const OpParams &
 // per counter with one or two lanes active -- 1,230 warp-instructions for 32
 // items at q7 n9 R4, most of them there.  The events go to a queue of the warp
 // instead and are worked 32 at a time: the move phase of one instance at q7 n9
-// R4 takes 34 us for 54 on a cluster of 8, 103 for 155 on one of 2; 64
-// instances together are bound by random DRAM sectors (3 TB/s) either way.
+// R4 takes 34 us for 54 on a cluster of 8, 103 for 155 on one of 2.
 __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpParams &P, Smem &S, uint32_t wid,
                                                uint32_t wstride, int &T, long long &dunc)
 {
@@ -755,31 +811,33 @@ __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpPara
     uint32_t *const qtag = S.ev_tag[threadIdx.x >> 5];
     const unsigned below = (1u << lane) - 1u;
     int qn = 0;                                    // events in the queue
-    constexpr int CH = 8;
+    const uint32_t inv = 65536u / (uint32_t)qm1 + 1u;
+    constexpr int CH = 8;                          // one chunk for q <= 9
     for (uint32_t t0 = wid * 32; t0 < nstep; t0 += wstride) {
         const uint32_t t = t0 + lane;
         const bool live = t < nit;
         int dt = 0;
         int key = -1;
         const uint8_t *ps = subp;
-        // every word of the item is distinct: all 2(q-1) counters are
+        // the words of a move are distinct: the counters of up to CH steps are
         // loaded before any is written, so the loads are in flight together
-        CovItem it = cov_item(d, subp, R, live ? t : 0, P.base, P.pc);
+        const CovItem it = cov_item(d, subp, R, live ? t : 0, P.base, P.pc);
         if (live) {
             key = (int)(t / d.ppow[R - 1]);
             ps = it.ps;
         }
-        // values of the last position in chunks of CH (one chunk for q <= 9)
+        const ItemRow row = item_row(d, it);
+        const int items = (int)min(32u, nit - t0);
         for (int kb = 0; kb < qm1; kb += CH) {
-            uint32_t oa[CH], ob[CH];
-            if (live) {
+            uint32_t oa[CH], ob[CH], wa[CH];
 #pragma unroll
-                for (int kc = 0; kc < CH; kc++) {
-                    if (kb + kc < qm1) {
-                        uint32_t a; uint64_t pka;
-                        cov_item_word(d, it, kb + kc, a, pka);
-                        oa[kc] = cov_ldcg(&d.cw[a]);
-                        ob[kc] = cov_ldcg(&d.cw[a + P.dv]);
+            for (int kc = 0; kc < CH; kc++) {
+                if (kb + kc < qm1) {
+                    const ItemStep st = item_step(kb + kc, qm1, inv);
+                    wa[kc] = step_word(row, st);
+                    if (st.src < items) {
+                        oa[kc] = cov_ldcg(&d.cw[wa[kc]]);
+                        ob[kc] = cov_ldcg(&d.cw[wa[kc] + P.dv]);
                     }
                 }
             }
@@ -787,16 +845,15 @@ __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpPara
 #pragma unroll
             for (int kc = 0; kc < CH; kc++) {
                 if (kb + kc < qm1) {
+                    const ItemStep st = item_step(kb + kc, qm1, inv);
                     int evd = -1, evi = -1;
                     uint32_t kd = 0, ki = 0;
-                    uint64_t pka = 0;
-                    if (live) {
-                        uint32_t a;
-                        cov_item_word(d, it, kb + kc, a, pka);
-                        const uint32_t o1 = oa[kc], o2 = ob[kc];
+                    bool out1 = false, in0 = false;
+                    if (st.src < items) {
+                        const uint32_t a = wa[kc], o1 = oa[kc], o2 = ob[kc];
                         const uint32_t c1 = o1 & 0xffffu, c2 = o2 & 0xffffu;
-                        dt -= c1 == 1;
-                        dt += c2 == 0;
+                        out1 = c1 == 1;
+                        in0 = c2 == 0;
                         if (c1 == 0 || c2 == 0xffffu) {
                             set_error(d, COV_EDRIFT);
                         } else {
@@ -809,8 +866,11 @@ __device__ __forceinline__ void commit_pairs_lane(const CovSlot &d, const OpPara
                             else if (c2 == 1) { evi = EV_SHARED; ki = o2 >> 16; }
                         }
                     }
+                    const unsigned mine = item_lanes(kb + kc, qm1);
+                    dt += __popc(__ballot_sync(0xffffffffu, in0) & mine) - __popc(__ballot_sync(0xffffffffu, out1) & mine);
                     const unsigned md = __ballot_sync(0xffffffffu, evd >= 0), mi = __ballot_sync(0xffffffffu, evi >= 0);
                     if (md | mi) {
+                        const uint64_t pka = step_pk(row, st);
                         if (evd >= 0) {
                             const int at = qn + __popc(md & below);
                             qpk[at] = pka;
@@ -848,8 +908,9 @@ __device__ __forceinline__ void commit_pairs_warp(const CovSlot &d, const OpPara
     const uint32_t nstep = (nit + 31) / 32 * 32;
     const int qm1 = d.q - 1;
 
-        // many events: collected per warp into the shared table
+    // many events: collected per warp into the shared table
     const uint32_t unit = cov_cw_unit(P.mi);
+    const uint32_t inv = 65536u / (uint32_t)qm1 + 1u;
     constexpr int CH = 8;
     for (uint32_t t0 = wid * 32; t0 < nstep; t0 += wstride) {
         const uint32_t t = t0 + lane;
@@ -857,59 +918,59 @@ __device__ __forceinline__ void commit_pairs_warp(const CovSlot &d, const OpPara
         int dt = 0;
         int key = -1;
         const uint8_t *ps = subp;
-        // every word of the item is distinct: all 2(q-1) counters are
-        // loaded before any is written, so the loads are in flight together
-        CovItem it = cov_item(d, subp, R, live ? t : 0, P.base, P.pc);
+        const CovItem it = cov_item(d, subp, R, live ? t : 0, P.base, P.pc);
         if (live) {
             key = (int)(t / d.ppow[R - 1]);
             ps = it.ps;
         }
-        // values of the last position in chunks of CH (one chunk for q <= 9)
+        const ItemRow row = item_row(d, it);
+        const int items = (int)min(32u, nit - t0);
         for (int kb = 0; kb < qm1; kb += CH) {
-        uint32_t oa[CH], ob[CH];
-        if (live) {
+            uint32_t oa[CH], ob[CH], wa[CH];
 #pragma unroll
             for (int kc = 0; kc < CH; kc++) {
                 if (kb + kc < qm1) {
-                    uint32_t a; uint64_t pka;
-                    cov_item_word(d, it, kb + kc, a, pka);
-                    oa[kc] = cov_ldcg(&d.cw[a]);
-                    ob[kc] = cov_ldcg(&d.cw[a + P.dv]);
-                }
-            }
-        }
-        // leaving word a loses codeword i, entering word a + dv gains it
-        // (the steps of word_dec_v / word_inc_v, with the private-count
-        // events handed to the warp-wide adjust)
-#pragma unroll
-        for (int kc = 0; kc < CH; kc++) {
-            if (kb + kc < qm1) {
-                bool evd = false, evi = false;
-                int kd = 0, ki = 0;
-                uint64_t pka = 0;
-                if (live) {
-                    uint32_t a;
-                    cov_item_word(d, it, kb + kc, a, pka);
-                    const uint32_t o1 = oa[kc], o2 = ob[kc];
-                    const uint32_t c1 = o1 & 0xffffu, c2 = o2 & 0xffffu;
-                    dt -= c1 == 1;
-                    dt += c2 == 0;
-                    if (c1 == 0 || c2 == 0xffffu) {
-                        set_error(d, COV_EDRIFT);
-                    } else {
-                        const uint32_t n1 = o1 - unit;
-                        cov_stcg(&d.cw[a], n1);
-                        cov_stcg(&d.cw[a + P.dv], o2 + unit);
-                        if (c1 == 1) { ul_insert(d, P.ul_valid, a, pka); zb_set(d, a); dunc += 1; }
-                        else if (c1 == 2) { evd = true; kd = (int)(n1 >> 16); }
-                        if (c2 == 0) { zb_clear(d, a + P.dv); dunc -= 1; }
-                        else if (c2 == 1) { evi = true; ki = (int)(o2 >> 16); }
+                    const ItemStep st = item_step(kb + kc, qm1, inv);
+                    wa[kc] = step_word(row, st);
+                    if (st.src < items) {
+                        oa[kc] = cov_ldcg(&d.cw[wa[kc]]);
+                        ob[kc] = cov_ldcg(&d.cw[wa[kc] + P.dv]);
                     }
                 }
-                warp_private_adjust(d, tab, evd, kd, pka, +1);
-                warp_private_adjust(d, tab, evi, ki, cov_setnib(pka, P.mp, P.mv), -1);
             }
-        }
+            // leaving word a loses codeword i, entering word a + dv gains it
+            // (the steps of word_dec_v / word_inc_v, with the private-count
+            // events handed to the warp-wide adjust)
+#pragma unroll
+            for (int kc = 0; kc < CH; kc++) {
+                if (kb + kc < qm1) {
+                    const ItemStep st = item_step(kb + kc, qm1, inv);
+                    const uint64_t pka = step_pk(row, st);
+                    bool evd = false, evi = false, out1 = false, in0 = false;
+                    int kd = 0, ki = 0;
+                    if (st.src < items) {
+                        const uint32_t a = wa[kc], o1 = oa[kc], o2 = ob[kc];
+                        const uint32_t c1 = o1 & 0xffffu, c2 = o2 & 0xffffu;
+                        out1 = c1 == 1;
+                        in0 = c2 == 0;
+                        if (c1 == 0 || c2 == 0xffffu) {
+                            set_error(d, COV_EDRIFT);
+                        } else {
+                            const uint32_t n1 = o1 - unit;
+                            cov_stcg(&d.cw[a], n1);
+                            cov_stcg(&d.cw[a + P.dv], o2 + unit);
+                            if (c1 == 1) { ul_insert(d, P.ul_valid, a, pka); zb_set(d, a); dunc += 1; }
+                            else if (c1 == 2) { evd = true; kd = (int)(n1 >> 16); }
+                            if (c2 == 0) { zb_clear(d, a + P.dv); dunc -= 1; }
+                            else if (c2 == 1) { evi = true; ki = (int)(o2 >> 16); }
+                        }
+                    }
+                    const unsigned mine = item_lanes(kb + kc, qm1);
+                    dt += __popc(__ballot_sync(0xffffffffu, in0) & mine) - __popc(__ballot_sync(0xffffffffu, out1) & mine);
+                    warp_private_adjust(d, tab, evd, kd, pka, +1);
+                    warp_private_adjust(d, tab, evi, ki, cov_setnib(pka, P.mp, P.mv), -1);
+                }
+            }
         }
         T += dt;
         if (t0 < nit) group_add_h(S.partH, key, dt, ps, R, -1);
@@ -985,6 +1046,7 @@ __device__ __forceinline__ void op_move_t(const CovSlot &d, const OpParams &P, S
         } else {
             const uint8_t *subq = d.sub1 + (size_t)P.mp * d.nsub1 * d.rs;
             const uint32_t pq = d.ppow[R - 2];
+            const uint32_t inv = 65536u / (uint32_t)qm1 + 1u;
             const uint32_t nxy = (uint32_t)d.nsub1 * pq;
             const uint32_t nstep2 = (nxy + 31) / 32 * 32;
             // the turns go on where the pairs above left off (the first warps
@@ -997,23 +1059,36 @@ __device__ __forceinline__ void op_move_t(const CovSlot &d, const OpParams &P, S
                 int dy = 0;
                 int key = -1;
                 const uint8_t *ps = subq;
+                const CovItem it = cov_item(d, subq, R - 1, t < nxy ? t : 0, P.base, P.pc);
                 if (t < nxy) {
-                    CovItem it = cov_item(d, subq, R - 1, t, P.base, P.pc);
                     key = (int)(t / pq);
                     ps = it.ps;
-                    uint32_t cy[COV_MAXQ - 1], cx[COV_MAXQ - 1];
+                }
+                const ItemRow row = item_row(d, it);
+                const int items = (int)min(32u, nxy - t0);
+                constexpr int CH = 8;
+                for (int kb = 0; kb < qm1; kb += CH) {
+                    uint32_t cy[CH], cx[CH];
 #pragma unroll
-                    for (int kk = 0; kk < COV_MAXQ - 1; kk++) {
-                        if (kk < qm1) {
-                            uint32_t y; uint64_t pky;
-                            cov_item_word(d, it, kk, y, pky);
-                            cy[kk] = cov_ldcg(&d.cw[y]);
-                            cx[kk] = cov_ldcg(&d.cw[y + P.dv]);
+                    for (int kc = 0; kc < CH; kc++) {
+                        cy[kc] = cx[kc] = 0;
+                        if (kb + kc < qm1) {
+                            const ItemStep st = item_step(kb + kc, qm1, inv);
+                            const uint32_t y = step_word(row, st);
+                            if (st.src < items) {
+                                cy[kc] = cov_ldcg(&d.cw[y]);
+                                cx[kc] = cov_ldcg(&d.cw[y + P.dv]);
+                            }
                         }
                     }
 #pragma unroll
-                    for (int kk = 0; kk < COV_MAXQ - 1; kk++)
-                        if (kk < qm1) dy += (int)((cy[kk] & 0xffffu) == 1) - (int)((cx[kk] & 0xffffu) == 1);
+                    for (int kc = 0; kc < CH; kc++) {
+                        if (kb + kc < qm1) {
+                            const unsigned mine = item_lanes(kb + kc, qm1);
+                            dy += __popc(__ballot_sync(0xffffffffu, (cy[kc] & 0xffffu) == 1) & mine) -
+                                  __popc(__ballot_sync(0xffffffffu, (cx[kc] & 0xffffu) == 1) & mine);
+                        }
+                    }
                 }
                 T += dy;
                 if (t0 < nxy) group_add_h(S.partH, key, dy, ps, R - 1, P.mp);
