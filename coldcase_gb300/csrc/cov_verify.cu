@@ -1,19 +1,21 @@
 // cov_verify.cu -- GB300 (sm_103a) verification kernels for covering codes.
 //
 //   * exact per-word minimum distance to a code (the distance transform),
-//     computed as n axis passes of the line-min recurrence
-//         D'(x) = min(D(x), 1 + min_a D(x with x_j := a))
-//     over uint8 values.  After the passes over axes 0..n-1, D(x) is the
+//     computed as axis passes of the line-min recurrence
+//         D'(x) = min(D(x), 1 + min_a D(x with x_j := a)).
+//     After the passes over axes 0..n-1, D(x) is the
 //     Hamming distance from x to the nearest codeword -- the `best` array of
 //     cov/verify_independent.py:144-186 -- and #{x : D(x) > R} is the
 //     uncovered count that cov/verify_cov.py:109-230 returns.
-//     The n passes are grouped so that HBM is swept twice, not n times:
-//     the low axes of a contiguous tile, then the high axes of a column
-//     strip, each group worked in shared memory.  The histogram of D is
-//     folded into the last pass.
+//     Few codewords: every tile of the word space is made from the code
+//     alone, with the values of a line or of a block of two digits as masks,
+//     and each distance is written once.  Many: uint8 values, the low axes
+//     of a contiguous tile, then the high axes of column strips, each group
+//     worked in shared memory.  The histogram of D is folded into the last
+//     pass.
 //   * coverage multiplicity cnt[x] = #{i : d(x,c_i) <= R} by marking every
-//     codeword's ball (covsearch2e.c:353-380, 958-967), with 32-bit atomics
-//     on packed uint16 pairs.
+//     codeword's ball (covsearch2e.c:353-380, 958-967) tile by tile in shared
+//     memory (cov_tiles.cuh).
 #include <cmath>
 #include <mutex>
 #include <cstdio>
@@ -1081,8 +1083,11 @@ int geom(int q, int n, DtGeom &g)
 // between calls (more goes back at the next synchronisation).  The default
 // pool gives everything back at each, and a call that maps memory anew takes
 // 100 to 200 us longer; so did a cudaMalloc and cudaFree for each buffer
-// (6^6: 213 us for a transform of 11).
-#define SCRATCH_KEEP (16ull << 20)
+// (6^6: 213 us for a transform of 11).  A pool reserves 32 MB at a time and
+// goes by what it has reserved, so that a limit of 16 MB kept nothing over a
+// device synchronisation: a lone call took 264 us, and takes 62 with two such
+// pieces kept.
+#define SCRATCH_KEEP (64ull << 20)
 
 int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
 {
@@ -1449,12 +1454,13 @@ int64_t cov_count_above_dev(int32_t q, int32_t n, const uint8_t *d_dist, int32_t
     unsigned long long *d_c = nullptr, h = 0;
     rc = scratch_alloc((void **)&d_c, 8, st);
     if (rc) return rc;
-    CK(cudaMemsetAsync(d_c, 0, 8, st));
+    cudaError_t e = cudaMemsetAsync(d_c, 0, 8, st);
     k_count_above<<<std::max(1, cov_sm_count()) * 8, 256, 0, st>>>(d_dist, g.N, R, d_c);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(&h, d_c, 8, cudaMemcpyDeviceToHost, st));
-    CK(cudaFreeAsync(d_c, st));
-    CK(cudaStreamSynchronize(st));
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, d_c, 8, cudaMemcpyDeviceToHost, st);
+    cudaFreeAsync(d_c, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    CK(e);
     return (int64_t)h;
 }
 
@@ -1527,12 +1533,12 @@ int cov_count_dev(int32_t q, int32_t n, int32_t R, const uint8_t *d_code, int32_
     uint32_t *hi = (uint32_t *)(mid + M);
     if (M > 0) {
         k_count_records<<<std::min(1024, (M + 127) / 128), 128, 0, st>>>(d_code, M, q, n, g.nh, g.nl, mid, hi);
-        CK(cudaGetLastError());
     }
     ct_launch(g, BtCode{hi, mid}, d_cnt, st);
-    CK(cudaGetLastError());
-    CK(cudaStreamSynchronize(st));
-    CK(cudaFreeAsync(tmp, st));
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    cudaFreeAsync(tmp, st);
+    CK(e);
     return COV_OK;
 }
 
