@@ -383,10 +383,11 @@ def sym_cpu_measure(moves):
 
 
 def dt_pass_bytes(q, n):
-    """HBM bytes the distance transform's kernels must move per launch: the
-    code bitmap read (N/8), the low-axes tile pass writing every word once
-    (N), and one read + write of every word per high-axes strip pass (the
-    same grouping of axes as cov_verify.cu's dt_run)."""
+    """HBM bytes the distance transform of a dense code must move per launch
+    (k_dt_low, k_dt_high): the code bitmap read (N/8), the low-axes tile pass
+    writing every word once (N), and one read + write of every word per
+    high-axes strip pass (the same grouping of axes as cov_verify.cu's
+    dt_run).  The form for few codewords writes N and reads the code."""
     N = q ** n
     q4 = (q + 3) // 4 * 4
 
@@ -463,7 +464,7 @@ def coverage_bench(args, code79, dev):
         if unc_dt != unc_ct:
             raise RuntimeError("distance transform and count disagree at %d^%d: %d vs %d" % (q, n, unc_dt, unc_ct))
         algo = 2 * n * Nw                       # n per-axis uint8 read+write sweeps
-        need = dt_pass_bytes(q, n)
+        need = Nw                               # few codewords: each distance written once, tiles from the code
         cbytes = 2 * 2 * M * sum(math.comb(n, i) * (q - 1) ** i for i in range(R + 1))
         key = "q%dn%d" % (q, n)
         out[key] = dict(
@@ -476,8 +477,8 @@ def coverage_bench(args, code79, dev):
                                   pass_bytes=need, pass_frac=need / (dt_ms / 1e3) / 1e9 / peak,
                                   peak_source=kind + " (MEASURED_PEAKS.json hbm_gbs)",
                                   note="algorithmic bytes = 2 n N (n axis passes, uint8 read + write); "
-                                       "the kernels fuse the passes into %d HBM sweeps, pass_bytes" % (
-                                           1 + (need - Nw // 8 - Nw) // (2 * Nw)))),
+                                       "the kernels write each distance once, pass_bytes (a dense code's "
+                                       "sweeps would move %.1f bytes a word)" % (dt_pass_bytes(q, n) / Nw))),
             count=dict(ms=ct_ms, words_s=Nw / (ct_ms / 1e3),
                        roofline=dict(bound="hbm", achieved=cbytes / (ct_ms / 1e3) / 1e9, peak=peak, unit="GB/s",
                                      frac=cbytes / (ct_ms / 1e3) / 1e9 / peak, algorithmic_bytes=cbytes,
@@ -1035,7 +1036,7 @@ def gpu_bench(args, rank, world, dist):
                                      best_red_uncovered=int(st["best"]))
                     if not ge:
                         one[form]["us_per_move"] = {k: round(v / 2070.0, 1) for k, v in phases.items() if v}
-            one["grid"]["note"] = "estimates by a grid-wide launch per move, the rest on the cluster"
+            one["grid"]["note"] = "every bulk operation over the whole GPU in one cooperative launch"
         seeds = replicas.shard(list(range(1000, 1000 + args.sym_batch * world)), rank, world)
         with SymPool(len(seeds), cluster=args.sym_cluster, budget_s=120.0) as sp:
             slots = [sp.add(qq, qn, qR, qM, seed=sd) for sd in seeds]

@@ -573,8 +573,8 @@ __device__ __forceinline__ unsigned long long warp_max64(unsigned long long k)
 // gathers for 182,791 at q7 n9 R4, from 6.6 MB instead of 81 MB), and a step
 // costs its two grid barriers and some six dependent trips to L2 whatever the
 // number of candidates counted: 11 us for 25 candidates at 6^9, against 15 us
-// for one on a cluster of 8 CTAs.  The fill of 6^9 (651 words) spends 42 ms
-// here where the cluster took 247.
+// for one on a cluster of 8 CTAs.  The fill of 6^9 (651 words) spends some 28
+// ms here where the cluster took 247.
 __global__ void __launch_bounds__(GREEDY_NT) k_lns_greedy(GreedyArgs a)
 {
     extern __shared__ int gr_own[];                // [own] bounds, [own] epochs at which they were exact
@@ -1034,8 +1034,8 @@ double tiles_ps(const cov_lns *h, long long m)
 // off it; else the transform of the masks, some 22 ps a word and one launch
 // less (spaces below a million words gain nothing: 17 to 90 ms fills of 6^6 to
 // 7^7 with and without).  Map at 7^9: 0.92 ms by transform, 0.07 to 0.25 by
-// tiles of 10 to 3000 words.  Six rounds at 7^9 48 -> 29 ms, the fill of 6^9
-// 71 -> 65.
+// tiles of 10 to 3000 words.  Six rounds at 7^9 48 -> 29 ms (25 with fewer
+// exact counts before a refresh), the fill of 6^9 71 -> 65.
 // *tiled: the map came from tiles.
 int lns_greedy_map(cov_lns *h, long long left, long long gone, bool *tiled)
 {
@@ -1449,8 +1449,9 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
     a.wait_ns = 2000000000ull;
     a.st = h->seq;
     // exact counts for one placement past which a map is the better buy.
-    // Fills with limits of 64, 256 and 1000: 6^9 116, 114, 151 ms; 7^9 518,
-    // 444, 475; 4^11 45, 48, 70.  A quarter of it where tiles make the map
+    // Fills of 6^9 with limits of 25, 50, 100, 200 and 400: 78.6, 67.9, 66.0,
+    // 69.8, 82.0 ms; with 64, 256 and 1000, at maps of twice the time: 7^9
+    // 518, 444, 475; 4^11 45, 48, 70.  A quarter of it where tiles make the map
     // (six rounds at 7^9 with 40, 80, 160, 320: 24.8, 24.8, 25.6, 28.9 ms).
     const int evals_map = (int)std::max<long long>(64, std::min<long long>(1024, (long long)h->N / 131072));
     const int evals_tiles = std::max(64, evals_map / 4);

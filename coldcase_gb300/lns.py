@@ -6,9 +6,9 @@ every decision read off exact counts kept on the device (cov_lns_* in
 libcovgpu.so).  The search here is its own design:
 
   * recreate -- cov_lns_greedy: the lazy greedy placement runs on the device
-    (a persistent cluster kernel re-counts the best gain bound exactly until
-    it is current, then places it), so a placement costs no host round trip;
-    the host only asks for it.  Each placed word covers as many uncovered
+    (one kernel over the whole GPU re-counts the best gain bounds exactly
+    until the best is current, then places it), so a placement costs no host
+    round trip; the host only asks for it.  Each placed word covers as many uncovered
     words as any word can (ties to the lower index).
   * ruin -- k codewords leave, chosen by one of four rules drawn with fixed
     weights: a soft minimum of their exact losses (Gumbel top-k: codewords

@@ -317,9 +317,10 @@ int cov_lns_peel(cov_lns *h, const uint32_t *idx, int32_t k, uint8_t *removed, i
  * up to `room` words, each one of maximal exact gain (#uncovered words it
  * covers; ties to the lower index), until everything is covered or no word
  * gains.  Bounds come from the gain map: at most cand_cap candidates above a
- * threshold stay on the device, and a persistent cluster kernel re-counts
- * the best bound exactly until it is current, then places it; the host only
- * refreshes the map when the threshold is reached.  placed[] receives the
+ * threshold stay on the device, and one kernel over the whole GPU re-counts
+ * the best bounds exactly until the best is current, then places it; the
+ * host only refreshes the map, when the threshold is reached or so many
+ * counts were made that a map is cheaper.  placed[] receives the
  * words in order; stats (may be null): refreshes, exact counts. */
 int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed, int32_t *nplaced,
                    int64_t *uncovered, int64_t *stats);
