@@ -472,13 +472,13 @@ def coverage_bench(args, code79, dev):
             l2="resident (%.0f MB uint8 array)" % (Nw / 1e6) if Nw < 1.2e8 else
                "HBM-resident (%.0f MB uint8 array > L2)" % (Nw / 1e6),
             dt=dict(ms=dt_ms, words_s=Nw / (dt_ms / 1e3),
-                    roofline=dict(bound="hbm", achieved=algo / (dt_ms / 1e3) / 1e9, peak=peak, unit="GB/s",
-                                  frac=algo / (dt_ms / 1e3) / 1e9 / peak, algorithmic_bytes=algo,
-                                  pass_bytes=need, pass_frac=need / (dt_ms / 1e3) / 1e9 / peak,
+                    roofline=dict(bound="hbm", achieved=need / (dt_ms / 1e3) / 1e9, peak=peak, unit="GB/s",
+                                  frac=need / (dt_ms / 1e3) / 1e9 / peak, algorithmic_bytes=need,
+                                  axis_sweep_bytes=algo,
                                   peak_source=kind + " (MEASURED_PEAKS.json hbm_gbs)",
-                                  note="algorithmic bytes = 2 n N (n axis passes, uint8 read + write); "
-                                       "the kernels write each distance once, pass_bytes (a dense code's "
-                                       "sweeps would move %.1f bytes a word)" % (dt_pass_bytes(q, n) / Nw))),
+                                  note="algorithmic bytes = N (each distance written once); n uint8 axis sweeps "
+                                       "would move 2 n N, a dense code's fused sweeps %.1f bytes a word" % (
+                                           dt_pass_bytes(q, n) / Nw))),
             count=dict(ms=ct_ms, words_s=Nw / (ct_ms / 1e3),
                        roofline=dict(bound="hbm", achieved=cbytes / (ct_ms / 1e3) / 1e9, peak=peak, unit="GB/s",
                                      frac=cbytes / (ct_ms / 1e3) / 1e9 / peak, algorithmic_bytes=cbytes,
