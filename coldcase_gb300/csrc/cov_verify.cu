@@ -45,12 +45,26 @@ struct DtGeom {
 };
 
 // --------------------------------------------------------- code bitmap ----
+// Index of the word with the n digits c, all ones (which is no index) when a
+// digit lies outside the alphabet: the sum alone could be another word's, or
+// lie past the end of the scratch that it indexes.
+__device__ __forceinline__ uint32_t dt_word(const uint8_t *__restrict__ c, int n, uint32_t q)
+{
+    uint32_t x = 0;
+    bool word = true;
+    for (int j = 0; j < n; j++) {
+        const uint32_t a = c[j];
+        word = word && a < q;
+        x = x * q + a;
+    }
+    return word ? x : 0xffffffffu;
+}
+
 __global__ void k_dt_bitmap(const uint8_t *__restrict__ code, int M, DtGeom g, uint32_t *bm)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-        uint32_t x = 0;
-        for (int j = 0; j < g.n; j++) x = x * (uint32_t)g.q + code[(size_t)i * g.n + j];
-        atomicOr(&bm[x >> 5], 1u << (x & 31));
+        const uint32_t x = dt_word(code + (size_t)i * g.n, g.n, (uint32_t)g.q);
+        if (x != 0xffffffffu) atomicOr(&bm[x >> 5], 1u << (x & 31));
     }
 }
 
@@ -342,9 +356,7 @@ template <int Q>
 __global__ void k_dt_records(const uint8_t *__restrict__ code, int M, DtGeom g, int nl, uint2 *__restrict__ rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-        uint32_t x = 0;
-        for (int j = 0; j < g.n; j++) x = x * (uint32_t)Q + code[(size_t)i * g.n + j];
-        if (x >= g.N) x = 0xffffffffu;           // a digit outside the alphabet: no word
+        const uint32_t x = dt_word(code + (size_t)i * g.n, g.n, (uint32_t)Q);
         uint32_t hi = x / g.pw[nl], h = 0;
         const uint32_t lo = x - hi * g.pw[nl];
         for (int j = 0; j < g.n - nl; j++) { h |= (hi % (uint32_t)Q) << (4 * j); hi /= (uint32_t)Q; }
@@ -548,9 +560,7 @@ template <int Q>
 __global__ void k_dt_block_records(const uint8_t *__restrict__ code, int M, DtGeom g, int nl, uint2 *__restrict__ rec)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < M; i += gridDim.x * blockDim.x) {
-        uint32_t x = 0;
-        for (int j = 0; j < g.n; j++) x = x * (uint32_t)Q + code[(size_t)i * g.n + j];
-        if (x >= g.N) x = 0xffffffffu;           // a digit outside the alphabet: no word
+        const uint32_t x = dt_word(code + (size_t)i * g.n, g.n, (uint32_t)Q);
         uint32_t hi = x / g.pw[nl], h = 0;
         const uint32_t lo = x - hi * g.pw[nl];
         for (int j = 0; j < g.n - nl; j++) { h |= (hi % (uint32_t)Q) << (4 * j); hi /= (uint32_t)Q; }

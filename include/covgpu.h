@@ -212,6 +212,8 @@ int cov_mindist(int32_t q, int32_t n, const uint8_t *code, int32_t M,
  * OUT=2 map of cov/gemm2/dct.cu:360-411. */
 int cov_count(int32_t q, int32_t n, int32_t R, const uint8_t *code, int32_t M,
               uint16_t *cnt, int64_t *uncovered);
+/* A codeword with a digit outside 0..q-1 is no word of the space and is
+ * ignored (the host forms refuse it with COV_EINVAL). */
 int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M,
                     uint8_t *d_dist, void *stream);
 /* d_cnt is updated in aligned 32-bit pairs: it must have room for q^n
