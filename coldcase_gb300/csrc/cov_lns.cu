@@ -41,11 +41,6 @@ namespace cg = cooperative_groups;
 
 #define LNS_NT 256
 #define LNS_HIST_MAX 8192   // bins of cov_lns_map_hist (one shared-memory counter each)
-#define MAP_SMEM_MAX (200 * 1024)   // shared memory of one map tile (bytes)
-#define MAP_SMEM_LOW (84 * 1024)    // of a low tile: two CTAs an SM at least
-#define MAP_SMEM_HIGH (112 * 1024)  // of a strip: two
-#define MAP_W_MIN 8                 // narrowest strip
-#define MAP_L2_BYTES (80 << 20)     // layers of the parts that are in flight between two sweeps
 #define SEQ_NT 512
 #define SEQ_CL 8                    // CTAs of the sequence cluster
 #define CAND_CAP (1 << 17)          // candidate bounds kept on the device per refresh
@@ -79,14 +74,11 @@ struct RefreshInfo {
 };
 enum { SEQ_DONE = 0, SEQ_REFRESH = 1, SEQ_COVERED = 2, SEQ_TARGET = 3, SEQ_GUARD = 5 };
 
-struct cov_lns {
+struct cov_lns : MapPlan {
     int q, n, R;
     uint32_t N;
     uint32_t pw[COV_MAXN];          // q^(n-1-j)
     uint16_t *cnt = nullptr;        // coverage multiplicity (saturated)
-    int kl = 0, ng = 0, gs[COV_MAXN] = {}, slots[COV_MAXN] = {};   // low axes, strip groups: their axes and layers (map_plan)
-    uint32_t parts = 1, at_once = 1;
-    size_t scratch_ints = 0, whole_ints = 0;
     int32_t *map_scratch = nullptr;      // the layers between the sweeps of a part (two of them from three groups on)
     int32_t *map_whole = nullptr;        // the layers that reach the last sweep
     int32_t *map = nullptr;         // last map (gain or loss)
@@ -868,10 +860,6 @@ int grid_of(uint32_t N)
 
 CovDeviceFlags g_map_attr;      // shared-memory opt-in of the map kernels, per device
 
-// a sweep of `layers` layers: kernels for 3, 5, 7 and 9, so that the registers
-// and the shared memory of an element stay few where the layers are
-int map_slots(int layers) { return layers <= 3 ? 3 : layers <= 5 ? 5 : layers <= 7 ? 7 : 9; }
-
 void map_kernels(int q, int layers, MapLow *low, MapHigh *high)
 {
     switch (map_slots(layers)) {
@@ -896,48 +884,6 @@ int map_attrs()
         }
     g_map_attr.set(dev);
     return 0;
-}
-
-// layers that a strip sweep of axes j0 .. j0+gsz-1 holds of an element
-int map_strip_slots(int n, int R, int j0, int gsz) { return map_slots(map_hi(R, j0 + gsz) - map_lo(n, R, j0) + 1); }
-
-uint32_t map_cols(int q, int k) { return ((uint32_t)bt_ipow(q, k) + 3u) & ~3u; }
-
-// a low tile at `slots` layers an element: the layers, the table of the
-// blocks' balls, the masks
-size_t map_low_smem(int q, int slots, int k, int nb, uint32_t blk)
-{
-    return (size_t)map_cols(q, k) * slots * 4 + (size_t)blk * (nb + 1) * 8 + (size_t)bt_ipow(q, k) / blk * 8;
-}
-
-// How the axes are grouped: the low ones in tiles at two CTAs an SM or more,
-// the others in strips of at least eight columns at two, in as few groups as that
-// allows, the larger ones first.
-void map_plan(cov_lns *h)
-{
-    const int q = h->q, n = h->n, R = h->R;
-    h->kl = h->nb;
-    while (h->kl < n && map_low_smem(q, map_slots(map_hi(R, h->kl + 1) + 1), h->kl + 1, h->nb, h->blk) <= MAP_SMEM_LOW)
-        h->kl++;
-    const int m = n - h->kl;
-    int gmax = 1;
-    while (gmax < m && bt_ipow(q, gmax + 1) * MAP_W_MIN * map_slots(R + 1) * 4 <= MAP_SMEM_HIGH) gmax++;
-    h->ng = (m + gmax - 1) / gmax;
-    for (int i = 0, left = m; i < h->ng; i++) {
-        h->gs[i] = (left + h->ng - i - 1) / (h->ng - i);
-        left -= h->gs[i];
-    }
-    for (int i = 0, j0 = h->kl; i < h->ng; j0 += h->gs[i++]) h->slots[i] = map_strip_slots(n, R, j0, h->gs[i]);
-    // All groups but the last work within the words that share the last
-    // group's digits.  A few such parts at a time go through them, so that
-    // what a sweep writes is still in L2 when the next one reads it.
-    h->parts = h->ng >= 2 ? (uint32_t)bt_ipow(q, h->gs[h->ng - 1]) : 1u;
-    int most = 0;
-    for (int i = 0; i < std::max(1, h->ng - 1); i++) most = std::max(most, h->slots[i]);
-    const long long cols = (long long)(h->N / h->parts) / bt_ipow(q, h->kl) * map_cols(q, h->kl);
-    h->at_once = (uint32_t)std::max(1LL, std::min<long long>(h->parts, MAP_L2_BYTES / (cols * most * 4)));
-    h->scratch_ints = h->ng ? (size_t)cols * h->at_once * most : 0;
-    h->whole_ints = h->ng >= 2 ? (size_t)cols * h->parts * h->slots[h->ng - 1] : 0;
 }
 
 // The layered transform of the marked words (masks um) or of the word counts
@@ -972,8 +918,7 @@ int lns_transform(cov_lns *h, const int32_t *A0, int32_t *out, uint16_t *cnt16)
         CK(cudaGetLastError());
         return 0;
     };
-    // the low kernel works at the slots of its reader where they hold its layers
-    const int lslots = std::max(map_slots(map_hi(R, h->kl) + 1), h->ng ? h->slots[0] : 0);
+    const int lslots = h->low_slots(R);
     const size_t lsm = map_low_smem(q, lslots, h->kl, h->nb, h->blk);
     const uint32_t part_tiles = h->N / h->parts / g.T;
     for (uint32_t p = 0; p < h->parts; p += h->at_once) {
@@ -1178,7 +1123,7 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
             for (uint32_t u = x, v = y, k = 0; k < (uint32_t)h->nb; k++, u /= q, v /= q) d += u % q != v % q;
             for (int sg = d; sg <= h->nb; sg++) low[(size_t)x * (h->nb + 1) + sg] |= 1ull << y;
         }
-    map_plan(h);
+    map_plan(*h, q, n, R, h->N, h->nb, h->blk);
     bool ok = cudaMalloc(&h->cnt, (size_t)N * 2) == cudaSuccess &&
               cudaMalloc(&h->map, (size_t)N * 4) == cudaSuccess &&
               cudaMalloc(&h->ball, items.size() * 8) == cudaSuccess &&

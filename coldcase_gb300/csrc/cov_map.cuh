@@ -4,6 +4,7 @@
 #pragma once
 #include <cstdint>
 #include <cuda_runtime.h>
+#include "cov_map_plan.h"
 
 #define LNS_MAXR 8
 #define MAP_LOW_NT 256
@@ -15,10 +16,6 @@ struct MapGeom {
     int32_t *out;                   // the map, or
     uint16_t *cnt16;                // the counts (saturated)
 };
-
-// layers of a tile with `done` of the n axes done: map_lo .. map_hi
-__host__ __device__ __forceinline__ int map_lo(int n, int R, int done) { return R - (n - done) > 0 ? R - (n - done) : 0; }
-__host__ __device__ __forceinline__ int map_hi(int R, int done) { return done < R ? done : R; }
 
 typedef void (*MapLow)(MapGeom, int, int, uint32_t, const uint64_t *, const uint64_t *, const int32_t *, uint32_t,
                        uint32_t, int32_t *, int);
