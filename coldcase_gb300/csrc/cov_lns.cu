@@ -80,7 +80,7 @@ struct cov_lns : MapPlan {
     uint32_t pw[COV_MAXN];          // q^(n-1-j)
     uint16_t *cnt = nullptr;        // coverage multiplicity (saturated)
     int32_t *map_scratch = nullptr;      // the layers between the sweeps of a part (two of them from three groups on)
-    int32_t *map_whole = nullptr;        // the layers that reach the last sweep
+    int32_t *map_whole = nullptr;        // the layers that reach the last sweep (and word counts: MapPlan)
     int32_t *map = nullptr;         // last map (gain or loss)
     uint64_t *ball = nullptr;       // whole-ball groups (cov_tiles.cuh, no high digits)
     uint8_t *ball_last = nullptr;
@@ -1141,8 +1141,8 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
               cudaMalloc(&h->acc, 4 * (3 * (GREEDY_MAXG + 1) + 1)) == cudaSuccess &&
               cudaMalloc(&h->info, sizeof(RefreshInfo)) == cudaSuccess &&
               cudaMalloc(&h->seq, sizeof(SeqState)) == cudaSuccess;
-    if (ok && h->scratch_ints)
-        ok = cudaMalloc(&h->map_scratch, h->scratch_ints * 4 * (h->ng >= 3 ? 2 : 1)) == cudaSuccess;
+    if (ok)
+        ok = cudaMalloc(&h->map_scratch, (h->scratch_ints * (h->ng >= 3 ? 2 : 1) + h->counts_ints) * 4) == cudaSuccess;
     if (ok && h->whole_ints) ok = cudaMalloc(&h->map_whole, h->whole_ints * 4) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
@@ -1194,17 +1194,19 @@ int cov_lns_recount(cov_lns *h, const uint32_t *idx, int32_t m)
     }
     int rc = lns_scratch(h, (size_t)m * 4);
     if (rc) return rc;
-    int32_t *a0 = nullptr;
-    if (cudaMalloc(&a0, (size_t)h->N * 4) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
-    auto done = [&](int r) { cudaFree(a0); return r; };
-    if (cudaMemset(a0, 0, (size_t)h->N * 4) != cudaSuccess ||
-        cudaMemcpy(h->scratch, idx, (size_t)m * 4, cudaMemcpyHostToDevice) != cudaSuccess)
-        return done(-100);
+    // (in the handle's own memory: an allocation of 4 q^n bytes for the call
+    // took 150 of the 430 us of 200,000 words at 7^8 R5, and could fail)
+    int32_t *const a0 = h->ng >= 2 ? h->map_whole + h->counts_at : h->map_scratch + h->scratch_ints;
+    CK(cudaMemsetAsync(a0, 0, (size_t)h->N * 4));
+    CK(cudaMemcpy(h->scratch, idx, (size_t)m * 4, cudaMemcpyHostToDevice));
     k_lns_scatter<<<(m + 255) / 256, 256>>>(a0, (const uint32_t *)h->scratch, m);
+    CK(cudaGetLastError());
     if (h->R == 0) k_lns_narrow<<<grid_of(h->N), LNS_NT>>>(a0, h->N, h->cnt);
     else rc = lns_transform(h, a0, nullptr, h->cnt);
-    if (!rc && cudaDeviceSynchronize() != cudaSuccess) rc = -100;
-    return done(rc);
+    if (rc) return rc;
+    CK(cudaGetLastError());
+    CK(cudaDeviceSynchronize());
+    return COV_OK;
 }
 
 int cov_lns_map(cov_lns *h, int32_t target)

@@ -53,6 +53,12 @@ struct MapPlan {
     int kl = 0, ng = 0, gs[MAP_MAXN] = {}, slots[MAP_MAXN] = {};   // low axes, strip groups: their axes and layers
     uint32_t parts = 1, at_once = 1;
     size_t scratch_ints = 0, whole_ints = 0;
+    // The word counts that a transform may start from instead of the masks lie
+    // at the end of the memory of the layers that reach the last sweep (two
+    // groups or more: what a part writes there ends before the counts of the
+    // parts after it), else in words of their own behind the scratch.
+    size_t counts_at = 0;               // in the layers' memory, or behind scratch_ints
+    size_t counts_ints = 0;             // words of their own
 
     // the low kernel works at the slots of its reader where they hold its layers
     int low_slots(int R) const { return std::max(map_slots(map_hi(R, kl) + 1), ng ? slots[0] : 0); }
@@ -68,6 +74,7 @@ static inline void map_plan(MapPlan &p, int q, int n, int R, uint32_t N, int nb,
     p.kl = nb;
     while (p.kl < n && map_low_smem(q, map_slots(map_hi(R, p.kl + 1) + 1), p.kl + 1, nb, blk) <= MAP_SMEM_LOW) p.kl++;
     const int m = n - p.kl;
+    p.counts_ints = N;
     if (m == 0) return;                  // one tile holds the space: no strips, nothing between sweeps
     int gmax = 1;
     while (gmax < m && map_ipow(q, gmax + 1) * MAP_W_MIN * map_slots(R + 1) * 4 <= MAP_SMEM_HIGH) gmax++;
@@ -86,5 +93,8 @@ static inline void map_plan(MapPlan &p, int q, int n, int R, uint32_t N, int nb,
     const long long cols = (long long)(N / p.parts) / map_ipow(q, p.kl) * map_cols(q, p.kl);
     p.at_once = (uint32_t)std::max(1LL, std::min<long long>(p.parts, MAP_L2_BYTES / (cols * most * 4)));
     p.scratch_ints = (size_t)cols * p.at_once * most;
-    p.whole_ints = p.ng >= 2 ? (size_t)cols * p.parts * p.slots[p.ng - 1] : 0;
+    if (p.ng < 2) return;
+    p.whole_ints = (size_t)cols * p.parts * p.slots[p.ng - 1];
+    p.counts_ints = 0;
+    p.counts_at = p.whole_ints - N;
 }

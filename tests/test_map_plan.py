@@ -56,15 +56,59 @@ int main()
 """
 
 
-def test_plan_of_every_cell(tmp_path):
+# Where the word counts that a transform may start from lie: the sweeps of a
+# part read its own, and nothing that a part leaves in the layers of the last
+# sweep reaches the counts of a later one.
+COUNTS = r"""
+#include <cstdio>
+#include "cov_map_plan.h"
+#define NEED(x) do { if (!(x)) { printf("q=%d n=%d R=%d: %s\n", q, n, R, #x); return 1; } } while (0)
+int main()
+{
+    int several = 0;
+    for (int q = 2; q <= 16; q++)
+        for (int n = 1; n <= 16 && map_ipow(q, n) < (1LL << 31); n++)
+            for (int R = 0; R <= (n < 8 ? n : 8); R++) {
+                int nb = 0;
+                uint32_t blk = 1;
+                while (nb < n && (long long)blk * q <= 64) { nb++; blk *= (uint32_t)q; }
+                const long long N = map_ipow(q, n);
+                MapPlan p;
+                map_plan(p, q, n, R, (uint32_t)N, nb, blk);
+                if (p.ng < 2) {
+                    NEED((long long)p.counts_ints >= N);
+                    continue;
+                }
+                NEED(p.counts_ints == 0 && p.counts_at + N <= p.whole_ints);
+                const long long T = map_ipow(q, p.kl), Tp = map_cols(q, p.kl), part = N / p.parts / T;
+                for (uint32_t k = 0; k < p.parts; k += p.at_once, several++) {
+                    const long long t1 = std::min<long long>(k + p.at_once, p.parts) * part;
+                    NEED(t1 * Tp * p.slots[p.ng - 1] <= (long long)p.counts_at + t1 * T);
+                }
+            }
+    printf("%d\n", several);
+    return several < 100;
+}
+"""
+
+
+def run_program(tmp_path, text):
     cxx = shutil.which(os.environ.get("CXX", "g++"))
     if not cxx:
         pytest.skip("no C++ compiler")
     src, exe = tmp_path / "plan.cpp", tmp_path / "plan"
-    src.write_text(PROGRAM)
+    src.write_text(text)
     subprocess.run([cxx, "-std=c++17", "-O1", "-fsanitize=undefined", "-fsanitize-undefined-trap-on-error",
                     "-I", os.path.join(REPO, "coldcase_gb300", "csrc"), str(src), "-o", str(exe)], check=True)
     p = subprocess.run([str(exe)], capture_output=True, text=True)
     assert p.returncode == 0, p.stdout + p.stderr
-    cells, single = (int(w) for w in (p.stdout.split()[0], p.stdout.split()[2]))
-    assert cells > 300 and 50 < single < cells
+    return p.stdout.split()
+
+
+def test_plan_of_every_cell(tmp_path):
+    words = run_program(tmp_path, PROGRAM)
+    assert int(words[0]) > 300 and 50 < int(words[2]) < int(words[0])
+
+
+def test_place_of_the_word_counts(tmp_path):
+    run_program(tmp_path, COUNTS)
