@@ -1195,7 +1195,7 @@ int cov_lns_recount(cov_lns *h, const uint32_t *idx, int32_t m)
     int rc = lns_scratch(h, (size_t)m * 4);
     if (rc) return rc;
     // (in the handle's own memory: an allocation of 4 q^n bytes for the call
-    // took 150 of the 430 us of 200,000 words at 7^8 R5, and could fail)
+    // took 200 of the 508 us of 200,000 words at 7^8 R5, and could fail)
     int32_t *const a0 = h->ng >= 2 ? h->map_whole + h->counts_at : h->map_scratch + h->scratch_ints;
     CK(cudaMemsetAsync(a0, 0, (size_t)h->N * 4));
     CK(cudaMemcpy(h->scratch, idx, (size_t)m * 4, cudaMemcpyHostToDevice));

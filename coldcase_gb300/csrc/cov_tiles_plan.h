@@ -1,0 +1,70 @@
+// cov_tiles_plan.h -- the tiles of a coverage count (cov_tiles.cuh): their
+// limits and their geometry.  Host arithmetic only, so that it compiles
+// without CUDA.
+#pragma once
+#include <cstddef>
+#include <cstdint>
+#include <algorithm>
+
+#define BT_SMEM_MAX (200 * 1024)    // shared memory of a tile CTA
+#define BT_LCH 4096            // codewords of a tile listed at once
+#define BT_NT  512             // threads of a tile CTA
+#define BT_ITEMS 1024          // ball groups held in shared memory
+
+static inline long long bt_ipow(long long b, int e)
+{
+    long long r = 1;
+    while (e-- > 0) r *= b;
+    return r;
+}
+
+// digits of a block: the last two (one for words of one digit)
+static inline int bt_block_digits(int n) { return n < 2 ? n : 2; }
+
+// ball groups of nm middle digits
+static inline long long bt_groups(int q, int nm, int R)
+{
+    long long g = 0, c = (long long)nm * (nm - 1) / 2;      // C(nm, r) (q-1)^(r-2)
+    for (int r = 2; r <= nm && r <= R; r++) {
+        g += c;
+        c = c * (nm - r) / (r + 1) * (q - 1);
+    }
+    return g;
+}
+
+// dynamic shared memory of a tile CTA: the ball groups, the list, then A0,
+// the row and column counters and B
+static inline size_t bt_smem_bytes(int q, int n, uint32_t tw)
+{
+    const size_t nblk = tw / (size_t)bt_ipow(q, bt_block_digits(n));
+    return BT_ITEMS * 4 + BT_LCH * 2 + ((size_t)tw + 2 * nblk * q + nblk) * 4;   // bt_layout's words
+}
+
+// Tile geometry: the number of low digits with the least estimate, in SM
+// cycles, of a tile's prefix tests (about 23 lane-instructions a codeword) and
+// words (14 a word) at 64 lanes a cycle and the latency chain of its phases
+// (some 6000 cycles, shared by the CTAs resident together).  An SM that works
+// at all works a whole tile, so fewer tiles than SMs share nothing: with their
+// work counted as spread over the chip, 8^6 R3 with 60000 codewords took eight
+// tiles of 8^5 words and 1690 us, and takes 64 and 312; 3^12 R3 M3000 65 and
+// 38.  Of 38 cells counted at every number of digits the choice is within 1 %
+// of the best in 32 and within 11 % in the rest (before: 1.1 to 5.4 times as
+// long in nine).  At most eight high and eight middle digits, which are held
+// as 32-bit nibbles.
+static inline void bt_geom(int q, int n, int R, int M, int *nh, int *nl)
+{
+    const int nb = bt_block_digits(n);
+    double least = 1e300;
+    *nl = -1;
+    for (int l = nb > n - 8 ? nb : n - 8; l <= n && l - nb <= 8; l++) {
+        const long long tw = bt_ipow(q, l);
+        if (tw > (1 << 20) || bt_smem_bytes(q, n, (uint32_t)tw) > BT_SMEM_MAX || bt_groups(q, l - nb, R) > BT_ITEMS)
+            break;
+        const double tiles = (double)bt_ipow(q, n - l);
+        const int res = (int)std::min<size_t>(4, (227 * 1024) / (bt_smem_bytes(q, n, (uint32_t)tw) + 1536));
+        const double waves = (double)(long long)((tiles + 152 * res - 1) / (152 * res));
+        const double cyc = std::max(1.0, tiles / 152) * (M * 23.0 + tw * 14.0) / 64.0 + waves * (6000.0 + M * 0.05);
+        if (cyc < least) { least = cyc; *nl = l; }
+    }
+    *nh = n - *nl;
+}
