@@ -3720,7 +3720,7 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     uint8_t *dsub = (uint8_t *)take_(tables.size());
     uint8_t *dball = dsub + subs.size(), *dsub1 = dball + balls.size();
     d.sub = dsub; d.ball_sub = dball; d.sub1 = dsub1;
-    bt_geom(q, n, R, Mw, &d.bt_nh, &d.bt_nl);
+    bt_geom(q, n, R, Mw, std::max(1, cov_sm_count()), &d.bt_nh, &d.bt_nl);
     d.bt_tw = (uint32_t)ipow_h(q, d.bt_nl);
     bt_vcum_h(q, n, R, d.bt_nl, d.bt_v);
     d.st = pool->d_states + s;

@@ -966,7 +966,7 @@ int lns_map_of_masks(cov_lns *h)
 double tiles_ps(const cov_lns *h, long long m)
 {
     int nh, nl;
-    bt_geom(h->q, h->n, h->R, (int)std::min<long long>(m, 1 << 30), &nh, &nl);
+    bt_geom(h->q, h->n, h->R, (int)std::min<long long>(m, 1 << 30), std::max(1, cov_sm_count()), &nh, &nl);
     double v = 1, c = 1;
     const int np = h->n - bt_block_digits(h->n);
     for (int r = 0; r < std::min(h->R, np); r++) { c = c * (np - r) / (r + 1) * (h->q - 1); v += c; }

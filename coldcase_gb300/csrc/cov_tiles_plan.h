@@ -50,8 +50,8 @@ static inline size_t bt_smem_bytes(int q, int n, uint32_t tw)
 // 38.  Of 38 cells counted at every number of digits the choice is within 1 %
 // of the best in 32 and within 11 % in the rest (before: 1.1 to 5.4 times as
 // long in nine).  At most eight high and eight middle digits, which are held
-// as 32-bit nibbles.
-static inline void bt_geom(int q, int n, int R, int M, int *nh, int *nl)
+// as 32-bit nibbles.  sms: the device's SMs.
+static inline void bt_geom(int q, int n, int R, int M, int sms, int *nh, int *nl)
 {
     const int nb = bt_block_digits(n);
     double least = 1e300;
@@ -62,8 +62,8 @@ static inline void bt_geom(int q, int n, int R, int M, int *nh, int *nl)
             break;
         const double tiles = (double)bt_ipow(q, n - l);
         const int res = (int)std::min<size_t>(4, (227 * 1024) / (bt_smem_bytes(q, n, (uint32_t)tw) + 1536));
-        const double waves = (double)(long long)((tiles + 152 * res - 1) / (152 * res));
-        const double cyc = std::max(1.0, tiles / 152) * (M * 23.0 + tw * 14.0) / 64.0 + waves * (6000.0 + M * 0.05);
+        const double waves = (double)(long long)((tiles + sms * res - 1) / (sms * res));
+        const double cyc = std::max(1.0, tiles / sms) * (M * 23.0 + tw * 14.0) / 64.0 + waves * (6000.0 + M * 0.05);
         if (cyc < least) { least = cyc; *nl = l; }
     }
     *nh = n - *nl;

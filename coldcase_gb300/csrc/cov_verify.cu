@@ -1163,7 +1163,7 @@ CountGeom count_geom(int q, int n, int R, int M)
     CountGeom g;
     memset(&g, 0, sizeof g);
     g.q = q; g.n = n; g.R = R; g.M = M;
-    bt_geom(q, n, R, M, &g.nh, &g.nl);
+    bt_geom(q, n, R, M, std::max(1, cov_sm_count()), &g.nh, &g.nl);
     g.tw = (uint32_t)ipw(q, g.nl);
     bt_vcum_h(q, n, R, g.nl, g.vcum);
     return g;

@@ -29,15 +29,16 @@ int main()
     for (int q = 2; q <= 16; q++)
         for (int n = 1; n <= 16 && bt_ipow(q, n) < (1LL << 32) - 1; n++)
             for (int R = 0; R <= n; R++)
-                for (int M : {0, 1, 50, 700, 5000, 20000, 65535, 1 << 20, 1 << 30}) {
-                    int nh = 0, nl = 0;
-                    bt_geom(q, n, R, M, &nh, &nl);
-                    NEED(nl >= 1 && nh + nl == n && fits(q, n, R, nl));
-                    if (M > 65535) continue;
-                    cells++;
-                    for (int l = 1; l < nl; l++)
-                        NEED(!fits(q, n, R, l) || bt_ipow(q, n - l) > 152);
-                }
+                for (int M : {0, 1, 50, 700, 5000, 20000, 65535, 1 << 20, 1 << 30})
+                    for (int sms : {1, 16, 132, 152}) {
+                        int nh = 0, nl = 0;
+                        bt_geom(q, n, R, M, sms, &nh, &nl);
+                        NEED(nl >= 1 && nh + nl == n && fits(q, n, R, nl));
+                        if (M > 65535) continue;
+                        cells++;
+                        for (int l = 1; l < nl; l++)
+                            NEED(!fits(q, n, R, l) || bt_ipow(q, n - l) > sms);
+                    }
     printf("%d\n", cells);
     return 0;
 }
