@@ -47,8 +47,8 @@ namespace cg = cooperative_groups;
 #define GREEDY_NT 512
 #define GREEDY_MAXG 512             // most CTAs of the greedy kernel (one per SM)
 #define THR_BINS 1024               // histogram bins behind an extraction threshold
-#define MAP_PS_WORD 20.0            // time of a map by transform, ps a word of the space
-#define MAP_PS_LAUNCH 20e6
+#define MAP_TILES_N 1000000u        // words of the smallest space whose greedy maps may come from tiles
+#define MAP_PS_LAUNCH 20e6          // what such a map has to save, ps
 #define NOTE_CAP (1 << 16)          // most words whose balls a refresh counts by tiles
 #define EXT_CHUNK 8192              // words of one block of an ordered extraction
 
@@ -961,34 +961,23 @@ int lns_map_of_masks(cov_lns *h)
     return 0;
 }
 
-// Estimate of counting the balls of m words by the verifier's tiles, in ps a
-// word of the space: 1.6 + 0.9 a mark + 0.6 a codeword per word of a tile.
-double tiles_ps(const cov_lns *h, long long m)
-{
-    int nh, nl;
-    bt_geom(h->q, h->n, h->R, (int)std::min<long long>(m, 1 << 30), std::max(1, cov_sm_count()), &nh, &nl);
-    double v = 1, c = 1;
-    const int np = h->n - bt_block_digits(h->n);
-    for (int r = 0; r < std::min(h->R, np); r++) { c = c * (np - r) / (r + 1) * (h->q - 1); v += c; }
-    return 1.6 + 0.9 * (double)m * v / h->N + 0.6 * (double)m / (double)bt_ipow(h->q, nl);
-}
-
 // The greedy's map of the uncovered words (masks um, `left` of them).  Few
 // uncovered words are counted by tiles from their list; few words covered
 // since the last map (`gone` of them; < 0: there is no last map) are counted
-// off it; else the transform of the masks, some 22 ps a word and one launch
-// less (spaces below a million words gain nothing: 17 to 90 ms fills of 6^6 to
-// 7^7 with and without).  Map at 7^9: 0.92 ms by transform, 0.07 to 0.25 by
+// off it; else the transform of the masks, one launch less (spaces below a
+// million words gain nothing: 17 to 90 ms fills of 6^6 to 7^7 with and
+// without).  Map at 7^9: 0.92 ms by transform, 0.07 to 0.25 by
 // tiles of 10 to 3000 words.  Six rounds at 7^9 48 -> 29 ms (25 with fewer
 // exact counts before a refresh), the fill of 6^9 71 -> 65.
 // *tiled: the map came from tiles.
 int lns_greedy_map(cov_lns *h, long long left, long long gone, bool *tiled)
 {
-    const double all_ps = left <= NOTE_CAP ? tiles_ps(h, left) + 0.6 : 1e300;
-    const double off_ps = gone >= 0 && gone <= NOTE_CAP ? tiles_ps(h, gone) + 1.2 : 1e300;
+    const int sms = std::max(1, cov_sm_count());
+    const double all_ps = left <= NOTE_CAP ? bt_count_ps(h->q, h->n, h->R, left, sms) + 0.6 * h->N : 1e300;
+    const double off_ps = gone >= 0 && gone <= NOTE_CAP ? bt_count_ps(h->q, h->n, h->R, gone, sms) + 1.2 * h->N : 1e300;
     *tiled = false;
-    if (h->R == 0 || MAP_PS_WORD * h->N <= MAP_PS_LAUNCH) return lns_map_of_masks(h);
-    const bool tiles = (MAP_PS_WORD - std::min(all_ps, off_ps)) * h->N > MAP_PS_LAUNCH;
+    if (h->R == 0 || h->N <= MAP_TILES_N) return lns_map_of_masks(h);
+    const bool tiles = bt_transform_ps(h->R) * h->N - std::min(all_ps, off_ps) > MAP_PS_LAUNCH;
     const int how = !tiles ? -1 : all_ps <= off_ps ? 1 : 0;
     const uint32_t nblk = h->N / h->blk;
     CK(cudaMemsetAsync(&h->info->noted, 0, 4));
@@ -1180,8 +1169,8 @@ int cov_lns_recount(cov_lns *h, const uint32_t *idx, int32_t m)
     if (!h || m < 0 || (m > 0 && !idx)) return COV_EINVAL;
     for (int i = 0; i < m; i++) if (idx[i] >= h->N) return COV_EINVAL;
     // the verifier's tiles while the code is sparse, else the transform of its
-    // word counts (about 12 ps a word)
-    if (tiles_ps(h, m) < 12.0) {
+    // word counts
+    if (bt_tiles_pay(h->q, h->n, h->R, m, std::max(1, cov_sm_count()))) {
         int rc = lns_scratch(h, (size_t)m * (4 + BT_REC_BYTES) + 8);
         if (rc) return rc;
         uint2 *rec = (uint2 *)h->scratch;

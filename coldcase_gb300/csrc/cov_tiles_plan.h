@@ -68,3 +68,51 @@ static inline void bt_geom(int q, int n, int R, int M, int sms, int *nh, int *nl
     }
     *nh = n - *nl;
 }
+
+// words within R of a word of n digits
+static inline double bt_ball(int q, int n, int R)
+{
+    double v = 1, c = 1;
+    for (int r = 0; r < R && r < n; r++) { c = c * (n - r) / (r + 1) * (q - 1); v += c; }
+    return v;
+}
+
+// Estimate of counting the balls of m words by tiles, in ps: 1.53 a word of
+// the space, and for each of the m 1850 (the chunks of a list, the host's copy)
+// and, for each tile of an SM, 650 (its prefix test), 1420 where its ball
+// reaches the tile, 1150 a group walked there and 60 a mark, 150 where the
+// strides are powers of two and a warp's marks share banks.  Fitted to 548
+// counts of 10 to 60,000 words in 68 cells of 2^12 to 8^9 words, R = 1 to 8:
+// with 29 us a call, 0.8 to 1.12 times the measured time in eight of ten (0.5
+// in the worst, 4^11 R8, where 10,000 words take 8.8 ms).
+static inline double bt_count_ps(int q, int n, int R, long long m, int sms)
+{
+    int nh, nl;
+    bt_geom(q, n, R, (int)std::min<long long>(m, 1 << 30), sms, &nh, &nl);
+    const double tiles = (double)bt_ipow(q, nh);
+    const int nm = nl - bt_block_digits(n);
+    double groups = 0, c = 1;
+    for (int d = 0; d <= nh && d <= R; d++) {
+        groups += c * (double)bt_groups(q, nm, R - d);
+        c = c * (nh - d) / (d + 1) * (q - 1);
+    }
+    const double near = std::min(1.0, bt_ball(q, nh, R) / tiles), marks = bt_ball(q, nm + nh, R) / tiles;
+    const double mark = (q & (q - 1)) ? 60.0 : 150.0;
+    return 1.53 * tiles * (double)bt_ipow(q, nl) +
+           (double)m * (1850.0 + std::max(1.0, tiles / sms) *
+                                     (650.0 + 1420.0 * near + 1150.0 * groups / tiles + mark * marks));
+}
+
+// The transform of a map or of word counts, ps a word of the space: an axis
+// moves R + 1 layers at most (68 cells: 0.7 to 1.2 times the measured time).
+static inline double bt_transform_ps(int R) { return 8.8 + 3.3 * R; }
+
+// Whether the counts of m words come from tiles sooner than from the transform
+// of their word counts, which takes 13 us of launches and clearing more.
+// Measured (us, tiles against transform): 7^8 R1 10,000 words 73, 139, 200,000
+// 775, 262; 6^9 R2 3000 74, 198, 30,000 385, 232; 4^11 R4 300 45, 134, 10,000
+// 306, 144; 2^16 R5 300 38, 60, 3000 147, 69.
+static inline bool bt_tiles_pay(int q, int n, int R, long long m, int sms)
+{
+    return bt_count_ps(q, n, R, m, sms) < 13e6 + 720.0 * (double)m + bt_transform_ps(R) * (double)bt_ipow(q, n);
+}
