@@ -1426,7 +1426,7 @@ int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed,
         a.eval_cap = tiled ? evals_tiles : evals_map;
         a.room = room - total;
         a.list = h->list + total;
-        a.max_steps = 64LL * (room - total) + 4LL * cand_cap + 64;
+        a.max_steps = greedy_max_steps(room - total, a.eval_cap);
         void *args[] = {&a};
         CK(cudaLaunchCooperativeKernel((const void *)k_lns_greedy, dim3((unsigned)G), dim3(GREEDY_NT), args, smem, 0));
         CK(cudaMemcpy(&st, h->seq, sizeof st, cudaMemcpyDeviceToHost));

@@ -1,6 +1,7 @@
 // cov_map_plan.h -- how the sweeps of the transform engine's maps
 // (cov_map.cuh, cov_lns.cu) group the axes of a cell, and what memory they
-// take.  Host arithmetic only, so that it compiles without CUDA.
+// take; and the bound on the steps of its greedy.  Host arithmetic only, so
+// that it compiles without CUDA.
 #pragma once
 #include <cstddef>
 #include <cstdint>
@@ -98,3 +99,9 @@ static inline void map_plan(MapPlan &p, int q, int n, int R, uint32_t N, int nb,
     p.counts_ints = 0;
     p.counts_at = p.whole_ints - N;
 }
+
+// Most steps of a greedy launch that places up to `room` words and leaves for
+// a fresh map after eval_cap exact counts without a placement: a step that
+// places none counts one candidate at least, so eval_cap of them come before
+// a placement or the end.  (The kernel gives up beyond it.)
+static inline long long greedy_max_steps(int room, int eval_cap) { return ((long long)room + 1) * (eval_cap + 1LL); }

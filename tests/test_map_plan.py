@@ -92,6 +92,35 @@ int main()
 """
 
 
+# A greedy launch in which every placement, and the refresh at the end, comes
+# after as many steps of one count each as the kernel allows: it stays within
+# the bound at which the kernel gives up, and a launch that went on would not.
+STEPS = r"""
+#include <cstdio>
+#include "cov_map_plan.h"
+int main()
+{
+    for (int room : {1, 2, 7, 1000, 40000})
+        for (int eval_cap : {64, 76, 256, 1024}) {
+            long long steps = 0;
+            for (int placed = 0, since = 0;;) {
+                if (placed >= room) break;
+                steps++;
+                if (since < eval_cap) { since++; continue; }
+                placed++;
+                since = 0;
+            }
+            steps += eval_cap + 1;
+            if (steps > greedy_max_steps(room, eval_cap) || steps + eval_cap < greedy_max_steps(room, eval_cap)) {
+                printf("room=%d eval_cap=%d: %lld steps\n", room, eval_cap, steps);
+                return 1;
+            }
+        }
+    return 0;
+}
+"""
+
+
 def run_program(tmp_path, text):
     cxx = shutil.which(os.environ.get("CXX", "g++"))
     if not cxx:
@@ -112,3 +141,7 @@ def test_plan_of_every_cell(tmp_path):
 
 def test_place_of_the_word_counts(tmp_path):
     run_program(tmp_path, COUNTS)
+
+
+def test_bound_on_the_greedys_steps(tmp_path):
+    run_program(tmp_path, STEPS)
