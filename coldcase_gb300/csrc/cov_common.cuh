@@ -261,12 +261,6 @@ static inline int cov_sm_count()
     return v;
 }
 
-// Device memory of the library: where it runs short, what the verification
-// calls' scratch pool keeps is given back first (cov_verify.cu).
-cudaError_t cov_malloc_bytes(void **p, size_t bytes);
-template <class T>
-static inline cudaError_t cov_malloc(T **p, size_t bytes) { return cov_malloc_bytes(reinterpret_cast<void **>(p), bytes); }
-
 // One bit per device: set once a set-up step ran with that device current.
 struct CovDeviceFlags {
     unsigned long long bits = 0;

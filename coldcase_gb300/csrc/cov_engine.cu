@@ -3507,10 +3507,10 @@ int cov_pool_create(int32_t max_slots, int32_t cluster, cov_pool **out)
     p->max_slots = max_slots;
     p->cluster = cluster;
     p->slots.resize(max_slots);
-    if (cov_malloc(&p->d_slots, sizeof(CovSlot) * max_slots) != cudaSuccess ||
-        cov_malloc(&p->d_map, sizeof(int) * max_slots) != cudaSuccess ||
-        cov_malloc(&p->d_all, sizeof(int) * max_slots) != cudaSuccess ||
-        cov_malloc(&p->d_states, sizeof(CovSlotState) * max_slots) != cudaSuccess) {
+    if (cudaMalloc(&p->d_slots, sizeof(CovSlot) * max_slots) != cudaSuccess ||
+        cudaMalloc(&p->d_map, sizeof(int) * max_slots) != cudaSuccess ||
+        cudaMalloc(&p->d_all, sizeof(int) * max_slots) != cudaSuccess ||
+        cudaMalloc(&p->d_states, sizeof(CovSlotState) * max_slots) != cudaSuccess) {
         cudaFree(p->d_slots); cudaFree(p->d_map); cudaFree(p->d_all); cudaFree(p->d_states);
         delete p;
         return COV_ENOMEM;
@@ -3693,7 +3693,7 @@ static int slot_alloc(cov_pool *pool, const cov_params *prm, int cap, int *s_out
     p2.M = Mw;
     size_t need = cov_slot_bytes(&p2) + subs.size() + subs1.size() + balls.size() + 2048;
     void *arena = nullptr;
-    if (cov_malloc(&arena, need) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+    if (cudaMalloc(&arena, need) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
     size_t off = 0;
     auto take_ = [&](size_t x) { void *p = (char *)arena + off; off += (x + 255) / 256 * 256; return p; };
     d.cw = (uint32_t *)take_((size_t)N * 4);
@@ -3998,7 +3998,7 @@ int cov_pool_set_param(cov_pool *pool, const char *name, int64_t value)
         if (value < 0 || value > 1024) return COV_EINVAL;
         CK(cudaStreamSynchronize(pool->cur_stream()));
         if (value > 0 && !pool->d_gh) {
-            if (cov_malloc(&pool->d_gh, sizeof(GridHelp)) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+            if (cudaMalloc(&pool->d_gh, sizeof(GridHelp)) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
         }
         pool->grid_help = (int)value;
         if (pool->gexec) { cudaGraphExecDestroy(pool->gexec); pool->gexec = nullptr; }

@@ -995,7 +995,7 @@ int lns_scratch(cov_lns *h, size_t bytes)
     if (h->scratch) cudaFree(h->scratch);
     h->scratch = nullptr;
     h->scratch_bytes = 0;
-    if (cov_malloc(&h->scratch, bytes) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+    if (cudaMalloc(&h->scratch, bytes) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
     h->scratch_bytes = bytes;
     return 0;
 }
@@ -1039,8 +1039,8 @@ int list_room(cov_lns *h, int k)
         h->list = nullptr;
         h->flag = nullptr;
         h->list_cap = 0;
-        CK(cov_malloc(&h->list, (size_t)k * 4));
-        CK(cov_malloc(&h->flag, (size_t)k));
+        CK(cudaMalloc(&h->list, (size_t)k * 4));
+        CK(cudaMalloc(&h->flag, (size_t)k));
         h->list_cap = k;
     }
     return 0;
@@ -1113,26 +1113,26 @@ int cov_lns_create(int32_t q, int32_t n, int32_t R, cov_lns **out)
             for (int sg = d; sg <= h->nb; sg++) low[(size_t)x * (h->nb + 1) + sg] |= 1ull << y;
         }
     map_plan(*h, q, n, R, h->N, h->nb, h->blk);
-    bool ok = cov_malloc(&h->cnt, (size_t)N * 2) == cudaSuccess &&
-              cov_malloc(&h->map, (size_t)N * 4) == cudaSuccess &&
-              cov_malloc(&h->ball, items.size() * 8) == cudaSuccess &&
-              cov_malloc(&h->ball_last, last.size()) == cudaSuccess &&
-              cov_malloc(&h->d_red, 64 * 8) == cudaSuccess &&
-              cov_malloc(&h->cand, (size_t)CAND_CAP * 4) == cudaSuccess &&
-              cov_malloc(&h->bound, (size_t)CAND_CAP * 4) == cudaSuccess &&
-              cov_malloc(&h->um, (size_t)(N / h->blk) * 8) == cudaSuccess &&
-              cov_malloc(&h->um_map, (size_t)(N / h->blk) * 8) == cudaSuccess &&
-              cov_malloc(&h->note, (size_t)NOTE_CAP * (4 + BT_REC_BYTES)) == cudaSuccess &&
-              cov_malloc(&h->pball, pitems.size() * 8) == cudaSuccess &&
-              cov_malloc(&h->pball_last, plast.size()) == cudaSuccess &&
-              cov_malloc(&h->lowball, low.size() * 8) == cudaSuccess &&
-              cov_malloc(&h->nom, sizeof(unsigned long long) * 2 * GREEDY_MAXG) == cudaSuccess &&
-              cov_malloc(&h->acc, 4 * (3 * (GREEDY_MAXG + 1) + 1)) == cudaSuccess &&
-              cov_malloc(&h->info, sizeof(RefreshInfo)) == cudaSuccess &&
-              cov_malloc(&h->seq, sizeof(SeqState)) == cudaSuccess;
+    bool ok = cudaMalloc(&h->cnt, (size_t)N * 2) == cudaSuccess &&
+              cudaMalloc(&h->map, (size_t)N * 4) == cudaSuccess &&
+              cudaMalloc(&h->ball, items.size() * 8) == cudaSuccess &&
+              cudaMalloc(&h->ball_last, last.size()) == cudaSuccess &&
+              cudaMalloc(&h->d_red, 64 * 8) == cudaSuccess &&
+              cudaMalloc(&h->cand, (size_t)CAND_CAP * 4) == cudaSuccess &&
+              cudaMalloc(&h->bound, (size_t)CAND_CAP * 4) == cudaSuccess &&
+              cudaMalloc(&h->um, (size_t)(N / h->blk) * 8) == cudaSuccess &&
+              cudaMalloc(&h->um_map, (size_t)(N / h->blk) * 8) == cudaSuccess &&
+              cudaMalloc(&h->note, (size_t)NOTE_CAP * (4 + BT_REC_BYTES)) == cudaSuccess &&
+              cudaMalloc(&h->pball, pitems.size() * 8) == cudaSuccess &&
+              cudaMalloc(&h->pball_last, plast.size()) == cudaSuccess &&
+              cudaMalloc(&h->lowball, low.size() * 8) == cudaSuccess &&
+              cudaMalloc(&h->nom, sizeof(unsigned long long) * 2 * GREEDY_MAXG) == cudaSuccess &&
+              cudaMalloc(&h->acc, 4 * (3 * (GREEDY_MAXG + 1) + 1)) == cudaSuccess &&
+              cudaMalloc(&h->info, sizeof(RefreshInfo)) == cudaSuccess &&
+              cudaMalloc(&h->seq, sizeof(SeqState)) == cudaSuccess;
     if (ok)
-        ok = cov_malloc(&h->map_scratch, (h->scratch_ints * (h->ng >= 3 ? 2 : 1) + h->counts_ints) * 4) == cudaSuccess;
-    if (ok && h->whole_ints) ok = cov_malloc(&h->map_whole, h->whole_ints * 4) == cudaSuccess;
+        ok = cudaMalloc(&h->map_scratch, (h->scratch_ints * (h->ng >= 3 ? 2 : 1) + h->counts_ints) * 4) == cudaSuccess;
+    if (ok && h->whole_ints) ok = cudaMalloc(&h->map_whole, h->whole_ints * 4) == cudaSuccess;
     if (!ok) {
         cudaGetLastError();
         cov_lns_destroy(h);

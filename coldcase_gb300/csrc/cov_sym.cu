@@ -1397,10 +1397,10 @@ int cov_sym_create(int32_t max_slots, int32_t cluster, cov_sym **out)
     p->cluster = cluster;
     p->slots.resize(max_slots);
     SCK(cudaDeviceGetAttribute(&p->sms, cudaDevAttrMultiProcessorCount, dev));
-    cudaError_t e = cov_malloc(&p->d_slots, sizeof(SymSlot) * max_slots);
-    if (e == cudaSuccess) e = cov_malloc(&p->d_states, sizeof(SymState) * max_slots);
-    if (e == cudaSuccess) e = cov_malloc(&p->d_list, sizeof(int) * max_slots);
-    if (e == cudaSuccess) e = cov_malloc(&p->d_gop, sizeof(SymOp));
+    cudaError_t e = cudaMalloc(&p->d_slots, sizeof(SymSlot) * max_slots);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_states, sizeof(SymState) * max_slots);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_list, sizeof(int) * max_slots);
+    if (e == cudaSuccess) e = cudaMalloc(&p->d_gop, sizeof(SymOp));
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->stream, cudaStreamNonBlocking);
     if (e != cudaSuccess) {
         cudaFree(p->d_slots); cudaFree(p->d_states); cudaFree(p->d_list); cudaFree(p->d_gop);
@@ -1545,7 +1545,7 @@ int cov_sym_add(cov_sym *p, const cov_sym_params *prm, int32_t *slot)
     const size_t ncap = (size_t)norb * q * NR + 8;
     const size_t need = cov_sym_slot_bytes(prm) + w0.size() + w1.size() + bs.size() + 1024;
     void *arena = nullptr;
-    if (cov_malloc(&arena, need) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+    if (cudaMalloc(&arena, need) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
     size_t off = 0;
     auto take_ = [&](size_t x) { void *q2 = (char *)arena + off; off += (x + 255) / 256 * 256; return q2; };
     d.cnt2 = (uint32_t *)take_((size_t)((d.N + 1) / 2) * 4);
@@ -1671,7 +1671,7 @@ int cov_sym_get_cnt(cov_sym *p, int32_t slot, uint16_t *out)
     if (!p || !out || slot < 0 || slot >= p->max_slots || !p->slots[slot].used) return COV_EINVAL;
     const SymSlot &d = p->slots[slot].d;
     uint16_t *tmp = nullptr;
-    if (cov_malloc(&tmp, (size_t)d.N * 2) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
+    if (cudaMalloc(&tmp, (size_t)d.N * 2) != cudaSuccess) { cudaGetLastError(); return COV_ENOMEM; }
     k_sym_unpack<<<1024, 256, 0, p->stream>>>(d.cnt2, d.N, tmp);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(out, tmp, (size_t)d.N * 2, cudaMemcpyDeviceToHost, p->stream);

@@ -1099,17 +1099,16 @@ int geom(int q, int n, DtGeom &g)
 // pieces kept.
 #define SCRATCH_KEEP (64ull << 20)
 
-cudaMemPool_t g_scratch[COV_MAX_DEVICES];       // per device, made at the first call there
-std::mutex g_scratch_lock;
-
 int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
 {
+    static cudaMemPool_t pools[COV_MAX_DEVICES];
+    static std::mutex m;
     int dev = 0;
     CK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= COV_MAX_DEVICES) return COV_ENODEV;
     {
-        std::lock_guard<std::mutex> hold(g_scratch_lock);
-        if (!g_scratch[dev]) {
+        std::lock_guard<std::mutex> hold(m);
+        if (!pools[dev]) {
             cudaMemPoolProps props;
             memset(&props, 0, sizeof props);
             props.allocType = cudaMemAllocationTypePinned;
@@ -1119,10 +1118,10 @@ int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
             CK(cudaMemPoolCreate(&pool, &props));
             unsigned long long keep = SCRATCH_KEEP;
             CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
-            g_scratch[dev] = pool;
+            pools[dev] = pool;
         }
     }
-    if (cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), g_scratch[dev], st) != cudaSuccess) {
+    if (cudaMallocFromPoolAsync(p, std::max<size_t>(bytes, 1), pools[dev], st) != cudaSuccess) {
         cudaGetLastError();
         return COV_ENOMEM;
     }
@@ -1349,19 +1348,6 @@ int dt_run(const DtGeom &g, const DtPlan &plan, const uint8_t *d_code, int M, ui
 }
 
 }  // namespace
-
-cudaError_t cov_malloc_bytes(void **p, size_t bytes)
-{
-    cudaError_t e = cudaMalloc(p, bytes);
-    int dev = 0;
-    if (e != cudaErrorMemoryAllocation || cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= COV_MAX_DEVICES) return e;
-    std::lock_guard<std::mutex> hold(g_scratch_lock);
-    if (!g_scratch[dev]) return e;
-    cudaGetLastError();
-    // (pieces behind an allocation in use stay: other threads' calls go on)
-    if (cudaMemPoolTrimTo(g_scratch[dev], 0) != cudaSuccess) return e;
-    return cudaMalloc(p, bytes);
-}
 
 // the records of the m listed words and the geometry of their count
 static int words_records(int q, int n, int R, const uint32_t *d_idx, int m, uint2 *rec, cudaStream_t st, CountGeom &g,
@@ -1627,7 +1613,7 @@ int cov_finish(int32_t q, int32_t n, int32_t R, int32_t M, const uint8_t *code, 
     const size_t bib = bitems.size() * 8, blb = (blast.size() + 7) / 8 * 8;
     const size_t cb = ((size_t)dg.N * 2 + 15) / 16 * 16;
     char *buf = nullptr;
-    if (cov_malloc(&buf, trb + bib + blb + (size_t)M * 8 + cb + 16) != cudaSuccess) {
+    if (cudaMalloc(&buf, trb + bib + blb + (size_t)M * 8 + cb + 16) != cudaSuccess) {
         cudaGetLastError();
         return COV_ENOMEM;
     }
@@ -1676,8 +1662,8 @@ int cov_count(int32_t q, int32_t n, int32_t R, const uint8_t *code, int32_t M, u
     uint8_t *d_code = nullptr;
     uint16_t *d_cnt = nullptr;
     const size_t nb = ((size_t)g.N + 1) / 2 * 4;     // whole 32-bit pairs
-    if (cov_malloc(&d_code, (size_t)std::max(M, 1) * n) != cudaSuccess ||
-        cov_malloc(&d_cnt, nb) != cudaSuccess) {
+    if (cudaMalloc(&d_code, (size_t)std::max(M, 1) * n) != cudaSuccess ||
+        cudaMalloc(&d_cnt, nb) != cudaSuccess) {
         cudaGetLastError();
         cudaFree(d_code); cudaFree(d_cnt);
         return COV_ENOMEM;

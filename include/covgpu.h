@@ -197,9 +197,6 @@ int cov_pool_destroy(cov_pool *pool);
 /* ------------------------------------------------------------------------
  * Verification and transforms (host buffers in, host buffers out; the
  * *_dev forms take device pointers and a cudaStream_t passed as void*).
- * Their scratch comes from a memory pool of the library's own, which keeps
- * up to 64 MB a device between calls; the library gives it back when an
- * allocation of its own would fail otherwise.
  * --------------------------------------------------------------------- */
 /* Exact uncovered count of a code at radius R: cov/verify_cov.py:109-152
  * (verify_pure) and :169-230 (verify_numpy) return the same number. */
