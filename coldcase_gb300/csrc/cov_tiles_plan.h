@@ -82,7 +82,7 @@ static inline double bt_ball(int q, int n, int R)
 // and, for each tile of an SM, 650 (its prefix test), 1420 where its ball
 // reaches the tile, 1150 a group walked there and 60 a mark, 150 where the
 // strides are powers of two and a warp's marks share banks.  Fitted to 548
-// counts of 10 to 60,000 words in 68 cells of 2^12 to 8^9 words, R = 1 to 8:
+// counts of 10 to 60,000 words in 71 cells of 2^12 to 8^9 words, R = 1 to 8:
 // with 29 us a call, 0.8 to 1.12 times the measured time in eight of ten (0.5
 // in the worst, 4^11 R8, where 10,000 words take 8.8 ms).
 static inline double bt_count_ps(int q, int n, int R, long long m, int sms)
@@ -104,7 +104,7 @@ static inline double bt_count_ps(int q, int n, int R, long long m, int sms)
 }
 
 // The transform of a map or of word counts, ps a word of the space: an axis
-// moves R + 1 layers at most (68 cells: 0.7 to 1.2 times the measured time).
+// moves R + 1 layers at most (71 cells: 0.7 to 1.2 times the measured time).
 static inline double bt_transform_ps(int R) { return 8.8 + 3.3 * R; }
 
 // Whether the counts of m words come from tiles sooner than from the transform

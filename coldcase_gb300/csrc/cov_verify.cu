@@ -1414,14 +1414,17 @@ int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M, uint
 // framework's caching allocator that has reserved the whole GPU), or code
 // that runs where an allocation would break the surrounding contract (inside
 // an out-of-memory handler).  The one scratch buffer the transform needs --
-// the bitmap of codeword positions -- lives in a file-scope device array
-// instead of being allocated per call.
+// the codewords' records of the tile forms, or the bitmap of codeword
+// positions of the sweeps -- lives in a file-scope device array instead of
+// being allocated per call.
 //
-//  * Limit: q^n <= COV_DT_STATIC_MAX_WORDS (2^26 words, an 8 MiB bitmap that
-//    every GPU which loads the library keeps until the process exits).
+//  * Limit: q^n <= COV_DT_STATIC_MAX_WORDS (2^26 words, whose bitmap is the
+//    8 MiB of the array, which every GPU that loads the library keeps until
+//    the process exits).  A code with more records than the array holds (8
+//    bytes each, 2^20 codewords) takes the sweeps.
 //  * The first call on a device looks up the array's device address
 //    (cudaGetSymbolAddress, with that device current) and caches it.
-//  * Every call uses the same array and clears it before use: two calls
+//  * Every call writes the same array anew before it reads it: two calls
 //    whose work overlaps on the GPU (different streams, no ordering) race.
 #define COV_DT_STATIC_MAX_WORDS (1u << 26)
 #define COV_DT_STATIC_MAX_DEVICES 64

@@ -197,6 +197,9 @@ int cov_pool_destroy(cov_pool *pool);
 /* ------------------------------------------------------------------------
  * Verification and transforms (host buffers in, host buffers out; the
  * *_dev forms take device pointers and a cudaStream_t passed as void*).
+ * Their scratch comes from a memory pool of the library's own that keeps up
+ * to 64 MB a device between calls, until the process ends; the CUDA runtime
+ * takes that back for an allocation that would fail otherwise.
  * --------------------------------------------------------------------- */
 /* Exact uncovered count of a code at radius R: cov/verify_cov.py:109-152
  * (verify_pure) and :169-230 (verify_numpy) return the same number. */
@@ -216,8 +219,7 @@ int cov_count(int32_t q, int32_t n, int32_t R, const uint8_t *code, int32_t M,
  * ignored (the host forms refuse it with COV_EINVAL). */
 int cov_mindist_dev(int32_t q, int32_t n, const uint8_t *d_code, int32_t M,
                     uint8_t *d_dist, void *stream);
-/* d_cnt is updated in aligned 32-bit pairs: it must have room for q^n
- * entries rounded up to an even number. */
+/* d_cnt: q^n entries, at any 2-byte boundary. */
 int cov_count_dev(int32_t q, int32_t n, int32_t R, const uint8_t *d_code,
                   int32_t M, uint16_t *d_cnt, void *stream);
 int64_t cov_count_above_dev(int32_t q, int32_t n, const uint8_t *d_dist,
@@ -323,7 +325,12 @@ int cov_lns_peel(cov_lns *h, const uint32_t *idx, int32_t k, uint8_t *removed, i
  * the best bounds exactly until the best is current, then places it; the
  * host only refreshes the map, when the threshold is reached or so many
  * counts were made that a map is cheaper.  placed[] receives the
- * words in order; stats (may be null): refreshes, exact counts. */
+ * words in order; stats (may be null): refreshes, exact counts.
+ * The kernel is a cooperative launch of one block per SM: beside other work
+ * on the GPU it starts once every SM has room for a block, and holds one on
+ * each until it places no more or asks for a map.  Beside a search launch
+ * that fills the SMs it waits for that launch's end (cov_lns_recount and
+ * cov_lns_map wait for the device beside any). */
 int cov_lns_greedy(cov_lns *h, int32_t room, int64_t cand_cap, uint32_t *placed, int32_t *nplaced,
                    int64_t *uncovered, int64_t *stats);
 /* The uncovered words (cnt == 0) in increasing index order, at most cap of
@@ -345,8 +352,9 @@ int cov_finish(int32_t q, int32_t n, int32_t R, int32_t M, const uint8_t *code, 
 /* cov_mindist_dev without any device allocation, for callers that cannot
  * allocate (their device memory belongs to another allocator, or they run
  * where an allocation is not allowed).  No counterpart in the reference.
- * Its one scratch buffer is a file-scope device array: q^n must be at most
- * 2^26 (else COV_ERANGE); the first call on a device also looks up the
+ * Its one scratch buffer is a file-scope device array of 8 MiB, written anew
+ * by each call: q^n must be at most 2^26 (else COV_ERANGE); a code of more
+ * than 2^20 codewords takes the form whose scratch goes by q^n; the first call on a device also looks up the
  * array's device address on the host; calls that overlap on the GPU share
  * the array and race. */
 int cov_mindist_dev_static(int32_t q, int32_t n, const uint8_t *d_code,
