@@ -1115,9 +1115,16 @@ int scratch_alloc(void **p, size_t bytes, cudaStream_t st)
             props.location.type = cudaMemLocationTypeDevice;
             props.location.id = dev;
             cudaMemPool_t pool = nullptr;
-            CK(cudaMemPoolCreate(&pool, &props));
+            // the call may be one that a stream captures: making a pool is no
+            // work of the stream, but is refused unless the thread's mode is
+            // relaxed, and the capture is lost
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            CK(cudaThreadExchangeStreamCaptureMode(&mode));
+            cudaError_t e = cudaMemPoolCreate(&pool, &props);
             unsigned long long keep = SCRATCH_KEEP;
-            CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+            if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+            CK(cudaThreadExchangeStreamCaptureMode(&mode));
+            CK(e);
             pools[dev] = pool;
         }
     }
